@@ -10,62 +10,81 @@
 //     over columns c0..c1, applied to rows rho+1..c1;
 //   L op: a left reflector from column c0 over rows c0..c1, applied to
 //     columns c0+1..min(c0 + 2BW - 1, n - 1).
-// Op k of sweep j touches nothing that ops >= k+4 of sweep j-1 touch.
+// Op k of sweep j touches nothing that ops >= k+4 of sweep j-1 touch, and shares
+// with op k+3 one element: that op's pivot (its beta), which is element BW-1 of
+// op k's last row (R op) or column (L op).
 //
 // Layout of the work.  A CTA owns the sweeps j0 .. j0+G-1 (groups handed out
-// in order by a ticket); compute warp i runs sweep j0+i, op t - 4i at tick t,
-// so the G sweeps advance in lockstep with the minimal lag, and all their
-// data stays in a window of W columns of the band in shared memory (column c
-// in slot c mod W).  A producer warp moves the band between the window and
-// global memory: before tick t it has loaded (cp.async, 16-byte chunks, L2
-// only) every column the tick touches, and it prefetches the columns of tick
-// t+3; after tick t it marks as retired the columns that no sweep of the
-// group touches again (those left of the trailing sweep's next pivot).  A
-// publisher warp writes retired columns back and publishes the boundary in
-// retired[g] (fence, release), off the ticks' critical path.  The next
-// group's producer loads a column only once retired[g] has passed it, so it
-// sees every update of this group, and this group never touches a column
-// again once it is retired: the result is the sequential chase's, bit for
-// bit, whatever the timing.  Compute warps touch only shared memory;
-// named barriers hand each tick between the producer and the compute warps.
-// Every wait on another CTA is bounded (kDevTimeout).
+// in order by a ticket); WPS compute warps run sweep j0+i, op t - 3i at tick t,
+// and all the group's data stays in a window of W columns of the band in shared
+// memory (column c in slot c mod W).  A tick has two barriers of the compute
+// warps: before it, and between its phases.  Phase 1 reads the pivot, forms the
+// reflector and all of the dot products but elements 0 and BW-1, and writes the
+// new pivot; phase 2 reads element BW-1 (which may be the pivot that the sweep
+// ahead wrote in this tick's phase 1) and applies.  That is what lets
+// consecutive sweeps follow each other at three ops instead of four.
+// A producer warp moves the band between the window and global memory: before
+// tick t it has loaded (cp.async, 16-byte chunks, L2 only) every column the tick
+// touches, and it prefetches the columns of tick t+3; a publisher warp writes
+// back the columns that no sweep of the group touches again (those left of the
+// trailing sweep's next pivot) and publishes the boundary in retired[g] (fence,
+// release), off the ticks' critical path.  The next group's producer loads a
+// column only once retired[g] has passed it, so it sees every update of this
+// group, and this group never touches a column again once it is retired: the
+// result is the sequential chase's, whatever the timing.  Compute warps touch
+// only shared memory.  Every wait is bounded (kDevTimeout).
+//
+// What bounds it: the latency of one op times the ops on the critical path (3
+// per sweep, plus 5 to 6 and the hand-off per group); the band stays in L2 and
+// shared memory.  The op's chain is kept short: the reflector is used unscaled
+// (u = x with u_0 = alpha - beta), so the dot products do not wait for the norm;
+// the norm's butterfly merges compensated pairs without renormalising; the
+// scalars come from the hardware estimates with one residual each
+// (reflect.cuh); full ops that do not wrap in the window have immediate
+// addresses and no predicates.  H lanes share a row (column): with H = 2 a sweep
+// runs on two warps, each forming the reflector itself.
+// Measured (GB300, chase alone, before: one warp per sweep, scaled reflector,
+// four ops of lag, generic double-float square root and divisions): band 16,
+// double-float, n = 1024 12.3 -> 5.0 ms, n = 4096 50.4 -> 21.1 ms, n = 16384
+// 204 -> 93 ms; band 32, n = 256 7.6 -> 2.5 ms.
 //
 // Band storage in global memory: the element chase's compact form, A(r, c) at
 // AB[(r - c + 2BW - 1) + c * ldab], ldab = 3 BW.
 #include <algorithm>
+#include <type_traits>
 
 #include "avs_common.cuh"
 #include "chase_ar.cuh"
+#include "reflect.cuh"
 
 namespace avs {
 namespace {
 
-template <int BW, int G>
+template <int BW, int G, int H>
 struct WinCfg {
     static constexpr int KU = 2 * BW - 1;
+    static constexpr int LAG = 3;               // ticks between consecutive sweeps of a group
     static constexpr int LDAB = 3 * BW;         // storage rows per column (global)
     static constexpr int LDW = 3 * BW + 2;      // window column stride (16-byte multiple; odd stride - 1)
     static constexpr int W = 2 * G * BW + 2 * BW;  // window columns (span of a group's ops + prefetch)
-    static constexpr int NC = 32 * G;           // compute threads: one warp per sweep
-    static constexpr int D = 4;                 // ticks of the mbarrier ring (producer lookahead)
+    static constexpr int RL = 32 / H;           // rows (R op) / columns (L op) per warp, H lanes each
+    static constexpr int WPS = (2 * BW - 1 + RL - 1) / RL;  // warps per sweep
+    static constexpr int SEG = BW / H;          // reflector elements per lane
+    static constexpr int NC = 32 * G * WPS;     // compute threads
+    static constexpr int D = 4;                 // ops of the mbarrier ring (producer lookahead)
     static constexpr int NT = NC + 64;          // + the producer and the publisher warps
     static constexpr int CHUNKS = LDAB * 8 / 16;  // 16-byte chunks per column
-    static_assert(BW % 2 == 0 && BW <= 32, "window chase band");
-    static constexpr size_t smem_bytes() { return 8 * ((size_t)W * LDW + (size_t)G * 32); }
+    static_assert(BW % 2 == 0 && BW <= 32 && SEG >= 4, "window chase band");
+    static_assert(WPS == 1 || 3 + G <= 16, "named barriers");
+    static constexpr size_t smem_bytes() { return 8 * (size_t)W * LDW; }
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void bar_sync(int id, int cnt) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(cnt) : "memory"); }
-__device__ __forceinline__ void bar_arrive(int id, int cnt) {
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(cnt) : "memory");
-}
 
 // mbarriers of the tick ring: the producer's copies arrive on them
 // (cp.async.mbarrier.arrive.noinc: when all of the lane's earlier copies have
@@ -91,58 +110,94 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *m, unsigned pa
 
 __device__ __forceinline__ int ld_volatile_shared(const int *p) { return *(const volatile int *)p; }
 __device__ __forceinline__ void st_volatile_shared(int *p, int v) { *(volatile int *)p = v; }
+__device__ __forceinline__ int ld_acquire_shared(const int *p) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_shared(int *p, int v) {
+    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
+}
 __device__ __forceinline__ int ld_relaxed(const int *p) {
     int v;
     asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 
-// Bounded waits on a shared-memory counter written by another warp of the CTA
-// (kWaitNs of %globaltimer, kSpinLimit polls); on timeout kDevTimeout.
-__device__ __forceinline__ bool wait_shared_geq(const int *p, int target, int *err) {
-    const unsigned long long t0 = global_ns();
-    for (long long it = 0; ld_volatile_shared(p) < target; ++it) {
-        if (it > kSpinLimit || ((it & 255) == 255 && (long long)(global_ns() - t0) > kWaitNs)) {
-            atomicCAS(err, kDevOk, kDevTimeout);
-            return false;
-        }
-        __nanosleep(32);
+// Bounded waits of the CTA's warps on one another: kWaitCycles of the SM clock
+// (about 4 s; reading it costs a few cycles, %globaltimer hundreds) and
+// kSpinLimit polls.  A wait that runs out records kDevTimeout and raises *fail,
+// on which every later wait of the CTA returns at once: the group runs to its
+// end on whatever data it has.
+constexpr long long kWaitCycles = 8000000000ll;
+__device__ __forceinline__ bool wait_over(long long it, long long t0, int *fail, int *err) {
+    if (ld_volatile_shared(fail)) return true;
+    if (it > kSpinLimit || clock64() - t0 > kWaitCycles) {
+        atomicCAS(err, kDevOk, kDevTimeout);
+        st_volatile_shared(fail, 1);
+        return true;
     }
-    return true;
+    return false;
 }
-// Bounded wait for a phase of an mbarrier (kWaitNs, kSpinLimit polls); on
-// timeout kDevTimeout and false.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *m, unsigned parity, int *err) {
-    const unsigned long long t0 = global_ns();
-    for (long long it = 0; !mbar_try_wait(m, parity); ++it) {
-        if (it > kSpinLimit || ((it & 63) == 63 && (long long)(global_ns() - t0) > kWaitNs)) {
-            atomicCAS(err, kDevOk, kDevTimeout);
-            return false;
-        }
+// a shared-memory counter written (release) by another warp of the CTA
+__device__ __forceinline__ void wait_shared_geq(const int *p, int target, int *fail, int *err) {
+    if (ld_acquire_shared(p) >= target) return;
+    const long long t0 = clock64();
+#pragma unroll 1
+    for (long long it = 0; ld_acquire_shared(p) < target; ++it) {
+        if ((it & 63) == 63 && wait_over(it, t0, fail, err)) return;
+        if (it > 16) __nanosleep(20);
     }
-    return true;
 }
-// returns the counter once it exceeds v (or v after a timeout)
-__device__ __forceinline__ int wait_shared_gt(const int *p, int v, int *err) {
-    const unsigned long long t0 = global_ns();
-    for (long long it = 0;; ++it) {
-        const int x = ld_volatile_shared(p);
-        if (x > v) return x;
-        if (it > kSpinLimit || ((it & 255) == 255 && (long long)(global_ns() - t0) > kWaitNs)) {
-            atomicCAS(err, kDevOk, kDevTimeout);
-            return v;
-        }
-        __nanosleep(32);
-    }
+// a phase of an mbarrier
+__device__ __forceinline__ void mbar_wait(unsigned long long *m, unsigned parity, int *fail, int *err) {
+    if (mbar_try_wait(m, parity)) return;
+    const long long t0 = clock64();
+#pragma unroll 1
+    for (long long it = 0; !mbar_try_wait(m, parity); ++it)
+        if ((it & 63) == 63 && wait_over(it, t0, fail, err)) return;
 }
 
+// The chase's arithmetic beyond ChaseAr: merging dot-product accumulators
+// without renormalising between the levels of a butterfly, the reflector's
+// scalars, and a - w u with one renormalisation.
 template <typename S>
-__device__ __forceinline__ typename ChaseAr<S>::V wsum(typename ChaseAr<S>::V v) {
-    using Ar = ChaseAr<S>;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = Ar::add(v, Ar::shfl_xor(v, o));
-    return v;
-}
+struct WinAr;
+template <>
+struct WinAr<df64> {
+    using Acc = ChaseAr<df64>::Acc;
+    static __device__ __forceinline__ Acc merge_xor(Acc a, int o) {
+        const df64 t = two_sum(a.s, __shfl_xor_sync(0xffffffffu, a.s, o));
+        return Acc{t.hi, __fadd_rn(t.lo, __fadd_rn(a.c, __shfl_xor_sync(0xffffffffu, a.c, o)))};
+    }
+    static __device__ __forceinline__ bool positive(Acc s) {
+        const df64 v = two_sum(s.s, s.c);
+        return v.hi > 0.0f;
+    }
+    // s + alpha^2
+    static __device__ __forceinline__ df64 norm2(Acc s, df64 al) {
+        const float p = __fmul_rn(al.hi, al.hi);
+        const float e = __fmaf_rn(2.0f * al.hi, al.lo, __fmaf_rn(al.hi, al.hi, -p));
+        const df64 t = two_sum(p, s.s);
+        return fast_two_sum(t.hi, __fadd_rn(t.lo, __fadd_rn(e, s.c)));
+    }
+    static __device__ __forceinline__ df64 sub_mul(df64 a, df64 w, df64 u) {
+        const float p = __fmul_rn(w.hi, u.hi);
+        const float e = __fmaf_rn(w.lo, u.hi, __fmaf_rn(w.hi, u.lo, __fmaf_rn(w.hi, u.hi, -p)));
+        const df64 t = two_sum(a.hi, -p);
+        return fast_two_sum(t.hi, __fadd_rn(t.lo, __fsub_rn(a.lo, e)));
+    }
+};
+template <>
+struct WinAr<double> {
+    using Acc = double;
+    static __device__ __forceinline__ Acc merge_xor(Acc a, int o) { return a + __shfl_xor_sync(0xffffffffu, a, o); }
+    static __device__ __forceinline__ bool positive(Acc s) { return s > 0.0; }
+    static __device__ __forceinline__ double norm2(Acc s, double al) { return ::fma(al, al, s); }
+    static __device__ __forceinline__ double sub_mul(double a, double w, double u) { return ::fma(-w, u, a); }
+};
+
+constexpr int kAllDone = 1 << 30;
 
 // Per-sweep op geometry.
 struct WOp {
@@ -160,28 +215,28 @@ __device__ __forceinline__ WOp wop(int64_t n, int j, int k) {
     return o;
 }
 
-template <int BW, typename S, int G>
-__global__ void __launch_bounds__(WinCfg<BW, G>::NT, 1)
+template <int BW, typename S, int G, int H>
+__global__ void __launch_bounds__(WinCfg<BW, G, H>::NT, 1)
     chase_win_kernel(typename ChaseAr<S>::St *ab_base, int64_t n, int batch, int64_t sAB, int *ticket,
                      int *retired_base, int64_t sRet, int *err) {
-    using Cfg = WinCfg<BW, G>;
+    using Cfg = WinCfg<BW, G, H>;
     using Ar = ChaseAr<S>;
+    using Wa = WinAr<S>;
     using V = typename Ar::V;
     using St = typename Ar::St;
     static_assert(sizeof(St) == 8 && sizeof(V) == 8, "8-byte band elements");
-    constexpr int KU = Cfg::KU, LDW = Cfg::LDW, W = Cfg::W, NC = Cfg::NC, NT = Cfg::NT, LDAB = Cfg::LDAB;
+    constexpr int KU = Cfg::KU, LDW = Cfg::LDW, W = Cfg::W, LDAB = Cfg::LDAB, LAG = Cfg::LAG;
+    constexpr int CW = G * Cfg::WPS;  // compute warps; then the producer and the publisher
     extern __shared__ __align__(16) unsigned char smem_raw[];
     St *win = reinterpret_cast<St *>(smem_raw);  // [W][LDW]
-    V *vbuf = reinterpret_cast<V *>(win + (size_t)W * LDW);  // [G][32]: each compute warp's reflector
     __shared__ int s_g;
-    __shared__ int s_tick, s_wb;  // ticks the compute warps have finished; columns below s_wb written back
+    __shared__ int s_tick, s_wb, s_fail;  // ticks finished; columns below s_wb written back; a wait ran out
     __shared__ __align__(8) unsigned long long s_full[Cfg::D];  // tick t's columns are in: phase t / D of [t % D]
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (tid == 0)
         for (int d = 0; d < Cfg::D; ++d) mbar_init(&s_full[d], 32);
     const int nsweeps = (int)(n - 1);
     const int ngroups = (nsweeps + G - 1) / G;
-    auto A = [&](int r, int c) -> St * { return win + (size_t)(c % W) * LDW + (r - c + KU); };
 
     for (;;) {
         if (tid == 0) s_g = atomicAdd(ticket, 1);
@@ -197,38 +252,25 @@ __global__ void __launch_bounds__(WinCfg<BW, G>::NT, 1)
         if (tid == 0) {
             s_tick = 0;
             s_wb = j0 + 1;
+            s_fail = 0;
         }
         __syncthreads();
         const int gs = min(G, nsweeps - j0);
+        // the leading sweep's op t touches columns below need(t); every other sweep
+        // of the group is left of it, and its last op reaches column n - 1
+        const int ops0 = wops<BW>(n, j0);
         int nticks = 0;
-        for (int i = 0; i < gs; ++i) nticks = max(nticks, 4 * i + wops<BW>(n, j0 + i));
-        // columns [lo, .. ) not yet retired; the tick's highest column + 1
-        auto tick_need = [&](int t) -> int {
-            int need = 0;
-            for (int i = 0; i < gs; ++i) {
-                const int k = t - 4 * i;
-                if (k >= 0 && k < wops<BW>(n, j0 + i)) need = max(need, wop<BW>(n, j0 + i, k).hi + 1);
-            }
-            return need;
-        };
-        // after tick t: the lowest column any op of a later tick touches (n: none)
-        auto retire_after = [&](int t) -> int {
-            int lo = (int)n;
-            for (int i = 0; i < gs; ++i) {
-                const int k = t + 1 - 4 * i;
-                if (k < wops<BW>(n, j0 + i)) lo = min(lo, wop<BW>(n, j0 + i, max(k, 0)).c0);
-            }
-            return lo;
-        };
+        for (int i = 0; i < gs; ++i) nticks = max(nticks, LAG * i + wops<BW>(n, j0 + i));
+        auto need_of = [&](int t) -> int { return t < ops0 ? wop<BW>(n, j0, t).hi + 1 : (int)n; };
 
-        if (wid == G) {
+        if (wid == CW) {
             // ---------------- producer warp: global -> window ----------------
-            // Each tick's copies arrive on the tick's mbarrier as they land; the
-            // producer runs up to D - 1 ticks ahead of the compute warps (the
-            // mbarrier ring) and never sits between two ticks.
+            // The copies of each of the leading sweep's ops arrive on the op's mbarrier
+            // as they land; the producer runs up to D - 1 ops ahead of that sweep.  The
+            // other sweeps are left of it.
             int issued = j0 + 1;               // columns below are requested (cp.async)
             int rp = (g == 0) ? (int)n : 0;    // retired[g-1] as last observed
-            int rp_next = rp;                  // lane 0: a relaxed read in flight, used next tick
+            int rp_next = rp;                  // lane 0: a relaxed read in flight, used at the next op
             // copies of the columns [from, to) into their slots (one column per step, lanes over chunks)
             auto copy_in = [&](int from, int to) {
                 int sl = from % W;
@@ -239,56 +281,57 @@ __global__ void __launch_bounds__(WinCfg<BW, G>::NT, 1)
                 }
             };
             for (int t = 0; t < nticks; ++t) {
-                const int need = tick_need(t);
-                if (t >= Cfg::D) {  // the ring slot of tick t is free once the compute warps are past tick t - D
-                    if (lane == 0) wait_shared_geq(&s_tick, t - Cfg::D + 1, err);
+                const int need = need_of(t);
+                if (t >= Cfg::D) {  // the ring slot of tick t is free once tick t - D is done
+                    if (lane == 0) wait_shared_geq(&s_tick, t - Cfg::D + 1, &s_fail, err);
                     __syncwarp();
                 }
                 if (issued < need) {
                     // not prefetched (the previous group was behind): load now
                     if (rp < need) {
-                        if (lane == 0) wait_geq(retired + g - 1, need, err);
+                        if (lane == 0 && !wait_geq(retired + g - 1, need, err)) st_volatile_shared(&s_fail, 1);
                         __syncwarp();
                         rp = max(need, __shfl_sync(0xffffffffu, lane == 0 ? ld_acquire(retired + g - 1) : 0, 0));
                     }
                     if (need > ld_volatile_shared(&s_wb) + W) {  // free slots (bounded wait on the publisher)
-                        if (lane == 0) wait_shared_geq(&s_wb, need - W, err);
+                        if (lane == 0) wait_shared_geq(&s_wb, need - W, &s_fail, err);
                         __syncwarp();
                     }
                     copy_in(issued, need);
                     issued = need;
                 }
-                cp_async_mbar_arrive(&s_full[t % Cfg::D]);  // tick t: when this lane's copies so far have landed
-                // lane 0's read of the previous group's boundary, issued last tick.  The
+                cp_async_mbar_arrive(&s_full[t % Cfg::D]);  // op t: when this lane's copies so far have landed
+                // lane 0's read of the previous group's boundary, issued at the last op.  The
                 // copies of the columns it releases are issued only once the value has
                 // arrived (their range depends on it) and read L2, where the previous
                 // group's writes were made visible before its release.
                 rp = max(rp, __shfl_sync(0xffffffffu, rp_next, 0));
                 if (g > 0 && rp < (int)n && lane == 0) rp_next = ld_relaxed(retired + g - 1);
-                // prefetch the columns of the next three ticks that the previous group
+                // prefetch the columns of the next three ops that the previous group
                 // has retired and whose slots are free
-                const int tgt = min(min(tick_need(t + 3), rp), min(ld_volatile_shared(&s_wb) + W, (int)n));
+                const int tgt = min(min(need_of(t + 3), rp), min(ld_volatile_shared(&s_wb) + W, (int)n));
                 if (tgt > issued) {
                     copy_in(issued, tgt);
                     issued = tgt;
                 }
             }
             cp_wait_all();
-        } else if (wid == G + 1) {
+        } else if (wid == CW + 1) {
             // ---------------- publisher warp: window -> global, retired[g] ----------------
-            // Follows the compute warps' progress: after tick t-1 the columns left
-            // of retire_after(t-1) are final for this group; they are written back
-            // and the boundary is released for the next group.
-            int wb = j0 + 1, seen = 0;
-            for (;;) {
-                int tk = seen;
-                if (lane == 0) tk = wait_shared_gt(&s_tick, seen, err);
-                tk = __shfl_sync(0xffffffffu, tk, 0);
-                if (tk <= seen) break;  // only after a timeout (recorded)
-                seen = tk;
-                const int r = (tk >= nticks) ? (int)n : retire_after(tk - 1);
+            // Follows the sweeps' progress: columns left of every sweep's current op
+            // are final for this group; they are written back and the boundary is
+            // released for the next group.
+            int wb = j0 + 1;
+            long long t0 = 0;
+            for (long long it = 0;;) {
+                int r = (int)n;
+                if (lane < gs) {  // the lowest column this sweep's current and later ops touch
+                    const int k = max(ld_acquire_shared(&s_tick) - LAG * lane, 0);
+                    if (k < wops<BW>(n, j0 + lane)) r = wop<BW>(n, j0 + lane, k).c0;
+                }
+                r = __reduce_min_sync(0xffffffffu, r);
+                __syncwarp();  // what each lane acquired is visible to the copying lanes
                 if (r > wb) {
-                    __threadfence_block();
                     int sl = wb % W;
                     for (int c = wb; c < r; ++c) {
                         for (int h = lane; h < Cfg::CHUNKS; h += 32) {
@@ -300,119 +343,172 @@ __global__ void __launch_bounds__(WinCfg<BW, G>::NT, 1)
                     __syncwarp();
                     wb = r;
                     if (lane == 0) {
-                        st_volatile_shared(&s_wb, wb);  // the slots may be refilled
+                        st_release_shared(&s_wb, wb);  // the slots may be refilled
                         __threadfence();
                         st_release(retired + g, wb);
                     }
+                    it = 0;
+                    if (r >= (int)n) break;
+                } else {
+                    if (it == 0) t0 = clock64();
+                    int over = 0;
+                    if (lane == 0 && (it & 63) == 63) over = wait_over(it, t0, &s_fail, err);
+                    if (__shfl_sync(0xffffffffu, over, 0)) break;
+                    ++it;
+                    __nanosleep(20);
                 }
-                if (tk >= nticks) break;
             }
         } else {
-            // ---------------- compute warps: warp i runs sweep j0 + i ----------------
-            // (one warp per sweep: measured faster than two warps sharing a sweep's
-            // reflector and halving its apply, 239 vs 300 ms at n = 16384)
-            const int sw = wid;
+            // ---------------- compute warps: WPS warps run sweep j0 + sw ----------------
+            constexpr int SEG = Cfg::SEG, RL = Cfg::RL, WPS = Cfg::WPS;
+            const int sw = wid / WPS, sub = wid % WPS;
             const int j = j0 + sw;
             const int ops = (sw < gs) ? wops<BW>(n, j) : 0;
-            V *sv = vbuf + wid * 32;
+            const int seg = lane / RL;                 // which SEG elements of the reflector
+            const int rl = sub * RL + lane % RL;       // which row (R op) / column (L op)
             for (int t = 0; t < nticks; ++t) {
                 bar_sync(1, Cfg::NC);  // every compute warp is done with tick t-1
-                if (wid == 0 && lane == 0) {
-                    __threadfence_block();
-                    st_volatile_shared(&s_tick, t);  // ticks < t are done (publisher, producer)
-                }
-                mbar_wait(&s_full[t % Cfg::D], (unsigned)(t / Cfg::D) & 1u, err);  // tick t's columns are in
-                const int k = t - 4 * sw;
-                if (k >= 0 && k < ops) {
-                    const WOp o = wop<BW>(n, j, k);
-                    const int L = o.c1 - o.c0 + 1;
-                    if (L >= 2) {
-                        const bool rop = (k & 1) == 0;
-                        const int rho = rop ? ((k == 0) ? j : o.c0 - BW) : o.c0;
-                        // reflector input: row rho (R op) or column c0 (L op), columns/rows c0..c1
-                        V x = Ar::zero();
-                        if (lane < L) x = Ar::lds(rop ? A(rho, o.c0 + lane) : A(o.c0 + lane, o.c0));
-                        typename Ar::Acc acc = Ar::acc_zero();
-                        if (lane >= 1 && lane < L) Ar::acc_add(acc, x, x);
-                        const V s = wsum<S>(Ar::acc_value(acc));
-                        const V alpha = Ar::shfl(x, 0);
-                        V tau = Ar::zero(), beta = alpha, scal = Ar::zero();
-                        if (Ar::gt0(s)) {
-                            const V nrm = Ar::sqrt(Ar::fma(alpha, alpha, s));
-                            beta = Ar::ge0(alpha) ? Ar::neg(nrm) : nrm;
-                            tau = Ar::mul(Ar::sub(beta, alpha), Ar::rcp(beta));
-                            scal = Ar::rcp(Ar::sub(alpha, beta));
-                        }
-                        if (lane < L) sv[lane] = (lane == 0) ? Ar::one() : Ar::mul(x, scal);
-                        __syncwarp();
-                        if (!Ar::iszero(tau)) {
-                            // column c0 + i sits in slot s0 + i (wrapping at W): one modulo per op
-                            const int s0 = o.c0 % W;
-                            if (rop) {
-                                // lane = row r: A(r, c0 + i) at slot(c0 + i) * LDW + (r - c0 - i + KU);
-                                // from column to column the address moves by LDW - 1 (- W LDW at the wrap)
-                                for (int r = rho + 1 + lane; r <= o.c1; r += 32) {
-                                    St *p0 = win + (size_t)s0 * LDW + (r - o.c0 + KU);
-                                    V xv[BW];
-                                    typename Ar::Acc a = Ar::acc_zero();
-                                    {
-                                        St *p = p0;
-#pragma unroll
-                                        for (int i = 0; i < BW; ++i) {
-                                            if (i < L) {
-                                                xv[i] = Ar::lds(p);
-                                                Ar::acc_add(a, xv[i], sv[i]);
-                                            }
-                                            p += LDW - 1;
-                                            if (s0 + i + 1 == W) p -= (size_t)W * LDW;
-                                        }
-                                    }
-                                    const V w = Ar::mul(Ar::acc_value(a), tau);
-                                    St *p = p0;
-#pragma unroll
-                                    for (int i = 0; i < BW; ++i) {
-                                        if (i < L) Ar::st(p, Ar::sub(xv[i], Ar::mul(w, sv[i])));
-                                        p += LDW - 1;
-                                        if (s0 + i + 1 == W) p -= (size_t)W * LDW;
-                                    }
-                                }
-                            } else {
-                                // lane = column c: rows c0 .. c0+L-1 contiguous from A(c0, c)
-                                for (int c = o.c0 + 1 + lane; c <= o.hi; c += 32) {
-                                    int sl = s0 + (c - o.c0);
-                                    sl -= (sl >= W) ? W : 0;
-                                    St *p = win + (size_t)sl * LDW + (o.c0 - c + KU);
-                                    V xv[BW];
-                                    typename Ar::Acc a = Ar::acc_zero();
-#pragma unroll
-                                    for (int i = 0; i < BW; ++i) {
-                                        if (i < L) {
-                                            xv[i] = Ar::lds(p + i);
-                                            Ar::acc_add(a, sv[i], xv[i]);
-                                        }
-                                    }
-                                    const V w = Ar::mul(Ar::acc_value(a), tau);
-#pragma unroll
-                                    for (int i = 0; i < BW; ++i)
-                                        if (i < L) Ar::st(p + i, Ar::sub(xv[i], Ar::mul(w, sv[i])));
-                                }
-                            }
-                        }
-                        // the pivot row / column: beta and zeros (every lane has read it:
-                        // the norm's shuffles came after the reads)
-                        if (lane < L) {
-                            St *p = rop ? A(rho, o.c0 + lane) : A(o.c0 + lane, o.c0);
-                            Ar::st(p, lane == 0 ? beta : Ar::zero());
-                        }
+                if (tid == 0) st_release_shared(&s_tick, t);
+                mbar_wait(&s_full[t % Cfg::D], (unsigned)(t / Cfg::D) & 1u, &s_fail, err);  // tick t's columns are in
+                const int k = t - LAG * sw;
+                const bool run = k >= 0 && k < ops;
+                const WOp o = wop<BW>(n, j, max(k, 0));
+                const int L = o.c1 - o.c0 + 1;
+                const bool act = run && L >= 2;
+                const bool rop = (k & 1) == 0;
+                // element i of the pivot (row rho of an R op, column c0 of an L op)
+                // and of this lane's row / column at base + i * stride; an R op's
+                // columns past the window's last slot continue at slot 0
+                const int s0 = o.c0 % W;
+                const int iw = W - s0;
+                const bool fast = (L == BW) && (!rop || iw >= BW);
+                const int rho = rop ? ((k == 0) ? j : o.c0 - BW) : o.c0;
+                St *piv = win + (size_t)s0 * LDW + (rho - o.c0 + KU);
+                St *row = piv;
+                bool valid = false;
+                if (act) {
+                    if (rop) {
+                        valid = rho + 1 + rl <= o.c1;
+                        if (valid) row = piv + 1 + rl;
+                    } else {
+                        const int c = o.c0 + 1 + rl;
+                        valid = c <= o.hi;
+                        int sl = s0 + 1 + rl;
+                        sl -= (sl >= W) ? W : 0;
+                        if (valid) row = win + (size_t)sl * LDW + (o.c0 - c + KU);
                     }
                 }
-                __syncwarp();
+                // The op in two phases.  Phase 1 reads the pivot, forms the scalars and
+                // all of the dot product but elements 0 and BW-1; the new pivot then goes
+                // to the window and is posted.  Phase 2 reads element BW-1, which op k+2
+                // of the previous sweep wrote, or which is the pivot of its op k+3 (the
+                // only element that ops three apart share), and applies.
+                V xr[SEG], xv[SEG];
+                typename Ar::Acc a = Ar::acc_zero();
+                V u0 = Ar::zero(), beta = Ar::zero(), rn = Ar::zero(), inv = Ar::zero();
+                bool nz = false;
+                V a0 = Ar::zero(), xl = Ar::zero();
+                auto phase1 = [&](auto fast_c, auto rop_c) {
+                    constexpr bool FAST = decltype(fast_c)::value, ROP = decltype(rop_c)::value;
+                    constexpr int STR = ROP ? LDW - 1 : 1;
+                    auto off = [&](int i) -> int { return i * STR - ((!FAST && ROP && i >= iw) ? W * LDW : 0); };
+                    const V alpha = Ar::lds(piv);
+#pragma unroll
+                    for (int q = 0; q < SEG; ++q) {
+                        const int i = seg * SEG + q;
+                        xr[q] = (FAST || i < L) ? Ar::lds(piv + off(i)) : Ar::zero();
+                    }
+                    xl = (FAST || BW - 1 < L) ? Ar::lds(piv + off(BW - 1)) : Ar::zero();
+                    a0 = Ar::lds(row);
+#pragma unroll
+                    for (int q = 0; q < SEG; ++q) {
+                        const int i = seg * SEG + q;
+                        const bool inner = q > 0 || seg > 0;  // element BW-1 only in phase 2
+                        xv[q] = ((FAST || i < L) && inner && (q < SEG - 1 || seg < H - 1)) ? Ar::lds(row + off(i))
+                                                                                          : Ar::zero();
+                    }
+                    // ||x||^2 without element 0, one element per lane and a butterfly (fewer
+                    // instructions than summing it in every lane: 20.7 against 21.9 ms for
+                    // the chase at n = 4096), and the dot product without elements 0 and
+                    // BW-1 (their xv are zero here)
+                    typename Ar::Acc s = Ar::acc_zero();
+                    {
+                        const int il = lane % BW;
+                        const V xs = (il >= 1 && (FAST || il < L)) ? Ar::lds(piv + off(il)) : Ar::zero();
+                        Ar::acc_add(s, xs, xs);
+                    }
+#pragma unroll
+                    for (int sh = BW / 2; sh >= 1; sh >>= 1) s = Wa::merge_xor(s, sh);
+#pragma unroll
+                    for (int q = 0; q < SEG; ++q)
+                        if ((q > 0 || H > 1) && (q < SEG - 1 || H > 1)) Ar::acc_add(a, xv[q], xr[q]);
+#pragma unroll
+                    for (int sh = RL; sh < 32; sh <<= 1) a = Wa::merge_xor(a, sh);
+                    // H = I - u u^T / (||x|| (||x|| + |alpha|)), u = x with u_0 = alpha - beta,
+                    // beta = -sign(alpha) ||x||: u needs no scaling, so the dot products do
+                    // not wait for the norm
+                    nz = Wa::positive(s);
+                    beta = alpha;
+                    if (nz) {
+                        V nrm;
+                        rsqrt_sqrt(Wa::norm2(s, alpha), rn, nrm);
+                        const bool pos = Ar::ge0(alpha);
+                        const V u = Ar::add(pos ? alpha : Ar::neg(alpha), nrm);
+                        u0 = pos ? u : Ar::neg(u);
+                        beta = pos ? Ar::neg(nrm) : nrm;
+                    }
+                };
+                auto put_pivot = [&](auto fast_c, auto rop_c) {
+                    constexpr bool FAST = decltype(fast_c)::value, ROP = decltype(rop_c)::value;
+                    constexpr int STR = ROP ? LDW - 1 : 1;
+                    if (lane < (FAST ? BW : L))
+                        Ar::st(piv + lane * STR - ((!FAST && ROP && lane >= iw) ? W * LDW : 0),
+                               lane == 0 ? beta : Ar::zero());
+                };
+                auto phase2 = [&](auto fast_c, auto rop_c) {
+                    constexpr bool FAST = decltype(fast_c)::value, ROP = decltype(rop_c)::value;
+                    constexpr int STR = ROP ? LDW - 1 : 1;
+                    auto off = [&](int i) -> int { return i * STR - ((!FAST && ROP && i >= iw) ? W * LDW : 0); };
+                    const V al = (FAST || BW - 1 < L) ? Ar::lds(row + off(BW - 1)) : Ar::zero();
+                    Ar::acc_add(a, al, xl);
+                    const V w = Ar::mul(Ar::mul(Ar::acc_value(a), rn), inv);
+                    if (seg == 0) {
+                        xv[0] = a0;
+                        xr[0] = u0;
+                    }
+                    if (seg == H - 1) xv[SEG - 1] = al;
+                    if (valid) {
+#pragma unroll
+                        for (int q = 0; q < SEG; ++q) {
+                            const int i = seg * SEG + q;
+                            if (FAST || i < L) Ar::st(row + off(i), Wa::sub_mul(xv[q], w, xr[q]));
+                        }
+                    }
+                };
+                auto dispatch = [&](auto f) {
+                    if (fast) {
+                        if (rop) f(std::true_type{}, std::true_type{});
+                        else f(std::true_type{}, std::false_type{});
+                    } else {
+                        if (rop) f(std::false_type{}, std::true_type{});
+                        else f(std::false_type{}, std::false_type{});
+                    }
+                };
+                if (act) dispatch(phase1);
+                if (WPS > 1) bar_sync(3 + sw, 32 * WPS);  // every warp of the sweep has read the pivot
+                else __syncwarp();
+                if (act && sub == 0) dispatch(put_pivot);
+                if (act && nz) {
+                    // the rest of the scalars and element 0's term, while the previous sweep
+                    // reaches the pivot of its op k+3
+                    inv = rcp_est(Ar::ge0(u0) ? u0 : Ar::neg(u0));
+                    Ar::acc_add(a, a0, u0);
+                }
+                bar_sync(2, Cfg::NC);  // the tick's new pivots are in the window
+                if (act && nz) dispatch(phase2);
             }
             bar_sync(1, Cfg::NC);
-            if (wid == 0 && lane == 0) {
-                __threadfence_block();
-                st_volatile_shared(&s_tick, nticks);  // all ticks done
-            }
+            if (tid == 0) st_release_shared(&s_tick, kAllDone);
         }
         __syncthreads();
         if (tid == 0) {  // fresh phases for the next group
@@ -424,12 +520,12 @@ __global__ void __launch_bounds__(WinCfg<BW, G>::NT, 1)
     }
 }
 
-template <int BW, typename S, int G>
+template <int BW, typename S, int G, int H>
 int launch_win(typename ChaseAr<S>::St *dAB, int64_t n, const Stage2Work &w, cudaStream_t s, int num_sms, int batch,
                int64_t sAB) {
-    using Cfg = WinCfg<BW, G>;
+    using Cfg = WinCfg<BW, G, H>;
     const size_t smem = Cfg::smem_bytes();
-    auto kern = chase_win_kernel<BW, S, G>;
+    auto kern = chase_win_kernel<BW, S, G, H>;
     AVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Cfg::NT, smem) != cudaSuccess || per_sm < 1) {
@@ -455,14 +551,21 @@ static int chase_window(typename ChaseAr<S>::St *dAB, int64_t n, int bw, const S
     if (n < 2 || batch < 1) return AVS_SUCCESS;
     if (n > ((int64_t)1 << 30) || (int64_t)batch * n > ((int64_t)1 << 31) - 64) return AVS_ERR_UNSUPPORTED;
     AVS_CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(int) * (size_t)((n + 1) * (int64_t)batch + 1), s));
+    // Sweeps per CTA (G) and lanes per row (H), swept on GB300.  Double-float, band
+    // 16: more sweeps share the hand-off between groups, but the tick is issue-bound
+    // once a scheduler has four warps (G = 8, H = 2), and one warp per sweep (H = 1)
+    // has twice the instructions on its path: G x H = 4 x 2 21.1 ms, 8 x 1 23.3, 4 x 1
+    // 24.0, 2 x 2 25.8, 8 x 2 26.1 at n = 4096; batches agree within 10% (32 matrices
+    // of order 1024: 10.3 ms of stage 2, 8 x 2 10.7, 8 x 1 11.9).  FP64 is bound by
+    // the FP64 unit's issue (64 cycles a warp instruction): H = 1, which repeats no
+    // reflector, and few sweeps per SM (n = 512, band 16: 4 x 1 6.3 ms, 8 x 1 7.8, 4 x 2
+    // 7.6; band 32: 2 x 1 11.4, 3 x 1 11.5, 3 x 2 13.9).  The values do not depend on G
+    // or, with one matrix or many, on the batch.
+    constexpr bool df = std::is_same<S, df64>::value;
     switch (bw) {
-        case 8: return launch_win<8, S, 8>(dAB, n, w, s, num_sms, batch, sAB);
-        // band 16: 8 sweeps per CTA for one matrix (n = 16384: 322 ms of stage 2 against 334 with 4); 4 for
-        // batches, whose matrices give the launch enough groups (512 matrices of order 256: 31.8 against
-        // 35.8 ms); the values do not depend on it
-        case 16: return batch > 1 ? launch_win<16, S, 4>(dAB, n, w, s, num_sms, batch, sAB)
-                                  : launch_win<16, S, 8>(dAB, n, w, s, num_sms, batch, sAB);
-        case 32: return launch_win<32, S, 3>(dAB, n, w, s, num_sms, batch, sAB);
+        case 8: return launch_win<8, S, 8, 2>(dAB, n, w, s, num_sms, batch, sAB);
+        case 16: return launch_win<16, S, 4, df ? 2 : 1>(dAB, n, w, s, num_sms, batch, sAB);
+        case 32: return launch_win<32, S, df ? 3 : 2, df ? 2 : 1>(dAB, n, w, s, num_sms, batch, sAB);
         default: return AVS_ERR_UNSUPPORTED;
     }
 }
