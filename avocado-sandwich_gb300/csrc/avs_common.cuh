@@ -18,10 +18,9 @@ enum DeviceError : int {
 };
 
 // Bounds of any dependency wait: at most kSpinLimit polls (an acquire load and
-// a 32 ns sleep each, about 1 us with the load's latency) and at most
-// kWaitNs of %globaltimer, whichever comes first -- far beyond any legitimate
-// wait, short enough that a lost dependency returns AVS_ERR_TIMEOUT instead of
-// hanging the GPU.
+// a short sleep each, about 1 us with the load's latency) and at most kWaitNs,
+// whichever comes first -- far beyond any legitimate wait, short enough that a
+// lost dependency returns AVS_ERR_TIMEOUT instead of hanging the GPU.
 constexpr long long kSpinLimit = 1ll << 27;
 constexpr long long kWaitNs = 4000000000ll;  // 4 s
 
@@ -58,21 +57,23 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 // Bounded wait until *flag >= target.  Called by one thread; returns false on
 // timeout (after recording kDevTimeout in *err) or when another CTA already
-// failed.  Never spins forever: at most kSpinLimit polls and limit_ns of
-// %globaltimer.
+// failed.  Never spins forever: at most kSpinLimit polls and limit_ns, measured
+// on the SM's clock at 2 cycles per ns (its maximum is 2.07 GHz; reading it takes
+// a few cycles, %globaltimer hundreds).  The first polls follow one another at
+// the load's latency: most waits are shorter than a sleep.
 __device__ __forceinline__ bool wait_geq_n(const int *flag, int target, int *err, long long limit_ns) {
     if (ld_acquire(flag) >= target) return true;
-    const unsigned long long t0 = global_ns();
+    const long long t0 = clock64();
     for (long long it = 0;; ++it) {
         if (ld_acquire(flag) >= target) return true;
         if ((it & 15) == 15) {  // another CTA's failure, the bounds: every 16 polls
             if (ld_acquire(err) != kDevOk) return false;
-            if (it > kSpinLimit || (long long)(global_ns() - t0) > limit_ns) {
+            if (it > kSpinLimit || clock64() - t0 > 2 * limit_ns) {
                 atomicCAS(err, kDevOk, kDevTimeout);
                 return false;
             }
         }
-        __nanosleep(32);
+        if (it >= 16) __nanosleep(32);
     }
 }
 __device__ __forceinline__ bool wait_geq(const int *flag, int target, int *err) {

@@ -18,9 +18,8 @@
 // its column block cb as soon as role p-1 has finished block cb: the roles form
 // a systolic pipeline over the row tiles whose critical path is
 // (#tiles + b/16) block steps instead of #tiles * b reflector steps.  Within a
-// block the 16 reflectors are generated one column at a time, their
-// compact-WY factor T (16 x 16) is formed, and the block is applied to the rest
-// of the tile with it.  A role hands block cb on in two parts: the 16 x 16
+// block the 16 reflectors are generated one column at a time, and the block is
+// applied to the rest of the tile in compact-WY form (16 reflectors).  A role hands block cb on in two parts: the 16 x 16
 // diagonal block of the top rows right after its reflectors (all the next
 // role's reflectors read), and the trailing top rows after its apply (which the
 // next role reads only in its own apply), so the step between roles is one
@@ -49,6 +48,7 @@
 
 #include "avs_common.cuh"
 #include "df64.cuh"
+#include "reflect.cuh"
 
 namespace avs {
 namespace {
@@ -85,159 +85,172 @@ struct UpdateArgs {
     int64_t sA, sTblk;  // per-matrix strides (blockIdx.y = matrix)
 };
 
-__host__ __device__ inline int ldpad(int b) { return b + 1; }
+__host__ __device__ inline int ldpad(int b) { return b + 1; }  // update_kernel's strips
 
 // ---------------------------------------------------------------------------
-// Reflector scalars.  The reference's expressions (QRkernels.jl:27-31) in
-// closed form: n1 = ||x||, nu = alpha + sign(alpha) n1,
-// tau = 2 nu^2 / (s + nu^2) = |nu| / n1, tau / nu = sign(nu) / n1,
-// tau / nu^2 = 1 / (n1 |nu|), new diagonal beta = -sign(alpha) n1; evaluated in
-// FP64 for FP64 tiles and in double-float for FP32 tiles (GB300 issues FP64 at
-// 1/64 of the FP32 rate).
-
-// Reflector scalars from s = sum of squares of the sub-column (as a pair) and
-// alpha.  Writes nu, tau, tau/nu, tau/nu^2, 1/nu, beta (the new diagonal).
-struct PScalars {
-    double nu, tau, tc, f, inv, beta;
+// Panel arithmetic by compute type.  Sq: a sum of squares (compensated pairs
+// (sum, error) for FP32 and double-float, merged without renormalising between
+// levels; plain for FP64).  scalars: the reference's expressions
+// (QRkernels.jl:27-31) in closed form: n1 = ||x||, nu = alpha + sign(alpha) n1,
+// tau = 2 nu^2 / (s + nu^2) = |nu| / n1, tc = tau / nu = sign(nu) / n1,
+// f = tau / nu^2 = 1 / (n1 |nu|), inv = 1 / nu, beta = -sign(alpha) n1 (the new
+// diagonal); evaluated in double-float for FP32 tiles and rounded once, in FP64
+// for FP64 tiles (reflect.cuh: hardware estimates and one residual each).
+// mac / fin: products accumulated into Mac (double-float: the compensated
+// dot product of Ogita, Rump and Oishi) and the value of the accumulator.
+template <typename CT>
+struct PRefl {
+    CT nu, tc, f, inv, beta, tau;
 };
 
-__device__ __forceinline__ PScalars pscal_double(double s, double alpha) {
-    PScalars r;
-    const double n1 = sqrt(s + alpha * alpha);
-    const double sg = alpha < 0.0 ? -1.0 : 1.0;
-    r.nu = alpha + sg * n1;
-    if (r.nu == 0.0) {
-        r.tau = r.tc = r.f = r.inv = 0.0;
-        r.beta = alpha;
-        return r;
+template <typename CT>
+struct PAr;
+
+struct PSqPair {
+    using Sq = float2;
+    static __device__ __forceinline__ Sq merge(Sq a, Sq b) {
+        const df64 t = two_sum(a.x, b.x);
+        return make_float2(t.hi, __fadd_rn(t.lo, __fadd_rn(a.y, b.y)));
     }
-    const double rn1 = 1.0 / n1;
-    const double anu = fabs(r.nu);
-    r.tau = anu * rn1;
-    r.tc = (r.nu < 0.0 ? -rn1 : rn1);
-    r.inv = 1.0 / r.nu;
-    r.f = rn1 * fabs(r.inv);
-    r.beta = -sg * n1;
-    return r;
-}
-
-// FP32 tiles: the same closed forms in double-float, rounded to FP32 at the
-// end -- no FP64 instruction (GB300 runs those at 1/64 of the FP32 rate).
-struct PScalarsF {
-    float nu, tau, tc, f, inv, beta;
-};
-
-__device__ __forceinline__ PScalarsF pscal_float(df64 s, float alpha) {
-    PScalarsF r;
-    const df64 x = df_add(s, two_prod(alpha, alpha));  // n1^2
-    if (x.hi <= 0.0f) {  // zero column: identity reflector
-        r.nu = r.tau = r.tc = r.f = r.inv = 0.0f;
-        r.beta = alpha;
-        return r;
-    }
-    // 1/n1: hardware rsqrt estimate, one Newton step in double-float:
-    // y' = y + y (1 - x y^2) / 2
-    const float y0 = rsqrtf(x.hi);
-    const df64 e = df_sub(df64{1.0f, 0.0f}, df_mul(x, two_prod(y0, y0)));
-    const df64 rn1 = df_add(df64{y0, 0.0f}, df_mul_f(e, 0.5f * y0));
-    const df64 n1 = df_mul(x, rn1);
-    const bool neg = alpha < 0.0f;
-    const df64 a = df64{alpha, 0.0f};
-    const df64 nu = neg ? df_sub(a, n1) : df_add(a, n1);  // |nu| = |alpha| + n1 > 0
-    // 1/nu: hardware reciprocal estimate, one Newton step: z' = z + z (1 - nu z)
-    const float z0 = __fdividef(1.0f, nu.hi);
-    const df64 ez = df_sub(df64{1.0f, 0.0f}, df_mul_f(nu, z0));
-    const df64 inv = df_add(df64{z0, 0.0f}, df_mul_f(ez, z0));
-    const df64 anu = neg ? df_neg(nu) : nu;
-    const df64 ainv = neg ? df_neg(inv) : inv;
-    const df64 tau = df_mul(anu, rn1);
-    const df64 f = df_mul(rn1, ainv);
-    r.nu = nu.hi + nu.lo;
-    r.tau = tau.hi + tau.lo;
-    r.tc = neg ? -(rn1.hi + rn1.lo) : (rn1.hi + rn1.lo);
-    r.inv = inv.hi + inv.lo;
-    r.f = f.hi + f.lo;
-    r.beta = neg ? (n1.hi + n1.lo) : -(n1.hi + n1.lo);
-    return r;
-}
-
-template <typename T>
-struct PScal;
-template <>
-struct PScal<double> {
-    using Acc = double;
-    static __device__ __forceinline__ Acc zero() { return 0.0; }
-    static __device__ __forceinline__ Acc sq(double x, Acc a) { return fma(x, x, a); }
-    static __device__ __forceinline__ Acc shfl_add(Acc a, int o) { return a + __shfl_xor_sync(0xffffffffu, a, o); }
-    static __device__ __forceinline__ Acc shfl_add_local(Acc a, Acc b) { return a + b; }
-    static __device__ __forceinline__ void compute(Acc s, double alpha, double *out) {
-        const PScalars r = pscal_double(s, alpha);
-        out[0] = r.nu; out[1] = r.tc; out[2] = r.f; out[3] = r.inv; out[4] = r.beta; out[5] = r.tau;
+    static __device__ __forceinline__ Sq merge_xor(Sq a, int o) {
+        return merge(a, make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o)));
     }
 };
 template <>
-struct PScal<float> {
-    using Acc = df64;
-    static __device__ __forceinline__ Acc zero() { return df64{0.0f, 0.0f}; }
-    static __device__ __forceinline__ Acc sq(float x, Acc a) { return df_add(a, two_prod(x, x)); }
-    static __device__ __forceinline__ Acc shfl_add(Acc a, int o) {
-        return df_add(a, df64{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)});
+struct PAr<float> : PSqPair {
+    using Mac = float;
+    static __device__ __forceinline__ Sq sq(float x) {
+        const float p = __fmul_rn(x, x);
+        return make_float2(p, __fmaf_rn(x, x, -p));
     }
-    static __device__ __forceinline__ Acc shfl_add_local(Acc a, Acc b) { return df_add(a, b); }
-    static __device__ __forceinline__ void compute(Acc s, float alpha, float *out) {
-        const PScalarsF r = pscal_float(s, alpha);
-        out[0] = r.nu; out[1] = r.tc; out[2] = r.f; out[3] = r.inv; out[4] = r.beta; out[5] = r.tau;
+    // The two hardware estimates start as soon as their arguments are known to
+    // FP32 and everything else is a residual of them: with r ~ 1/n1 and z ~ 1/|nu|,
+    // n1 = x r (1 + g), 1/n1 = r (1 + g), 1/|nu| = z (1 + k); relative errors
+    // below 2^-44 before the one rounding of each result.
+    static __device__ __forceinline__ PRefl<float> scalars(Sq s, float alpha) {
+        PRefl<float> o;
+        const float xa = fmaf(alpha, alpha, s.x);  // n1^2 to FP32
+        if (xa <= 0.0f) {  // zero column: identity reflector
+            o.nu = o.tau = o.tc = o.f = o.inv = 0.0f;
+            o.beta = alpha;
+            return o;
+        }
+        const float r = rsqrt_hw(xa);
+        const df64 a2 = two_prod(alpha, alpha);
+        const df64 x = two_sum(a2.hi, s.x);
+        const float xl = __fadd_rn(x.lo, __fadd_rn(a2.lo, s.y));
+        const float t = __fmul_rn(x.hi, r);
+        const float tl = __fmaf_rn(xl, r, __fmaf_rn(x.hi, r, -t));
+        const float aa = fabsf(alpha);
+        const df64 u = two_sum(aa, t);
+        const float z = rcp_hw(u.hi);
+        const float e = __fmaf_rn(-tl, r, __fmaf_rn(-t, r, 1.0f));
+        const float g = __fmul_rn(e, __fmaf_rn(0.375f, e, 0.5f));
+        const float nl = __fmaf_rn(t, g, tl);   // n1 = t + nl
+        const float ul = __fadd_rn(u.lo, nl);   // |nu| = u.hi + ul
+        const float ez = __fmaf_rn(-ul, z, __fmaf_rn(-u.hi, z, 1.0f));
+        const float k = __fmaf_rn(ez, ez, ez);
+        const bool neg = alpha < 0.0f;
+        const float nu = __fadd_rn(u.hi, ul), n1 = __fadd_rn(t, nl);
+        const float rn = __fmaf_rn(r, g, r), inv = __fmaf_rn(z, k, z);
+        const float p = __fmul_rn(u.hi, r);
+        o.tau = __fadd_rn(p, __fmaf_rn(p, g, __fmaf_rn(ul, r, __fmaf_rn(u.hi, r, -p))));
+        const float q = __fmul_rn(r, z);
+        o.f = __fadd_rn(q, __fmaf_rn(q, __fadd_rn(g, k), __fmaf_rn(r, z, -q)));
+        o.nu = neg ? -nu : nu;
+        o.tc = neg ? -rn : rn;
+        o.inv = neg ? -inv : inv;
+        o.beta = neg ? n1 : -n1;
+        return o;
     }
+    static __device__ __forceinline__ Mac mac0() { return 0.0f; }
+    static __device__ __forceinline__ Mac mac_from(float x) { return x; }
+    static __device__ __forceinline__ void mac(Mac &a, float x, float y) { a = fmaf(x, y, a); }
+    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) { return a + b; }
+    static __device__ __forceinline__ float fin(Mac a) { return a; }
 };
-
-// FP64 tiles in double-float arithmetic (AVS_PREC_FP64X2): the same closed
-// forms with alpha and the results as double-float values.
-struct PScalarsD {
-    df64 nu, tau, tc, f, inv, beta;
-};
-
-__device__ __forceinline__ PScalarsD pscal_df(df64 s, df64 alpha) {
-    PScalarsD r;
-    const df64 x = df_add(s, df_mul(alpha, alpha));  // n1^2
-    const df64 z{0.0f, 0.0f};
-    if (x.hi <= 0.0f) {  // zero column: identity reflector
-        r.nu = r.tau = r.tc = r.f = r.inv = z;
-        r.beta = alpha;
+// FP64 tiles in double-float arithmetic (AVS_PREC_FP64X2)
+template <>
+struct PAr<dfx> : PSqPair {
+    using Mac = df64;
+    static __device__ __forceinline__ Sq sq(dfx v) {
+        const df64 x = v.v;
+        const float p = __fmul_rn(x.hi, x.hi);
+        return make_float2(p, __fmaf_rn(2.0f * x.hi, x.lo, __fmaf_rn(x.hi, x.hi, -p)));
+    }
+    static __device__ __forceinline__ PRefl<dfx> scalars(Sq s, dfx al) {
+        PRefl<dfx> r;
+        const df64 alpha = al.v;
+        const Sq m = merge(s, sq(al));
+        const df64 x = fast_two_sum(m.x, m.y);
+        if (x.hi <= 0.0f) {
+            r.nu = r.tau = r.tc = r.f = r.inv = dfx(0);
+            r.beta = al;
+            return r;
+        }
+        df64 rn, n1;
+        rsqrt_sqrt(x, rn, n1);
+        const bool neg = df_lt0(alpha);
+        const df64 u = df_add(neg ? df_neg(alpha) : alpha, n1);
+        const df64 iu = rcp_est(u);
+        r.nu = dfx(neg ? df_neg(u) : u);
+        r.tau = dfx(df_mul(u, rn));
+        r.tc = dfx(neg ? df_neg(rn) : rn);
+        r.inv = dfx(neg ? df_neg(iu) : iu);
+        r.f = dfx(df_mul(rn, iu));
+        r.beta = dfx(neg ? n1 : df_neg(n1));
         return r;
     }
-    // 1/n1 and 1/nu: FP32 estimates refined by one Newton step in double-float
-    const float y0 = rsqrtf(x.hi);
-    const df64 e = df_sub(df64{1.0f, 0.0f}, df_mul(x, two_prod(y0, y0)));
-    const df64 rn1 = df_add(df64{y0, 0.0f}, df_mul_f(e, 0.5f * y0));
-    const df64 n1 = df_mul(x, rn1);
-    const bool neg = df_lt0(alpha);
-    const df64 nu = neg ? df_sub(alpha, n1) : df_add(alpha, n1);  // |nu| = |alpha| + n1 > 0
-    const df64 inv = df_rcp(nu);
-    const df64 anu = neg ? df_neg(nu) : nu;
-    const df64 ainv = neg ? df_neg(inv) : inv;
-    r.nu = nu;
-    r.tau = df_mul(anu, rn1);
-    r.tc = neg ? df_neg(rn1) : rn1;
-    r.inv = inv;
-    r.f = df_mul(rn1, ainv);
-    r.beta = neg ? n1 : df_neg(n1);
-    return r;
-}
-
+    static __device__ __forceinline__ Mac mac0() { return df64{0.0f, 0.0f}; }
+    static __device__ __forceinline__ Mac mac_from(dfx x) { return x.v; }
+    static __device__ __forceinline__ void mac(Mac &a, dfx x, dfx y) {
+        const float p = __fmul_rn(x.v.hi, y.v.hi);
+        float ep = __fmaf_rn(x.v.hi, y.v.hi, -p);
+        ep = __fmaf_rn(x.v.hi, y.v.lo, ep);
+        ep = __fmaf_rn(x.v.lo, y.v.hi, ep);
+        const df64 t = two_sum(a.hi, p);
+        a.hi = t.hi;
+        a.lo = __fadd_rn(a.lo, __fadd_rn(t.lo, ep));
+    }
+    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) {
+        const df64 t = two_sum(a.hi, b.hi);
+        return df64{t.hi, __fadd_rn(t.lo, __fadd_rn(a.lo, b.lo))};
+    }
+    static __device__ __forceinline__ dfx fin(Mac a) { return dfx(two_sum(a.hi, a.lo)); }
+};
 template <>
-struct PScal<dfx> {
-    using Acc = df64;
-    static __device__ __forceinline__ Acc zero() { return df64{0.0f, 0.0f}; }
-    static __device__ __forceinline__ Acc sq(dfx x, Acc a) { return df_add(a, df_mul(x.v, x.v)); }
-    static __device__ __forceinline__ Acc shfl_add(Acc a, int o) {
-        return df_add(a, df64{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)});
+struct PAr<double> {
+    using Sq = double;
+    using Mac = double;
+    static __device__ __forceinline__ Sq sq(double x) { return x * x; }
+    static __device__ __forceinline__ Sq merge(Sq a, Sq b) { return a + b; }
+    static __device__ __forceinline__ Sq merge_xor(Sq a, int o) { return a + __shfl_xor_sync(0xffffffffu, a, o); }
+    static __device__ __forceinline__ PRefl<double> scalars(Sq s, double alpha) {
+        PRefl<double> r;
+        const double x = fma(alpha, alpha, s);
+        if (x == 0.0) {
+            r.nu = r.tau = r.tc = r.f = r.inv = 0.0;
+            r.beta = alpha;
+            return r;
+        }
+        double rn, n1;
+        rsqrt_sqrt(x, rn, n1);
+        const bool neg = alpha < 0.0;
+        const double u = fabs(alpha) + n1;
+        const double iu = rcp_est(u);
+        r.nu = neg ? -u : u;
+        r.tau = u * rn;
+        r.tc = neg ? -rn : rn;
+        r.inv = neg ? -iu : iu;
+        r.f = rn * iu;
+        r.beta = neg ? n1 : -n1;
+        return r;
     }
-    static __device__ __forceinline__ Acc shfl_add_local(Acc a, Acc b) { return df_add(a, b); }
-    static __device__ __forceinline__ void compute(Acc s, dfx alpha, dfx *out) {
-        const PScalarsD r = pscal_df(s, alpha.v);
-        out[0] = dfx(r.nu); out[1] = dfx(r.tc); out[2] = dfx(r.f); out[3] = dfx(r.inv); out[4] = dfx(r.beta);
-        out[5] = dfx(r.tau);
-    }
+    static __device__ __forceinline__ Mac mac0() { return 0.0; }
+    static __device__ __forceinline__ Mac mac_from(double x) { return x; }
+    static __device__ __forceinline__ void mac(Mac &a, double x, double y) { a = fma(x, y, a); }
+    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) { return a + b; }
+    static __device__ __forceinline__ double fin(Mac a) { return a; }
 };
 
 // Warp shuffles and finiteness of the panel's compute types.
@@ -246,116 +259,241 @@ __device__ __forceinline__ double vshfl_xor(double v, int o) { return __shfl_xor
 __device__ __forceinline__ dfx vshfl_xor(dfx v, int o) {
     return dfx(df64{__shfl_xor_sync(0xffffffffu, v.v.hi, o), __shfl_xor_sync(0xffffffffu, v.v.lo, o)});
 }
-__device__ __forceinline__ float vshfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ double vshfl(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ dfx vshfl(dfx v, int src) {
-    return dfx(df64{__shfl_sync(0xffffffffu, v.v.hi, src), __shfl_sync(0xffffffffu, v.v.lo, src)});
-}
 __device__ __forceinline__ bool vfinite(float v) { return isfinite(v); }
 __device__ __forceinline__ bool vfinite(double v) { return isfinite(v); }
 __device__ __forceinline__ bool vfinite(dfx v) { return isfinite(v.v.hi) && isfinite(v.v.lo); }
 
-// ---------------------------------------------------------------------------
-// Panel kernel (roles, schedule and outputs as described at the top):
-//   * every thread owns one row of the 16-column slice (b <= 256 rows, 256
-//     threads); the 16 dot products of a reflector step are reduced with a
-//     warp reduce-scatter (16 shuffles) and one double-buffered shared-memory
-//     pass across warps: one barrier per reflector;
-//   * the masked reflector block Y is written once per block (row-major, so the
-//     apply reads a row of it as 16 consecutive values);
-//   * the apply to the rest of the tile is Z = Y^T C (thread j owns column j; C
-//     streams through shared memory in row chunks, cp.async ring issued at the
-//     start of the block), W = T^T Z (+ top rows), C -= Y W (threads own rows,
-//     W broadcast from shared memory).
-
+// 16-byte vectors: VN values of T from / to shared or global memory.
 template <typename T>
-__device__ __forceinline__ void ld4(const T *p, T (&v)[4]) {
-    if (sizeof(T) == 4) {
+struct PVec;
+template <>
+struct PVec<float> {
+    static constexpr int VN = 4;
+    static __device__ __forceinline__ void ld(const float *p, float *v) {
+        const float4 x = *reinterpret_cast<const float4 *>(p);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    }
+    static __device__ __forceinline__ void ldcg(const float *p, float *v) {
         const float4 x = __ldcg(reinterpret_cast<const float4 *>(p));
         v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-    } else {
+    }
+    static __device__ __forceinline__ void st(float *p, const float *v) {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+};
+template <>
+struct PVec<double> {
+    static constexpr int VN = 2;
+    static __device__ __forceinline__ void ld(const double *p, double *v) {
+        const double2 x = *reinterpret_cast<const double2 *>(p);
+        v[0] = x.x; v[1] = x.y;
+    }
+    static __device__ __forceinline__ void ldcg(const double *p, double *v) {
         const double2 x = __ldcg(reinterpret_cast<const double2 *>(p));
-        const double2 y = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
-        v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+        v[0] = x.x; v[1] = x.y;
+    }
+    static __device__ __forceinline__ void st(double *p, const double *v) {
+        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    }
+};
+template <>
+struct PVec<dfx> {
+    static constexpr int VN = 2;
+    static __device__ __forceinline__ void ld(const dfx *p, dfx *v) {
+        const float4 x = *reinterpret_cast<const float4 *>(p);
+        v[0] = dfx(df64{x.x, x.y}); v[1] = dfx(df64{x.z, x.w});
+    }
+    static __device__ __forceinline__ void st(dfx *p, const dfx *v) {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0].v.hi, v[0].v.lo, v[1].v.hi, v[1].v.lo);
+    }
+};
+// two sums of squares at a 16-byte aligned address
+template <typename Sq>
+struct PSq2;
+template <>
+struct PSq2<float2> {
+    static __device__ __forceinline__ void ld(const float2 *p, float2 &a, float2 &b) {
+        const float4 x = *reinterpret_cast<const float4 *>(p);
+        a = make_float2(x.x, x.y);
+        b = make_float2(x.z, x.w);
+    }
+};
+template <>
+struct PSq2<double> {
+    static __device__ __forceinline__ void ld(const double *p, double &a, double &b) {
+        const double2 x = *reinterpret_cast<const double2 *>(p);
+        a = x.x;
+        b = x.y;
+    }
+};
+// 16 consecutive values of CT at a 16-byte aligned address in shared memory.
+template <typename CT>
+__device__ __forceinline__ void ld16(const CT *p, CT (&v)[kIB]) {
+#pragma unroll
+    for (int q = 0; q < kIB; q += PVec<CT>::VN) PVec<CT>::ld(p + q, v + q);
+}
+template <typename CT>
+__device__ __forceinline__ void st16(CT *p, const CT (&v)[kIB]) {
+#pragma unroll
+    for (int q = 0; q < kIB; q += PVec<CT>::VN) PVec<CT>::st(p + q, v + q);
+}
+// RPL rows of one column of the view (LAYOUT 0: contiguous, 16-byte aligned).
+template <typename T, int LAYOUT, typename CT, int RPL>
+__device__ __forceinline__ void load_col(const View<T, LAYOUT> &V, int64_t r, int64_t c, CT (&v)[RPL]) {
+    if (LAYOUT == 0) {
+#pragma unroll
+        for (int q = 0; q < RPL; q += PVec<T>::VN) {
+            T w[PVec<T>::VN];
+            PVec<T>::ldcg(&V(r + q, c), w);
+#pragma unroll
+            for (int e = 0; e < PVec<T>::VN; ++e) v[q + e] = CT(w[e]);
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < RPL; ++q) v[q] = CT(__ldcg(&V(r + q, c)));
+    }
+}
+template <typename T, int LAYOUT, typename CT, int RPL>
+__device__ __forceinline__ void store_col(const View<T, LAYOUT> &V, int64_t r, int64_t c, const CT (&v)[RPL]) {
+    if (LAYOUT == 0) {
+#pragma unroll
+        for (int q = 0; q < RPL; q += PVec<T>::VN) {
+            T w[PVec<T>::VN];
+#pragma unroll
+            for (int e = 0; e < PVec<T>::VN; ++e) w[e] = (T)v[q + e];
+            PVec<T>::st(&V(r + q, c), w);
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < RPL; ++q) V(r + q, c) = (T)v[q];
     }
 }
 
-// Rows of the trailing tile staged per chunk in the apply's first product
-// (two chunks in flight), and the padded leading dimension of a chunk.
-template <typename T>
-__host__ __device__ constexpr int chunk_rows() { return sizeof(T) == 8 ? 16 : 32; }
-template <typename T, int LAYOUT>
-__host__ __device__ inline int chunk_ld(int b) { return LAYOUT == 0 ? chunk_rows<T>() + 4 : b + 4; }
-// chunks in flight: the first ones are issued when a block starts, so their
-// loads overlap the block's reflectors
-template <typename T>
-__host__ __device__ constexpr int chunk_bufs() { return sizeof(T) == 8 ? 2 : 4; }
-template <typename T>
-__host__ __device__ inline size_t chunk_elems(int b) {
-    // the larger of the two layouts: [b][CR + 4] or [CR][b + 4]
-    const size_t a0 = (size_t)b * (chunk_rows<T>() + 4), a1 = (size_t)chunk_rows<T>() * (b + 4);
-    return a0 > a1 ? a0 : a1;
+__device__ __forceinline__ void bar_named(int id, int cnt) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(cnt) : "memory");
 }
 
-template <typename T>
-size_t panel3_smem_bytes(int b) {
-    return sizeof(T) * (32 /* tau, scalars */ + (size_t)ldpad(b) * kIB /* X */ + (size_t)b * kIB /* Yr */ +
-                        (size_t)kIB * b /* Rt */ + (size_t)kIB * b /* Ws */ + 2 * kIB * kIB /* Tm, G */ +
-                        16 * kIB /* part */ + 8 + 2 * kIB /* spart, dsum, rvs */ + 4 /* align */ +
-                        chunk_bufs<T>() * chunk_elems<T>(b) /* C chunks */) +
-           sizeof(double) * 16;
-}
+// ---------------------------------------------------------------------------
+// Panel kernel (roles, schedule and outputs as described at the top).
+//
+// What bounds it: latency.  The critical path is (P - 1) reflector loops of 16
+// steps with a hand-off each, plus b/16 whole blocks (reflectors, Gram matrix,
+// apply), all on one SM per role.  So:
+//   * the block's 16 columns live in registers, a lane owning one column's rows
+//     of its half of the warp's 32 rows: a step's dot products and updates are in
+//     the lane (one shuffle joins the halves), against the reflector's column
+//     broadcast through shared memory; the norm is one butterfly of compensated
+//     pairs beside them.  (With a row per lane the 16 dot products took a warp
+//     reduce-scatter of 423 cycles a step.)  Across warps one shared-memory pass
+//     and one barrier of the b / 32 reflector warps, none for tiles 16 and 32;
+//   * a TSQRT step changes one row of the diagonal block only, so that block is
+//     read once per block and each new row goes straight to global memory;
+//   * the block reflector is applied from the Gram matrix, not from T: with
+//     G = Y^T Y and T^-1 = diag(1/tau) + striu(G), W = T^T Z is the forward
+//     substitution w_l = tau_l (z_l - sum_{m<l} G_ml w_m), one thread per
+//     column; 16 unit right-hand sides beside them give T (an output, for the
+//     trailing update);
+//   * the trailing columns of the tile stay in shared memory for the role's
+//     whole life: all of them for tiles up to 128, the last 128 of an FP32 tile of
+//     256 (its first ones, and those of an 8-byte tile of 256, are read from L2);
+//     the next block's 16 columns go from the apply to the next block in
+//     registers;
+//   * Z = Y^T C is split over column pairs and row ranges so that all warps
+//     work whatever the columns left; C -= Y W runs two rows per thread.
+// Measured (GB300; stage 1 of one call, before: runtime tile size, columns in
+// shared memory, a row per lane, explicit T): FP32 n = 1296 tile 16 195 -> 75 ms,
+// n = 1024 tile 64 20.4 -> 14.1, n = 4096 tile 128 91.8 -> 63.8, split BF16 n =
+// 5760 tile 128 96.8 -> 49.8, n = 16384 tile 256 344 -> 276; FP64 n = 1024 tile 64
+// 78.0 -> 43.0, double-float n = 2048 tile 128 103 -> 66.  A block of 16
+// reflectors: 9.5 k cycles (tile 16), 14.5 k (64), 17 k (128), 21 k (256), before
+// about 48 k.
+template <typename CT, int B>
+struct PanelCfg {
+    static constexpr int NB = B / kIB;
+    static constexpr int NWR = B >= 32 ? B / 32 : 1;  // reflector warps
+    static constexpr int RPL = (B >= 32 ? 32 : B) / 2;  // rows per lane
+    static constexpr int NT = B >= 128 ? 256 : (B == 64 ? 128 : (B == 32 ? 64 : 32));
+    static constexpr int NW = NT / 32;
+    static constexpr bool F4 = sizeof(CT) == 4;
+    static constexpr int YLD = F4 ? 20 : 18;      // row stride of Y and W (16-byte rows, conflict-free vectors)
+    static constexpr int CLD = B + (F4 ? 4 : 2);  // resident trailing columns: [column][row]
+    static constexpr int RESC = B <= 128 ? B - kIB : (F4 ? 128 : 0);  // resident columns, the last of the tile
+    static constexpr int S0 = B - RESC;           // first resident column
+    static constexpr int KSMAX = F4 ? 8 : 4;
+    static constexpr int NR = B > kIB ? B - kIB : kIB;  // trailing columns at most
+    static constexpr bool STREAM = NB > 1 && RESC < NR;
+    // split of Z = Y^T C over nw warps: wcol warps of 64 columns, ks row ranges
+    __host__ __device__ static constexpr int wcol(int nc) { return (nc + 63) / 64; }
+    __host__ __device__ static constexpr int ks(int nc, int nw) {
+        const int k = nc > 0 ? nw / wcol(nc) : 1;
+        const int k2 = k >= 8 ? 8 : (k >= 4 ? 4 : (k >= 2 ? 2 : 1));
+        return k2 < KSMAX ? k2 : KSMAX;
+    }
+    // streamed columns of the nrest trailing ones, and the warps of each part
+    __host__ __device__ static constexpr int nstream(int nrest) {
+        return nrest > RESC ? nrest - RESC : 0;
+    }
+    __host__ __device__ static constexpr int warps_r(int nrest) { return nstream(nrest) > 0 ? (RESC > 0 ? NW / 2 : 0) : NW; }
+    __host__ __device__ static constexpr int zsize(int nrest) {  // columns x row ranges of the partial Z
+        const int ns = nstream(nrest), nr = nrest - ns, wr = warps_r(nrest);
+        return (nr > 0 ? nr * ks(nr, wr) : 0) + (ns > 0 ? ns * ks(ns, NW - wr) : 0);
+    }
+    static constexpr int zcols() {
+        int m = 0;
+        for (int r = kIB; r <= NR; r += kIB) m = zsize(r) > m ? zsize(r) : m;
+        return m;
+    }
+    static constexpr size_t smem_bytes() {  // in the order of the kernel's carving
+        return 16 * NWR + sizeof(CT) * (2 * NWR * kIB + 2 * NWR * 32 + 2 * kIB + kIB + kIB * (kIB + 4) + kIB * kIB +
+                                       (F4 ? NW * kIB * kIB : 0) + (size_t)B * YLD +
+                                       (NB > 1 ? (size_t)NR * YLD + (size_t)kIB * zcols() + (size_t)RESC * CLD : 0));
+    }
+};
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
-                 "l"(gmem)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-template <typename T, int LAYOUT, typename CT = T>
-__global__ void __launch_bounds__(kNT) panel3_kernel(PanelArgs args) {
+template <typename T, int LAYOUT, typename CT, int B>
+__global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs args) {
+    using Cfg = PanelCfg<CT, B>;
+    using Ar = PAr<CT>;
+    using Sq = typename Ar::Sq;
+    using Mac = typename Ar::Mac;
+    constexpr int NB = Cfg::NB, NWR = Cfg::NWR, NT = Cfg::NT, NW = Cfg::NW, YLD = Cfg::YLD, CLD = Cfg::CLD;
+    constexpr int RPL = Cfg::RPL, RESC = Cfg::RESC, S0 = Cfg::S0;
+    constexpr int TV = PVec<T>::VN, CV = PVec<CT>::VN;
+    static_assert(sizeof(Sq) == 8 && sizeof(CT) == sizeof(T), "panel types");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int b = args.b;
-    const int nb = b / kIB;
-    const int ldx = ldpad(b);
-    using Acc = typename PScal<CT>::Acc;
-    Acc *spart = reinterpret_cast<Acc *>(smem_raw);         // 8 warps
-    CT *stau = reinterpret_cast<CT *>(smem_raw + sizeof(double) * 16);
-    CT *scal = stau + kIB;                                   // 16
-    CT *X = scal + 16;                                       // ldx * kIB (column-major)
-    CT *Yr = X + (size_t)ldx * kIB;                          // b * kIB (row-major: Yr[t*16 + l])
-    CT *Rt = Yr + (size_t)b * kIB;                           // kIB * b, Rt[l + j*kIB]
-    CT *Ws = Rt + (size_t)kIB * b;                           // kIB * b, Ws[l + j*kIB]
-    CT *Tm = Ws + (size_t)kIB * b;                           // kIB * kIB, Tm[l + i*kIB]
-    CT *G = Tm + kIB * kIB;                                  // kIB * kIB
-    CT *part = G + kIB * kIB;                                // 2 x 8 * kIB (double-buffered)
-    CT *dsum = part + 16 * kIB;                              // end of the small arrays
-    // C chunks (16-byte aligned): LAYOUT 0 [column][row], LAYOUT 1 [row][column]
-    T *cbuf0 = reinterpret_cast<T *>((reinterpret_cast<uintptr_t>(dsum + 2 * kIB + 8) + 15) & ~(uintptr_t)15);
+    Sq *spart = reinterpret_cast<Sq *>(smem_raw);                 // [2][NWR]
+    CT *part = reinterpret_cast<CT *>(spart + 2 * NWR);           // [2][16][NWR]
+    CT *xs = part + 2 * NWR * kIB;                                // [2][NWR][32] the step's column
+    CT *rowb = xs + 2 * NWR * 32;                                 // [2][16]
+    CT *stau = rowb + 2 * kIB;                                    // [16]
+    CT *Rts = stau + kIB;                                         // [16][20], Rts[l * 20 + j]
+    CT *G = Rts + kIB * (kIB + 4);                                // [16][16], G[l * 16 + m] = y_l^T y_m
+    CT *Gp = G + kIB * kIB;                                       // FP32: [NW][16][16]
+    CT *Yr = Gp + (Cfg::F4 ? NW * kIB * kIB : 0);                 // [B][YLD]
+    CT *Ws = Yr + (size_t)B * YLD;                                // [columns][YLD]
+    CT *Zp = Ws + (NB > 1 ? (size_t)Cfg::NR * YLD : 0);           // [row range][16][columns], both parts
+    CT *Cs = Zp + (NB > 1 ? (size_t)kIB * Cfg::zcols() : 0);      // [column - S0][CLD]
 
-    __shared__ int s_role, s_ok;
+    __shared__ int s_role, s_ok, s_fail;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int64_t zb = blockIdx.y;
-    int *ticket = args.ticket + zb * args.sFlags;
     int *progress = args.progress + zb * args.sFlags;
-    if (tid == 0) s_role = atomicAdd(ticket, 1) + args.first_role;
+    if (tid == 0) {
+        s_role = atomicAdd(args.ticket + zb * args.sFlags, 1) + args.first_role;
+        s_fail = 0;
+    }
     __syncthreads();
     const int p = s_role;
     if (p >= args.P) return;
 
     View<T, LAYOUT> V{reinterpret_cast<T *>(args.a) + zb * args.sA, args.lda};
-    const int64_t row0 = (int64_t)(args.pr + p) * b;
-    const int64_t top0 = (int64_t)args.pr * b;
-    const int64_t col0 = (int64_t)args.pc * b;
+    const int64_t row0 = (int64_t)(args.pr + p) * B;
+    const int64_t top0 = (int64_t)args.pr * B;
+    const int64_t col0 = (int64_t)args.pc * B;
     const bool geqrt = (p == 0);
-    T *tau_out = reinterpret_cast<T *>(args.tau) + zb * args.sTau + (size_t)p * b;
-    T *tblk_out = reinterpret_cast<T *>(args.tblk) + zb * args.sTblk + (size_t)p * nb * kIB * kIB;
-    const int t = tid;  // my row (b <= 256)
+    const bool follow = !geqrt && p > args.first_role;  // another role runs ahead
+    T *tau_out = reinterpret_cast<T *>(args.tau) + zb * args.sTau + (size_t)p * B;
+    T *tblk_out = reinterpret_cast<T *>(args.tblk) + zb * args.sTblk + (size_t)p * NB * kIB * kIB;
 
     if (args.ready) {  // the tile is still being written by the previous update's chain
         if (tid == 0) s_ok = wait_geq(args.ready + p, args.ready_need, args.err);
@@ -363,379 +501,535 @@ __global__ void __launch_bounds__(kNT) panel3_kernel(PanelArgs args) {
         if (!s_ok) return;
     }
     int *full = progress + args.P;  // per role: block cb's trailing top rows are final
-    for (int cb = 0; cb < nb; ++cb) {
+
+    // my column of the block and my rows of it (reflector warps)
+    const bool refl = wid < NWR;
+    const int jc = lane & (kIB - 1), half = lane >> 4;
+    const int rb = wid * 32 + half * RPL;
+    CT col[RPL];
+    if (refl) load_col<T, LAYOUT, CT, RPL>(V, row0 + rb, col0 + jc, col);
+    if constexpr (RESC > 0 && NB > 1) {  // the trailing columns, kept until the role is done
+        constexpr int U = 16;
+        constexpr int NC = RESC, TOT = NC * B;
+        for (int base = tid; base < TOT; base += NT * U) {
+            T v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int idx = base + u * NT;
+                const int tt = LAYOUT == 0 ? idx % B : idx / NC;
+                const int j = LAYOUT == 0 ? idx / B : idx % NC;
+                v[u] = idx < TOT ? __ldcg(&V(row0 + tt, col0 + S0 + j)) : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int idx = base + u * NT;
+                const int tt = LAYOUT == 0 ? idx % B : idx / NC;
+                const int j = LAYOUT == 0 ? idx / B : idx % NC;
+                if (idx < TOT) Cs[(size_t)j * CLD + tt] = CT(v[u]);
+            }
+        }
+    }
+
+    for (int cb = 0; cb < NB; ++cb) {
         const int c0 = cb * kIB;
-        // ---- the role's own tile (no other role writes it): the block's 16
-        // columns and the first chunks of its trailing columns load while the
-        // role waits for the previous one
-        for (int idx = tid; idx < b * kIB; idx += kNT) {
-            int tt, l;
-            if (LAYOUT == 0) { tt = idx % b; l = idx / b; } else { l = idx % kIB; tt = idx / kIB; }
-            X[tt + l * ldx] = CT(__ldcg(&V(row0 + tt, col0 + c0 + l)));
-        }
         const int jbase = c0 + kIB;
-        const int nrest = b - jbase;
-        const int tstart = geqrt ? c0 : 0;  // rows above c0 have Y = 0 for GEQRT
-        constexpr int CR = chunk_rows<T>();
-        constexpr int NBUF = chunk_bufs<T>();
-        const int cld = chunk_ld<T, LAYOUT>(b);
-        const int nch = nrest > 0 ? (b - tstart + CR - 1) / CR : 0;
-        auto issue = [&](int ch) {  // one cp.async group per chunk (empty past the last)
-            if (ch < nch) {
-                constexpr int VEC = 16 / (int)sizeof(T);  // elements per 16-byte copy
-                T *buf = cbuf0 + (size_t)(ch % NBUF) * chunk_elems<T>(b);
-                const int t0 = tstart + ch * CR;
-                const int rows = min(CR, b - t0);
-                if (LAYOUT == 0) {  // column j: rows t0.. contiguous
-                    const int per = rows / VEC;
-                    for (int idx = tid; idx < nrest * per; idx += kNT) {
-                        const int j = idx / per, r = (idx % per) * VEC;
-                        cp_async16(buf + j * cld + r, &V(row0 + t0 + r, col0 + jbase + j));
-                    }
-                } else {  // row t: columns contiguous
-                    const int per = nrest / VEC;
-                    for (int idx = tid; idx < rows * per; idx += kNT) {
-                        const int r = idx / per, j = (idx % per) * VEC;
-                        cp_async16(buf + r * cld + j, &V(row0 + t0 + r, col0 + jbase + j));
-                    }
-                }
-            }
-            cp_async_commit();
-        };
-        if (nrest > 0) {
-#pragma unroll
-            for (int q = 0; q < NBUF; ++q) issue(q);
-        }
-        // ---- the diagonal 16 x 16 block of the top rows, once the previous
-        // role's reflectors of this block are in it (TSQRT)
-        if (tid == 0) {
-            bool ok = true;
-            if (p > args.first_role) ok = wait_geq(progress + p - 1, cb + 1, args.err);
-            s_ok = ok;
-        }
-        __syncthreads();
-        if (!s_ok) {
-            cp_async_wait<0>();
-            return;
-        }
-        if (!geqrt) {
-            for (int idx = tid; idx < kIB * kIB; idx += kNT) {
-                int l, j;
-                if (LAYOUT == 0) { l = idx % kIB; j = idx / kIB; } else { j = idx % kIB; l = idx / kIB; }
-                Rt[l + (c0 + j) * kIB] = CT(__ldcg(&V(top0 + c0 + l, col0 + c0 + j)));
-            }
-        }
-        __syncthreads();
+        const int nrest = B - jbase;
+        const int ns = Cfg::nstream(nrest), nr = nrest - ns;  // columns jbase.. streamed, the last nr resident
+        const int wr = Cfg::warps_r(nrest);
+        const int KR = Cfg::ks(nr, wr), KST = Cfg::ks(ns, NW - wr);
+        CT *ZpS = Zp + (size_t)kIB * KR * nr;  // the streamed part's partial Z
 
-        // ---- the 16 reflectors of the block, one per step, all threads.  One
-        // barrier per reflector: the warp partial sums are double-buffered, and
-        // every warp forms the (identical) scalars and column sums itself.
-        // Every warp reads the pivot row (alpha and the row the reflector
-        // updates) after the step's barrier, so warp 0 keeps the updated pivot
-        // row in registers and stores it after the next barrier: no later step
-        // reads that row before the Gram matrix below.
-        CT *pend_at = nullptr;
-        CT pend_v = CT(0);
-        for (int i = 0; i < kIB; ++i) {
-            const int c = c0 + i;
-            const int pb = i & 1;
-            if (geqrt && c == b - 1) {
-                if (tid == 0) stau[i] = CT(0);
-                continue;
-            }
-            const bool live = (t < b) && (geqrt ? (t > c) : true);
-            const CT x = live ? X[t + i * ldx] : CT(0);
-            CT pv[kIB];
-#pragma unroll
-            for (int jj = 0; jj < kIB; ++jj) pv[jj] = (live && jj > i) ? x * X[t + jj * ldx] : CT(0);
-            Acc sq = PScal<CT>::zero();
-            if (live) sq = PScal<CT>::sq(x, sq);
-            // warp reduce-scatter of pv[0..15]: lane L ends with the warp sum of pv[L & 15]
-#pragma unroll
-            for (int h = 8; h >= 1; h >>= 1) {
-                const bool upper = (lane & h) != 0;
-#pragma unroll
-                for (int q = 0; q < h; ++q) {
-                    const CT send = upper ? pv[q] : pv[q + h];
-                    const CT keep = upper ? pv[q + h] : pv[q];
-                    pv[q] = keep + vshfl_xor(send, h);
+        if (refl) {
+            // ---- the diagonal 16 x 16 block of the top rows, once the previous
+            // role's reflectors of this block are in it (TSQRT)
+            if (!geqrt) {
+                if (follow) {
+                    if (lane == 0 && !wait_geq(progress + p - 1, cb + 1, args.err)) s_fail = 1;
+                    __syncwarp();
                 }
-            }
-            pv[0] += vshfl_xor(pv[0], 16);
+                {
+                    constexpr int RU = kIB * kIB / (NWR * 32);  // all loads in flight
+                    T v[RU];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sq = PScal<CT>::shfl_add(sq, o);
-            if (lane < kIB) part[pb * 8 * kIB + wid * kIB + lane] = pv[0];  // lane L holds index L & 15
-            if (lane == 0) spart[pb * 8 + wid] = sq;
-            __syncthreads();
-            if (pend_at) {  // the previous step's pivot row, read by every warp before this barrier
-                *pend_at = pend_v;
-                pend_at = nullptr;
-            }
-            const CT alpha = geqrt ? X[c + i * ldx] : Rt[i + c * kIB];
-            CT out[6];
-            if constexpr (!std::is_same<CT, double>::value) {
-                // FP32 tiles: every lane forms the (double-float) scalars -- no
-                // divergence, and the loads below overlap them.  The 8 warp
-                // partials are summed by a 3-level shuffle tree; df_add is
-                // commutative, so every lane of every warp gets the same sum.
-                Acc s_all = spart[pb * 8 + (lane & 7)];
-                s_all = PScal<CT>::shfl_add(s_all, 1);
-                s_all = PScal<CT>::shfl_add(s_all, 2);
-                s_all = PScal<CT>::shfl_add(s_all, 4);
-                PScal<CT>::compute(s_all, alpha, out);
-                if (!vfinite(out[5]) || !vfinite(out[0])) {
-                    if (tid == 0) atomicCAS(args.err, kDevOk, kDevNonfinite);
-                    out[5] = out[1] = out[2] = out[3] = CT(0);
-                    out[4] = alpha;
-                }
-            } else {
-                // FP64 tiles: lane 0 of each warp forms the scalars (FP64 is
-                // costly on every lane), the warp reads them with shuffles
-                if (lane == 0) {
-                    Acc s_all = PScal<CT>::zero();
+                    for (int u = 0; u < RU; ++u) {
+                        const int idx = tid + u * NWR * 32;
+                        const int l = LAYOUT == 0 ? idx % kIB : idx / kIB;
+                        const int j = LAYOUT == 0 ? idx / kIB : idx % kIB;
+                        v[u] = __ldcg(&V(top0 + c0 + l, col0 + c0 + j));
+                    }
 #pragma unroll
-                    for (int w = 0; w < kNT / 32; ++w) s_all = PScal<CT>::shfl_add_local(s_all, spart[pb * 8 + w]);
-                    PScal<CT>::compute(s_all, alpha, out);
-                    if (!vfinite(out[5]) || !vfinite(out[0])) {
-                        if (tid == 0) atomicCAS(args.err, kDevOk, kDevNonfinite);
-                        out[5] = out[1] = out[2] = out[3] = CT(0);
-                        out[4] = alpha;
+                    for (int u = 0; u < RU; ++u) {
+                        const int idx = tid + u * NWR * 32;
+                        const int l = LAYOUT == 0 ? idx % kIB : idx / kIB;
+                        const int j = LAYOUT == 0 ? idx / kIB : idx % kIB;
+                        Rts[l * (kIB + 4) + j] = CT(v[u]);
                     }
                 }
+                // a hardware barrier for one warp too: after the divergent wait it puts the
+                // warp back in step (with __syncwarp alone a block of a 16-wide tile took
+                // 65 us instead of 7)
+                bar_named(1, NWR * 32);
+            }
+            // ---- the 16 reflectors of the block, one per step: a loop, not unrolled
+            // (a step is some 200 instructions, and straight-line code that a single
+            // warp runs once per block is bound by instruction fetch).  GEQRT: rows at
+            // or above the pivot row do not take part (zeros in the broadcast column);
+            // the pivot row is row i % RPL of the lanes of its segment.
+            CT myinv = CT(0), mytau = CT(0);
+            bool bad = false;
+            auto put_x = [&](int i) {  // column i's live rows for every lane of the warp
+                if (jc == i) {
+                    CT *dst = xs + ((i & 1) * NWR + wid) * 32 + half * RPL;
+                    if (!geqrt) {
 #pragma unroll
-                for (int q = 0; q < 6; ++q) out[q] = vshfl(out[q], 0);
-            }
-            // column sums of the 16 dot products: lane L sums column L & 15
-            CT dmine = CT(0);
+                        for (int r = 0; r < RPL; r += CV) PVec<CT>::st(dst + r, col + r);
+                    } else {
 #pragma unroll
-            for (int w = 0; w < kNT / 32; ++w) dmine += part[pb * 8 * kIB + w * kIB + (lane & 15)];
-            CT rvr[kIB];
-#pragma unroll
-            for (int jj = 0; jj < kIB; ++jj) rvr[jj] = geqrt ? X[c + jj * ldx] : Rt[i + (c0 + jj) * kIB];
-            const CT tv = out[5];
-            if (tid == 0) stau[i] = tv;
-            if (tv == CT(0)) {
-                if (live) X[t + i * ldx] = CT(0);
-                continue;  // the next step reads only own rows until its barrier
-            }
-            const CT nu = out[0], tc = out[1], f = out[2], inv = out[3];
-            CT dsv[kIB];
-#pragma unroll
-            for (int jj = 0; jj < kIB; ++jj) dsv[jj] = vshfl(dmine, jj);
-            if (live) {
-#pragma unroll
-                for (int jj = 0; jj < kIB; ++jj)
-                    if (jj > i) X[t + jj * ldx] -= x * (f * (nu * rvr[jj] + dsv[jj]));
-                X[t + i * ldx] = x * inv;
-            }
-            if (tid < kIB && tid >= i) {
-                pend_v = (tid == i) ? out[4] : rvr[tid] - tc * (nu * rvr[tid] + dmine);
-                pend_at = geqrt ? &X[c + tid * ldx] : &Rt[i + (c0 + tid) * kIB];
-            }
-        }
-        __syncthreads();
-        if (pend_at) *pend_at = pend_v;
-        __syncthreads();
-        // the diagonal block of the top rows is final for this role: back to
-        // global memory and handed on -- a TSQRT role's successor needs only
-        // this block for its own reflectors
-        if (!geqrt) {
-            for (int idx = tid; idx < kIB * kIB; idx += kNT) {
-                int l, jx;
-                if (LAYOUT == 0) { l = idx % kIB; jx = idx / kIB; } else { jx = idx % kIB; l = idx / kIB; }
-                V(top0 + c0 + l, col0 + c0 + jx) = (T)Rt[l + (c0 + jx) * kIB];
-            }
-            __syncthreads();
-            if (tid == 0) {
-                __threadfence();
-                st_release(progress + p, cb + 1);
-            }
-        }
-
-        // ---- Gram matrix of the block's reflectors, CT (warp 0), masked Y
-        {
-            const int pi = tid >> 1, h = tid & 1;
-            int l = -1, i = 0;
-            if (pi < kIB * (kIB - 1) / 2) {
-                int acc = 0;
-                for (int ii = 1; ii < kIB; ++ii) {
-                    if (pi < acc + ii) { i = ii; l = pi - acc; break; }
-                    acc += ii;
+                        for (int r = 0; r < RPL; ++r) dst[r] = (rb + r > c0 + i) ? col[r] : CT(0);
+                    }
                 }
-            }
-            CT pt = CT(0);
-            if (l >= 0) {
-                const int half = (b + 1) / 2;
-                const int tlo = h * half, thi = min(b, tlo + half);
-                for (int tt = tlo; tt < thi; ++tt)
-                    if (geqrt ? (tt > c0 + i) : true) pt += X[tt + l * ldx] * X[tt + i * ldx];
-            }
-            pt += vshfl_xor(pt, 1);
-            if (l >= 0 && h == 0) G[l + i * kIB] = pt + (geqrt ? X[c0 + i + l * ldx] : CT(0));
-        }
-        if (tid < kIB * kIB) Tm[tid] = CT(0);
-        for (int idx = tid; idx < b * kIB; idx += kNT) {
-            const int tt = idx / kIB, l = idx % kIB;
-            CT y = X[tt + l * ldx];
-            if (geqrt) y = (tt == c0 + l) ? CT(1) : (tt > c0 + l ? y : CT(0));
-            Yr[tt * kIB + l] = y;
-        }
-        __syncthreads();
-        if (wid == 0) {
-            if (lane < kIB) Tm[lane + lane * kIB] = stau[lane];
+            };
+            put_x(0);
             __syncwarp();
-            for (int i = 1; i < kIB; ++i) {
-                if (lane < i) {
-                    CT acc = CT(0);
-                    for (int m = lane; m < i; ++m) acc += Tm[lane + m * kIB] * G[m + i * kIB];
-                    Tm[lane + i * kIB] = -stau[i] * acc;
+            const int nstep = (geqrt && cb == NB - 1) ? kIB - 1 : kIB;  // the last column has no reflector
+            T *ptop = &V(top0 + c0, col0 + c0 + jc);
+            const int64_t dtop = LAYOUT == 0 ? 1 : args.lda;
+            const bool out_top = !geqrt && tid < kIB;
+#pragma unroll 1
+            for (int i = 0; i < nstep; ++i) {
+                const int pb = i & 1;
+                const bool own = geqrt && rb == c0 + i - i % RPL;
+                const CT *xw = xs + (pb * NWR + wid) * 32;
+                CT xr[RPL];
+#pragma unroll
+                for (int r = 0; r < RPL; r += CV) PVec<CT>::ld(xw + half * RPL + r, xr + r);
+                Sq sq = Ar::sq(xw[lane & (2 * RPL - 1)]);
+                if (geqrt) {
+                    CT piv = col[0];
+#pragma unroll
+                    for (int r = 1; r < RPL; ++r) piv = (i % RPL == r) ? col[r] : piv;
+                    if (own) rowb[pb * kIB + jc] = piv;
                 }
+#pragma unroll
+                for (int o = RPL; o > 0; o >>= 1) sq = Ar::merge_xor(sq, o);
+                CT d;
+                {
+                    constexpr int NA = Cfg::F4 ? 4 : 2;
+                    Mac a[NA];
+#pragma unroll
+                    for (int u = 0; u < NA; ++u) a[u] = Ar::mac0();
+#pragma unroll
+                    for (int r = 0; r < RPL; ++r) Ar::mac(a[r % NA], xr[r], col[r]);
+#pragma unroll
+                    for (int h2 = NA / 2; h2 >= 1; h2 >>= 1)
+#pragma unroll
+                        for (int u = 0; u < h2; ++u) a[u] = Ar::mac_merge(a[u], a[u + h2]);
+                    d = Ar::fin(a[0]);
+                    d = d + vshfl_xor(d, 16);
+                }
+                if (NWR > 1) {
+                    if (lane < kIB) part[(pb * kIB + lane) * NWR + wid] = d;
+                    if (lane == 0) spart[pb * NWR + wid] = sq;
+                    bar_named(1, NWR * 32);
+                    Sq sw[NWR];
+                    CT dw[NWR];
+#pragma unroll
+                    for (int w = 0; w < NWR; w += 2) PSq2<Sq>::ld(spart + pb * NWR + w, sw[w], sw[w + 1]);
+                    if constexpr (NWR >= CV) {
+#pragma unroll
+                        for (int w = 0; w < NWR; w += CV) PVec<CT>::ld(part + (pb * kIB + jc) * NWR + w, dw + w);
+                    } else {
+#pragma unroll
+                        for (int w = 0; w < NWR; ++w) dw[w] = part[(pb * kIB + jc) * NWR + w];
+                    }
+#pragma unroll
+                    for (int h2 = NWR / 2; h2 >= 1; h2 >>= 1)
+#pragma unroll
+                        for (int w = 0; w < h2; ++w) {
+                            sw[w] = Ar::merge(sw[w], sw[w + h2]);
+                            dw[w] = dw[w] + dw[w + h2];
+                        }
+                    sq = sw[0];
+                    d = dw[0];
+                } else {
+                    __syncwarp();
+                }
+                const CT *prow = geqrt ? rowb + pb * kIB : Rts + i * (kIB + 4);
+                const CT rj = prow[jc];
+                const PRefl<CT> r = Ar::scalars(sq, prow[i]);
+                bad = bad || !vfinite(r.tau) || !vfinite(r.nu);
+                const CT h = r.nu * rj + d;
+                const CT w = jc > i ? r.f * h : CT(0);  // columns up to i are finished
+#pragma unroll
+                for (int q = 0; q < RPL; ++q) col[q] = col[q] - xr[q] * w;
+                const CT top = jc > i ? rj - r.tc * h : r.beta;  // the pivot row's new value
+                if (geqrt) {
+#pragma unroll
+                    for (int q = 0; q < RPL; ++q) col[q] = (own && jc >= i && i % RPL == q) ? top : col[q];
+                }
+                if (i < kIB - 1) put_x(i + 1);
+                if (out_top && jc >= i) ptop[i * dtop] = (T)top;
+                mytau = jc == i ? r.tau : mytau;
+                myinv = jc == i ? r.inv : myinv;
                 __syncwarp();
             }
+            if (bad && lane == 0) atomicCAS(args.err, kDevOk, kDevNonfinite);
+            if (tid < kIB) stau[tid] = mytau;
+            __syncwarp();
+            // the diagonal block of the top rows is final for this role: handed on -- a
+            // TSQRT role's successor needs only this block for its own reflectors
+            if (!geqrt && tid == 0) st_release(progress + p, cb + 1);
+            // ---- V (each column scaled by its 1 / nu) back to the tile, and the
+            // masked Y (unit lower for GEQRT)
+#pragma unroll
+            for (int r = 0; r < RPL; ++r)
+                if (!geqrt || rb + r > c0 + jc) col[r] = col[r] * myinv;
+            if (!geqrt || rb >= c0) store_col<T, LAYOUT, CT, RPL>(V, row0 + rb, col0 + c0 + jc, col);
+#pragma unroll
+            for (int r = 0; r < RPL; ++r) {
+                CT y = col[r];
+                if (geqrt) y = (rb + r == c0 + jc) ? CT(1) : (rb + r > c0 + jc ? y : CT(0));
+                Yr[(size_t)(rb + r) * YLD + jc] = y;
+            }
         }
-        for (int idx = tid; idx < b * kIB; idx += kNT) {
-            int tt, l;
-            if (LAYOUT == 0) { tt = idx % b; l = idx / b; } else { l = idx % kIB; tt = idx / kIB; }
-            if (!geqrt || tt >= c0) V(row0 + tt, col0 + c0 + l) = (T)X[tt + l * ldx];
-        }
-        if (tid < kIB) tau_out[c0 + tid] = (T)stau[tid];
         __syncthreads();
-        if (geqrt && tid == 0) {  // the block's rows of the top tile are written back above
-            __threadfence();
-            st_release(progress, cb + 1);
-        }
-        if (tid < kIB * kIB) tblk_out[(size_t)cb * kIB * kIB + tid] = (T)Tm[tid];
+        if (s_fail) return;
+        // the block's rows of the top tile are written back above (the release
+        // covers what the barrier ordered before it)
+        if (geqrt && tid == 0) st_release(progress, cb + 1);
+        if (tid < kIB) tau_out[c0 + tid] = (T)stau[tid];
 
-        // ---- apply to the rest of the tile
-        if (nrest > 0) {
-            // (a) Z = Y^CT C: the rows tstart..b-1 of C stream through shared
-            // memory in chunks of CR rows (cp.async ring of NBUF chunks, issued
-            // since the block started); thread j owns column j and all 16
-            // reflectors (Y rows broadcast).
-            {
-                CT z[kIB];
+        // ---- Gram matrix of the block's reflectors
+        if constexpr (Cfg::F4) {
+            // 4 x 4 blocks, two row halves per warp, a range of rows per warp
+            constexpr int RW = B / NW;
+            const int lb = (lane >> 2) & 3, ib = lane & 3;
+            CT g[4][4];
 #pragma unroll
-                for (int l = 0; l < kIB; ++l) z[l] = CT(0);
-                for (int ch = 0; ch < nch; ++ch) {
-                    cp_async_wait<NBUF - 1>();
-                    __syncthreads();
-                    const T *buf = cbuf0 + (size_t)(ch % NBUF) * chunk_elems<T>(b);
-                    const int t0 = tstart + ch * CR;
-                    const int rows = min(CR, b - t0);
-                    const int j = tid;
-                    if (j < nrest) {
-                        for (int r = 0; r < rows; ++r) {
-                            const CT cv = CT(LAYOUT == 0 ? buf[j * cld + r] : buf[r * cld + j]);
-                            const CT *yrow = Yr + (t0 + r) * kIB;
+            for (int u = 0; u < 4; ++u)
 #pragma unroll
-                            for (int l = 0; l < kIB; ++l) z[l] += yrow[l] * cv;
-                        }
-                    }
-                    __syncthreads();
-                    issue(ch + NBUF);
-                }
-                cp_async_wait<0>();
-                if (tid < nrest) {
+                for (int v = 0; v < 4; ++v) g[u][v] = CT(0);
+#pragma unroll 4
+            for (int r = half; r < RW; r += 2) {
+                const CT *yr = Yr + (size_t)(wid * RW + r) * YLD;
+                CT a[4], e[4];
+                PVec<CT>::ld(yr + 4 * lb, a);
+                PVec<CT>::ld(yr + 4 * ib, e);
 #pragma unroll
-                    for (int l = 0; l < kIB; ++l) Ws[l + tid * kIB] = z[l];
-                }
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) g[u][v] += a[u] * e[v];
             }
-            __syncthreads();
-            // the trailing top rows, once the previous role's (b) is in them
-            if (!geqrt) {
-                if (tid == 0) s_ok = (p > args.first_role) ? wait_geq(full + p - 1, cb + 1, args.err) : true;
-                __syncthreads();
-                if (!s_ok) return;
-                for (int idx = tid; idx < kIB * nrest; idx += kNT) {
-                    int l, j;
-                    if (LAYOUT == 0) { l = idx % kIB; j = idx / kIB; } else { j = idx % nrest; l = idx / nrest; }
-                    Rt[l + (jbase + j) * kIB] = CT(__ldcg(&V(top0 + c0 + l, col0 + jbase + j)));
-                }
-                __syncthreads();
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+#pragma unroll
+                for (int v = 0; v < 4; ++v) g[u][v] += vshfl_xor(g[u][v], 16);
+                if (half == 0) PVec<CT>::st(Gp + wid * kIB * kIB + (4 * lb + u) * kIB + 4 * ib, g[u]);
             }
-            // (b) W = CT^CT (Z + top rows); top rows -= W
-            for (int jr = tid; jr < nrest; jr += kNT) {
-                CT zc[kIB];
-#pragma unroll
-                for (int l = 0; l < kIB; ++l) {
-                    zc[l] = Ws[l + jr * kIB];
-                    if (!geqrt) zc[l] += Rt[l + (jbase + jr) * kIB];
+        } else {
+            // one pair l < m per thread (two threads per pair from 256 threads on)
+            constexpr int HS = NT >= 256 ? 2 : 1;
+            constexpr int NP = kIB * (kIB - 1) / 2;
+            for (int idx = tid; idx < (NP * HS + 31) / 32 * 32; idx += NT) {
+                const int pi = idx / HS, h = idx % HS;
+                int l = 0, m = 0;
+                if (pi < NP) {
+                    m = 1;
+                    while (m * (m + 1) / 2 <= pi) ++m;
+                    l = pi - m * (m - 1) / 2;
                 }
-#pragma unroll
-                for (int l = 0; l < kIB; ++l) {
-                    CT acc = CT(0);
-#pragma unroll
-                    for (int m = 0; m <= l; ++m) acc += Tm[m + l * kIB] * zc[m];
-                    Ws[l + jr * kIB] = acc;
-                    if (!geqrt) Rt[l + (jbase + jr) * kIB] -= acc;
+                Mac acc = Ar::mac0();
+                if (pi < NP) {
+                    constexpr int RH = B / HS;
+                    const CT *yr = Yr + (size_t)h * RH * YLD;
+#pragma unroll 4
+                    for (int r = 0; r < RH; ++r) Ar::mac(acc, yr[r * YLD + l], yr[r * YLD + m]);
                 }
+                CT v = Ar::fin(acc);
+                if (HS == 2) v = v + vshfl_xor(v, 1);
+                if (pi < NP && h == 0) G[l * kIB + m] = v;
             }
-            __syncthreads();
-            // The trailing top rows are final for this block: a TSQRT role
-            // hands them to the next role now, before updating its own tile (c).
-            if (!geqrt) {
-                for (int idx = tid; idx < kIB * nrest; idx += kNT) {
-                    int l, jx;
-                    if (LAYOUT == 0) { l = idx % kIB; jx = idx / kIB; } else { jx = idx % nrest; l = idx / nrest; }
-                    V(top0 + c0 + l, col0 + jbase + jx) = (T)Rt[l + (jbase + jx) * kIB];
-                }
-                __syncthreads();
-                if (tid == 0) {
-                    __threadfence();
-                    st_release(full + p, cb + 1);
-                }
-            }
-            // (c) C -= Y W: thread owns row t; 16 columns per group, the next
-            // group's loads issued before the current group's arithmetic
-            if (t >= tstart && t < b) {
-                CT yv[kIB];
+        }
+
+        // ---- Z = Y^T C over the trailing columns of the tile: thread = columns
+        // jA, jA + 32 of its warp's 64, rows of its range
+        if constexpr (NB > 1) {
+            if (nrest > 0) {
+                const bool res = wid < wr;
+                const int nc = res ? nr : ns, K = res ? KR : KST, w0 = res ? wid : wid - wr;
+                const int wcol = Cfg::wcol(nc);
+                const int wc = wcol > 0 ? w0 % wcol : 0, kseg = wcol > 0 ? w0 / wcol : 0;
+                const int jA = wc * 64 + lane, jB = jA + 32;
+                const bool onA = kseg < K && jA < nc, onB = kseg < K && jB < nc;
+                const int RK = B / K;
+                CT *zp = (res ? Zp : ZpS) + (size_t)kseg * kIB * nc;
+                Mac z0[kIB], z1[kIB];
 #pragma unroll
-                for (int l = 0; l < kIB; ++l) yv[l] = Yr[t * kIB + l];
-                CT cur[16], nxt[16];
-                auto load16 = [&](int jr, CT (&v)[16]) {
-                    if (LAYOUT == 0) {
+                for (int l = 0; l < kIB; ++l) z0[l] = z1[l] = Ar::mac0();
+                auto row_mac = [&](int r, CT va, CT vb) {
+                    CT y[kIB];
+                    ld16<CT>(Yr + (size_t)r * YLD, y);
 #pragma unroll
-                        for (int q = 0; q < 16; ++q) v[q] = CT(__ldcg(&V(row0 + t, col0 + jbase + jr + q)));
-                    } else {
-#pragma unroll
-                        for (int q4 = 0; q4 < 4; ++q4) {
-                            T w4[4];
-                            ld4(&V(row0 + t, col0 + jbase + jr + 4 * q4), w4);
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) v[4 * q4 + q] = CT(w4[q]);
-                        }
+                    for (int l = 0; l < kIB; ++l) {
+                        Ar::mac(z0[l], y[l], va);
+                        Ar::mac(z1[l], y[l], vb);
                     }
                 };
-                load16(0, cur);
-                for (int jr = 0; jr < nrest; jr += 16) {
-                    if (jr + 16 < nrest) load16(jr + 16, nxt);
+                if (onA) {
+                    if (RESC > 0 && res) {
+                        const CT *pA = Cs + (size_t)(B - nr - S0 + jA) * CLD;
+                        const CT *pB = onB ? pA + (size_t)32 * CLD : pA;
+#pragma unroll 1
+                        for (int r = kseg * RK; r < (kseg + 1) * RK; r += CV) {
+                            CT cA[CV], cB[CV];
+                            PVec<CT>::ld(pA + r, cA);
+                            PVec<CT>::ld(pB + r, cB);
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        CT s2 = CT(0);
+                            for (int u = 0; u < CV; ++u) row_mac(r + u, cA[u], cB[u]);
+                        }
+                    } else if (Cfg::STREAM) {
+                        // streamed columns: from L2, the next SU rows in flight
+                        constexpr int SU = Cfg::F4 ? 8 : 4;
+                        const int64_t cA0 = col0 + jbase + jA, cB0 = onB ? cA0 + 32 : cA0;
+                        T bA[SU], bB[SU], nA[SU], nB[SU];
+                        auto fetch = [&](int r, T (&a)[SU], T (&b)[SU]) {
+                            if (LAYOUT == 0) {
 #pragma unroll
-                        for (int l = 0; l < kIB; ++l) s2 += yv[l] * Ws[l + (jr + q) * kIB];
-                        cur[q] -= s2;
+                                for (int u = 0; u < SU; u += TV) {
+                                    PVec<T>::ldcg(&V(row0 + r + u, cA0), a + u);
+                                    PVec<T>::ldcg(&V(row0 + r + u, cB0), b + u);
+                                }
+                            } else {
+#pragma unroll
+                                for (int u = 0; u < SU; ++u) {
+                                    a[u] = __ldcg(&V(row0 + r + u, cA0));
+                                    b[u] = __ldcg(&V(row0 + r + u, cB0));
+                                }
+                            }
+                        };
+                        const int rend = (kseg + 1) * RK;
+                        fetch(kseg * RK, bA, bB);
+#pragma unroll 1
+                        for (int r = kseg * RK; r < rend; r += SU) {
+                            if (r + SU < rend) fetch(r + SU, nA, nB);
+#pragma unroll
+                            for (int u = 0; u < SU; ++u) row_mac(r + u, CT(bA[u]), CT(bB[u]));
+#pragma unroll
+                            for (int u = 0; u < SU; ++u) {
+                                bA[u] = nA[u];
+                                bB[u] = nB[u];
+                            }
+                        }
                     }
-                    if (LAYOUT == 0) {
+                }
 #pragma unroll
-                        for (int q = 0; q < 16; ++q) V(row0 + t, col0 + jbase + jr + q) = (T)cur[q];
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 16; ++q) V(row0 + t, col0 + jbase + jr + q) = (T)cur[q];
-                    }
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) cur[q] = nxt[q];
+                for (int l = 0; l < kIB; ++l) {
+                    if (onA) zp[(size_t)l * nc + jA] = Ar::fin(z0[l]);
+                    if (onB) zp[(size_t)l * nc + jB] = Ar::fin(z1[l]);
                 }
             }
-        } else if (!geqrt) {
-            // no columns right of the block (the diagonal block went back above)
-            if (tid == 0) st_release(full + p, cb + 1);
+        }
+        CT nx[RPL];  // the next block's columns, loaded ahead of their update
+        if constexpr (NB > 1) {
+            if (nrest > 0 && refl) {
+                if (Cfg::STREAM && ns > 0) {
+                    load_col<T, LAYOUT, CT, RPL>(V, row0 + rb, col0 + jbase + jc, nx);
+                } else if (RESC > 0) {
+#pragma unroll
+                    for (int r = 0; r < RPL; r += CV)
+                        PVec<CT>::ld(Cs + (size_t)(jbase - S0 + jc) * CLD + rb + r, nx + r);
+                }
+            }
         }
         __syncthreads();
-        if (geqrt && tid == 0) {
-            __threadfence();
-            st_release(full, cb + 1);
+        if constexpr (Cfg::F4) {
+            for (int idx = tid; idx < kIB * kIB; idx += NT) {
+                CT v = Gp[idx];
+#pragma unroll
+                for (int w = 1; w < NW; ++w) v += Gp[w * kIB * kIB + idx];
+                G[idx] = v;
+            }
         }
+        // the trailing top rows, once the previous role's are in them
+        if (tid == 0) s_ok = (follow && nrest > 0) ? wait_geq(full + p - 1, cb + 1, args.err) : true;
+        __syncthreads();
+        if (!s_ok) return;
+
+        // ---- W = T^T (Z + top rows) by forward substitution; top rows -= W.  The 16
+        // unit right-hand sides after the columns give the rows of T.
+        for (int j = tid; j < nrest + kIB; j += NT) {
+            CT z[kIB], top[kIB];
+            Mac zz[kIB];
+            const bool unit = j >= nrest;
+            if (unit) {
+#pragma unroll
+                for (int l = 0; l < kIB; ++l) zz[l] = Ar::mac_from(CT(j - nrest == l ? 1 : 0));
+            } else {
+                if (!geqrt) load_col<T, LAYOUT, CT, kIB>(V, top0 + c0, col0 + jbase + j, top);
+                const bool str = j < ns;
+                const CT *zp = str ? ZpS + j : Zp + (j - ns);
+                const int nc = str ? ns : nr, K = str ? KST : KR;
+#pragma unroll
+                for (int l = 0; l < kIB; ++l) z[l] = zp[(size_t)l * nc];
+                for (int k = 1; k < K; ++k) {
+#pragma unroll
+                    for (int l = 0; l < kIB; ++l) z[l] = z[l] + zp[(size_t)(k * kIB + l) * nc];
+                }
+                if (!geqrt) {
+#pragma unroll
+                    for (int l = 0; l < kIB; ++l) z[l] = z[l] + top[l];
+                }
+#pragma unroll
+                for (int l = 0; l < kIB; ++l) zz[l] = Ar::mac_from(z[l]);
+            }
+#pragma unroll
+            for (int l = 0; l < kIB; ++l) {
+                z[l] = stau[l] * Ar::fin(zz[l]);
+                const CT nz = -z[l];
+#pragma unroll
+                for (int m = l + 1; m < kIB; ++m) Ar::mac(zz[m], G[l * kIB + m], nz);
+            }
+            if (unit) {
+#pragma unroll
+                for (int k = 0; k < kIB; ++k) tblk_out[(size_t)cb * kIB * kIB + (j - nrest) + k * kIB] = (T)z[k];
+            } else if constexpr (NB > 1) {
+                st16<CT>(Ws + (size_t)j * YLD, z);
+                if (!geqrt) {
+#pragma unroll
+                    for (int l = 0; l < kIB; ++l) top[l] = top[l] - z[l];
+                    store_col<T, LAYOUT, CT, kIB>(V, top0 + c0, col0 + jbase + j, top);
+                }
+            }
+        }
+        __syncthreads();
+        if constexpr (NB > 1) {
+            // a TSQRT role hands the trailing top rows on before updating its own tile
+            if (!geqrt && tid == 0) st_release(full + p, cb + 1);
+            if (nrest > 0) {
+                // ---- C -= Y W: the next block's 16 columns first, into registers
+                if (refl) {
+                    if constexpr (!std::is_same<CT, dfx>::value) {
+                        CT w[kIB];
+                        ld16<CT>(Ws + (size_t)jc * YLD, w);
+#pragma unroll
+                        for (int r = 0; r < RPL; ++r) {
+                            CT y[kIB];
+                            ld16<CT>(Yr + (size_t)(rb + r) * YLD, y);
+                            Mac acc = Ar::mac0();
+#pragma unroll
+                            for (int l = 0; l < kIB; ++l) Ar::mac(acc, y[l], w[l]);
+                            col[r] = nx[r] - Ar::fin(acc);
+                        }
+                    } else {  // reflectors in a loop: unrolled, its code is bound by instruction fetch
+                        Mac acc[RPL];
+#pragma unroll
+                        for (int r = 0; r < RPL; ++r) acc[r] = Ar::mac0();
+#pragma unroll 1
+                        for (int l = 0; l < kIB; ++l) {
+                            const CT wl = Ws[(size_t)jc * YLD + l];
+#pragma unroll
+                            for (int r = 0; r < RPL; ++r) Ar::mac(acc[r], Yr[(size_t)(rb + r) * YLD + l], wl);
+                        }
+#pragma unroll
+                        for (int r = 0; r < RPL; ++r) col[r] = nx[r] - Ar::fin(acc[r]);
+                    }
+                    // GEQRT: rows c0 .. c0+15 of these columns are final
+                    if (geqrt && rb == c0) store_col<T, LAYOUT, CT, RPL>(V, row0 + rb, col0 + jbase + jc, col);
+                }
+                // ---- the other columns, two rows per thread
+                if (nrest > kIB) {
+                    constexpr int RS = B >= 64 ? B / 2 : B;
+                    constexpr int CG = NT / RS > 0 ? NT / RS : 1;
+                    const int slot = tid % RS, grp = tid / RS;
+                    CT ya[kIB], yb[kIB];
+                    ld16<CT>(Yr + (size_t)slot * YLD, ya);
+                    ld16<CT>(Yr + (size_t)(slot + B / 2) * YLD, yb);
+                    auto apply = [&](int j, CT &a, CT &b) {
+                        CT w[kIB];
+                        ld16<CT>(Ws + (size_t)j * YLD, w);
+                        Mac a0 = Ar::mac0(), a1 = Ar::mac0();
+#pragma unroll
+                        for (int l = 0; l < kIB; ++l) {
+                            Ar::mac(a0, ya[l], w[l]);
+                            Ar::mac(a1, yb[l], w[l]);
+                        }
+                        a = a - Ar::fin(a0);
+                        b = b - Ar::fin(a1);
+                    };
+                    // GEQRT: only rows from c0 on belong to this role
+                    const bool wa = !geqrt || slot >= c0, wb = !geqrt || slot + B / 2 >= c0;
+                    if (Cfg::STREAM && ns > kIB) {  // streamed columns, NQ per turn, the next ones in flight
+                        constexpr int NQ = 4;
+                        T ga[NQ], gb[NQ], ha[NQ], hb[NQ];
+                        auto fetch = [&](int j, T (&a)[NQ], T (&b)[NQ]) {
+                            const int64_t c = col0 + jbase + j;
+                            if (LAYOUT == 0) {
+#pragma unroll
+                                for (int e = 0; e < NQ; ++e) {
+                                    a[e] = __ldcg(&V(row0 + slot, c + e));
+                                    b[e] = __ldcg(&V(row0 + slot + B / 2, c + e));
+                                }
+                            } else {
+#pragma unroll
+                                for (int e = 0; e < NQ; e += TV) {
+                                    PVec<T>::ldcg(&V(row0 + slot, c + e), a + e);
+                                    PVec<T>::ldcg(&V(row0 + slot + B / 2, c + e), b + e);
+                                }
+                            }
+                        };
+                        const int jbeg = kIB + grp * NQ;  // 16 columns at least, a multiple of 16
+                        if (jbeg < ns) fetch(jbeg, ga, gb);
+#pragma unroll 1
+                        for (int j = jbeg; j < ns; j += CG * NQ) {
+                            if (j + CG * NQ < ns) fetch(j + CG * NQ, ha, hb);
+#pragma unroll
+                            for (int e = 0; e < NQ; ++e) {
+                                CT a = CT(ga[e]), b = CT(gb[e]);
+                                apply(j + e, a, b);
+                                ga[e] = (T)a;
+                                gb[e] = (T)b;
+                            }
+                            const int64_t c = col0 + jbase + j;
+                            if (LAYOUT == 0) {
+#pragma unroll
+                                for (int e = 0; e < NQ; ++e) {
+                                    if (wa) V(row0 + slot, c + e) = ga[e];
+                                    if (wb) V(row0 + slot + B / 2, c + e) = gb[e];
+                                }
+                            } else {
+#pragma unroll
+                                for (int e = 0; e < NQ; e += TV) {
+                                    if (wa) PVec<T>::st(&V(row0 + slot, c + e), ga + e);
+                                    if (wb) PVec<T>::st(&V(row0 + slot + B / 2, c + e), gb + e);
+                                }
+                            }
+#pragma unroll
+                            for (int e = 0; e < NQ; ++e) {
+                                ga[e] = ha[e];
+                                gb[e] = hb[e];
+                            }
+                        }
+                    }
+                    if constexpr (RESC > 0) {
+                        // GEQRT: rows c0 .. c0+15 of the columns are final and go out
+                        const bool oa = geqrt && slot >= c0 && slot < jbase;
+                        const bool ob = geqrt && slot + B / 2 >= c0 && slot + B / 2 < jbase;
+#pragma unroll 2
+                        for (int j = (ns > kIB ? ns : kIB) + grp; j < nrest; j += CG) {
+                            CT *pc = Cs + (size_t)(jbase - S0 + j) * CLD + slot;
+                            CT a = pc[0], b = pc[B / 2];
+                            apply(j, a, b);
+                            pc[0] = a;
+                            pc[B / 2] = b;
+                            if (oa) V(row0 + slot, col0 + jbase + j) = (T)a;
+                            if (ob) V(row0 + slot + B / 2, col0 + jbase + j) = (T)b;
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        if (geqrt && tid == 0) st_release(full, cb + 1);
     }
 }
 
@@ -856,6 +1150,34 @@ __global__ void __launch_bounds__(kNT) update_kernel(UpdateArgs args) {
     store_strip(Top, top0);
 }
 
+// One panel kernel per tile size.
+template <typename T, int LAYOUT, typename CT, int B>
+int launch_panel_b(const PanelArgs &a, dim3 grid, cudaStream_t s) {
+    using Cfg = PanelCfg<CT, B>;
+    static std::atomic<bool> attr_set{false};
+    constexpr size_t smem = Cfg::smem_bytes();
+    static_assert(smem <= 227 * 1024, "panel shared memory");
+    if (!attr_set) {
+        AVS_CUDA_TRY(cudaFuncSetAttribute(panel_kernel<T, LAYOUT, CT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+        attr_set = true;
+    }
+    panel_kernel<T, LAYOUT, CT, B><<<grid, Cfg::NT, smem, s>>>(a);
+    AVS_CUDA_TRY(cudaGetLastError());
+    return AVS_SUCCESS;
+}
+template <typename T, int LAYOUT, typename CT>
+int launch_panel_ct(const PanelArgs &a, dim3 grid, cudaStream_t s) {
+    switch (a.b) {
+        case 16: return launch_panel_b<T, LAYOUT, CT, 16>(a, grid, s);
+        case 32: return launch_panel_b<T, LAYOUT, CT, 32>(a, grid, s);
+        case 64: return launch_panel_b<T, LAYOUT, CT, 64>(a, grid, s);
+        case 128: return launch_panel_b<T, LAYOUT, CT, 128>(a, grid, s);
+        case 256: return launch_panel_b<T, LAYOUT, CT, 256>(a, grid, s);
+        default: return AVS_ERR_UNSUPPORTED;
+    }
+}
+
 // FP64 tiles with the double-float trailing updates (AVS_PREC_FP64X2) run
 // the panel in double-float arithmetic too (CT = dfx: FP64 storage, each value
 // converted on load and rounded back on store); GB300 issues FP64 at 1/64 of
@@ -863,18 +1185,7 @@ __global__ void __launch_bounds__(kNT) update_kernel(UpdateArgs args) {
 template <typename T, int LAYOUT>
 int launch_panel(T *dA, int64_t lda, int b, int pr, int pc, int P, int first_role, const Stage1Work &w,
                  cudaStream_t s, const int *ready = nullptr) {
-    static std::atomic<bool> attr_set{false};
-    const size_t smem = panel3_smem_bytes<T>(b);
     const bool dfp = sizeof(T) == 8 && w.df_update;
-    if (!attr_set) {
-        AVS_CUDA_TRY(cudaFuncSetAttribute(panel3_kernel<T, LAYOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)panel3_smem_bytes<T>(256)));
-        if constexpr (sizeof(T) == 8)
-            AVS_CUDA_TRY(cudaFuncSetAttribute(panel3_kernel<T, LAYOUT, dfx>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)panel3_smem_bytes<T>(256)));
-        attr_set = true;
-    }
     const int batch = w.batch > 0 ? w.batch : 1;
     AVS_CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(int) * (size_t)(batch > 1 ? w.sFlags * batch : 2 * P + 1), s));
     PanelArgs a;
@@ -896,16 +1207,11 @@ int launch_panel(T *dA, int64_t lda, int b, int pr, int pc, int P, int first_rol
     a.sFlags = w.sFlags;
     a.ready = ready;
     a.ready_need = b / kChainStrip;
+    const dim3 grid(P - first_role, batch);
     if constexpr (sizeof(T) == 8) {
-        if (dfp) {
-            panel3_kernel<T, LAYOUT, dfx><<<dim3(P - first_role, batch), kNT, smem, s>>>(a);
-            AVS_CUDA_TRY(cudaGetLastError());
-            return AVS_SUCCESS;
-        }
+        if (dfp) return launch_panel_ct<T, LAYOUT, dfx>(a, grid, s);
     }
-    panel3_kernel<T, LAYOUT><<<dim3(P - first_role, batch), kNT, smem, s>>>(a);
-    AVS_CUDA_TRY(cudaGetLastError());
-    return AVS_SUCCESS;
+    return launch_panel_ct<T, LAYOUT, T>(a, grid, s);
 }
 
 template <typename T, int LAYOUT>
