@@ -294,8 +294,10 @@ int run_stages23(avs_handle *h, const Layout &L, int64_t n, int b, const S *W, i
     }
     AVS_CUDA_TRY(cudaEventRecord(h->ev[2], s));
     double *sig = reinterpret_cast<double *>(ws_at(h, L.off_sig));
-    if (fp64_stages)
-        rc = stage3_bisect(dd, de, n, rel_tol, sig, reinterpret_cast<double *>(ws_at(h, L.off_scr)), s, launches);
+    if (fp64_stages)  // the squares take the narrow band's place (stage 2 is done with it)
+        rc = stage3_bisect(dd, de, n, rel_tol, sig, reinterpret_cast<double *>(ws_at(h, L.off_scr)),
+                           reinterpret_cast<float2 *>(ws_at(h, L.off_pairs)),
+                           reinterpret_cast<double *>(ws_at(h, L.off_ab2)), s, launches);
     else
         rc = stage3_bisect_df(dd, de, n, rel_tol, sig, reinterpret_cast<double *>(ws_at(h, L.off_scr)),
                               reinterpret_cast<float2 *>(ws_at(h, L.off_pairs)), s, launches);
@@ -1101,7 +1103,9 @@ int avs_bidiag_svals_dev(avs_handle *h, int64_t n, const double *dd, const doubl
     if (n > 1) AVS_CUDA_TRY(cudaMemcpyAsync(te, de, sizeof(double) * (size_t)(n - 1), cudaMemcpyDeviceToDevice, s));
     int64_t launches = 0;
     AVS_CUDA_TRY(cudaEventRecord(h->ev[0], s));
-    rc = stage3_bisect(dd, te, n, rel_tol, dsigma, reinterpret_cast<double *>(ws_at(h, L.off_scr)), s, &launches);
+    rc = stage3_bisect(dd, te, n, rel_tol, dsigma, reinterpret_cast<double *>(ws_at(h, L.off_scr)),
+                       reinterpret_cast<float2 *>(ws_at(h, L.off_pairs)),
+                       reinterpret_cast<double *>(ws_at(h, L.off_ab2)), s, &launches);
     if (rc != AVS_SUCCESS) return rc;
     AVS_CUDA_TRY(cudaEventRecord(h->ev[1], s));
     AVS_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1291,7 +1295,9 @@ int group_launches(avs_handle *h, const BatchLayout &L, int64_t n, int b, int cn
     }
     double *sig = reinterpret_cast<double *>(base + L.sig);
     if (sizeof(T) == 8 && f64_stages)
-        rc = stage3_bisect_batched(dd, de, n, cnt, tol, sig, reinterpret_cast<double *>(base + L.scr), s, launches);
+        rc = stage3_bisect_batched(dd, de, n, cnt, tol, sig, reinterpret_cast<double *>(base + L.scr),
+                                   reinterpret_cast<float2 *>(base + L.pairs),
+                                   reinterpret_cast<double *>(base + L.ab2), s, launches);
     else
         rc = stage3_bisect_df_batched(dd, de, n, cnt, tol, sig, reinterpret_cast<double *>(base + L.scr),
                                       reinterpret_cast<float2 *>(base + L.pairs), s, launches);

@@ -291,13 +291,13 @@ int stage2_chase_fp64_batched(const double *dW, int64_t n, int bw, int batch, do
                               double *de, const Stage2Work &w, cudaStream_t s, int num_sms, int64_t *launches,
                               int tbw, bool window, double *dAB2);
 int stage3_bisect_batched(const double *dd, const double *de, int64_t n, int batch, double rel_tol, double *dsigma,
-                          double *dscratch, cudaStream_t s, int64_t *launches);
+                          double *dscratch, float2 *dpairs, double *dsq, cudaStream_t s, int64_t *launches);
 int bidiag_svals_noalloc(int64_t n, const double *dd, const double *de, double *dsigma, double rel_tol,
                          cudaStream_t s);
 int stage3_bisect_df(const double *dd, const double *de, int64_t n, double rel_tol, double *dsigma, double *dscratch,
                      float2 *dpairs, cudaStream_t s, int64_t *launches);
 int stage3_bisect(const double *dd, const double *de, int64_t n, double rel_tol, double *dsigma, double *dscratch,
-                  cudaStream_t s, int64_t *launches);
+                  float2 *dpairs, double *dsq, cudaStream_t s, int64_t *launches);
 
 template <typename T>
 int cast_from_double(const double *src, T *dst, int64_t n, cudaStream_t s);

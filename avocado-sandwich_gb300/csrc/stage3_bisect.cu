@@ -5,8 +5,16 @@
 // Replaces LAPACK.bdsdc!('U','N', d, e) (KAbasedSVD/src/bulgechasing.jl:50-53,
 // CUDAbasedSVD/SVD_GPU.jl:267,281), which the reference runs on the CPU.
 // Method: Sturm counts from the LDL^T pivots of TGK - x I with the pivot guard
-// of LAPACK dstebz (Kahan's bisection); one thread per singular value, every
-// loop bounded.  Output is descending, like bdsdc.
+// of LAPACK dstebz (Kahan's bisection), every loop bounded.  Output is
+// descending, like bdsdc.
+//
+// B is scaled by a power of two so that every singular value lies in [0, 1), and
+// a value is found as the cell of a dyadic grid that contains it: FP32 counts
+// first, double-float counts on the cell and its neighbours, and for FP64 results
+// FP64 counts on that cell and its neighbours, each on a group of G lanes that
+// splits the bracket at G K points a pass.  A bracket whose edges a finer
+// arithmetic does not confirm is dropped and that arithmetic starts again from
+// [0, 1).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -17,7 +25,8 @@
 namespace avs {
 namespace {
 
-// scratch[0] = Gershgorin bound of TGK, scratch[1] = pivmin (one block).
+// scratch[0] = Gershgorin bound of TGK, scratch[1] = pivmin, scratch[2] = exponent k
+// of the scaling by 2^-k (one block).
 __device__ void tgk_bound_body(const double *d, const double *e, int64_t n, double *scratch) {
     __shared__ double sb[32], sm[32];
     double bound = 0.0, maxsq = 0.0;
@@ -45,6 +54,8 @@ __device__ void tgk_bound_body(const double *d, const double *e, int64_t n, doub
         }
         scratch[0] = b2;
         scratch[1] = DBL_MIN * fmax(m2, 1.0);
+        // exponent of the scale: b2 2^-k < 1, with room for the bound's rounding
+        scratch[2] = (b2 > 0.0 && b2 <= DBL_MAX) ? (double)(ilogb(b2 * (1.0 + 1e-6)) + 1) : 0.0;
     }
 }
 
@@ -112,8 +123,10 @@ __device__ __forceinline__ int tgk_count_f32(const double *__restrict__ d, const
     return cnt;
 }
 
-// The k-th largest singular value of the upper bidiagonal (d, e) of order n,
-// from the bound and pivot guard in scratch[0..1].
+// The k-th largest singular value of the upper bidiagonal (d, e) of order n by one
+// thread, from the bound and pivot guard in scratch[0..1]: the allocation-free
+// call's form, which has no room for the squared off-diagonals the multisection
+// below reads.
 __device__ double bisect_value(const double *d, const double *e, int64_t n, int64_t k, double rel_tol,
                                const double *scratch) {
     const double bound = scratch[0];
@@ -152,175 +165,294 @@ __device__ double bisect_value(const double *d, const double *e, int64_t n, int6
     return 0.5 * (lo + hi);
 }
 
-__global__ void bisect_kernel(const double *d, const double *e, int64_t n, double rel_tol, const double *scratch,
-                              double *sigma) {
+__global__ void bisect_thread_kernel(const double *d, const double *e, int64_t n, double rel_tol,
+                                     const double *scratch, double *sigma) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n) return;
     sigma[k] = bisect_value(d, e, n, k, rel_tol, scratch);
 }
 
-// ---- double-float bisection (the pipeline's stage 3 for FP32-class modes) ----
-// B is scaled by 1/bound so every quantity stays inside FP32's exponent range;
-// the squared TGK off-diagonals a_i = (off_i / bound)^2 are formed once in FP64
-// and stored as df64 pairs.  A count costs ~60 FP32 instructions per pivot
-// instead of an FP64 division; relative errors of ~1e-14 per pivot keep the
-// count exact for a matrix within ~1e-14 of TGK(B) (the backward-stability
-// argument of the FP64 recurrence).
-__global__ void tgk_prep_df_kernel(const double *d, const double *e, int64_t n, const double *scratch, float2 *a) {
-    const double inv = scratch[0] > 0.0 ? 1.0 / scratch[0] : 0.0;
+// ---- multisection on the scaled problem (every pipeline call) -----------------
+// The squared scaled off-diagonals a_i = (off_i 2^-k)^2: as double-float pairs,
+// and in FP64 for FP64 results (sq, may be null).
+__device__ __forceinline__ void tgk_prep_one(double off, int k, int64_t i, float2 *a, double *sq) {
+    const double o = scalbn(off, -k);
+    const double v = o * o;
+    const float h = (float)v;
+    a[i] = make_float2(h, (float)(v - (double)h));
+    if (sq) sq[i] = v;
+}
+__global__ void tgk_prep_kernel(const double *d, const double *e, int64_t n, const double *scratch, float2 *a,
+                                double *sq) {
+    const int k = (int)scratch[2];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 2 * n - 1;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const double off = ((i & 1) ? e[i >> 1] : d[i >> 1]) * inv;
-        const double sq = off * off;
-        const float h = (float)sq;
-        a[i] = make_float2(h, (float)(sq - (double)h));
-    }
+         i += (int64_t)gridDim.x * blockDim.x)
+        tgk_prep_one((i & 1) ? e[i >> 1] : d[i >> 1], k, i, a, sq);
 }
 
-// 1 / q in double-float: hardware reciprocal estimate of q.hi (relative error
-// ~2^-23) refined by one Newton-Raphson step r' = r + r (1 - q r) in df64.
-__device__ __forceinline__ df64 df_rcp_fast(df64 q) {
+__device__ __forceinline__ float rcp_ftz(float x) {
     float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q.hi));
-    const df64 e = df_sub(df64{1.0f, 0.0f}, df_mul_f(q, r));
-    return df_add(df64{r, 0.0f}, df_mul_f(e, r));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((127 + e) << 23); }  // |e| <= 126
+__device__ __forceinline__ double pow2d(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
-// Sturm counts of TGK at K shifts at once (one pass over a, K independent
-// recurrences interleaved for instruction-level parallelism).
+// Sturm counts at K shifts at once (one pass over a, K interleaved recurrences
+// q = -x - a / q).  The a_i are at most 1 and |q| is kept at 1e-36 or more, so no
+// quotient overflows.
 template <int K>
-__device__ __forceinline__ void tgk_count_df_k(const float2 *__restrict__ a, int64_t m, const df64 (&x)[K],
-                                               float pivmin, int (&cnt)[K]) {
-    df64 nx[K], q[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-        nx[j] = df_neg(x[j]);
-        q[j] = nx[j];
-        if (fabsf(q[j].hi) < pivmin) q[j] = df64{-pivmin, 0.0f};
-        cnt[j] = df_lt0(q[j]);
-    }
-    for (int64_t i = 0; i < m; ++i) {
-        const float2 ai = __ldg(a + i);
-        const df64 av{ai.x, ai.y};
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            q[j] = df_sub(nx[j], df_mul(av, df_rcp_fast(q[j])));
-            if (fabsf(q[j].hi) < pivmin) q[j] = df64{-pivmin, 0.0f};
-            cnt[j] += df_lt0(q[j]);
-        }
-    }
-}
-
-template <int K>
-__device__ __forceinline__ void tgk_count_f_k(const float2 *__restrict__ a, int64_t m, const float (&x)[K],
-                                              float pivmin, int (&cnt)[K]) {
+__device__ __forceinline__ void tgk_count_f(const float2 *__restrict__ a, int m, const float (&x)[K], int (&cnt)[K]) {
+    constexpr float pivmin = 1e-36f;
     float q[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-        q[j] = -x[j];
-        if (fabsf(q[j]) < pivmin) q[j] = -pivmin;
-        cnt[j] = (q[j] < 0.0f);
+        q[j] = x[j] < pivmin ? -pivmin : -x[j];
+        cnt[j] = 1;
     }
-    for (int64_t i = 0; i < m; ++i) {
+#pragma unroll 4
+    for (int i = 0; i < m; ++i) {
         const float ai = __ldg(a + i).x;
 #pragma unroll
         for (int j = 0; j < K; ++j) {
-            q[j] = -x[j] - __fdividef(ai, q[j]);
-            if (fabsf(q[j]) < pivmin || !isfinite(q[j])) q[j] = -pivmin;
-            cnt[j] += (q[j] < 0.0f);
+            q[j] = fmaf(-ai, rcp_ftz(q[j]), -x[j]);
+            if (fabsf(q[j]) < pivmin) q[j] = -pivmin;
+            cnt[j] += __float_as_uint(q[j]) >> 31;
         }
     }
 }
-
-// k-th largest singular value of the scaled problem (a = squared scaled
-// off-diagonals, bound = the scale), returned unscaled.  Multisection by a
-// group of G consecutive lanes: each lane counts at K = 3 shifts (one pass
-// over a, three interleaved recurrences), so a pass splits the bracket into
-// G*K + 1 parts; the group agrees on the first shift whose count exceeds the
-// target with G-lane shuffles.  FP32 passes first (to ~1e-6 of the scale),
-// then a double-float verified bracket and double-float passes to rel_tol.
-template <int G>
-__device__ double bisect_df_grp(const float2 *a, int64_t n, int64_t k, double rel_tol, double bound, int gl,
-                                unsigned gmask) {
-    if (bound == 0.0) return 0.0;
-    constexpr int K = 3, NSH = G * K, NI = NSH + 1;
-    const int64_t m = 2 * n - 1;
-    const float pivmin = 1e-36f;
-    const int64_t target = 2 * n - 1 - k;
-    auto group_first = [&](const int (&c)[K]) {
-        int first = NSH;
+// In double-float: the quotient is t = a r with r ~ 1/q plus its residual
+// (a - t q) r, about 20 instructions a pivot and 75 cycles of chain where a
+// reciprocal refined in double-float and a product take 60 and 200; its relative
+// error is below 2^-46 (r is refined once in FP32), so the counts are exact for a
+// matrix within about 1e-14 of TGK(B), as those of the FP64 recurrence are.
+template <int K>
+__device__ __forceinline__ void tgk_count_df(const float2 *__restrict__ a, int m, const df64 (&x)[K],
+                                             int (&cnt)[K]) {
+    constexpr float pivmin = 1e-36f;
+    df64 q[K];
 #pragma unroll
-        for (int j = K - 1; j >= 0; --j)
-            if (c[j] > target) first = gl * K + j;
-#pragma unroll
-        for (int o = G / 2; o >= 1; o >>= 1) first = min(first, __shfl_xor_sync(gmask, first, o));
-        return first;
-    };
-    // FP32 phase on the scaled problem (all values in [0, 1]); count(x) > target <=> x > sigma_k
-    float flo = 0.0f, fhi = 1.0f + 1e-6f;
-    for (int it = 0; it < 24 && fhi - flo > 1e-6f; ++it) {
-        const float w = (fhi - flo) * (1.0f / NI);
-        if (!(flo + w > flo) || !(fhi - w < fhi)) break;
-        float x[K];
-#pragma unroll
-        for (int j = 0; j < K; ++j) x[j] = flo + w * (float)(gl * K + j + 1);
-        int c[K];
-        tgk_count_f_k<K>(a, m, x, pivmin, c);
-        const int first = group_first(c);
-        const float nlo = flo + w * (float)first;
-        const float nhi = first == NSH ? fhi : flo + w * (float)(first + 1);
-        flo = nlo;
-        fhi = nhi;
+    for (int j = 0; j < K; ++j) {
+        q[j] = x[j].hi < pivmin ? df64{-pivmin, 0.0f} : df_neg(x[j]);
+        cnt[j] = 1;
     }
-    // verified bracket in double-float
-    df64 lo = df64{0.0f, 0.0f}, hi = df64{1.0f + 1e-6f, 0.0f};
-    {
-        const float w = fmaxf(fhi - flo, 4e-7f);
-        df64 t[2] = {df64{fmaxf(0.0f, flo - w), 0.0f}, df64{fminf(1.0f + 1e-6f, fhi + w), 0.0f}};
-        int c[2];
-        tgk_count_df_k<2>(a, m, t, pivmin, c);
-        if (c[0] <= target) lo = t[0];
-        if (c[1] > target) hi = t[1];
-    }
-    const float tol = (float)fmax(rel_tol, 1e-15);
-    for (int it = 0; it < 60; ++it) {
-        const df64 width = df_sub(hi, lo);
-        if (width.hi <= tol) break;
-        const df64 q = df64{width.hi * (1.0f / NI), width.lo * (1.0f / NI)};
-        df64 x[K];
+#pragma unroll 2
+    for (int i = 0; i < m; ++i) {
+        const float2 ai = __ldg(a + i);
 #pragma unroll
-        for (int j = 0; j < K; ++j) x[j] = df_add(lo, df_mul_f(q, (float)(gl * K + j + 1)));
-        int c[K];
-        tgk_count_df_k<K>(a, m, x, pivmin, c);
-        const int first = group_first(c);
-        const df64 nlo = first == 0 ? lo : df_add(lo, df_mul_f(q, (float)first));
-        const df64 nhi = first == NSH ? hi : df_add(lo, df_mul_f(q, (float)(first + 1)));
-        lo = nlo;
-        hi = nhi;
+        for (int j = 0; j < K; ++j) {
+            float r = rcp_ftz(q[j].hi);
+            r = fmaf(r, fmaf(-q[j].hi, r, 1.0f), r);
+            const float t = __fmul_rn(ai.x, r);
+            const float rem = __fadd_rn(__fmaf_rn(-t, q[j].lo, __fmaf_rn(-t, q[j].hi, ai.x)), ai.y);
+            const df64 s = two_sum(-x[j].hi, -t);
+            const float lo = __fsub_rn(s.lo, __fmaf_rn(rem, r, x[j].lo));
+            q[j] = fast_two_sum(s.hi, lo);
+            if (fabsf(q[j].hi) < pivmin) q[j] = df64{-pivmin, 0.0f};
+            cnt[j] += __float_as_uint(q[j].hi) >> 31;
+        }
     }
-    const df64 c = df_add(lo, hi);
-    return bound * 0.5 * df_to_double(c);
+}
+// In FP64: q = -x - a r (2 - q r) with r ~ 1/q from FP32 (one refinement, relative
+// error 2^-23, so 2^-46 after the step): three FP64 instructions a pivot.  GB300
+// issues an FP64 warp instruction in 64 cycles per scheduler, conversions
+// included, so q's FP32 image and r's FP64 one are made with integer operations.
+__device__ __forceinline__ double tgk_step_d(double a, double q, double x) {
+    const unsigned hi = (unsigned)__double2hiint(q), lo = (unsigned)__double2loint(q);
+    const unsigned ex = (hi >> 20) & 0x7ffu;
+    if (ex - (1023u - 115u) < 230u) {
+        const unsigned sgn = hi & 0x80000000u;
+        const unsigned mag = ((((hi & 0x7fffffffu) - (896u << 20)) << 3) | (lo >> 29)) + ((lo >> 28) & 1u);
+        const float qf = __uint_as_float(mag | sgn);
+        float r = rcp_ftz(qf);
+        r = fmaf(r, fmaf(-qf, r, 1.0f), r);
+        const unsigned rb = __float_as_uint(r);
+        const double rd =
+            __hiloint2double((int)((((rb & 0x7fffffffu) >> 3) + (896u << 20)) | sgn), (int)(rb << 29));
+        return fma(-(a * rd), fma(-q, rd, 2.0), -x);
+    }
+    return -x - a / q;
+}
+__device__ __forceinline__ int tgk_count_d(const double *__restrict__ sq, int m, double x) {
+    double q = x < DBL_MIN ? -DBL_MIN : -x;
+    int cnt = 1;
+#pragma unroll 2
+    for (int i = 0; i < m; ++i) {
+        q = tgk_step_d(__ldg(sq + i), q, x);
+        // |q| < DBL_MIN (no exponent): the pivot guard
+        if ((__double2hiint(q) & 0x7ff00000) == 0) q = -DBL_MIN;
+        cnt += (unsigned)__double2hiint(q) >> 31;
+    }
+    return cnt;
 }
 
-// Lanes per value, a function of the order alone: the single-matrix and the
-// batched calls of one order run the same multisection, so a matrix's values
-// are identical alone and in a batch (the final bracket depends on G).  A group
-// of G lanes does more counts per value (about 1.3, 2.3 and 3.2 times those of
-// one lane for G = 2, 4, 8) in fewer dependent passes; G = 2 measured fastest
-// at n = 16384 on GB300 (121 ms with G = 1, 98 ms with G = 2, 146 ms with
-// G = 4) and keeps the batched workloads, where values are plentiful, close
-// to the one-lane work.
-inline int bisect_group(int64_t n) { return n >= 65536 ? 1 : 2; }
+// A bracket [lo, lo + 2^c) in units of 2^-depth; top: its upper edge is confirmed.
+struct Bracket {
+    long long lo;
+    int depth, c;
+    bool top;
+};
 
-template <int G>
-__global__ void bisect_df_kernel(const float2 *a, int64_t n, double rel_tol, const double *scratch, double *sigma) {
+constexpr int kDepthF = 18;      // cells of the FP32 phase: its counts err by up to a few 1e-7
+constexpr int kDepthDfMax = 47;  // the double-float grid: shifts are exact pairs
+constexpr int kDepthDfD = 40;    // double-float cells before the FP64 phase
+
+// One group (G consecutive lanes) splits the bracket at G K points per pass until
+// its cell has the wanted depth.  exceed(v0, depth, ex): ex[j] = count at
+// (v0 + j) 2^-depth > target.  Returns false when the lower edge turns out to lie
+// above the value or the upper edge is never confirmed.
+template <int G, int K, typename F>
+__device__ __forceinline__ bool multisect(Bracket &b, int want, int gl, unsigned gmask, F exceed) {
+    constexpr int NI = G * K;
+    constexpr int P = NI >= 128 ? 7 : NI >= 64 ? 6 : NI >= 32 ? 5 : NI >= 16 ? 4 : NI >= 8 ? 3 : 2;
+    static_assert(NI == (1 << P), "parts");
+    while (b.depth < want || b.c > 0) {
+        const int p = min(P, want - b.depth + b.c);
+        const long long lo = b.lo << (p - b.c);
+        const int depth = b.depth + p - b.c;
+        bool ex[K];
+        exceed(lo + gl * K, depth, ex);
+        int first = NI;
+#pragma unroll
+        for (int j = K - 1; j >= 0; --j)
+            if (ex[j] && lo + gl * K + j > 0) first = gl * K + j;
+#pragma unroll
+        for (int o = G / 2; o >= 1; o >>= 1) first = min(first, __shfl_xor_sync(gmask, first, o));
+        if (first == 0) return false;
+        const int parts = 1 << p;
+        if (first <= parts && first < NI) b.top = true;
+        b.lo = lo + min(first, parts) - 1;
+        b.depth = depth;
+        b.c = 0;
+    }
+    return b.top;
+}
+// The cell and its neighbours: one cell below, two above.
+__device__ __forceinline__ Bracket widen(const Bracket &b) {
+    return Bracket{b.lo > 0 ? b.lo - 1 : 0, b.depth, 2, false};
+}
+
+// k-th largest singular value.  F64: FP64 result (sq given), else double-float.
+template <int G, bool F64>
+__device__ double bisect_grp(const float2 *a, const double *sq, int64_t n, int64_t k, double rel_tol,
+                             const double *scratch, int gl, unsigned gmask) {
+    const double bound = scratch[0];
+    if (!(bound > 0.0)) return bound;  // 0, or NaN
+    const int ke = (int)scratch[2];
+    const int m = (int)(2 * n - 1);
+    const int target = (int)(2 * n - 1 - k);  // TGK index (ascending) of the k-th largest sigma
+    // depth whose cells are at most rel_tol * bound wide
+    const double tol = fmin(fmax(rel_tol * scalbn(bound, -ke), 1e-17), 0.5);
+    int want = -ilogb(tol);
+    if (pow2d(-want) > tol) ++want;
+    want = max(want, kDepthF + 2);
+
+    Bracket b{0, 0, 0, true};
+    constexpr int K = 4;
+    multisect<G, K>(b, kDepthF, gl, gmask, [&](long long v0, int depth, bool(&ex)[K]) {
+        float x[K];
+        int c[K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) x[j] = (float)(int)(v0 + j) * pow2f(-depth);
+        tgk_count_f<K>(a, m, x, c);
+#pragma unroll
+        for (int j = 0; j < K; ++j) ex[j] = c[j] > target;
+    });
+    auto ex_df = [&](long long v0, int depth, bool(&ex)[K]) {
+        df64 x[K];
+        int c[K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {  // 24 + 23 bits, both exact
+            const long long v = v0 + j;
+            x[j] = fast_two_sum((float)(int)(v >> 24) * pow2f(24 - depth), (float)(int)(v & 0xffffff) * pow2f(-depth));
+        }
+        tgk_count_df<K>(a, m, x, c);
+#pragma unroll
+        for (int j = 0; j < K; ++j) ex[j] = c[j] > target;
+    };
+    const int wdf = F64 ? min(kDepthDfD, want) : min(want, kDepthDfMax);
+    b = widen(b);
+    if (!multisect<G, K>(b, wdf, gl, gmask, ex_df)) {
+        b = Bracket{0, 0, 0, true};
+        multisect<G, K>(b, wdf, gl, gmask, ex_df);
+    }
+    if constexpr (F64) {
+        const int wd = min(max(want, kDepthDfD + 2), 52);
+        auto ex_d = [&](long long v0, int depth, bool(&ex)[1]) {
+            ex[0] = tgk_count_d(sq, m, (double)v0 * pow2d(-depth)) > target;
+        };
+        b = widen(b);
+        if (!multisect<G, 1>(b, wd, gl, gmask, ex_d)) {
+            b = Bracket{0, 0, 0, true};
+            multisect<G, 1>(b, wd, gl, gmask, ex_d);
+        }
+    }
+    return scalbn(((double)b.lo + 0.5) * pow2d(-b.depth), ke);
+}
+
+// Lanes per value.  A pass costs one count's latency while every scheduler has
+// one warp or so, and its issue beyond; the shifts counted per resolved bit grow
+// with G (G K shifts for log2(G K) bits).  So: as many lanes as fill the GPU about
+// once.  Measured (GB300, double-float, tolerance 1e-10, ms): n = 128 G = 32 0.11,
+// 8 0.14, 2 0.19; n = 1024 G = 16 0.71, 8 0.91, 32 1.04; n = 4096 G = 4 4.4, 2 5.2,
+// 8 5.3; n = 5760 G = 2 7.3, 4 9.1; above n = 12288 the pivots no longer fit in L1
+// and a second warp hides their latency: n = 16384 G = 2 39, 1 42, 4 51.  FP64: n =
+// 512 G = 32 0.92, 16 1.09; n = 1024 G = 16 2.2, 32 2.6; n = 4096 G = 8 14.9, 16
+// 20.3.  Before (two lanes, double-float reciprocals; FP64: one thread per value):
+// n = 128 0.39, 1024 2.9, 4096 11.7, 16384 65 ms; FP64 n = 1024 31.8, 4096 127 ms.
+// The value found is the grid's cell whatever G is, as long as the counts at
+// neighbouring grid points are ordered, i.e. the cells are wider than the counts'
+// errors (about 2n 1e-14 at the very worst): so for tolerances of 5e-11 and more
+// and orders up to 2048 the batch may take part in the choice (256 matrices of order
+// 256: G = 1 1.4 ms, 2 1.5, 4 2.5) and a matrix still gets the values of its single
+// call bit for bit; otherwise G depends on the order alone.
+inline int bisect_lanes(int64_t n, int64_t batch, double rel_tol, bool f64) {
+    const int64_t nv = (!f64 && rel_tol >= 5e-11 && n <= 2048) ? n * batch : n;
+    const int least = f64 ? 8 : (n > 12288 ? 2 : 1);
+    int g = 32;
+    while (g > least && nv * g > (f64 ? 16384 : 20480)) g >>= 1;
+    return g;
+}
+
+template <int G, bool F64>
+__global__ void __launch_bounds__(128) bisect_kernel(const float2 *a, const double *sq, int64_t n, int64_t batch,
+                                                     int64_t sA, int64_t sScr, double rel_tol, const double *scratch,
+                                                     double *sigma) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t k = t / G;
+    const int64_t g = t / G;
+    if (g >= n * batch) return;  // whole groups: G divides the block size
     const int gl = (int)(t % G);
-    if (k >= n) return;  // whole groups: G divides the block size
-    const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
-    const double v = bisect_df_grp<G>(a, n, k, rel_tol, scratch[0], gl, gmask);
-    if (gl == 0) sigma[k] = v;
+    const int64_t zb = g / n, k = g % n;
+    const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
+    const double v = bisect_grp<G, F64>(a + zb * sA, F64 ? sq + zb * sA : nullptr, n, k, rel_tol, scratch + zb * sScr,
+                                        gl, gmask);
+    if (gl == 0) sigma[g] = v;
+}
+
+template <bool F64>
+int launch_bisect(const float2 *a, const double *sq, int64_t n, int64_t batch, int64_t sA, int64_t sScr,
+                  double rel_tol, const double *scratch, double *sigma, cudaStream_t s) {
+    const int G = bisect_lanes(n, batch, rel_tol, F64);
+    const unsigned blocks = (unsigned)((n * batch * G + 127) / 128);
+    switch (G) {
+        case 1:
+            if constexpr (!F64)
+                bisect_kernel<1, F64><<<blocks, 128, 0, s>>>(a, sq, n, batch, sA, sScr, rel_tol, scratch, sigma);
+            break;
+        case 2:
+            if constexpr (!F64)
+                bisect_kernel<2, F64><<<blocks, 128, 0, s>>>(a, sq, n, batch, sA, sScr, rel_tol, scratch, sigma);
+            break;
+        case 4:
+            if constexpr (!F64)
+                bisect_kernel<4, F64><<<blocks, 128, 0, s>>>(a, sq, n, batch, sA, sScr, rel_tol, scratch, sigma);
+            break;
+        case 8: bisect_kernel<8, F64><<<blocks, 128, 0, s>>>(a, sq, n, batch, sA, sScr, rel_tol, scratch, sigma); break;
+        case 16: bisect_kernel<16, F64><<<blocks, 128, 0, s>>>(a, sq, n, batch, sA, sScr, rel_tol, scratch, sigma); break;
+        default: bisect_kernel<32, F64><<<blocks, 128, 0, s>>>(a, sq, n, batch, sA, sScr, rel_tol, scratch, sigma); break;
+    }
+    AVS_CUDA_TRY(cudaGetLastError());
+    return AVS_SUCCESS;
 }
 
 template <typename T>
@@ -345,17 +477,29 @@ inline int bisect_threads(int64_t n) {
 
 }  // namespace
 
-int stage3_bisect(const double *dd, const double *de, int64_t n, double rel_tol, double *dsigma, double *dscratch,
-                  cudaStream_t s, int64_t *launches) {
+// FP64 results (dsq: 2n doubles) or double-float ones (dsq null); dpairs 2n pairs.
+static int bisect_single(const double *dd, const double *de, int64_t n, double rel_tol, double *dsigma,
+                         double *dscratch, float2 *dpairs, double *dsq, cudaStream_t s, int64_t *launches) {
     if (n <= 0) return AVS_SUCCESS;
-    if (!(rel_tol > 0.0)) rel_tol = 2.0 * DBL_EPSILON;
+    if (n > ((int64_t)1 << 29)) return AVS_ERR_UNSUPPORTED;  // pivots are counted in 32 bits
     tgk_bound_kernel<<<1, 1024, 0, s>>>(dd, de, n, dscratch);
     AVS_CUDA_TRY(cudaGetLastError());
-    const int threads = bisect_threads(n);
-    bisect_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, s>>>(dd, de, n, rel_tol, dscratch, dsigma);
+    const int pb = (int)std::min<int64_t>((2 * n + 255) / 256, 1024);
+    tgk_prep_kernel<<<pb, 256, 0, s>>>(dd, de, n, dscratch, dpairs, dsq);
     AVS_CUDA_TRY(cudaGetLastError());
-    if (launches) *launches += 2;
-    return AVS_SUCCESS;
+    if (launches) *launches += 3;
+    return dsq ? launch_bisect<true>(dpairs, dsq, n, 1, 0, 0, rel_tol, dscratch, dsigma, s)
+               : launch_bisect<false>(dpairs, nullptr, n, 1, 0, 0, rel_tol, dscratch, dsigma, s);
+}
+int stage3_bisect(const double *dd, const double *de, int64_t n, double rel_tol, double *dsigma, double *dscratch,
+                  float2 *dpairs, double *dsq, cudaStream_t s, int64_t *launches) {
+    if (!(rel_tol > 0.0)) rel_tol = 2.0 * DBL_EPSILON;
+    return bisect_single(dd, de, n, rel_tol, dsigma, dscratch, dpairs, dsq, s, launches);
+}
+int stage3_bisect_df(const double *dd, const double *de, int64_t n, double rel_tol, double *dsigma, double *dscratch,
+                     float2 *dpairs, cudaStream_t s, int64_t *launches) {
+    if (!(rel_tol > 0.0)) rel_tol = 1e-14;
+    return bisect_single(dd, de, n, rel_tol, dsigma, dscratch, dpairs, nullptr, s, launches);
 }
 
 // ---------------------------------------------------------------------------
@@ -422,34 +566,9 @@ int bidiag_svals_noalloc(int64_t n, const double *dd, const double *de, double *
     tgk_bound_kernel<<<1, 1024, 0, s>>>(dd, te, n, scr);
     AVS_CUDA_TRY(cudaGetLastError());
     const int threads = bisect_threads(n);
-    bisect_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, s>>>(dd, te, n, rel_tol, scr, dsigma);
+    bisect_thread_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, s>>>(dd, te, n, rel_tol, scr, dsigma);
     AVS_CUDA_TRY(cudaGetLastError());
     AVS_CUDA_TRY(cudaStreamSynchronize(s));
-    return AVS_SUCCESS;
-}
-
-int stage3_bisect_df(const double *dd, const double *de, int64_t n, double rel_tol, double *dsigma, double *dscratch,
-                     float2 *dpairs, cudaStream_t s, int64_t *launches) {
-    if (n <= 0) return AVS_SUCCESS;
-    if (!(rel_tol > 0.0)) rel_tol = 1e-14;
-    tgk_bound_kernel<<<1, 1024, 0, s>>>(dd, de, n, dscratch);
-    AVS_CUDA_TRY(cudaGetLastError());
-    const int pb = (int)std::min<int64_t>((2 * n + 255) / 256, 1024);
-    tgk_prep_df_kernel<<<pb, 256, 0, s>>>(dd, de, n, dscratch, dpairs);
-    AVS_CUDA_TRY(cudaGetLastError());
-    const int G = bisect_group(n);
-    const int64_t nt = n * G;
-    const unsigned blocks = (unsigned)((nt + 127) / 128);
-    if (G == 1)
-        bisect_df_kernel<1><<<blocks, 128, 0, s>>>(dpairs, n, rel_tol, dscratch, dsigma);
-    else if (G == 2)
-        bisect_df_kernel<2><<<blocks, 128, 0, s>>>(dpairs, n, rel_tol, dscratch, dsigma);
-    else if (G == 4)
-        bisect_df_kernel<4><<<blocks, 128, 0, s>>>(dpairs, n, rel_tol, dscratch, dsigma);
-    else
-        bisect_df_kernel<8><<<blocks, 128, 0, s>>>(dpairs, n, rel_tol, dscratch, dsigma);
-    AVS_CUDA_TRY(cudaGetLastError());
-    if (launches) *launches += 3;
     return AVS_SUCCESS;
 }
 
@@ -479,92 +598,48 @@ template int copy_convert_2d<double, float>(const double *, int64_t, float *, in
                                             cudaStream_t);
 
 // ---------------------------------------------------------------------------
-// Batched double-float bisection: `batch` bidiagonals of order n stacked at
-// stride n (d, e), singular values to dsigma (stride n).
+// Batched: `batch` bidiagonals of order n stacked at stride n (d, e), singular
+// values to dsigma (stride n); pairs and squares at stride 2n.
 namespace {
 __global__ void tgk_bound_batched(const double *d, const double *e, int64_t n, double *scratch) {
     const int64_t zb = blockIdx.x;
     tgk_bound_body(d + zb * n, e + zb * n, n, scratch + zb * 4);
 }
-__global__ void tgk_prep_df_batched(const double *d, const double *e, int64_t n, int batch, const double *scratch,
-                                    float2 *a) {
+__global__ void tgk_prep_batched(const double *d, const double *e, int64_t n, int batch, const double *scratch,
+                                 float2 *a, double *sq) {
     const int64_t m = 2 * n - 1;
     const int64_t total = m * (int64_t)batch;
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
         const int64_t zb = g / m, i = g % m;
-        const double bnd = scratch[zb * 4];
-        const double inv = bnd > 0.0 ? 1.0 / bnd : 0.0;
-        const double off = ((i & 1) ? e[zb * n + (i >> 1)] : d[zb * n + (i >> 1)]) * inv;
-        const double sq = off * off;
-        const float h = (float)sq;
-        a[zb * (2 * n) + i] = make_float2(h, (float)(sq - (double)h));
+        tgk_prep_one((i & 1) ? e[zb * n + (i >> 1)] : d[zb * n + (i >> 1)], (int)scratch[zb * 4 + 2], i,
+                     a + zb * 2 * n, sq ? sq + zb * 2 * n : nullptr);
     }
 }
-template <int G>
-__global__ void bisect_df_batched(const float2 *a, int64_t n, int batch, double rel_tol, const double *scratch,
-                                  double *sigma) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t g = t / G;
-    const int gl = (int)(t % G);
-    if (g >= n * (int64_t)batch) return;
-    const int64_t zb = g / n, k = g % n;
-    const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
-    const double v = bisect_df_grp<G>(a + zb * (2 * n), n, k, rel_tol, scratch[zb * 4], gl, gmask);
-    if (gl == 0) sigma[g] = v;
-}
 }  // namespace
 
-// Batched FP64 bisection: the single-matrix kernel's per-value code, one
-// thread per value of every matrix (values identical to stage3_bisect's).
-namespace {
-__global__ void bisect_batched(const double *d, const double *e, int64_t n, int batch, double rel_tol,
-                               const double *scratch, double *sigma) {
-    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (g >= n * (int64_t)batch) return;
-    const int64_t zb = g / n, k = g % n;
-    sigma[g] = bisect_value(d + zb * n, e + zb * n, n, k, rel_tol, scratch + zb * 4);
-}
-}  // namespace
-
-int stage3_bisect_batched(const double *dd, const double *de, int64_t n, int batch, double rel_tol, double *dsigma,
-                          double *dscratch, cudaStream_t s, int64_t *launches) {
+static int bisect_batch(const double *dd, const double *de, int64_t n, int batch, double rel_tol, double *dsigma,
+                        double *dscratch, float2 *dpairs, double *dsq, cudaStream_t s, int64_t *launches) {
     if (n <= 0 || batch <= 0) return AVS_SUCCESS;
-    if (!(rel_tol > 0.0)) rel_tol = 2.0 * DBL_EPSILON;
-    tgk_bound_batched<<<batch, 256, 0, s>>>(dd, de, n, dscratch);
-    AVS_CUDA_TRY(cudaGetLastError());
-    const int64_t nv = n * (int64_t)batch;
-    const int threads = bisect_threads(nv);
-    bisect_batched<<<(unsigned)((nv + threads - 1) / threads), threads, 0, s>>>(dd, de, n, batch, rel_tol, dscratch,
-                                                                               dsigma);
-    AVS_CUDA_TRY(cudaGetLastError());
-    if (launches) *launches += 2;
-    return AVS_SUCCESS;
-}
-
-int stage3_bisect_df_batched(const double *dd, const double *de, int64_t n, int batch, double rel_tol,
-                             double *dsigma, double *dscratch, float2 *dpairs, cudaStream_t s, int64_t *launches) {
-    if (n <= 0 || batch <= 0) return AVS_SUCCESS;
-    if (!(rel_tol > 0.0)) rel_tol = 4e-14;
+    if (n > ((int64_t)1 << 29)) return AVS_ERR_UNSUPPORTED;
     tgk_bound_batched<<<batch, 256, 0, s>>>(dd, de, n, dscratch);
     AVS_CUDA_TRY(cudaGetLastError());
     const int64_t total = (2 * n - 1) * (int64_t)batch;
-    tgk_prep_df_batched<<<(unsigned)std::min<int64_t>((total + 255) / 256, 8192), 256, 0, s>>>(dd, de, n, batch,
-                                                                                              dscratch, dpairs);
-    AVS_CUDA_TRY(cudaGetLastError());
-    const int64_t nv = n * (int64_t)batch;
-    const int G = bisect_group(n);
-    const unsigned blocks = (unsigned)((nv * G + 127) / 128);
-    if (G == 1)
-        bisect_df_batched<1><<<blocks, 128, 0, s>>>(dpairs, n, batch, rel_tol, dscratch, dsigma);
-    else if (G == 2)
-        bisect_df_batched<2><<<blocks, 128, 0, s>>>(dpairs, n, batch, rel_tol, dscratch, dsigma);
-    else if (G == 4)
-        bisect_df_batched<4><<<blocks, 128, 0, s>>>(dpairs, n, batch, rel_tol, dscratch, dsigma);
-    else
-        bisect_df_batched<8><<<blocks, 128, 0, s>>>(dpairs, n, batch, rel_tol, dscratch, dsigma);
+    tgk_prep_batched<<<(unsigned)std::min<int64_t>((total + 255) / 256, 8192), 256, 0, s>>>(dd, de, n, batch, dscratch,
+                                                                                           dpairs, dsq);
     AVS_CUDA_TRY(cudaGetLastError());
     if (launches) *launches += 3;
-    return AVS_SUCCESS;
+    return dsq ? launch_bisect<true>(dpairs, dsq, n, batch, 2 * n, 4, rel_tol, dscratch, dsigma, s)
+               : launch_bisect<false>(dpairs, nullptr, n, batch, 2 * n, 4, rel_tol, dscratch, dsigma, s);
+}
+int stage3_bisect_batched(const double *dd, const double *de, int64_t n, int batch, double rel_tol, double *dsigma,
+                          double *dscratch, float2 *dpairs, double *dsq, cudaStream_t s, int64_t *launches) {
+    if (!(rel_tol > 0.0)) rel_tol = 2.0 * DBL_EPSILON;
+    return bisect_batch(dd, de, n, batch, rel_tol, dsigma, dscratch, dpairs, dsq, s, launches);
+}
+int stage3_bisect_df_batched(const double *dd, const double *de, int64_t n, int batch, double rel_tol,
+                             double *dsigma, double *dscratch, float2 *dpairs, cudaStream_t s, int64_t *launches) {
+    if (!(rel_tol > 0.0)) rel_tol = 4e-14;
+    return bisect_batch(dd, de, n, batch, rel_tol, dsigma, dscratch, dpairs, nullptr, s, launches);
 }
 
 }  // namespace avs
