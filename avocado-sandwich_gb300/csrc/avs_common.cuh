@@ -106,6 +106,8 @@ struct Stage1Work {
     void *tau;        // [nt][b] of T
     void *tblk;       // [nt][b/ib][ib*ib] of T
     int *flags;       // ticket (1) + two progress counters per tile (2 nt), reset per launch
+    int *uflags = nullptr;  // optional: counters of the update of tiles 16-64 (n / 8 + 1 ints, stage 2's flags)
+    int64_t sUflags = 0;    // ints between matrices (batched)
     int *err;         // device status word (shared with other stages)
     void *tfull;      // [nt][b*b] of T: full compact-WY factors (tiles 128, 256)
     void *tc_ws = nullptr;  // tensor-core update buffers (stage1_tc_bytes), FP32 tiles

@@ -49,12 +49,12 @@
 #include "avs_common.cuh"
 #include "df64.cuh"
 #include "reflect.cuh"
+#include "vec16.cuh"
 
 namespace avs {
 namespace {
 
 constexpr int kIB = 16;    // reflectors per compact-WY block
-constexpr int kNT = 256;   // threads per CTA (16 columns x 16 row groups)
 
 struct PanelArgs {
     void *a;
@@ -80,12 +80,14 @@ struct UpdateArgs {
     int b;
     int pr, pc, P;
     int first_role;  // 1: the top tile's own (GEQRT) blocks were applied earlier
-    int width;       // strip width
+    int nstrip;      // column strips
+    int group;       // consecutive tiles per CTA
     const void *tblk;
-    int64_t sA, sTblk;  // per-matrix strides (blockIdx.y = matrix)
+    int fine;        // 1: a counter per block of a strip, 0: one per strip
+    int *flags;      // [0] ticket, then the counters: tiles done with the block (the strip); zeroed
+    int *err;
+    int64_t sA, sTblk, sFlags;  // per-matrix strides (blockIdx.y = matrix)
 };
-
-__host__ __device__ inline int ldpad(int b) { return b + 1; }  // update_kernel's strips
 
 // ---------------------------------------------------------------------------
 // Panel arithmetic by compute type.  Sq: a sum of squares (compensated pairs
@@ -263,50 +265,6 @@ __device__ __forceinline__ bool vfinite(float v) { return isfinite(v); }
 __device__ __forceinline__ bool vfinite(double v) { return isfinite(v); }
 __device__ __forceinline__ bool vfinite(dfx v) { return isfinite(v.v.hi) && isfinite(v.v.lo); }
 
-// 16-byte vectors: VN values of T from / to shared or global memory.
-template <typename T>
-struct PVec;
-template <>
-struct PVec<float> {
-    static constexpr int VN = 4;
-    static __device__ __forceinline__ void ld(const float *p, float *v) {
-        const float4 x = *reinterpret_cast<const float4 *>(p);
-        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-    }
-    static __device__ __forceinline__ void ldcg(const float *p, float *v) {
-        const float4 x = __ldcg(reinterpret_cast<const float4 *>(p));
-        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-    }
-    static __device__ __forceinline__ void st(float *p, const float *v) {
-        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    }
-};
-template <>
-struct PVec<double> {
-    static constexpr int VN = 2;
-    static __device__ __forceinline__ void ld(const double *p, double *v) {
-        const double2 x = *reinterpret_cast<const double2 *>(p);
-        v[0] = x.x; v[1] = x.y;
-    }
-    static __device__ __forceinline__ void ldcg(const double *p, double *v) {
-        const double2 x = __ldcg(reinterpret_cast<const double2 *>(p));
-        v[0] = x.x; v[1] = x.y;
-    }
-    static __device__ __forceinline__ void st(double *p, const double *v) {
-        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
-    }
-};
-template <>
-struct PVec<dfx> {
-    static constexpr int VN = 2;
-    static __device__ __forceinline__ void ld(const dfx *p, dfx *v) {
-        const float4 x = *reinterpret_cast<const float4 *>(p);
-        v[0] = dfx(df64{x.x, x.y}); v[1] = dfx(df64{x.z, x.w});
-    }
-    static __device__ __forceinline__ void st(dfx *p, const dfx *v) {
-        *reinterpret_cast<float4 *>(p) = make_float4(v[0].v.hi, v[0].v.lo, v[1].v.hi, v[1].v.lo);
-    }
-};
 // two sums of squares at a 16-byte aligned address
 template <typename Sq>
 struct PSq2;
@@ -1033,121 +991,263 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
     }
 }
 
-template <typename T>
-size_t update_smem_bytes(int b, int width) {
-    return sizeof(T) * ((size_t)2 * ldpad(b) * width + (size_t)ldpad(b) * kIB + 2 * (size_t)kIB * width +
-                        (size_t)kIB * kIB);
-}
-
-template <typename T, int LAYOUT>
-__global__ void __launch_bounds__(kNT) update_kernel(UpdateArgs args) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int b = args.b;
-    const int nb = b / kIB;
-    const int ld = ldpad(b);
-    const int W = args.width;
-    T *Top = reinterpret_cast<T *>(smem_raw);  // ld * W
-    T *Ap = Top + (size_t)ld * W;              // ld * W
-    T *Vs = Ap + (size_t)ld * W;               // ld * kIB
-    T *Zs = Vs + (size_t)ld * kIB;             // kIB * W
-    T *Ws = Zs + (size_t)kIB * W;              // kIB * W
-    T *Tm = Ws + (size_t)kIB * W;              // kIB * kIB
-
-    const int tid = threadIdx.x;
-    const int64_t j0 = (int64_t)(args.pc + 1) * b + (int64_t)blockIdx.x * W;
-    const int wc = (int)min((int64_t)W, args.n - j0);
-    if (wc <= 0) return;
-    const int64_t zb = blockIdx.y;
-    View<T, LAYOUT> V{reinterpret_cast<T *>(args.a) + zb * args.sA, args.lda};
-    const int64_t top0 = (int64_t)args.pr * b;
-    const int64_t col0 = (int64_t)args.pc * b;
-    const T *tblk = reinterpret_cast<const T *>(args.tblk) + zb * args.sTblk;
-
-    auto load_strip = [&](T *S, int64_t r0) {
-        for (int idx = tid; idx < b * wc; idx += kNT) {
-            int t, c;
-            if (LAYOUT == 0) { t = idx % b; c = idx / b; } else { c = idx % wc; t = idx / wc; }
-            S[t + c * ld] = V(r0 + t, j0 + c);
-        }
-    };
-    auto store_strip = [&](const T *S, int64_t r0) {
-        for (int idx = tid; idx < b * wc; idx += kNT) {
-            int t, c;
-            if (LAYOUT == 0) { t = idx % b; c = idx / b; } else { c = idx % wc; t = idx / wc; }
-            V(r0 + t, j0 + c) = S[t + c * ld];
-        }
-    };
-
-    load_strip(Top, top0);
-    for (int p = args.first_role; p < args.P; ++p) {
-        const bool geqrt = (p == 0);
-        const int64_t r0 = (int64_t)(args.pr + p) * b;
-        T *Tp = geqrt ? Top : Ap;
-        if (!geqrt) load_strip(Ap, r0);
-        for (int cb = 0; cb < nb; ++cb) {
-            const int c0 = cb * kIB;
-            for (int idx = tid; idx < b * kIB; idx += kNT) {
-                int t, l;
-                if (LAYOUT == 0) { t = idx % b; l = idx / b; } else { l = idx % kIB; t = idx / kIB; }
-                Vs[t + l * ld] = V(r0 + t, col0 + c0 + l);
-            }
-            if (tid < kIB * kIB) Tm[tid] = tblk[((size_t)p * nb + cb) * kIB * kIB + tid];
-            __syncthreads();
-            // Z = Y^T Tp (+ top rows for TSQRT blocks)
-            for (int o = tid; o < kIB * wc; o += kNT) {
-                const int l = o % kIB, c = o / kIB;
-                T z;
-                if (geqrt) {
-                    const int ts = c0 + l;
-                    z = Tp[ts + c * ld];
-                    for (int t = ts + 1; t < b; ++t) z += Vs[t + l * ld] * Tp[t + c * ld];
-                } else {
-                    z = Top[c0 + l + c * ld];
-                    for (int t = 0; t < b; ++t) z += Vs[t + l * ld] * Tp[t + c * ld];
-                }
-                Zs[l + c * kIB] = z;
-            }
-            __syncthreads();
-            // W = T^T Z
-            for (int o = tid; o < kIB * wc; o += kNT) {
-                const int l = o % kIB, c = o / kIB;
-                T w = T(0);
-                for (int m = 0; m <= l; ++m) w += Tm[m + l * kIB] * Zs[m + c * kIB];
-                Ws[l + c * kIB] = w;
-            }
-            __syncthreads();
-            // Tp -= Y W ; top rows -= W (TSQRT)
-            for (int idx = tid; idx < b * wc; idx += kNT) {
-                const int t = idx % b, c = idx / b;
-                if (geqrt) {
-                    if (t >= c0) {
-                        const int lmax = min(kIB - 1, t - c0);
-                        T acc = T(0);
-                        for (int l = 0; l <= lmax; ++l) {
-                            const T y = (t == c0 + l) ? T(1) : Vs[t + l * ld];
-                            acc += y * Ws[l + c * kIB];
-                        }
-                        Tp[t + c * ld] -= acc;
-                    }
-                } else {
-                    T acc = T(0);
-#pragma unroll
-                    for (int l = 0; l < kIB; ++l) acc += Vs[t + l * ld] * Ws[l + c * kIB];
-                    Tp[t + c * ld] -= acc;
-                }
-            }
-            if (!geqrt) {
-                for (int o = tid; o < kIB * wc; o += kNT) {
-                    const int l = o % kIB, c = o / kIB;
-                    Top[c0 + l + c * ld] -= Ws[l + c * kIB];
-                }
-            }
-            __syncthreads();
-        }
-        if (!geqrt) store_strip(Ap, r0);
-        __syncthreads();
+// ---------------------------------------------------------------------------
+// Trailing update of tiles 16, 32 and 64, 16 reflectors at a time (tiles 128 and
+// 256: the full-T update).
+//
+// A CTA takes a column strip and `group` consecutive tiles; a thread owns 16 rows
+// of one column of the current tile, in registers from its load to its store.
+// Per block of 16 reflectors: Z = V^T A over the thread's rows, the row segments
+// joined through shared memory, W = T^T (Z + top rows) (FP32: by every segment's
+// thread, so W needs no second exchange; FP64: by the first segment's), top rows
+// -= W, A -= V W.  The top rows of the strip stay in shared memory while the CTA
+// works through its group and pass from group to group block by block: the next
+// group needs a block's top rows only when it forms that block's W, so the chain
+// through the tiles is one load, one 16 x 16 product and one store per tile and
+// block (a counter per block: one for the whole strip would not grow
+// monotonically).
+// V and T of the next blocks are staged ahead (three buffers: one barrier per
+// block).  (tile group, strip) pairs come from a ticket in group-major order, so a
+// CTA only waits on one that already runs.
+//
+// What bounds it: the chain of W through the tiles (about 1.5 us a tile), the FP32
+// pipe in large batches, the FP64 unit for FP64.  Measured (GB300, all of a call's
+// updates, before: one CTA per strip looping over the tiles, every product from
+// shared memory with three barriers a block): FP32 n = 1024 tile 64 11.3 -> 1.35
+// ms, n = 1296 tile 16 39 -> 11 ms; FP64 n = 1024 tile 64 22.5 -> 7.2 ms.
+template <typename T, int B>
+struct UpdCfg {
+    static constexpr int NB = B / kIB;             // blocks per tile = row segments
+    static constexpr bool F4 = sizeof(T) == 4;
+    static constexpr int W = F4 ? 64 : 32;         // columns of a strip
+    static constexpr int NT = W * NB;
+    static constexpr int LDV = F4 ? 20 : 18;       // row stride of V (16-byte rows)
+    static constexpr int VSZ = B * LDV + kIB * kIB;  // one staged block: V, then T (row l: T(0..15, l))
+    static constexpr int PER = (B * kIB + NT - 1) / NT;
+    static constexpr int MINB = F4 ? (B == 64 ? 2 : (B == 32 ? 3 : 6)) : 1;  // CTAs per SM the registers allow
+    static constexpr size_t smem_bytes() {
+        return sizeof(T) * (3 * (size_t)VSZ + (size_t)B * W + (NB > 1 ? 2 * (size_t)NB * kIB * W + kIB * W : 0));
     }
-    store_strip(Top, top0);
+};
+
+template <typename T, int LAYOUT, int B>
+__global__ void __launch_bounds__(UpdCfg<T, B>::NT, UpdCfg<T, B>::MINB) update_kernel(UpdateArgs args) {
+    using C = UpdCfg<T, B>;
+    constexpr int NB = C::NB, W = C::W, NT = C::NT, LDV = C::LDV, PER = C::PER;
+    constexpr int VN = PVec<T>::VN;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *Vs = reinterpret_cast<T *>(smem_raw);  // [3][VSZ]
+    T *Top = Vs + 3 * C::VSZ;                 // [B][W]
+    T *Zp = Top + B * W;                      // [2][NB][16][W]
+    T *Wx = Zp + 2 * NB * kIB * W;            // [16][W] (FP64)
+    __shared__ int s_t, s_ok;
+    const int tid = threadIdx.x;
+    const int64_t zb = blockIdx.y;
+    int *flags = args.flags + zb * args.sFlags;
+    if (tid == 0) {
+        s_t = atomicAdd(flags, 1);
+        s_ok = 1;
+    }
+    __syncthreads();
+    const int grp = s_t / args.nstrip, strip = s_t % args.nstrip;
+    const int p0 = args.first_role + grp * args.group;
+    if (p0 >= args.P) return;
+    const int p1 = min(args.P, p0 + args.group);
+    int *done = flags + 1 + strip * (args.fine ? NB : 1);
+    const int64_t j0 = (int64_t)(args.pc + 1) * B + (int64_t)strip * W;
+    const int col = tid % W, seg = tid / W;
+    const bool live = j0 + col < args.n;
+    View<T, LAYOUT> V{reinterpret_cast<T *>(args.a) + zb * args.sA, args.lda};
+    const int64_t top0 = (int64_t)args.pr * B, col0 = (int64_t)args.pc * B;
+    const int64_t jc = live ? j0 + col : j0;  // dead columns repeat the first one and store nothing
+    const T *tblk = reinterpret_cast<const T *>(args.tblk) + zb * args.sTblk;
+    const int nblk = (p1 - p0) * NB;
+
+    // staging of block u of the group (tile p0 + u / NB, block u % NB): V masked to
+    // unit lower for the top tile, and T
+    T sv[PER];
+    T st[kIB * kIB / NT > 0 ? kIB * kIB / NT : 1];
+    auto fetch = [&](int u) {
+        const int p = p0 + u / NB, c0 = (u % NB) * kIB;
+        const int64_t r0 = (int64_t)(args.pr + p) * B;
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int idx = tid + e * NT;
+            const int r = LAYOUT == 0 ? idx % B : idx / kIB, l = LAYOUT == 0 ? idx / B : idx % kIB;
+            T v = __ldcg(&V(r0 + r, col0 + c0 + l));
+            if (p == 0) v = r == c0 + l ? T(1) : (r > c0 + l ? v : T(0));
+            sv[e] = v;
+        }
+#pragma unroll
+        for (int e = 0; e < (int)(sizeof(st) / sizeof(T)); ++e) {
+            const int idx = tid + e * NT;
+            if (idx < kIB * kIB) st[e] = __ldcg(tblk + ((size_t)p * NB + u % NB) * kIB * kIB + idx);
+        }
+    };
+    auto stage = [&](int u) {
+        T *buf = Vs + (u % 3) * C::VSZ;
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int idx = tid + e * NT;
+            const int r = LAYOUT == 0 ? idx % B : idx / kIB, l = LAYOUT == 0 ? idx / B : idx % kIB;
+            buf[r * LDV + l] = sv[e];
+        }
+#pragma unroll
+        for (int e = 0; e < (int)(sizeof(st) / sizeof(T)); ++e) {
+            const int idx = tid + e * NT;
+            if (idx < kIB * kIB) buf[B * LDV + idx] = st[e];
+        }
+    };
+    static_assert(B * kIB % NT == 0, "staging split");
+
+    T a[kIB], an[kIB];
+    auto load_tile = [&](int p, T (&v)[kIB]) {
+        load_col<T, LAYOUT, T, kIB>(V, (int64_t)(args.pr + p) * B + seg * kIB, jc, v);
+    };
+    load_tile(p0, a);
+    fetch(0);
+    stage(0);
+    if (nblk > 1) {
+        fetch(1);
+        stage(1);
+    }
+    if (nblk > 2) fetch(2);
+    __syncthreads();
+    T pend[kIB];       // new top rows, stored once every thread has read the old ones
+    int pend_row = -1;
+    for (int u = 0; u < nblk; ++u) {
+        const int p = p0 + u / NB, cb = u % NB, c0 = cb * kIB;
+        const bool head = p == 0;                    // the top tile itself (GEQRT)
+        const bool in_global = !head && p == p0;     // the top rows come from the previous group
+        const T *vb = Vs + (u % 3) * C::VSZ, *tb = vb + B * LDV;
+        if (cb == 0 && p + 1 < p1) load_tile(p + 1, an);
+        // Z over my rows
+        T z[kIB];
+#pragma unroll
+        for (int l = 0; l < kIB; ++l) z[l] = T(0);
+#pragma unroll
+        for (int r = 0; r < kIB; ++r) {
+            T y[kIB];
+            ld16<T>(vb + (seg * kIB + r) * LDV, y);
+#pragma unroll
+            for (int l = 0; l < kIB; ++l) z[l] += y[l] * a[r];
+        }
+        if (NB > 1) {
+            T *zp = Zp + ((u & 1) * NB + seg) * kIB * W + col;
+#pragma unroll
+            for (int l = 0; l < kIB; ++l) zp[l * W] = z[l];
+        }
+        if (tid == 0 && in_global && p > args.first_role && (args.fine || cb == 0))
+            s_ok = wait_geq(done + (args.fine ? cb : 0), p - args.first_role, args.err);
+        __syncthreads();
+        if (!s_ok) return;
+        if (pend_row >= 0) {
+#pragma unroll
+            for (int l = 0; l < kIB; ++l) Top[(pend_row + l) * W + col] = pend[l];
+            pend_row = -1;
+        }
+        if (u + 2 < nblk) {
+            stage(u + 2);
+            if (u + 3 < nblk) fetch(u + 3);
+        }
+        // another group follows: each block's counter only grows tile by tile
+        const bool release = p + 1 == p1 && p + 1 < args.P && (args.fine || cb == NB - 1);
+        // W = T^T (Z + top rows); top rows -= W
+        T w[kIB];
+        if (C::F4 || seg == 0) {
+            T top[kIB];
+            if (!head) {
+                if (in_global) {
+                    load_col<T, LAYOUT, T, kIB>(V, top0 + c0, jc, top);
+                } else {
+#pragma unroll
+                    for (int l = 0; l < kIB; ++l) top[l] = Top[(c0 + l) * W + col];
+                }
+            }
+            if (NB > 1) {
+#pragma unroll
+                for (int l = 0; l < kIB; ++l) {
+                    const T *zp = Zp + (u & 1) * NB * kIB * W + l * W + col;
+                    z[l] = zp[0];
+#pragma unroll
+                    for (int q = 1; q < NB; ++q) z[l] += zp[q * kIB * W];
+                }
+            }
+            if (!head) {
+#pragma unroll
+                for (int l = 0; l < kIB; ++l) z[l] += top[l];
+                // every segment has read the rows that the first one overwrites below
+                if (C::F4 && NB > 1 && in_global && p + 1 == p1) __syncthreads();
+            }
+#pragma unroll
+            for (int l = 0; l < kIB; ++l) {  // T(m, l) at tb[m + 16 l]
+                T tl[kIB];
+#pragma unroll
+                for (int q = 0; q <= l; q += VN) PVec<T>::ld(tb + l * kIB + q, tl + q);
+                T acc = T(0);
+#pragma unroll
+                for (int m = 0; m <= l; ++m) acc += tl[m] * z[m];
+                w[l] = acc;
+            }
+            if (!head) {
+                // out: the last tile of the group hands the rows on (and the last tile
+                // of the panel leaves them final)
+                if (seg == 0) {
+#pragma unroll
+                    for (int l = 0; l < kIB; ++l) pend[l] = top[l] - w[l];
+                    if (p + 1 == p1) {
+                        if (live) store_col<T, LAYOUT, T, kIB>(V, top0 + c0, jc, pend);
+                        if (release) {
+                            bar_named(1, W);
+                            if (col == 0) st_release(done + (args.fine ? cb : 0), p - args.first_role + 1);
+                        }
+                    } else {
+                        pend_row = c0;
+                    }
+                }
+            }
+            if (!C::F4 && NB > 1) {
+#pragma unroll
+                for (int l = 0; l < kIB; ++l) Wx[l * W + col] = w[l];
+            }
+        }
+        if (!C::F4 && NB > 1) {
+            __syncthreads();
+            if (seg > 0) {
+#pragma unroll
+                for (int l = 0; l < kIB; ++l) w[l] = Wx[l * W + col];
+            }
+        }
+        // A -= V W
+#pragma unroll
+        for (int r = 0; r < kIB; ++r) {
+            T y[kIB];
+            ld16<T>(vb + (seg * kIB + r) * LDV, y);
+            T acc = T(0);
+#pragma unroll
+            for (int l = 0; l < kIB; ++l) acc += y[l] * w[l];
+            a[r] -= acc;
+        }
+        if (head) {
+            // rows c0 .. c0+15 of the top tile are final for this tile
+            if (p + 1 == p1) {
+                if (seg == cb && live) store_col<T, LAYOUT, T, kIB>(V, top0 + c0, jc, a);
+                if (release) {
+                    __syncthreads();
+                    if (tid == 0) st_release(done + (args.fine ? cb : 0), p - args.first_role + 1);
+                }
+            } else if (seg == cb) {
+#pragma unroll
+                for (int l = 0; l < kIB; ++l) Top[(c0 + l) * W + col] = a[l];
+            }
+        }
+        if (cb == NB - 1) {
+            if (!head && live)
+                store_col<T, LAYOUT, T, kIB>(V, (int64_t)(args.pr + p) * B + seg * kIB, jc, a);
+#pragma unroll
+            for (int r = 0; r < kIB; ++r) a[r] = an[r];
+        }
+    }
 }
 
 // One panel kernel per tile size.
@@ -1214,19 +1314,49 @@ int launch_panel(T *dA, int64_t lda, int b, int pr, int pc, int P, int first_rol
     return launch_panel_ct<T, LAYOUT, T>(a, grid, s);
 }
 
+template <typename T, int LAYOUT, int B>
+int launch_update_b(UpdateArgs a, int64_t ncols, const Stage1Work &w, cudaStream_t s) {
+    using C = UpdCfg<T, B>;
+    static std::atomic<bool> attr_set{false};
+    constexpr size_t smem = C::smem_bytes();
+    static_assert(smem <= 227 * 1024, "update shared memory");
+    if (!attr_set) {
+        AVS_CUDA_TRY(cudaFuncSetAttribute(update_kernel<T, LAYOUT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+        attr_set = true;
+    }
+    const int batch = w.batch > 0 ? w.batch : 1;
+    a.nstrip = (int)((ncols + C::W - 1) / C::W);
+    // Tiles per CTA.  Passing the strip on costs about what a 16-wide FP32 tile costs,
+    // so those go to one CTA per strip (n = 1296: stage 1 49 ms, one tile per CTA
+    // 54).  Otherwise one tile per CTA where latency counts (FP32 n = 1024 tile 64
+    // 5.0 ms, all tiles in one CTA 6.5; FP64 n = 512 tile 32 18.0 against 27.7, and
+    // FP64 always: its tiles take long), and all of them once the strips fill the GPU
+    // twice over by themselves (32 matrices of order 1024 tile 64 10.5 ms against
+    // 15.0, 256 of order 256 tile 32 2.2 against 3.0).  The values do not depend on it.
+    const bool whole = C::F4 && (B == 16 || (int64_t)a.nstrip * batch >= 304);
+    a.group = whole ? a.P : 1;
+    // ticket and counters: one per block and strip in the work's own array, else (out
+    // of core) one per strip in the panel's flags, which are free again
+    a.fine = w.uflags != nullptr;
+    a.flags = a.fine ? w.uflags : w.flags;
+    a.sFlags = a.fine ? w.sUflags : w.sFlags;
+    const size_t fb = sizeof(int) * (size_t)(1 + a.nstrip * (a.fine ? C::NB : 1));
+    if (batch > 1)
+        AVS_CUDA_TRY(cudaMemset2DAsync(a.flags, sizeof(int) * (size_t)a.sFlags, 0, fb, batch, s));
+    else
+        AVS_CUDA_TRY(cudaMemsetAsync(a.flags, 0, fb, s));
+    const int ngrp = (a.P - a.first_role + a.group - 1) / a.group;
+    update_kernel<T, LAYOUT, B><<<dim3((unsigned)a.nstrip * ngrp, batch), C::NT, smem, s>>>(a);
+    AVS_CUDA_TRY(cudaGetLastError());
+    return AVS_SUCCESS;
+}
 template <typename T, int LAYOUT>
 int launch_update(T *dA, int64_t lda, int64_t n, int b, int pr, int pc, int P, const Stage1Work &w,
                   cudaStream_t s, int first_role = 0) {
-    const int width = sizeof(T) == 8 ? 32 : 64;
-    static std::atomic<bool> attr_set{false};
-    if (!attr_set) {
-        AVS_CUDA_TRY(cudaFuncSetAttribute(update_kernel<T, LAYOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)update_smem_bytes<T>(256, width)));
-        attr_set = true;
-    }
     const int64_t ncols = n - (int64_t)(pc + 1) * b;
-    if (ncols <= 0) return AVS_SUCCESS;
-    UpdateArgs a;
+    if (ncols <= 0 || P <= first_role) return AVS_SUCCESS;
+    UpdateArgs a{};
     a.a = dA;
     a.lda = lda;
     a.n = n;
@@ -1235,14 +1365,16 @@ int launch_update(T *dA, int64_t lda, int64_t n, int b, int pr, int pc, int P, c
     a.pc = pc;
     a.P = P;
     a.first_role = first_role;
-    a.width = width;
     a.tblk = w.tblk;
+    a.err = w.err;
     a.sA = w.sA;
     a.sTblk = w.sTblk;
-    const unsigned grid = (unsigned)((ncols + width - 1) / width);
-    update_kernel<T, LAYOUT><<<dim3(grid, w.batch > 0 ? w.batch : 1), kNT, update_smem_bytes<T>(b, width), s>>>(a);
-    AVS_CUDA_TRY(cudaGetLastError());
-    return AVS_SUCCESS;
+    switch (b) {
+        case 16: return launch_update_b<T, LAYOUT, 16>(a, ncols, w, s);
+        case 32: return launch_update_b<T, LAYOUT, 32>(a, ncols, w, s);
+        case 64: return launch_update_b<T, LAYOUT, 64>(a, ncols, w, s);
+        default: return AVS_ERR_UNSUPPORTED;  // the full-T update
+    }
 }
 
 // The tau of the panel just launched (roles 0..P-1 of half-step k, tile index

@@ -16,17 +16,29 @@
 // forms the same T for FP32 tiles with T's upper block triangle in shared
 // memory.
 //
-// update_full_kernel: one CTA per column strip keeps the strip of the top tile
-// row in shared memory for the whole half-step; each of the three products is
-// a register-blocked GEMM (8 rows x CB columns per thread, K = b streamed
-// through shared memory in chunks that the next chunk's loads overlap).  FP64
-// tiles use 16-column strips when 32-column strips would leave SMs idle; in
-// double-float the products accumulate with the compensated dot product.
+// update_full_kernel: one CTA per (tile, column strip).  Only W and the strip of
+// the top tile row pass from tile to tile (W_p needs Top after tile p-1), so
+// V_p^T A_p runs as soon as the CTA starts, then the CTA waits for the previous
+// tile's release of the strip, forms W, hands the strip on and updates its own
+// tile.  CTAs take (tile, strip) pairs in tile-major order from a ticket, so a
+// CTA only waits on one that already runs.  What bounded it with one CTA per strip
+// looping over the tiles: the strips were the launch's only parallelism (64
+// columns each, 2 to 62 CTAs on 152 SMs at n = 4096) and every tile's three
+// products ran in sequence.  Now the FP32 pipe while there are many tiles (n = 4096:
+// about 19 TFLOP/s in the first half-steps), the chain of W (about 6 us a tile)
+// towards the end.  Measured (GB300, all updates of a call, before -> after): FP32 n
+// = 4096 tile 128 45.8 -> 20.2 ms, double-float n = 2048 tile 128 34.5 -> 24.0 ms.
+// Each of the three products is a register-blocked GEMM (8 rows x CB columns per
+// thread, K = b streamed through shared memory in chunks that the next chunk's
+// loads overlap); T's zeros are skipped by row groups.  FP64 tiles use 16-column
+// strips when 32-column strips would leave SMs idle; in double-float the products
+// accumulate with the compensated dot product.
 #include <algorithm>
 #include <type_traits>
 
 #include "avs_common.cuh"
 #include "df64.cuh"
+#include "vec16.cuh"
 
 namespace avs {
 namespace {
@@ -354,6 +366,10 @@ struct UpdFullArgs {
     const void *tfull;
     int64_t sA, sTfull;  // per-matrix strides (blockIdx.y = matrix)
     int first_role;      // 1: the top tile's own reflectors were applied earlier
+    int nstrip;
+    int *flags;          // [0] ticket, [1 + strip] tiles finished with the top strip; zeroed
+    int64_t sFlags;      // ints between matrices
+    int *err;
 };
 
 // A-operand sources for the three products.
@@ -367,7 +383,13 @@ struct UCfg {
     static constexpr int TM = B / MB;             // threads along rows
     static constexpr int TC = kWNT / TM;          // threads along columns
     static constexpr int CB = W / TC;             // columns per thread
-    static constexpr int LDB = B + 4;             // leading dimension of strip buffers (rows)
+    // A thread's 8 rows are groups of VN consecutive ones, B VN / 8 apart, and the strip
+    // buffers are row-major: a product's operands are 16-byte loads, 3 for 32
+    // products in FP32 (12 single ones bound it by shared memory)
+    static constexpr int VN = sizeof(T) == 4 ? 4 : 2;
+    static constexpr int GS = B * VN / MB;        // rows between a thread's groups
+    static __device__ __forceinline__ int row(int m0, int i) { return (i / VN) * GS + m0 * VN + i % VN; }
+    static constexpr int LDW = W + VN;            // row stride of the strip buffers
     static constexpr int LDC = B + 4;             // leading dimension of A chunks (m)
     static constexpr int PER = KC * B / kWNT;     // chunk elements per thread
     static_assert(CB >= 1 && PER >= 1, "update configuration");
@@ -403,13 +425,28 @@ struct UpdCtx {
 
 // acc (+|-)= A(k, m)^T-view ... : acc[i][j] += sign * sum_k A(k, m0+i) * Bop(k, c0+j)
 template <typename T, int LAYOUT, int B, int WW = WCfg<T>::W, typename CT = T>
-__device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, int src,
+__device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, const int src,
                                      CT (&acc)[8][UCfg<T, B, WW>::CB], const CT *Bop, CT *chunk0, CT *chunk1,
                                      bool neg) {
     using C = UCfg<T, B, WW>;
     const int tid = threadIdx.x;
-    const int m0 = tid % C::TM;  // rows m0 + TM*i: consecutive lanes, consecutive rows
+    const int m0 = tid % C::TM;
     const int c0 = (tid / C::TM) * C::CB;
+    // rows and columns of the products at chunk row k
+    auto load_av = [&](const CT *cur, int k, CT (&av)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; i += C::VN) PVec<CT>::ld(cur + k * C::LDC + C::row(m0, i), av + i);
+    };
+    auto load_bv = [&](int k, CT (&bv)[C::CB]) {
+        const CT *p = Bop + k * C::LDW + c0;
+        if constexpr (C::CB % C::VN == 0) {
+#pragma unroll
+            for (int j = 0; j < C::CB; j += C::VN) PVec<CT>::ld(p + j, bv + j);
+        } else {
+#pragma unroll
+            for (int j = 0; j < C::CB; ++j) bv[j] = p[j];
+        }
+    };
     CT pre[C::PER];
     // prologue: chunk 0 into registers
 #pragma unroll
@@ -446,15 +483,14 @@ __device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, in
 #pragma unroll 4
             for (int k = 0; k < C::KC; ++k) {
                 CT av[8], bv[C::CB];
+                load_av(cur, k, av);
+                load_bv(k0 + k, bv);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) av[i] = cur[k * C::LDC + m0 + C::TM * i];
-#pragma unroll
-                for (int j = 0; j < C::CB; ++j) {
-                    bv[j] = Bop[(k0 + k) + (c0 + j) * C::LDB];
+                for (int j = 0; j < C::CB; ++j)
                     if (neg) bv[j] = -bv[j];
-                }
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+                for (int i = 0; i < 8; ++i) {
+                    if (src == kTrows && (i / C::VN + 1) * C::GS <= k0) continue;  // T(k, m) = 0 below the diagonal
 #pragma unroll
                     for (int j = 0; j < C::CB; ++j) {
                         const df64 x = av[i].v, y = bv[j].v;
@@ -469,16 +505,15 @@ __device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, in
                         a.hi = t;
                         a.lo = __fadd_rn(a.lo, __fadd_rn(es, ep));
                     }
+                }
             }
             continue;
         }
 #pragma unroll 4
         for (int k = 0; k < C::KC; ++k) {
             CT av[8], bv[C::CB];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) av[i] = cur[k * C::LDC + m0 + C::TM * i];
-#pragma unroll
-            for (int j = 0; j < C::CB; ++j) bv[j] = Bop[(k0 + k) + (c0 + j) * C::LDB];
+            load_av(cur, k, av);
+            load_bv(k0 + k, bv);
             if (neg) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
@@ -486,9 +521,11 @@ __device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, in
                     for (int j = 0; j < C::CB; ++j) acc[i][j] -= av[i] * bv[j];
             } else {
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+                for (int i = 0; i < 8; ++i) {
+                    if (src == kTrows && (i / C::VN + 1) * C::GS <= k0) continue;  // T(k, m) = 0 below the diagonal
 #pragma unroll
                     for (int j = 0; j < C::CB; ++j) acc[i][j] += av[i] * bv[j];
+                }
             }
         }
     }
@@ -506,15 +543,21 @@ __global__ void __launch_bounds__(kWNT) update_full_kernel(UpdFullArgs args) {
     using C = UCfg<T, B, WW>;
     static_assert(sizeof(CT) == sizeof(T), "compute type of the element's size");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    CT *Top = reinterpret_cast<CT *>(smem_raw);    // LDB x W, column-major
-    CT *Buf = Top + (size_t)C::LDB * C::W;         // LDB x W
-    CT *ch0 = Buf + (size_t)C::LDB * C::W;         // KC x LDC
+    CT *Buf = reinterpret_cast<CT *>(smem_raw);    // B x LDW, row-major: the tile's strip
+    CT *Zb = Buf + (size_t)B * C::LDW;             // B x LDW: top strip, Z, W
+    CT *ch0 = Zb + (size_t)B * C::LDW;             // KC x LDC
     CT *ch1 = ch0 + (size_t)C::KC * C::LDC;
+    __shared__ int s_t, s_ok;
     const int tid = threadIdx.x;
-    const int64_t j0 = (int64_t)(args.pc + 1) * B + (int64_t)blockIdx.x * C::W;
-    const int wc = (int)min((int64_t)C::W, args.n - j0);
-    if (wc <= 0) return;
     const int64_t zb = blockIdx.y;
+    int *flags = args.flags + zb * args.sFlags;
+    if (tid == 0) s_t = atomicAdd(flags, 1);
+    __syncthreads();
+    const int p = args.first_role + s_t / args.nstrip, strip = s_t % args.nstrip;
+    if (p >= args.P) return;
+    int *done = flags + 1 + strip;
+    const int64_t j0 = (int64_t)(args.pc + 1) * B + (int64_t)strip * C::W;
+    const int wc = (int)min((int64_t)C::W, args.n - j0);
     View<T, LAYOUT> V{reinterpret_cast<T *>(args.a) + zb * args.sA, args.lda};
     const int64_t top0 = (int64_t)args.pr * B;
     const int m0 = tid % C::TM;
@@ -524,27 +567,27 @@ __global__ void __launch_bounds__(kWNT) update_full_kernel(UpdFullArgs args) {
         for (int idx = tid; idx < B * C::W; idx += kWNT) {
             int t, c;
             if (LAYOUT == 0) { t = idx % B; c = idx / B; } else { c = idx % C::W; t = idx / C::W; }
-            S[t + c * C::LDB] = (c < wc) ? CT(V(r0 + t, j0 + c)) : CT(0);
+            S[t * C::LDW + c] = (c < wc) ? CT(__ldcg(&V(r0 + t, j0 + c))) : CT(0);
         }
     };
     auto store_strip = [&](const CT *S, int64_t r0) {
         for (int idx = tid; idx < B * C::W; idx += kWNT) {
             int t, c;
             if (LAYOUT == 0) { t = idx % B; c = idx / B; } else { c = idx % C::W; t = idx / C::W; }
-            if (c < wc) V(r0 + t, j0 + c) = (T)S[t + c * C::LDB];
+            if (c < wc) V(r0 + t, j0 + c) = (T)S[t * C::LDW + c];
         }
     };
     auto get_blk = [&](const CT *S, CT (&r)[8][C::CB]) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < C::CB; ++j) r[i][j] = S[(m0 + C::TM * i) + (c0 + j) * C::LDB];
+            for (int j = 0; j < C::CB; ++j) r[i][j] = S[C::row(m0, i) * C::LDW + c0 + j];
     };
     auto put_blk = [&](CT *S, const CT (&r)[8][C::CB]) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < C::CB; ++j) S[(m0 + C::TM * i) + (c0 + j) * C::LDB] = r[i][j];
+            for (int j = 0; j < C::CB; ++j) S[C::row(m0, i) * C::LDW + c0 + j] = r[i][j];
     };
     auto zero = [&](CT (&r)[8][C::CB]) {
 #pragma unroll
@@ -553,66 +596,71 @@ __global__ void __launch_bounds__(kWNT) update_full_kernel(UpdFullArgs args) {
             for (int j = 0; j < C::CB; ++j) r[i][j] = CT(0);
     };
 
-    load_strip(Top, top0);
-    __syncthreads();
     CT acc[8][C::CB];
-    CT apr[8][C::CB];
-    for (int p = args.first_role; p < args.P; ++p) {
-        UpdCtx<T, LAYOUT, B, WW, CT> ctx;
-        ctx.V = V;
-        ctx.Tf = reinterpret_cast<const T *>(args.tfull) + zb * args.sTfull + (size_t)p * B * B;
-        ctx.row0 = (int64_t)(args.pr + p) * B;
-        ctx.col0 = (int64_t)args.pc * B;
-        ctx.geqrt = (p == 0);
-        if (p == 0) {
-            zero(acc);
-            gemm(ctx, kVrows, acc, Top, ch0, ch1, false);   // Z = Y0^T Top
-            put_blk(Buf, acc);
-            __syncthreads();
-            zero(acc);
-            gemm(ctx, kTrows, acc, Buf, ch0, ch1, false);   // W = T0^T Z
-            put_blk(Buf, acc);
-            __syncthreads();
-            get_blk(Top, acc);
-            gemm(ctx, kVcols, acc, Buf, ch0, ch1, true);    // Top -= Y0 W
-            put_blk(Top, acc);
-            __syncthreads();
-        } else {
-            load_strip(Buf, ctx.row0);
-            __syncthreads();
-            get_blk(Top, acc);
-            gemm(ctx, kVrows, acc, Buf, ch0, ch1, false);   // Z = Top + V^T A_p
-            get_blk(Buf, apr);
-            __syncthreads();
-            put_blk(Buf, acc);
-            __syncthreads();
-            zero(acc);
-            gemm(ctx, kTrows, acc, Buf, ch0, ch1, false);   // W = T^T Z
-            {
-                CT tp[8][C::CB];
-                get_blk(Top, tp);
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int j = 0; j < C::CB; ++j) tp[i][j] -= acc[i][j];
-                put_blk(Top, tp);                                             // Top -= W
-            }
-            put_blk(Buf, acc);
-            __syncthreads();
-            gemm(ctx, kVcols, apr, Buf, ch0, ch1, true);    // A_p -= V W
-            put_blk(Buf, apr);
-            __syncthreads();
-            store_strip(Buf, ctx.row0);
-            __syncthreads();
-        }
+    CT blk[8][C::CB];
+    UpdCtx<T, LAYOUT, B, WW, CT> ctx;
+    ctx.V = V;
+    ctx.Tf = reinterpret_cast<const T *>(args.tfull) + zb * args.sTfull + (size_t)p * B * B;
+    ctx.row0 = (int64_t)(args.pr + p) * B;
+    ctx.col0 = (int64_t)args.pc * B;
+    ctx.geqrt = (p == 0);
+    load_strip(Buf, ctx.row0);
+    __syncthreads();
+    zero(acc);
+    gemm(ctx, kVrows, acc, Buf, ch0, ch1, false);   // V_p^T A_p (the top tile: Y0^T Top)
+    if (p == 0) {
+        put_blk(Zb, acc);
+        __syncthreads();
+        zero(acc);
+        gemm(ctx, kTrows, acc, Zb, ch0, ch1, false);   // W = T0^T Z
+        put_blk(Zb, acc);
+        __syncthreads();
+        get_blk(Buf, acc);
+        gemm(ctx, kVcols, acc, Zb, ch0, ch1, true);    // Top -= Y0 W
+        put_blk(Buf, acc);
+        __syncthreads();
+        store_strip(Buf, top0);
+        __syncthreads();
+        if (tid == 0) st_release(done, 1);
+        return;
     }
-    store_strip(Top, top0);
+    // the top strip, once the previous tile is done with it
+    if (tid == 0) s_ok = p > args.first_role ? wait_geq(done, p - args.first_role, args.err) : true;
+    __syncthreads();
+    if (!s_ok) return;
+    load_strip(Zb, top0);
+    __syncthreads();
+    get_blk(Zb, blk);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < C::CB; ++j) acc[i][j] += blk[i][j];
+    put_blk(Zb, acc);                                // Z = Top + V^T A_p (each thread its own entries)
+    __syncthreads();
+    zero(acc);
+    gemm(ctx, kTrows, acc, Zb, ch0, ch1, false);    // W = T^T Z
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < C::CB; ++j) blk[i][j] -= acc[i][j];
+    put_blk(Zb, blk);                                // Top -= W, handed on
+    __syncthreads();
+    store_strip(Zb, top0);
+    __syncthreads();
+    if (tid == 0) st_release(done, p - args.first_role + 1);
+    put_blk(Zb, acc);
+    __syncthreads();
+    get_blk(Buf, blk);
+    gemm(ctx, kVcols, blk, Zb, ch0, ch1, true);     // A_p -= V W
+    put_blk(Buf, blk);
+    __syncthreads();
+    store_strip(Buf, ctx.row0);
 }
 
 template <typename T, int B, int WW = WCfg<T>::W>
 size_t upd_full_smem() {
     using C = UCfg<T, B, WW>;
-    return sizeof(T) * (2 * (size_t)C::LDB * C::W + 2 * (size_t)C::KC * C::LDC);
+    return sizeof(T) * (2 * (size_t)B * C::LDW + 2 * (size_t)C::KC * C::LDC);
 }
 
 template <typename T, int LAYOUT, int B, typename CT = T, int WW = WCfg<T>::W>
@@ -628,17 +676,28 @@ int launch_upd_full(T *dA, int64_t lda, int64_t n, int pr, int pc, int P, const 
     }
     const int64_t ncols = n - (int64_t)(pc + 1) * B;
     if (ncols <= 0) return AVS_SUCCESS;
-    UpdFullArgs a{dA, lda, n, B, pr, pc, P, w.tfull, w.sA, w.sTfull, first_role};
-    const unsigned gx = (unsigned)((ncols + C::W - 1) / C::W);
-    update_full_kernel<T, LAYOUT, B, CT, WW><<<dim3(gx, w.batch > 0 ? w.batch : 1), kWNT, smem, s>>>(a);
+    const int nstrip = (int)((ncols + C::W - 1) / C::W);
+    const int batch = w.batch > 0 ? w.batch : 1;
+    // ticket and strip counters take the place of the panel's 16 x 16 T blocks,
+    // which the T build has read
+    const int64_t sFl = w.sTblk * (int64_t)(sizeof(T) / sizeof(int));
+    if (sizeof(int) * (size_t)(1 + nstrip) > sizeof(T) * (size_t)(P - first_role) * (B / kWIB) * kWIB * kWIB)
+        return AVS_ERR_INTERNAL;
+    int *flags = reinterpret_cast<int *>(w.tblk);
+    if (batch > 1)
+        AVS_CUDA_TRY(cudaMemset2DAsync(flags, sizeof(int) * (size_t)sFl, 0, sizeof(int) * (size_t)(1 + nstrip), batch, s));
+    else
+        AVS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)(1 + nstrip), s));
+    UpdFullArgs a{dA, lda, n, B, pr, pc, P, w.tfull, w.sA, w.sTfull, first_role, nstrip, flags, sFl, w.err};
+    update_full_kernel<T, LAYOUT, B, CT, WW><<<dim3((unsigned)nstrip * (P - first_role), batch), kWNT, smem, s>>>(a);
     AVS_CUDA_TRY(cudaGetLastError());
     return AVS_SUCCESS;
 }
 
 // FP64 tiles: the update in FP64, or in double-float when the work asks for it.
 // FP64 tiles: 32-column strips, or 16 when the 32-column strips (times the
-// batch) would not give every SM two CTAs -- a strip runs its P tiles in
-// sequence, so the strips are the launch's only parallelism.  A column's values
+// batch) would not give every SM two CTAs: a strip's tiles follow one another
+// through W, which takes half as long for half the columns.  A column's values
 // do not depend on the strip width (columns are independent, the sums run in
 // the same order), so single and batched calls agree bit for bit.
 template <typename T, int LAYOUT, int B>
