@@ -211,10 +211,9 @@ __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 
 template <typename S>
-__device__ __forceinline__ typename ChaseAr<S>::V warp_sum_s(typename ChaseAr<S>::V v) {
-    using Ar = ChaseAr<S>;
+__device__ __forceinline__ typename ChaseAr<S>::Acc warp_sum_acc(typename ChaseAr<S>::Acc v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = Ar::add(v, Ar::shfl_xor(v, o));
+    for (int o = 16; o > 0; o >>= 1) v = ChaseRefl<S>::merge_xor(v, o);
     return v;
 }
 
@@ -245,14 +244,19 @@ __device__ __forceinline__ void warp_reflector(const BandT<S> &A, bool row, int6
         const int i = lane + 32 * t;
         if (i >= 1 && i < L) Ar::acc_add(acc, x[t], x[t]);
     }
-    const V s = warp_sum_s<S>(Ar::acc_value(acc));
+    const typename Ar::Acc s = warp_sum_acc<S>(acc);
     const V alpha = Ar::shfl(x[0], 0);
     V tau = Ar::zero(), beta = alpha, scal = Ar::zero();
-    if (Ar::gt0(s)) {
-        const V nrm = Ar::sqrt(Ar::fma(alpha, alpha, s));
-        beta = Ar::ge0(alpha) ? Ar::neg(nrm) : nrm;
-        tau = Ar::mul(Ar::sub(beta, alpha), Ar::rcp(beta));
-        scal = Ar::rcp(Ar::sub(alpha, beta));
+    if (ChaseRefl<S>::positive(s)) {
+        // tau = 1 + |alpha| / ||x||, 1 / (alpha - beta) = sign(alpha) / (|alpha| + ||x||)
+        V rn, nrm;
+        rsqrt_sqrt(ChaseRefl<S>::norm2(s, alpha), rn, nrm);
+        const bool pos = Ar::ge0(alpha);
+        const V aa = pos ? alpha : Ar::neg(alpha);
+        beta = pos ? Ar::neg(nrm) : nrm;
+        tau = Ar::fma(aa, rn, Ar::one());
+        const V inv = rcp_est(Ar::add(aa, nrm));
+        scal = pos ? inv : Ar::neg(inv);
     }
 #pragma unroll
     for (int t = 0; t < PER; ++t) {
@@ -400,7 +404,7 @@ __global__ void __launch_bounds__(ChaseCfg<BW, CC, NTT>::NT, ChaseCfg<BW, CC, NT
                             const int ri = lane + 32 * t;
                             if (ri < L) Ar::acc_add(acc, sv[ri], vals[k][t]);
                         }
-                        const V w = Ar::mul(warp_sum_s<S>(Ar::acc_value(acc)), tau);
+                        const V w = Ar::mul(Ar::acc_value(warp_sum_acc<S>(acc)), tau);
                         if (c <= cend) {
 #pragma unroll
                             for (int t = 0; t < Cfg::RPL; ++t) {

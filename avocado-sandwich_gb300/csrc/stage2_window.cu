@@ -55,7 +55,6 @@
 
 #include "avs_common.cuh"
 #include "chase_ar.cuh"
-#include "reflect.cuh"
 
 namespace avs {
 namespace {
@@ -158,45 +157,6 @@ __device__ __forceinline__ void mbar_wait(unsigned long long *m, unsigned parity
         if ((it & 63) == 63 && wait_over(it, t0, fail, err)) return;
 }
 
-// The chase's arithmetic beyond ChaseAr: merging dot-product accumulators
-// without renormalising between the levels of a butterfly, the reflector's
-// scalars, and a - w u with one renormalisation.
-template <typename S>
-struct WinAr;
-template <>
-struct WinAr<df64> {
-    using Acc = ChaseAr<df64>::Acc;
-    static __device__ __forceinline__ Acc merge_xor(Acc a, int o) {
-        const df64 t = two_sum(a.s, __shfl_xor_sync(0xffffffffu, a.s, o));
-        return Acc{t.hi, __fadd_rn(t.lo, __fadd_rn(a.c, __shfl_xor_sync(0xffffffffu, a.c, o)))};
-    }
-    static __device__ __forceinline__ bool positive(Acc s) {
-        const df64 v = two_sum(s.s, s.c);
-        return v.hi > 0.0f;
-    }
-    // s + alpha^2
-    static __device__ __forceinline__ df64 norm2(Acc s, df64 al) {
-        const float p = __fmul_rn(al.hi, al.hi);
-        const float e = __fmaf_rn(2.0f * al.hi, al.lo, __fmaf_rn(al.hi, al.hi, -p));
-        const df64 t = two_sum(p, s.s);
-        return fast_two_sum(t.hi, __fadd_rn(t.lo, __fadd_rn(e, s.c)));
-    }
-    static __device__ __forceinline__ df64 sub_mul(df64 a, df64 w, df64 u) {
-        const float p = __fmul_rn(w.hi, u.hi);
-        const float e = __fmaf_rn(w.lo, u.hi, __fmaf_rn(w.hi, u.lo, __fmaf_rn(w.hi, u.hi, -p)));
-        const df64 t = two_sum(a.hi, -p);
-        return fast_two_sum(t.hi, __fadd_rn(t.lo, __fsub_rn(a.lo, e)));
-    }
-};
-template <>
-struct WinAr<double> {
-    using Acc = double;
-    static __device__ __forceinline__ Acc merge_xor(Acc a, int o) { return a + __shfl_xor_sync(0xffffffffu, a, o); }
-    static __device__ __forceinline__ bool positive(Acc s) { return s > 0.0; }
-    static __device__ __forceinline__ double norm2(Acc s, double al) { return ::fma(al, al, s); }
-    static __device__ __forceinline__ double sub_mul(double a, double w, double u) { return ::fma(-w, u, a); }
-};
-
 constexpr int kAllDone = 1 << 30;
 
 // Per-sweep op geometry.
@@ -221,7 +181,7 @@ __global__ void __launch_bounds__(WinCfg<BW, G, H>::NT, 1)
                      int *retired_base, int64_t sRet, int *err) {
     using Cfg = WinCfg<BW, G, H>;
     using Ar = ChaseAr<S>;
-    using Wa = WinAr<S>;
+    using Wa = ChaseRefl<S>;
     using V = typename Ar::V;
     using St = typename Ar::St;
     static_assert(sizeof(St) == 8 && sizeof(V) == 8, "8-byte band elements");
