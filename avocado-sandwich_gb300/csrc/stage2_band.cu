@@ -24,10 +24,16 @@
 // result is bit-identical to running the sweeps one after another.
 //
 // One thread-block cluster of C CTAs owns a sweep.  Every CTA loads the
-// panel and factors it itself (same data, same code: the same bits), builds
-// the compact-WY factor T (LAPACK xLARFT, forward, columnwise), then applies
-// the block reflector to its share of the rows (R op) or columns (L op) as
-// two small GEMMs on the FP32 (or FP64) pipe, operands in shared memory.
+// panel and factors it itself (same data, same code: the same bits) and applies
+// the block reflector to its share of the rows (R op) or columns (L op): W = A V (Z
+// = V^T A), Y = W T (T^T Z) by forward substitution from the Gram matrix that the
+// factorisation leaves (T^-1 = diag(1/tau) + striu(V^T V), one thread per row or
+// column), A -= Y V^T (V Y); operands in shared memory, on the FP32 (or FP64) pipe.
+// What bounds it: the latency of an op along the sweep wavefront (the panel's 16
+// reflectors are half of it: 12 to 15 k of about 20 to 37 k cycles).  Measured (GB300,
+// the whole stage, before: every column's work inside the panel's chain, T formed
+// by one warp, one reflector per thread in the first product): band 64 n = 1024 3.3
+// -> 2.4 ms, 128 n = 4096 15.4 -> 11.6 ms, 256 n = 16384 115 -> 84 ms.
 // The band is in compact storage A(r, c) at AB[(r - c + 2B) + c * ldab],
 // ldab = 3B + 1 (band_ku / band_ldab): rows c-2B .. c+B of column c (band,
 // upper bulge up to 2B-1, lower bulge up to B-1), laid out so that every
@@ -42,6 +48,7 @@
 #include <type_traits>
 
 #include "avs_common.cuh"
+#include "reflect.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -61,10 +68,11 @@ struct BandCfg {
     static constexpr int LDA_L = B + 4;           // L op staging: column stride (B rows)
     static constexpr int ASZ = (B * LDA_R > RPC * LDA_L) ? B * LDA_R : RPC * LDA_L;
     static constexpr int LDW = RPC + 4;           // W / Y buffer: [k][r or cc]
-    // GEMM 1 / Y: 4 rows (R op) or 4 columns (L op) x KPT reflectors per thread
+    // GEMM 1: 4 rows (R op) or 4 columns (L op) x 4 reflectors per thread, the sum
+    // over the band's width split KS ways (partial W joined by the substitution)
     static constexpr int NG4 = RPC / 4;
-    static constexpr int NKG = NT / NG4;
-    static constexpr int KPT = (T >= NKG) ? T / NKG : 1;
+    static constexpr int KS = NT / (NG4 * (T / 4));
+    static constexpr int BK = B / KS;
     // GEMM 2, R op: 4 rows x CPT2R columns per thread
     static constexpr int NCG_R = NT / NG4;
     static constexpr int CPT2R = B / NCG_R;
@@ -73,12 +81,12 @@ struct BandCfg {
     static constexpr int NCG_L = NT / NIG;
     static constexpr int CPT2L = RPC / NCG_L;
     static_assert(B % 32 == 0 && T <= 32 && T < B && B % T == 0, "band stage shape");
-    static_assert(NT % NG4 == 0 && (T >= NKG ? T % NKG == 0 : true), "GEMM 1 split");
+    static_assert(KS >= 1 && KS * NG4 * (T / 4) == NT && BK % 4 == 0 && RPC <= NT, "GEMM 1 split");
     static_assert(CPT2R % 4 == 0 && CPT2R * NCG_R == B, "R op GEMM 2 split");
     static_assert(NT % NIG == 0 && CPT2L % 4 == 0 && CPT2L * NCG_L == RPC, "L op GEMM 2 split");
     template <typename R>
     static constexpr size_t smem_bytes() {
-        return sizeof(R) * ((size_t)T * LDP + ASZ + (size_t)T * LDW + (size_t)T * (T + 1) * 2 + T);
+        return sizeof(R) * ((size_t)T * LDP + ASZ + (size_t)KS * T * LDW + (size_t)T * (T + 1) + T);
     }
 };
 
@@ -173,24 +181,29 @@ __device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.a
 
 // Scalars of the LAPACK-convention reflector of x = (alpha, x2) with s =
 // ||x2||^2 > 0: beta = -sign(alpha) ||x||, tau = (beta - alpha) / beta =
-// 1 + |alpha| / ||x||, scal = 1 / (alpha - beta).  FP32: the norm from the
-// hardware reciprocal square root with one Newton step (about 0.5 ulp), the
-// reciprocals correctly rounded -- a short dependent chain on the panel's
-// critical path; FP64: divisions and sqrt.
+// 1 + |alpha| / ||x||, scal = 1 / (alpha - beta): the hardware estimates with one
+// Newton step each in FP32 (within an ulp), reflect.cuh's in FP64 -- a short
+// dependent chain on the panel's critical path.
 __device__ __forceinline__ void reflector_scalars(float alpha, float s, float &tau, float &beta, float &scal) {
     const float a2s = fmaf(alpha, alpha, s);
-    const float r = rsqrtf(a2s);
-    float nrm = a2s * r;
-    nrm = fmaf(0.5f * r, fmaf(-nrm, nrm, a2s), nrm);
+    const float r = rsqrt_hw(a2s);
+    const float t = a2s * r;
+    const float h = 0.5f * fmaf(-t, r, 1.0f);
+    const float nrm = fmaf(t, h, t), rn = fmaf(r, h, r);
+    const float u = fabsf(alpha) + nrm;
+    float z = rcp_hw(u);
+    z = fmaf(z, fmaf(-u, z, 1.0f), z);
     beta = alpha >= 0.0f ? -nrm : nrm;
-    scal = __frcp_rn(alpha - beta);
-    tau = fmaf(fabsf(alpha), __frcp_rn(nrm), 1.0f);
+    scal = alpha >= 0.0f ? z : -z;
+    tau = fmaf(fabsf(alpha), rn, 1.0f);
 }
 __device__ __forceinline__ void reflector_scalars(double alpha, double s, double &tau, double &beta, double &scal) {
-    const double nrm = sqrt(fma(alpha, alpha, s));
+    double rn, nrm;
+    rsqrt_sqrt(fma(alpha, alpha, s), rn, nrm);
     beta = alpha >= 0.0 ? -nrm : nrm;
-    tau = (beta - alpha) / beta;
-    scal = 1.0 / (alpha - beta);
+    tau = fma(fabs(alpha), rn, 1.0);
+    const double z = rcp_est(fabs(alpha) + nrm);
+    scal = alpha >= 0.0 ? z : -z;
 }
 
 // Householder QR of the panel P (B rows x T columns, column k at P + k*LDP,
@@ -199,8 +212,11 @@ __device__ __forceinline__ void reflector_scalars(double alpha, double s, double
 // tau = (beta - alpha) / beta; tau = 0 when the part below the diagonal is
 // zero.  On return P holds R on and above the diagonal and V below it;
 // s_tau the taus; gram[j * (T+1) + k] = v_j^T v_k for j < k.  Warp w owns
-// columns w, w + NW, ...; lane l rows l, l + 32, ...; one barrier per
-// reflector.
+// columns w, w + NW, ...; lane l rows l, l + 32, ....  The owner of column k+1
+// applies H_k to that column first, forms H_{k+1}, publishes it (arrives at a named
+// barrier) and only then applies H_k to its other columns: a step's chain is one
+// dot product, one norm and the scalars (with the other columns' work on it, the
+// panel took 16.4 k cycles at B = 128).
 template <typename R, int B, int T, int NW>
 __device__ __forceinline__ void panel_qr(R *P, R *s_tau, R *gram) {
     constexpr int LDP = B + 4;
@@ -214,81 +230,108 @@ __device__ __forceinline__ void panel_qr(R *P, R *s_tau, R *gram) {
 #pragma unroll
         for (int u = 0; u < RPL; ++u) x[jj][u] = (j < T) ? P[j * LDP + lane + 32 * u] : R(0);
     }
+    // H_k of column k in slot JK of its owner
+    auto generate = [&](auto slot_c, int k) {
+        constexpr int JK = decltype(slot_c)::value;
+        R s = R(0);
 #pragma unroll
-    for (int k = 0; k < T; ++k) {
-        const int ow = k % NW, jk = k / NW;
-        if (w == ow) {
-            R s = R(0);
-#pragma unroll
-            for (int u = 0; u < RPL; ++u) {
-                const int i = lane + 32 * u;
-                if (i > k) s = fma(x[jk][u], x[jk][u], s);
-            }
-            s = warp_sum(s);
-            const R alpha = __shfl_sync(0xffffffffu, x[jk][k / 32], k % 32);
-            R tau = R(0), beta = alpha, scal = R(0);
-            if (s > R(0)) reflector_scalars(alpha, s, tau, beta, scal);
-#pragma unroll
-            for (int u = 0; u < RPL; ++u) {
-                const int i = lane + 32 * u;
-                if (i > k) x[jk][u] *= scal;
-                else if (i == k) x[jk][u] = beta;
-                P[k * LDP + i] = x[jk][u];
-            }
-            if (lane == 0) s_tau[k] = tau;
+        for (int u = 0; u < RPL; ++u) {
+            const int i = lane + 32 * u;
+            if (i > k) s = fma(x[JK][u], x[JK][u], s);
         }
-        __syncthreads();
-        const R tau = s_tau[k];
-        R v[RPL];
+        s = warp_sum(s);
+        const R alpha = __shfl_sync(0xffffffffu, x[JK][0], k);  // T <= 32: row k is in slot 0
+        R tau = R(0), beta = alpha, scal = R(0);
+        if (s > R(0)) reflector_scalars(alpha, s, tau, beta, scal);
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+            const int i = lane + 32 * u;
+            if (i > k) x[JK][u] *= scal;
+            else if (i == k) x[JK][u] = beta;
+            P[k * LDP + i] = x[JK][u];
+        }
+        if (lane == 0) s_tau[k] = tau;
+        __syncwarp();
+    };
+    R v[RPL], tau;
+    // H_k (v, tau) to the column in slot JJ: right of k the apply, left of k the Gram
+    // entry v_j^T v_k (x holds v_j below its diagonal)
+    auto apply = [&](auto slot_c, int j, int k) {
+        constexpr int JJ = decltype(slot_c)::value;
+        R d = R(0);
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) d = fma(v[u], x[JJ][u], d);
+        d = warp_sum(d);
+        if (j > k) {
+            const R t = d * tau;
+#pragma unroll
+            for (int u = 0; u < RPL; ++u) x[JJ][u] = fma(-t, v[u], x[JJ][u]);
+        } else if (lane == 0) {
+            gram[j * (T + 1) + k] = d;
+        }
+    };
+    auto slots = [&](auto f) {  // f for every column slot of the warp
+        f(std::integral_constant<int, 0>{});
+        if constexpr (CPW > 1) f(std::integral_constant<int, 1>{});
+        if constexpr (CPW > 2) f(std::integral_constant<int, 2>{});
+        if constexpr (CPW > 3) f(std::integral_constant<int, 3>{});
+    };
+    static_assert(CPW <= 4 && T % NW == 0, "panel columns");
+    // barriers 1 and 2 in turn: column k's owner arrives, the other warps wait
+    auto publish = [&](int k) {
+        asm volatile("bar.arrive %0, %1;" ::"r"(1 + (k & 1)), "n"(32 * NW) : "memory");
+    };
+    if (w == 0) {
+        generate(std::integral_constant<int, 0>{}, 0);
+        publish(0);
+    }
+#pragma unroll 1
+    for (int k = 0; k < T; ++k) {
+        if (w != k % NW) asm volatile("bar.sync %0, %1;" ::"r"(1 + (k & 1)), "n"(32 * NW) : "memory");
+        tau = s_tau[k];
 #pragma unroll
         for (int u = 0; u < RPL; ++u) {
             const int i = lane + 32 * u;
             v[u] = (i > k) ? P[k * LDP + i] : (i == k ? R(1) : R(0));
         }
-        // columns right of k get H_k (column k+1's slot first: the critical path);
-        // columns left of k give the Gram entries v_j^T v_k
-#pragma unroll
-        for (int jj0 = 0; jj0 < CPW; ++jj0) {
-            const int jj = (jj0 + ((k + 1) / NW)) % CPW;
-            const int j = w + NW * jj;
-            if (j < T && j != k) {
-                R d = R(0);
-#pragma unroll
-                for (int u = 0; u < RPL; ++u) d = fma(v[u], x[jj][u], d);
-                d = warp_sum(d);
-                if (j > k) {
-                    const R t = d * tau;
-#pragma unroll
-                    for (int u = 0; u < RPL; ++u) x[jj][u] = fma(-t, v[u], x[jj][u]);
-                } else if (lane == 0) {
-                    gram[j * (T + 1) + k] = d;  // x holds v_j below its diagonal
+        const int kn = k + 1;
+        const bool next = kn < T && w == kn % NW;
+        if (next) {
+            slots([&](auto sl) {
+                if (kn / NW == decltype(sl)::value) {
+                    apply(sl, kn, k);
+                    generate(sl, kn);
                 }
-            }
+            });
+            publish(kn);
         }
+        slots([&](auto sl) {
+            const int j = w + NW * decltype(sl)::value;
+            if (j != k && !(next && j == kn)) apply(sl, j, k);
+        });
     }
 }
 
-// Compact-WY factor of the panel's reflectors (LAPACK xLARFT, forward,
-// columnwise): Tm[i*(T+1)+k], upper triangular, T[k][k] = tau_k, T[0:k, k] =
-// -tau_k T[0:k, 0:k] (V^T v_k)[0:k].  Warp 0, lane i builds row i.
-template <typename R, int T>
-__device__ __forceinline__ void build_t(const R *s_tau, const R *gram, R *Tm) {
-    const int i = threadIdx.x;
-    if (i >= 32) return;
-    R row[T];
+// Y from the partial W of one row (R op: Y = W T) or column (L op: Y = T^T Z): the
+// same forward substitution y_k = tau_k (w_k - sum_{l<k} G_lk y_l).  Wy: KS
+// partial sums [k][LDW] in, Y in the first on return; one thread per row.
+template <typename R, int T, int KS, int LDW>
+__device__ __forceinline__ void substitute(const R *s_tau, const R *gram, R *Wy, int row) {
+    R w[T];
 #pragma unroll
     for (int k = 0; k < T; ++k) {
-        const R tk = s_tau[k];
-        R acc = R(0);
+        w[k] = Wy[k * LDW + row];
 #pragma unroll
-        for (int l = 0; l < k; ++l)
-            if (l >= i) acc = fma(row[l], gram[l * (T + 1) + k], acc);
-        row[k] = (i < k) ? -tk * acc : (i == k ? tk : R(0));
+        for (int q = 1; q < KS; ++q) w[k] += Wy[(q * T + k) * LDW + row];
     }
-    if (i < T) {
 #pragma unroll
-        for (int k = 0; k < T; ++k) Tm[i * (T + 1) + k] = row[k];
+    for (int k = 0; k < T; ++k) {
+        w[k] = s_tau[k] * w[k];
+#pragma unroll
+        for (int m = k + 1; m < T; ++m) w[m] = fma(-gram[k * (T + 1) + m], w[k], w[m]);
     }
+#pragma unroll
+    for (int k = 0; k < T; ++k) Wy[k * LDW + row] = w[k];
 }
 
 template <int B, int T, typename R, int C>
@@ -301,9 +344,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *P = reinterpret_cast<R *>(smem_raw);  // [T][LDP] panel (QR form), then V
     R *As = P + T * LDP;                      // apply staging
-    R *Wy = As + Cfg::ASZ;                    // [T][LDW]: W / Z, then Y
-    R *Tm = Wy + T * LDW;                     // [T][T+1]
-    R *gram = Tm + T * (T + 1);               // [T][T+1]
+    R *Wy = As + Cfg::ASZ;                    // [KS][T][LDW]: partial W / Z, then Y in the first
+    R *gram = Wy + Cfg::KS * T * LDW;         // [T][T+1]
     R *s_tau = gram + T * (T + 1);            // [T]
     __shared__ int s_j;
     cg::cluster_group cluster = cg::this_cluster();
@@ -372,13 +414,10 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                 cl_arrive();  // done reading the pivot rows
                 panel_qr<R, B, T, NW>(P, s_tau, gram);
                 __syncthreads();
-                build_t<R, T>(s_tau, gram, Tm);
-                cl_wait();  // every CTA has read the pivot rows: CTA 0 stores L and zeros
-                if (q == 0) {
-                    for (int idx = tid; idx < T * L; idx += NT) {
-                        const int k = idx % T, j = idx / T;
-                        *at(rho + k, c0 + j) = (j <= k) ? P[k * LDP + j] : R(0);
-                    }
+                cl_wait();  // every CTA has read the pivot rows: L and zeros, a share per CTA
+                for (int idx = q * (T * B / C) + tid; idx < (q + 1) * (T * B / C); idx += NT) {
+                    const int k = idx % T, j = idx / T;
+                    if (j < L) *at(rho + k, c0 + j) = (j <= k) ? P[k * LDP + j] : R(0);
                 }
                 __syncthreads();
                 for (int idx = tid; idx < T * T; idx += NT) {  // explicit V: unit diagonal, zeros above
@@ -386,66 +425,35 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                     if (i <= k) P[k * LDP + i] = (i == k) ? R(1) : R(0);
                 }
                 __syncthreads();
-                // W = A V: thread = 4 rows x KPT reflectors
+                // W = A V: thread = 4 rows x 4 reflectors, BK columns of the sum
                 {
-                    constexpr int KPT = Cfg::KPT;
-                    const int g = tid % Cfg::NG4, kg = tid / Cfg::NG4;
-                    const int k0 = kg * KPT;
-                    if (k0 < T) {
-                        R acc[KPT][4];
+                    const int g = tid % Cfg::NG4, k0 = (tid / Cfg::NG4) % (T / 4) * 4, ks = tid / (Cfg::NG4 * (T / 4));
+                    R acc[4][4];
 #pragma unroll
-                        for (int a = 0; a < KPT; ++a)
+                    for (int a = 0; a < 4; ++a)
 #pragma unroll
-                            for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = R(0);
+                        for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = R(0);
 #pragma unroll 2
-                        for (int c = 0; c < B; c += 4) {
-                            R a4[4][4], v4[KPT][4];
+                    for (int c = ks * Cfg::BK; c < (ks + 1) * Cfg::BK; c += 4) {
+                        R a4[4][4], v4[4][4];
 #pragma unroll
-                            for (int cc = 0; cc < 4; ++cc) Vec4<R>::ld(As + (c + cc) * Cfg::LDA_R + 4 * g, a4[cc]);
+                        for (int cc = 0; cc < 4; ++cc) Vec4<R>::ld(As + (c + cc) * Cfg::LDA_R + 4 * g, a4[cc]);
 #pragma unroll
-                            for (int kk = 0; kk < KPT; ++kk) Vec4<R>::ld(P + (k0 + kk) * LDP + c, v4[kk]);
+                        for (int kk = 0; kk < 4; ++kk) Vec4<R>::ld(P + (k0 + kk) * LDP + c, v4[kk]);
 #pragma unroll
-                            for (int kk = 0; kk < KPT; ++kk)
+                        for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                                for (int cc = 0; cc < 4; ++cc)
+                            for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-                                    for (int rr = 0; rr < 4; ++rr)
-                                        acc[kk][rr] = fma(a4[cc][rr], v4[kk][cc], acc[kk][rr]);
-                        }
-#pragma unroll
-                        for (int kk = 0; kk < KPT; ++kk)
-#pragma unroll
-                            for (int rr = 0; rr < 4; ++rr) Wy[(k0 + kk) * LDW + 4 * g + rr] = acc[kk][rr];
+                                for (int rr = 0; rr < 4; ++rr) acc[kk][rr] = fma(a4[cc][rr], v4[kk][cc], acc[kk][rr]);
                     }
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                        for (int rr = 0; rr < 4; ++rr) Wy[(ks * T + k0 + kk) * LDW + 4 * g + rr] = acc[kk][rr];
                 }
                 __syncthreads();
-                // Y = W T (all reads before the barrier, then in place)
-                {
-                    constexpr int KPT = Cfg::KPT;
-                    const int g = tid % Cfg::NG4, kg = tid / Cfg::NG4;
-                    const int k0 = kg * KPT;
-                    R y[KPT][4];
-                    if (k0 < T) {
-#pragma unroll
-                        for (int kk = 0; kk < KPT; ++kk) {
-                            const int k = k0 + kk;
-#pragma unroll
-                            for (int rr = 0; rr < 4; ++rr) y[kk][rr] = R(0);
-                            for (int l = 0; l <= k; ++l) {
-                                const R t = Tm[l * (T + 1) + k];
-#pragma unroll
-                                for (int rr = 0; rr < 4; ++rr) y[kk][rr] = fma(Wy[l * LDW + 4 * g + rr], t, y[kk][rr]);
-                            }
-                        }
-                    }
-                    __syncthreads();
-                    if (k0 < T) {
-#pragma unroll
-                        for (int kk = 0; kk < KPT; ++kk)
-#pragma unroll
-                            for (int rr = 0; rr < 4; ++rr) Wy[(k0 + kk) * LDW + 4 * g + rr] = y[kk][rr];
-                    }
-                }
+                if (tid < RPC) substitute<R, T, Cfg::KS, LDW>(s_tau, gram, Wy, tid);
                 __syncthreads();
                 // A -= Y V^T: thread = 4 rows x CPT2R columns; straight to global
                 {
@@ -531,13 +539,10 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                 cl_arrive();  // done reading the pivot columns
                 panel_qr<R, B, T, NW>(P, s_tau, gram);
                 __syncthreads();
-                build_t<R, T>(s_tau, gram, Tm);
-                cl_wait();  // CTA 0 stores R and zeros
-                if (q == 0) {
-                    for (int idx = tid; idx < Tc * L; idx += NT) {
-                        const int i = idx % L, k = idx / L;
-                        *at(c0 + i, c0 + k) = (i <= k) ? P[k * LDP + i] : R(0);
-                    }
+                cl_wait();  // R and zeros, a share per CTA
+                for (int idx = q * (T * B / C) + tid; idx < (q + 1) * (T * B / C); idx += NT) {
+                    const int i = idx % B, k = idx / B;
+                    if (i < L && k < Tc) *at(c0 + i, c0 + k) = (i <= k) ? P[k * LDP + i] : R(0);
                 }
                 __syncthreads();
                 for (int idx = tid; idx < T * T; idx += NT) {
@@ -546,68 +551,36 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                 }
                 __syncthreads();
                 // Z = V^T A: thread = 4 columns (g + cc NG4: lanes one column apart, so
-                // their column reads spread over the banks) x KPT reflectors
+                // their column reads spread over the banks) x 4 reflectors, BK rows of the sum
                 {
-                    constexpr int KPT = Cfg::KPT;
-                    const int g = tid % Cfg::NG4, kg = tid / Cfg::NG4;
-                    const int k0 = kg * KPT;
-                    if (k0 < T) {
-                        R acc[KPT][4];
+                    const int g = tid % Cfg::NG4, k0 = (tid / Cfg::NG4) % (T / 4) * 4, ks = tid / (Cfg::NG4 * (T / 4));
+                    R acc[4][4];
 #pragma unroll
-                        for (int a = 0; a < KPT; ++a)
+                    for (int a = 0; a < 4; ++a)
 #pragma unroll
-                            for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = R(0);
+                        for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = R(0);
 #pragma unroll 2
-                        for (int i = 0; i < B; i += 4) {
-                            R a4[4][4], v4[KPT][4];
+                    for (int i = ks * Cfg::BK; i < (ks + 1) * Cfg::BK; i += 4) {
+                        R a4[4][4], v4[4][4];
+#pragma unroll
+                        for (int cc = 0; cc < 4; ++cc)
+                            Vec4<R>::ld(As + (g + cc * Cfg::NG4) * Cfg::LDA_L + i, a4[cc]);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) Vec4<R>::ld(P + (k0 + kk) * LDP + i, v4[kk]);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
                             for (int cc = 0; cc < 4; ++cc)
-                                Vec4<R>::ld(As + (g + cc * Cfg::NG4) * Cfg::LDA_L + i, a4[cc]);
 #pragma unroll
-                            for (int kk = 0; kk < KPT; ++kk) Vec4<R>::ld(P + (k0 + kk) * LDP + i, v4[kk]);
-#pragma unroll
-                            for (int kk = 0; kk < KPT; ++kk)
-#pragma unroll
-                                for (int cc = 0; cc < 4; ++cc)
-#pragma unroll
-                                    for (int ii = 0; ii < 4; ++ii)
-                                        acc[kk][cc] = fma(v4[kk][ii], a4[cc][ii], acc[kk][cc]);
-                        }
-#pragma unroll
-                        for (int kk = 0; kk < KPT; ++kk)
-#pragma unroll
-                            for (int cc = 0; cc < 4; ++cc) Wy[(k0 + kk) * LDW + g + cc * Cfg::NG4] = acc[kk][cc];
+                                for (int ii = 0; ii < 4; ++ii) acc[kk][cc] = fma(v4[kk][ii], a4[cc][ii], acc[kk][cc]);
                     }
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                        for (int cc = 0; cc < 4; ++cc) Wy[(ks * T + k0 + kk) * LDW + g + cc * Cfg::NG4] = acc[kk][cc];
                 }
                 __syncthreads();
-                // Y = T^T Z
-                {
-                    constexpr int KPT = Cfg::KPT;
-                    const int g = tid % Cfg::NG4, kg = tid / Cfg::NG4;
-                    const int k0 = kg * KPT;
-                    R y[KPT][4];
-                    if (k0 < T) {
-#pragma unroll
-                        for (int kk = 0; kk < KPT; ++kk) {
-                            const int k = k0 + kk;
-#pragma unroll
-                            for (int cc = 0; cc < 4; ++cc) y[kk][cc] = R(0);
-                            for (int l = 0; l <= k; ++l) {
-                                const R t = Tm[l * (T + 1) + k];
-#pragma unroll
-                                for (int cc = 0; cc < 4; ++cc)
-                                    y[kk][cc] = fma(t, Wy[l * LDW + g + cc * Cfg::NG4], y[kk][cc]);
-                            }
-                        }
-                    }
-                    __syncthreads();
-                    if (k0 < T) {
-#pragma unroll
-                        for (int kk = 0; kk < KPT; ++kk)
-#pragma unroll
-                            for (int cc = 0; cc < 4; ++cc) Wy[(k0 + kk) * LDW + g + cc * Cfg::NG4] = y[kk][cc];
-                    }
-                }
+                if (tid < RPC) substitute<R, T, Cfg::KS, LDW>(s_tau, gram, Wy, tid);
                 __syncthreads();
                 // A -= V Y: thread = 4 rows x CPT2L columns; straight to global
                 {
