@@ -98,8 +98,6 @@ struct UpdateArgs {
 // f = tau / nu^2 = 1 / (n1 |nu|), inv = 1 / nu, beta = -sign(alpha) n1 (the new
 // diagonal); evaluated in double-float for FP32 tiles and rounded once, in FP64
 // for FP64 tiles (reflect.cuh: hardware estimates and one residual each).
-// mac / fin: products accumulated into Mac (double-float: the compensated
-// dot product of Ogita, Rump and Oishi) and the value of the accumulator.
 template <typename CT>
 struct PRefl {
     CT nu, tc, f, inv, beta, tau;
@@ -119,8 +117,7 @@ struct PSqPair {
     }
 };
 template <>
-struct PAr<float> : PSqPair {
-    using Mac = float;
+struct PAr<float> : PSqPair, MacAr<float> {
     static __device__ __forceinline__ Sq sq(float x) {
         const float p = __fmul_rn(x, x);
         return make_float2(p, __fmaf_rn(x, x, -p));
@@ -165,16 +162,10 @@ struct PAr<float> : PSqPair {
         o.beta = neg ? n1 : -n1;
         return o;
     }
-    static __device__ __forceinline__ Mac mac0() { return 0.0f; }
-    static __device__ __forceinline__ Mac mac_from(float x) { return x; }
-    static __device__ __forceinline__ void mac(Mac &a, float x, float y) { a = fmaf(x, y, a); }
-    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) { return a + b; }
-    static __device__ __forceinline__ float fin(Mac a) { return a; }
 };
 // FP64 tiles in double-float arithmetic (AVS_PREC_FP64X2)
 template <>
-struct PAr<dfx> : PSqPair {
-    using Mac = df64;
+struct PAr<dfx> : PSqPair, MacAr<dfx> {
     static __device__ __forceinline__ Sq sq(dfx v) {
         const df64 x = v.v;
         const float p = __fmul_rn(x.hi, x.hi);
@@ -203,27 +194,10 @@ struct PAr<dfx> : PSqPair {
         r.beta = dfx(neg ? n1 : df_neg(n1));
         return r;
     }
-    static __device__ __forceinline__ Mac mac0() { return df64{0.0f, 0.0f}; }
-    static __device__ __forceinline__ Mac mac_from(dfx x) { return x.v; }
-    static __device__ __forceinline__ void mac(Mac &a, dfx x, dfx y) {
-        const float p = __fmul_rn(x.v.hi, y.v.hi);
-        float ep = __fmaf_rn(x.v.hi, y.v.hi, -p);
-        ep = __fmaf_rn(x.v.hi, y.v.lo, ep);
-        ep = __fmaf_rn(x.v.lo, y.v.hi, ep);
-        const df64 t = two_sum(a.hi, p);
-        a.hi = t.hi;
-        a.lo = __fadd_rn(a.lo, __fadd_rn(t.lo, ep));
-    }
-    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) {
-        const df64 t = two_sum(a.hi, b.hi);
-        return df64{t.hi, __fadd_rn(t.lo, __fadd_rn(a.lo, b.lo))};
-    }
-    static __device__ __forceinline__ dfx fin(Mac a) { return dfx(two_sum(a.hi, a.lo)); }
 };
 template <>
-struct PAr<double> {
+struct PAr<double> : MacAr<double> {
     using Sq = double;
-    using Mac = double;
     static __device__ __forceinline__ Sq sq(double x) { return x * x; }
     static __device__ __forceinline__ Sq merge(Sq a, Sq b) { return a + b; }
     static __device__ __forceinline__ Sq merge_xor(Sq a, int o) { return a + __shfl_xor_sync(0xffffffffu, a, o); }
@@ -248,11 +222,6 @@ struct PAr<double> {
         r.beta = neg ? n1 : -n1;
         return r;
     }
-    static __device__ __forceinline__ Mac mac0() { return 0.0; }
-    static __device__ __forceinline__ Mac mac_from(double x) { return x; }
-    static __device__ __forceinline__ void mac(Mac &a, double x, double y) { a = fma(x, y, a); }
-    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) { return a + b; }
-    static __device__ __forceinline__ double fin(Mac a) { return a; }
 };
 
 // Warp shuffles and finiteness of the panel's compute types.

@@ -9,12 +9,10 @@
 //   GEQRT tile:  Z = Y0^T Top,          W = T0^T Z,  Top -= Y0 W
 //   TSQRT tile:  Z = Top + V_p^T A_p,   W = T_p^T Z, Top -= W, A_p -= V_p W
 //
-// tbuild_kernel forms T_p (b x b, upper triangular) from the 16 x 16 diagonal
-// blocks the panel kernel produced and the Gram matrix G = Y_p^T Y_p:
-// T[0:c0, J] = -T[0:c0, 0:c0] G[0:c0, J] T_JJ for the column blocks J (FP64
-// tiles; in double-float with the double-float updates); tbuild_f32_kernel
-// forms the same T for FP32 tiles with T's upper block triangle in shared
-// memory.
+// The T build forms T_p (b x b, upper triangular) from the 16 x 16 diagonal blocks
+// the panel kernel produced and the Gram matrix G = Y_p^T Y_p: by doubling
+// (gram_kernel, tdouble_kernel), or column block by column block, T[0:c0, J] =
+// -T[0:c0, 0:c0] G[0:c0, J] T_JJ (tbuild_kernel: 8-byte tiles of 256).
 //
 // update_full_kernel: one CTA per (tile, column strip).  Only W and the strip of
 // the top tile row pass from tile to tile (W_p needs Top after tile p-1), so
@@ -64,7 +62,7 @@ struct TBuildArgs {
 };
 
 // ---------------------------------------------------------------------------
-// T build.  One CTA per tile.
+// T build of 8-byte tiles of 256.  One CTA per tile.
 template <typename T, int LAYOUT, typename CT = T>
 __global__ void __launch_bounds__(kWNT) tbuild_kernel(TBuildArgs args) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -184,174 +182,208 @@ __global__ void __launch_bounds__(kWNT) tbuild_kernel(TBuildArgs args) {
 }
 
 // ---------------------------------------------------------------------------
-// T build in shared memory (FP32 tiles).  One CTA per tile, the same T as
-// tbuild_kernel with T's upper block triangle held in shared memory, packed by
-// 16-column blocks (column block J: rows 0 .. 16(J+1), column-major, at
-// offset 256 J (J+1) / 2):
-//   1. the Gram blocks G_IJ = Y_I^T Y_J (I < J) in two passes over the tile's
-//      rows (8 x 8 output tiles per thread, rows of Y staged 32 at a time with
-//      the next chunk's loads in flight during the current chunk's products),
-//      written straight into their places in the packed T;
-//   2. the diagonal blocks T_JJ from the panel;
-//   3. column blocks J = 1.. in order: H = G[0:c0, J] T_JJ, then
-//      T[0:c0, J] = -T[0:c0, 0:c0] H, one thread per row, every operand in
-//      shared memory (the recurrence is latency-bound when it reads T back
-//      from global memory);
-//   4. T to tfull (zeros below the diagonal blocks), coalesced.
-constexpr int kTbKC = 32;  // rows of Y per staged chunk
+// T build by doubling (FP32 tiles of 128 and 256, FP64 and double-float tiles of
+// 128).  gram_kernel forms the Gram matrix's 64 x 64 tiles on or above the diagonal,
+// one CTA each, into the upper triangle of tfull; tdouble_kernel, one CTA per tile,
+// starts from the 16 x 16 diagonal blocks and joins neighbours of size s = 16, 32,
+// ..: T = [T1, -T1 G12 T2; 0, T2], two products per level with all pairs in
+// parallel, T's upper block triangle packed in shared memory by 16-column blocks
+// (column block J: rows 0 .. 16(J+1), column-major, at offset 256 J (J+1) / 2).
+// What bounded the build column block by column block: b/16 - 1 dependent steps on
+// one SM per tile, after a Gram matrix on the same SM.  Measured (GB300, a whole
+// panel's T, before -> after): FP32 tile 256 295 -> 130 us, tile 128 61 -> 32 us;
+// double-float tile 128 500 -> 150 us.
+constexpr int kGT = 64;    // Gram tile
+constexpr int kGK = 32;    // rows per staged chunk
 
-__host__ __device__ constexpr int tb_off(int J) { return 256 * J * (J + 1) / 2; }
-inline size_t tbuild_f32_smem(int b) {
-    const int nb = b / kWIB;
-    return sizeof(float) * ((size_t)tb_off(nb) + (size_t)kTbKC * (b + 4));
-}
-
-template <int LAYOUT>
-__global__ void __launch_bounds__(kWNT) tbuild_f32_kernel(TBuildArgs args) {
+template <typename T, int LAYOUT, typename CT>
+__global__ void __launch_bounds__(kWNT) gram_kernel(TBuildArgs args) {
+    using M = MacAr<CT>;
+    constexpr int LD = kGT + 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    CT *sI = reinterpret_cast<CT *>(smem_raw);  // [kGK][LD]
+    CT *sJ = sI + kGK * LD;
     const int b = args.b;
-    const int nb = b / kWIB;
-    const int p = blockIdx.x + args.first_role;
-    const int64_t zb = blockIdx.y;
+    int J = 0;
+    while ((J + 1) * (J + 2) / 2 <= (int)blockIdx.x) ++J;
+    const int I = (int)blockIdx.x - J * (J + 1) / 2;  // tile pair I <= J
+    const int p = blockIdx.y + args.first_role;
+    const int64_t zb = blockIdx.z;
     const bool geqrt = (p == 0);
     const int tid = threadIdx.x;
-    View<const float, LAYOUT> V{reinterpret_cast<const float *>(args.a) + zb * args.sA, args.lda};
+    View<const T, LAYOUT> V{reinterpret_cast<const T *>(args.a) + zb * args.sA, args.lda};
     const int64_t row0 = (int64_t)(args.pr + p) * b;
     const int64_t col0 = (int64_t)args.pc * b;
-    float *Tf = reinterpret_cast<float *>(args.tfull) + zb * args.sTfull + (size_t)p * b * b;
-    const float *tb = reinterpret_cast<const float *>(args.tblk) + zb * args.sTblk + (size_t)p * nb * kWIB * kWIB;
-    float *Tp = reinterpret_cast<float *>(smem_raw);  // packed upper block triangle
-    float *ch = Tp + tb_off(nb);                        // [kTbKC][b + 4] rows of Y, then H
-    const int ldc = b + 4;
-    auto tp = [&](int r, int i) -> float & {  // T(r, i), r < 16 (i / 16 + 1)
-        const int J = i / kWIB;
-        return Tp[tb_off(J) + (i % kWIB) * (kWIB * (J + 1)) + r];
+    T *Tf = reinterpret_cast<T *>(args.tfull) + zb * args.sTfull + (size_t)p * b * b;
+    constexpr int PER = kGK * kGT / kWNT;
+    T nI[PER], nJ[PER];
+    auto fetch = [&](int k0, int m0, T (&v)[PER]) {
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int idx = tid + e * kWNT;
+            const int k = LAYOUT == 0 ? idx % kGK : idx / kGT, m = LAYOUT == 0 ? idx / kGK : idx % kGT;
+            const int t = k0 + k, c = m0 + m;
+            T x = __ldcg(&V(row0 + t, col0 + c));
+            if (geqrt) x = (t == c) ? T(1) : (t > c ? x : T(0));
+            v[e] = x;
+        }
     };
-
-    // ---- 1. Gram blocks
-    const int ntiles = 2 * nb * (nb - 1);  // 8 x 8 tiles: 4 per block pair
-    const int per = kTbKC * b / kWNT;      // staged values per thread and chunk
-    for (int base = 0; base < ntiles; base += kWNT) {
-        const int u = base + tid;
-        int l0 = -1, i0 = -1;
-        if (u < ntiles) {
-            const int pair = u >> 2;
-            int J = 1;
-            while (J * (J + 1) / 2 <= pair) ++J;
-            const int I = pair - J * (J - 1) / 2;
-            l0 = I * kWIB + 8 * ((u >> 1) & 1);
-            i0 = J * kWIB + 8 * (u & 1);
+    auto stage = [&](CT *s, const T (&v)[PER]) {
+#pragma unroll
+        for (int e = 0; e < PER; ++e) {
+            const int idx = tid + e * kWNT;
+            const int k = LAYOUT == 0 ? idx % kGK : idx / kGT, m = LAYOUT == 0 ? idx / kGK : idx % kGT;
+            s[k * LD + m] = CT(v[e]);
         }
-        float g[8][8];
+    };
+    const int l0 = 4 * (tid % 16), i0 = 4 * (tid / 16);
+    const CT *bJ = I == J ? sI : sJ;
+    typename M::Mac g[4][4];
 #pragma unroll
-        for (int x = 0; x < 8; ++x)
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-            for (int y = 0; y < 8; ++y) g[x][y] = 0.0f;
-        // staged value e of this thread: (k, m) = (k_0 + e dk, m_0 + e dm), one
-        // pointer stepped by a fixed stride (coalesced along the tile's storage)
-        const int k_0 = (LAYOUT == 0) ? tid % kTbKC : tid / b;
-        const int m_0 = (LAYOUT == 0) ? tid / kTbKC : tid % b;
-        const int dk = (LAYOUT == 0) ? 0 : kWNT / b;
-        const int dm = (LAYOUT == 0) ? kWNT / kTbKC : 0;
-        const int64_t dp = (LAYOUT == 0) ? (int64_t)dm * args.lda : (int64_t)dk * args.lda;
-        float nx[32];
-        auto fetch = [&](int k0) {
-            const float *ptr = &V(row0 + k0 + k_0, col0 + m_0);
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-                if (e < per) {
-                    float v = __ldcg(ptr + e * dp);
-                    if (geqrt) {
-                        const int t = k0 + k_0 + e * dk, m = m_0 + e * dm;
-                        v = (t == m) ? 1.0f : (t > m ? v : 0.0f);
-                    }
-                    nx[e] = v;
-                }
-            }
-        };
-        fetch(0);
-        for (int k0 = 0; k0 < b; k0 += kTbKC) {
-            __syncthreads();  // the previous chunk's products are done
-#pragma unroll
-            for (int e = 0; e < 32; ++e)
-                if (e < per) ch[(k_0 + e * dk) * ldc + m_0 + e * dm] = nx[e];
-            __syncthreads();
-            if (k0 + kTbKC < b) fetch(k0 + kTbKC);
-            if (l0 >= 0) {
+        for (int y = 0; y < 4; ++y) g[x][y] = M::mac0();
+    fetch(0, I * kGT, nI);
+    if (I != J) fetch(0, J * kGT, nJ);
+    for (int k0 = 0; k0 < b; k0 += kGK) {
+        __syncthreads();
+        stage(sI, nI);
+        if (I != J) stage(sJ, nJ);
+        __syncthreads();
+        if (k0 + kGK < b) {
+            fetch(k0 + kGK, I * kGT, nI);
+            if (I != J) fetch(k0 + kGK, J * kGT, nJ);
+        }
 #pragma unroll 4
-                for (int k = 0; k < kTbKC; ++k) {
-                    const float4 a0 = *reinterpret_cast<const float4 *>(ch + k * ldc + l0);
-                    const float4 a1 = *reinterpret_cast<const float4 *>(ch + k * ldc + l0 + 4);
-                    const float4 c0 = *reinterpret_cast<const float4 *>(ch + k * ldc + i0);
-                    const float4 c1 = *reinterpret_cast<const float4 *>(ch + k * ldc + i0 + 4);
-                    const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                    const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        for (int k = 0; k < kGK; ++k) {
+            CT a[4], c[4];
 #pragma unroll
-                    for (int x = 0; x < 8; ++x)
-#pragma unroll
-                        for (int y = 0; y < 8; ++y) g[x][y] = fmaf(a[x], c[y], g[x][y]);
-                }
+            for (int q = 0; q < 4; q += PVec<CT>::VN) {
+                PVec<CT>::ld(sI + k * LD + l0 + q, a + q);
+                PVec<CT>::ld(bJ + k * LD + i0 + q, c + q);
             }
-        }
-        if (l0 >= 0) {
 #pragma unroll
-            for (int y = 0; y < 8; ++y)
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
-                for (int x = 0; x < 8; ++x) tp(l0 + x, i0 + y) = g[x][y];
+                for (int y = 0; y < 4; ++y) M::mac(g[x][y], a[x], c[y]);
         }
     }
-    // ---- 2. diagonal blocks
-    for (int idx = tid; idx < nb * kWIB * kWIB; idx += kWNT) {
-        const int J = idx / (kWIB * kWIB), e = idx % (kWIB * kWIB), r = e % kWIB, q = e / kWIB;
-        tp(J * kWIB + r, J * kWIB + q) = tb[idx];
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+            Tf[I * kGT + l0 + x + (size_t)(J * kGT + i0 + y) * b] = (T)M::fin(g[x][y]);
+}
+
+__host__ __device__ constexpr int tb_off(int J) { return 128 * J * (J + 1); }
+
+template <typename CT, int B>
+constexpr size_t tdouble_smem() {  // packed T, then the products G12 T2 of a level
+    return sizeof(CT) * ((size_t)tb_off(B / kWIB) + (size_t)B * B / 4);
+}
+
+template <typename T, typename CT, int B>
+__global__ void __launch_bounds__(kWNT) tdouble_kernel(TBuildArgs args) {
+    using M = MacAr<CT>;
+    constexpr int NB = B / kWIB, VN = PVec<CT>::VN;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CT *Tp = reinterpret_cast<CT *>(smem_raw);
+    CT *X = Tp + tb_off(NB);
+    const int p = blockIdx.x + args.first_role;
+    const int64_t zb = blockIdx.y;
+    const int tid = threadIdx.x;
+    T *Tf = reinterpret_cast<T *>(args.tfull) + zb * args.sTfull + (size_t)p * B * B;
+    const T *tb = reinterpret_cast<const T *>(args.tblk) + zb * args.sTblk + (size_t)p * NB * kWIB * kWIB;
+    auto col = [&](int i) -> CT * { return Tp + tb_off(i / kWIB) + (i % kWIB) * (kWIB * (i / kWIB + 1)); };
+    // the Gram blocks above the diagonal blocks, and the diagonal blocks of T
+    for (int idx = tid; idx < B * B; idx += kWNT) {
+        const int r = idx % B, i = idx / B;
+        if (r / kWIB < i / kWIB) col(i)[r] = CT(__ldcg(Tf + r + (size_t)i * B));
+    }
+    for (int idx = tid; idx < NB * kWIB * kWIB; idx += kWNT) {
+        const int J = idx / (kWIB * kWIB), e = idx % (kWIB * kWIB);
+        col(J * kWIB + e / kWIB)[J * kWIB + e % kWIB] = CT(tb[idx]);
     }
     __syncthreads();
-    // ---- 3. column blocks
-    float *H = ch;  // [c0][16]
-    for (int J = 1; J < nb; ++J) {
-        const int c0 = J * kWIB;
-        const int r = tid;
-        if (r < c0) {  // H[r] = G[r, J] T_JJ (T_JJ upper triangular)
-            float gq[kWIB], h[kWIB];
+#pragma unroll 1
+    for (int s = kWIB; s < B; s *= 2) {
+        const int per = (s / 4) * (s / 4);  // 4 x 4 tiles of a pair
+        const int tasks = B / (2 * s) * per;
+        for (int u = tid; u < tasks; u += kWNT) {  // X = G12 T2 (T2 upper triangular)
+            const int q = u / per, r = 4 * (u % per % (s / 4)), c = 4 * (u % per / (s / 4));
+            const int r1 = q * 2 * s, r2 = r1 + s;
+            typename M::Mac a[4][4];
 #pragma unroll
-            for (int q = 0; q < kWIB; ++q) gq[q] = tp(r, c0 + q);
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
-            for (int q = 0; q < kWIB; ++q) {
-                float v = 0.0f;
+                for (int y = 0; y < 4; ++y) a[x][y] = M::mac0();
+            const CT *t0 = col(r2 + c) + r2, *t1 = col(r2 + c + 1) + r2, *t2 = col(r2 + c + 2) + r2,
+                     *t3 = col(r2 + c + 3) + r2;
+            const int mend = c / kWIB * kWIB + kWIB;
+#pragma unroll 2
+            for (int m = 0; m < mend; ++m) {
+                CT g[4];
+                const CT *gp = col(r2 + m) + r1 + r;
 #pragma unroll
-                for (int qq = 0; qq <= q; ++qq) v = fmaf(gq[qq], tp(c0 + qq, c0 + q), v);
-                h[q] = v;
+                for (int e = 0; e < 4; e += VN) PVec<CT>::ld(gp + e, g + e);
+                const CT tv[4] = {t0[m], t1[m], t2[m], t3[m]};
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) M::mac(a[x][y], g[x], tv[y]);
             }
 #pragma unroll
-            for (int q = 0; q < kWIB; q += 4)
-                *reinterpret_cast<float4 *>(H + r * kWIB + q) = make_float4(h[q], h[q + 1], h[q + 2], h[q + 3]);
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 4; y += VN) {
+                    CT v[VN];
+#pragma unroll
+                    for (int e = 0; e < VN; ++e) v[e] = M::fin(a[x][y + e]);
+                    PVec<CT>::st(X + (size_t)(q * s + r + x) * s + c + y, v);
+                }
         }
         __syncthreads();
-        if (r < c0) {  // T[r, J] = -sum_{m >= block start of r} T(r, m) H[m]
-            float acc[kWIB];
+        for (int u = tid; u < tasks; u += kWNT) {  // T12 = -T1 X (T1 upper triangular)
+            const int q = u / per, r = 4 * (u % per % (s / 4)), c = 4 * (u % per / (s / 4));
+            const int r1 = q * 2 * s, r2 = r1 + s;
+            typename M::Mac a[4][4];
 #pragma unroll
-            for (int q = 0; q < kWIB; ++q) acc[q] = 0.0f;
-            for (int m = (r / kWIB) * kWIB; m < c0; ++m) {
-                const float t = tp(r, m);
-                const float4 *hm = reinterpret_cast<const float4 *>(H + m * kWIB);
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
-                for (int q4 = 0; q4 < kWIB / 4; ++q4) {
-                    const float4 hv = hm[q4];
-                    acc[4 * q4] = fmaf(t, hv.x, acc[4 * q4]);
-                    acc[4 * q4 + 1] = fmaf(t, hv.y, acc[4 * q4 + 1]);
-                    acc[4 * q4 + 2] = fmaf(t, hv.z, acc[4 * q4 + 2]);
-                    acc[4 * q4 + 3] = fmaf(t, hv.w, acc[4 * q4 + 3]);
+                for (int y = 0; y < 4; ++y) a[x][y] = M::mac0();
+#pragma unroll 2
+            for (int m = r / kWIB * kWIB; m < s; ++m) {
+                CT t[4], xv[4];
+                const CT *tp = col(r1 + m) + r1 + r;
+                const CT *xp = X + (size_t)(q * s + m) * s + c;
+#pragma unroll
+                for (int e = 0; e < 4; e += VN) {
+                    PVec<CT>::ld(tp + e, t + e);
+                    PVec<CT>::ld(xp + e, xv + e);
                 }
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) M::mac(a[x][y], t[x], xv[y]);
             }
 #pragma unroll
-            for (int q = 0; q < kWIB; ++q) tp(r, c0 + q) = -acc[q];
+            for (int y = 0; y < 4; ++y) {
+                CT *dst = col(r2 + c + y) + r1 + r;
+#pragma unroll
+                for (int x = 0; x < 4; x += VN) {
+                    CT v[VN];
+#pragma unroll
+                    for (int e = 0; e < VN; ++e) v[e] = -M::fin(a[x + e][y]);
+                    PVec<CT>::st(dst + x, v);
+                }
+            }
         }
         __syncthreads();
     }
-    // ---- 4. out, zeros below the diagonal blocks
-    for (int idx = tid; idx < b * b; idx += kWNT) {
-        const int l = idx % b, i = idx / b;
-        Tf[l + (size_t)i * b] = (l < kWIB * (i / kWIB + 1)) ? tp(l, i) : 0.0f;
+    // out, zeros below the diagonal blocks
+    for (int idx = tid; idx < B * B; idx += kWNT) {
+        const int r = idx % B, i = idx / B;
+        Tf[idx] = (r < kWIB * (i / kWIB + 1)) ? (T)col(i)[r] : T(0);
     }
 }
 
@@ -721,46 +753,56 @@ int launch_upd_full_any(T *dA, int64_t lda, int64_t n, int pr, int pc, int P, co
     return launch_upd_full<T, LAYOUT, B>(dA, lda, n, pr, pc, P, w, s, first_role);
 }
 
+template <typename T, int LAYOUT, typename CT, int B>
+int launch_tdouble(const TBuildArgs &a, int nrole, int batch, cudaStream_t s) {
+    static std::atomic<bool> attr{false};
+    constexpr size_t smem = tdouble_smem<CT, B>(), gsm = sizeof(CT) * 2 * kGK * (kGT + 4);
+    static_assert(smem <= 227 * 1024 && gsm <= 48 * 1024, "T build shared memory");
+    if (!attr) {
+        AVS_CUDA_TRY(cudaFuncSetAttribute(tdouble_kernel<T, CT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+        attr = true;
+    }
+    constexpr int NG = (B / kGT) * (B / kGT + 1) / 2;
+    gram_kernel<T, LAYOUT, CT><<<dim3(NG, nrole, batch), kWNT, gsm, s>>>(a);
+    AVS_CUDA_TRY(cudaGetLastError());
+    tdouble_kernel<T, CT, B><<<dim3(nrole, batch), kWNT, smem, s>>>(a);
+    AVS_CUDA_TRY(cudaGetLastError());
+    return AVS_SUCCESS;
+}
+
+// Tiles of 128, and FP32 tiles of 256, by doubling; 8-byte tiles of 256, whose
+// packed T does not fit in shared memory, column block by column block.  FP64
+// tiles with the double-float updates build T in double-float too (FP64 storage;
+// GB300 issues FP64 at 1/64 of the FP32 rate).
 template <typename T, int LAYOUT>
 int launch_tbuild(const T *dA, int64_t lda, int b, int pr, int pc, int P, const Stage1Work &w, cudaStream_t s,
                   int first_role = 0) {
+    const int batch = w.batch > 0 ? w.batch : 1, nrole = P - first_role;
+    TBuildArgs a{dA, lda, b, pr, pc, P, w.tblk, w.tfull, w.sA, w.sTblk, w.sTfull, first_role};
     if constexpr (sizeof(T) == 4) {
-        static std::atomic<bool> attr32{false};
-        if (!attr32) {
-            AVS_CUDA_TRY(cudaFuncSetAttribute(tbuild_f32_kernel<LAYOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)tbuild_f32_smem(256)));
-            attr32 = true;
+        return b == 256 ? launch_tdouble<T, LAYOUT, float, 256>(a, nrole, batch, s)
+                        : launch_tdouble<T, LAYOUT, float, 128>(a, nrole, batch, s);
+    } else {
+        if (b == 128)
+            return w.df_update ? launch_tdouble<T, LAYOUT, dfx, 128>(a, nrole, batch, s)
+                               : launch_tdouble<T, LAYOUT, double, 128>(a, nrole, batch, s);
+        static std::atomic<bool> attr{false};
+        constexpr size_t smem = sizeof(T) * (size_t)32 * (256 + 1);
+        if (!attr) {
+            AVS_CUDA_TRY(cudaFuncSetAttribute(tbuild_kernel<T, LAYOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)smem));
+            AVS_CUDA_TRY(cudaFuncSetAttribute(tbuild_kernel<T, LAYOUT, dfx>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            attr = true;
         }
-        TBuildArgs a{dA, lda, b, pr, pc, P, w.tblk, w.tfull, w.sA, w.sTblk, w.sTfull, first_role};
-        tbuild_f32_kernel<LAYOUT><<<dim3(P - first_role, w.batch > 0 ? w.batch : 1), kWNT, tbuild_f32_smem(b), s>>>(a);
+        if (w.df_update)
+            tbuild_kernel<T, LAYOUT, dfx><<<dim3(nrole, batch), kWNT, smem, s>>>(a);
+        else
+            tbuild_kernel<T, LAYOUT><<<dim3(nrole, batch), kWNT, smem, s>>>(a);
         AVS_CUDA_TRY(cudaGetLastError());
         return AVS_SUCCESS;
     }
-    static std::atomic<bool> attr{false};
-    const size_t smem = sizeof(T) * (size_t)32 * (256 + 1) > sizeof(T) * (size_t)256 * 256 / 16
-                            ? sizeof(T) * (size_t)32 * (256 + 1)
-                            : sizeof(T) * (size_t)256 * 16;
-    if (!attr) {
-        AVS_CUDA_TRY(
-            cudaFuncSetAttribute(tbuild_kernel<T, LAYOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if constexpr (sizeof(T) == 8)
-            AVS_CUDA_TRY(cudaFuncSetAttribute(tbuild_kernel<T, LAYOUT, dfx>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr = true;
-    }
-    TBuildArgs a{dA, lda, b, pr, pc, P, w.tblk, w.tfull, w.sA, w.sTblk, w.sTfull, first_role};
-    if constexpr (sizeof(T) == 8) {
-        // FP64 tiles with the double-float updates: the T build in double-float
-        // too (FP64 storage; GB300 issues FP64 at 1/64 of the FP32 rate)
-        if (w.df_update) {
-            tbuild_kernel<T, LAYOUT, dfx><<<dim3(P - first_role, w.batch > 0 ? w.batch : 1), kWNT, smem, s>>>(a);
-            AVS_CUDA_TRY(cudaGetLastError());
-            return AVS_SUCCESS;
-        }
-    }
-    tbuild_kernel<T, LAYOUT><<<dim3(P - first_role, w.batch > 0 ? w.batch : 1), kWNT, smem, s>>>(a);
-    AVS_CUDA_TRY(cudaGetLastError());
-    return AVS_SUCCESS;
 }
 
 }  // namespace

@@ -1,5 +1,5 @@
-// 16-byte vectors of the kernels' element types: VN values of T from / to shared
-// or global memory (16-byte aligned).
+// Element types of the stage-1 kernels: 16-byte vectors (VN values of T from / to
+// shared or global memory, 16-byte aligned) and sums of products.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -51,4 +51,47 @@ struct PVec<dfx> {
         *reinterpret_cast<float4 *>(p) = make_float4(v[0].v.hi, v[0].v.lo, v[1].v.hi, v[1].v.lo);
     }
 };
+// Sums of products: mac accumulates into Mac (double-float: the compensated dot
+// product of Ogita, Rump and Oishi, an unnormalised pair), fin gives the value.
+template <typename CT>
+struct MacAr;
+template <>
+struct MacAr<float> {
+    using Mac = float;
+    static __device__ __forceinline__ Mac mac0() { return 0.0f; }
+    static __device__ __forceinline__ Mac mac_from(float x) { return x; }
+    static __device__ __forceinline__ void mac(Mac &a, float x, float y) { a = fmaf(x, y, a); }
+    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) { return a + b; }
+    static __device__ __forceinline__ float fin(Mac a) { return a; }
+};
+template <>
+struct MacAr<dfx> {
+    using Mac = df64;
+    static __device__ __forceinline__ Mac mac0() { return df64{0.0f, 0.0f}; }
+    static __device__ __forceinline__ Mac mac_from(dfx x) { return x.v; }
+    static __device__ __forceinline__ void mac(Mac &a, dfx x, dfx y) {
+        const float p = __fmul_rn(x.v.hi, y.v.hi);
+        float ep = __fmaf_rn(x.v.hi, y.v.hi, -p);
+        ep = __fmaf_rn(x.v.hi, y.v.lo, ep);
+        ep = __fmaf_rn(x.v.lo, y.v.hi, ep);
+        const df64 t = two_sum(a.hi, p);
+        a.hi = t.hi;
+        a.lo = __fadd_rn(a.lo, __fadd_rn(t.lo, ep));
+    }
+    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) {
+        const df64 t = two_sum(a.hi, b.hi);
+        return df64{t.hi, __fadd_rn(t.lo, __fadd_rn(a.lo, b.lo))};
+    }
+    static __device__ __forceinline__ dfx fin(Mac a) { return dfx(two_sum(a.hi, a.lo)); }
+};
+template <>
+struct MacAr<double> {
+    using Mac = double;
+    static __device__ __forceinline__ Mac mac0() { return 0.0; }
+    static __device__ __forceinline__ Mac mac_from(double x) { return x; }
+    static __device__ __forceinline__ void mac(Mac &a, double x, double y) { a = fma(x, y, a); }
+    static __device__ __forceinline__ Mac mac_merge(Mac a, Mac b) { return a + b; }
+    static __device__ __forceinline__ double fin(Mac a) { return a; }
+};
+
 }  // namespace avs
