@@ -14,6 +14,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "avs_common.cuh"
+#include "df64.cuh"
 #include "tc_gemm.cuh"
 
 namespace avs {
@@ -274,10 +275,21 @@ int run_stages23(avs_handle *h, const Layout &L, int64_t n, int b, const S *W, i
         if (band_ran) *band_ran = true;
     } else if (tbw > 0 && sizeof(S) == 4 && !fp64_stages) {
         // the FP32 band of width b in the first half of AB (3b x n floats)
-        if ((rc = stage2_chase_hier_df(reinterpret_cast<const float *>(W), n, ldw, b, tbw,
-                                       reinterpret_cast<float *>(AB), reinterpret_cast<float2 *>(ws_at(h, L.off_ab2)),
-                                       dd, de, w2, s, h->num_sms, launches, !(flags & AVS_FLAG_CLUSTER_CHASE),
-                                       h->ev[6])) != AVS_SUCCESS)
+        if ((rc = stage2_chase_hier_df<float, float>(
+                 reinterpret_cast<const float *>(W), n, ldw, b, tbw, reinterpret_cast<float *>(AB),
+                 reinterpret_cast<float2 *>(ws_at(h, L.off_ab2)), dd, de, w2, s, h->num_sms, launches,
+                 !(flags & AVS_FLAG_CLUSTER_CHASE), h->ev[6])) != AVS_SUCCESS)
+            return rc;
+        if (band_ran) *band_ran = true;
+    } else if (tbw > 0 && sizeof(S) == 8 && !fp64_stages) {
+        // FP64 tiles, double-float stages: the block stage in double-float too.  One
+        // stage against two (GB300, stage 2): tile 64 n = 256 3.3 / 2.9 ms, n = 1024 15.1
+        // / 13.2; tile 128 n = 512 8.1 / 6.6, n = 2048 36.6 / 29.0; tile 256 n = 2048 72.5
+        // / 37.0.
+        if ((rc = stage2_chase_hier_df<double, dfx>(
+                 reinterpret_cast<const double *>(W), n, ldw, b, tbw, reinterpret_cast<dfx *>(AB),
+                 reinterpret_cast<float2 *>(ws_at(h, L.off_ab2)), dd, de, w2, s, h->num_sms, launches,
+                 !(flags & AVS_FLAG_CLUSTER_CHASE), h->ev[6])) != AVS_SUCCESS)
             return rc;
         if (band_ran) *band_ran = true;
     } else if (fp64_stages) {
@@ -1284,7 +1296,8 @@ int group_launches(avs_handle *h, const BatchLayout &L, int64_t n, int b, int cn
                                            reinterpret_cast<double *>(base + L.ab2));
         else
             rc = stage2_chase_df_batched(W, n, b, cnt, reinterpret_cast<float2 *>(base + L.ab), 3 * (int64_t)b, dd,
-                                         de, w2, s, h->num_sms, launches, window);
+                                         de, w2, s, h->num_sms, launches, tbw, window,
+                                         reinterpret_cast<float2 *>(base + L.ab2));
     } else {
         rc = stage2_chase_df_batched(W, n, b, cnt, reinterpret_cast<float2 *>(base + L.ab), 3 * (int64_t)b, dd, de,
                                      w2, s, h->num_sms, launches, tbw, window, reinterpret_cast<float2 *>(base + L.ab2));

@@ -243,8 +243,8 @@ int stage2_chase_df_batched(const float *dW, int64_t n, int bw, int batch, float
                             bool window, float2 *dAB2);
 // FP64 tiles, double-float chase (the batched groups of AVS_PREC_FP64X2)
 int stage2_chase_df_batched(const double *dW, int64_t n, int bw, int batch, float2 *dAB, int64_t ldab, double *dd,
-                            double *de, const Stage2Work &w, cudaStream_t s, int num_sms, int64_t *launches,
-                            bool window);
+                            double *de, const Stage2Work &w, cudaStream_t s, int num_sms, int64_t *launches, int tbw,
+                            bool window, float2 *dAB2);
 // Blocked band reduction bw -> tbw (stage2_band.cu), on a compact band with
 // 16-byte aligned column segments: A(r, c) at dAB[(r - c + band_ku(bw)) + c *
 // ldab], ldab = band_ldab(bw) (rows c-2bw .. c+bw of column c; a segment that
@@ -268,12 +268,14 @@ template <typename R>
 int band_to_dense(const R *dAB, int64_t n, int bw, int64_t ldab, R *dA, int64_t lda, cudaStream_t s);
 // Hierarchical stage 2 (stage2_chase.cu): the band of width bw of dW
 // (W[r + c*ldw]) -> width tbw by the blocked band reduction, then the element
-// chase tbw -> 1; d and e out.  _df: FP32 band reduction, double-float chase;
-// _fp64: FP64 throughout.  dAB1 holds 3 bw x n elements, dAB2 3 tbw x n.
+// chase tbw -> 1; d and e out.  _df: band reduction in FP32 (R = float, FP32 tiles)
+// or double-float (R = dfx, FP64 tiles), double-float chase; _fp64: FP64
+// throughout.  dAB1 holds 3 bw x n elements, dAB2 3 tbw x n.
 // window: the narrow band's element chase by the windowed multi-sweep kernel
 // (stage2_window.cu) instead of the cluster kernel.
 // after_band (optional): recorded on s between the band reduction and the chase.
-int stage2_chase_hier_df(const float *dW, int64_t n, int64_t ldw, int bw, int tbw, float *dAB1, float2 *dAB2,
+template <typename T, typename R>
+int stage2_chase_hier_df(const T *dW, int64_t n, int64_t ldw, int bw, int tbw, R *dAB1, float2 *dAB2,
                          double *dd, double *de, const Stage2Work &w, cudaStream_t s, int num_sms, int64_t *launches,
                          bool window, cudaEvent_t after_band = nullptr);
 int stage2_chase_hier_fp64(const double *dW, int64_t n, int64_t ldw, int bw, int tbw, double *dAB1, double *dAB2,

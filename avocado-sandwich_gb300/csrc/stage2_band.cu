@@ -29,6 +29,8 @@
 // = V^T A), Y = W T (T^T Z) by forward substitution from the Gram matrix that the
 // factorisation leaves (T^-1 = diag(1/tau) + striu(V^T V), one thread per row or
 // column), A -= Y V^T (V Y); operands in shared memory, on the FP32 (or FP64) pipe.
+// In double-float every product chain keeps an unnormalised pair (12 instead of 15
+// instructions a multiply-add; n = 2048, band 128: 20.3 -> 18.8 ms).
 // What bounds it: the latency of an op along the sweep wavefront (the panel's 16
 // reflectors are half of it: 12 to 15 k of about 20 to 37 k cycles).  Measured (GB300,
 // the whole stage, before: every column's work inside the panel's chain, T formed
@@ -41,14 +43,17 @@
 // 16-byte vectors.
 //
 // Arithmetic: the element type R throughout (FP32 for the FP32-class modes,
-// FP64 for the FP64 path), reflector scalars included.
+// double-float for AVS_PREC_FP64X2, FP64 for the FP64 path), reflector scalars
+// included.
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <type_traits>
 
 #include "avs_common.cuh"
+#include "df64.cuh"
 #include "reflect.cuh"
+#include "vec16.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -90,6 +95,25 @@ struct BandCfg {
     }
 };
 
+// Multiply-adds run on MacAr<R> accumulators (double-float: an unnormalised
+// pair); the sum of one over a warp, and the value of lane src.
+__device__ __forceinline__ bool positive(float a) { return a > 0.0f; }
+__device__ __forceinline__ bool positive(double a) { return a > 0.0; }
+__device__ __forceinline__ bool positive(dfx a) { return a.v.hi > 0.0f; }
+__device__ __forceinline__ float wsum(float v) { return warp_sum(v); }
+__device__ __forceinline__ double wsum(double v) { return warp_sum(v); }
+__device__ __forceinline__ dfx wsum(df64 s) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        s = MacAr<dfx>::mac_merge(s, df64{__shfl_xor_sync(0xffffffffu, s.hi, o), __shfl_xor_sync(0xffffffffu, s.lo, o)});
+    return MacAr<dfx>::fin(s);
+}
+__device__ __forceinline__ float wshfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ double wshfl(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ dfx wshfl(dfx v, int src) {
+    return dfx(df64{__shfl_sync(0xffffffffu, v.v.hi, src), __shfl_sync(0xffffffffu, v.v.lo, src)});
+}
+
 template <typename R>
 struct Vec4;
 template <>
@@ -114,7 +138,19 @@ struct Vec4<double> {
     }
 };
 
-// 16-byte vectors of the element type: 4 floats or 2 doubles.
+template <>
+struct Vec4<dfx> {
+    static __device__ __forceinline__ void ld(const dfx *p, dfx (&o)[4]) {
+        const float4 a = *reinterpret_cast<const float4 *>(p);
+        const float4 b = *reinterpret_cast<const float4 *>(p + 2);
+        o[0] = dfx(df64{a.x, a.y});
+        o[1] = dfx(df64{a.z, a.w});
+        o[2] = dfx(df64{b.x, b.y});
+        o[3] = dfx(df64{b.z, b.w});
+    }
+};
+
+// 16-byte vectors of the element type: 4 floats, 2 doubles or 2 pairs.
 template <typename R>
 struct Vec16;
 template <>
@@ -141,6 +177,19 @@ struct Vec16<double> {
     }
     static __device__ __forceinline__ void st(double *p, const double (&v)[2]) {
         *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    }
+};
+
+template <>
+struct Vec16<dfx> {
+    static constexpr int N = 2;
+    static __device__ __forceinline__ void ld(const dfx *p, dfx (&o)[2]) {
+        const float4 v = __ldcg(reinterpret_cast<const float4 *>(p));
+        o[0] = dfx(df64{v.x, v.y});
+        o[1] = dfx(df64{v.z, v.w});
+    }
+    static __device__ __forceinline__ void st(dfx *p, const dfx (&v)[2]) {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0].v.hi, v[0].v.lo, v[1].v.hi, v[1].v.lo);
     }
 };
 
@@ -206,6 +255,17 @@ __device__ __forceinline__ void reflector_scalars(double alpha, double s, double
     scal = alpha >= 0.0 ? z : -z;
 }
 
+__device__ __forceinline__ void reflector_scalars(dfx al, dfx s, dfx &tau, dfx &beta, dfx &scal) {
+    df64 rn, nrm;
+    rsqrt_sqrt((al * al + s).v, rn, nrm);
+    const bool neg = df_lt0(al.v);
+    const df64 aa = neg ? df_neg(al.v) : al.v;
+    beta = dfx(neg ? nrm : df_neg(nrm));
+    tau = dfx(aa) * dfx(rn) + dfx(1);
+    const df64 z = rcp_est(df_add(aa, nrm));
+    scal = dfx(neg ? df_neg(z) : z);
+}
+
 // Householder QR of the panel P (B rows x T columns, column k at P + k*LDP,
 // zero rows below the valid part), LAPACK convention per column: beta =
 // -sign(alpha) ||x||, v = x / (alpha - beta) below the diagonal, v_k = 1,
@@ -233,20 +293,20 @@ __device__ __forceinline__ void panel_qr(R *P, R *s_tau, R *gram) {
     // H_k of column k in slot JK of its owner
     auto generate = [&](auto slot_c, int k) {
         constexpr int JK = decltype(slot_c)::value;
-        R s = R(0);
+        auto sq = MacAr<R>::mac0();
 #pragma unroll
         for (int u = 0; u < RPL; ++u) {
             const int i = lane + 32 * u;
-            if (i > k) s = fma(x[JK][u], x[JK][u], s);
+            if (i > k) MacAr<R>::mac(sq, x[JK][u], x[JK][u]);
         }
-        s = warp_sum(s);
-        const R alpha = __shfl_sync(0xffffffffu, x[JK][0], k);  // T <= 32: row k is in slot 0
+        const R s = wsum(sq);
+        const R alpha = wshfl(x[JK][0], k);  // T <= 32: row k is in slot 0
         R tau = R(0), beta = alpha, scal = R(0);
-        if (s > R(0)) reflector_scalars(alpha, s, tau, beta, scal);
+        if (positive(s)) reflector_scalars(alpha, s, tau, beta, scal);
 #pragma unroll
         for (int u = 0; u < RPL; ++u) {
             const int i = lane + 32 * u;
-            if (i > k) x[JK][u] *= scal;
+            if (i > k) x[JK][u] = x[JK][u] * scal;
             else if (i == k) x[JK][u] = beta;
             P[k * LDP + i] = x[JK][u];
         }
@@ -258,14 +318,18 @@ __device__ __forceinline__ void panel_qr(R *P, R *s_tau, R *gram) {
     // entry v_j^T v_k (x holds v_j below its diagonal)
     auto apply = [&](auto slot_c, int j, int k) {
         constexpr int JJ = decltype(slot_c)::value;
-        R d = R(0);
+        auto dot = MacAr<R>::mac0();
 #pragma unroll
-        for (int u = 0; u < RPL; ++u) d = fma(v[u], x[JJ][u], d);
-        d = warp_sum(d);
+        for (int u = 0; u < RPL; ++u) MacAr<R>::mac(dot, v[u], x[JJ][u]);
+        const R d = wsum(dot);
         if (j > k) {
-            const R t = d * tau;
+            const R t = -(d * tau);
 #pragma unroll
-            for (int u = 0; u < RPL; ++u) x[JJ][u] = fma(-t, v[u], x[JJ][u]);
+            for (int u = 0; u < RPL; ++u) {
+                auto m = MacAr<R>::mac_from(x[JJ][u]);
+                MacAr<R>::mac(m, t, v[u]);
+                x[JJ][u] = MacAr<R>::fin(m);
+            }
         } else if (lane == 0) {
             gram[j * (T + 1) + k] = d;
         }
@@ -317,21 +381,20 @@ __device__ __forceinline__ void panel_qr(R *P, R *s_tau, R *gram) {
 // partial sums [k][LDW] in, Y in the first on return; one thread per row.
 template <typename R, int T, int KS, int LDW>
 __device__ __forceinline__ void substitute(const R *s_tau, const R *gram, R *Wy, int row) {
-    R w[T];
+    typename MacAr<R>::Mac w[T];
 #pragma unroll
     for (int k = 0; k < T; ++k) {
-        w[k] = Wy[k * LDW + row];
+        w[k] = MacAr<R>::mac_from(Wy[k * LDW + row]);
 #pragma unroll
-        for (int q = 1; q < KS; ++q) w[k] += Wy[(q * T + k) * LDW + row];
+        for (int q = 1; q < KS; ++q) w[k] = MacAr<R>::mac_merge(w[k], MacAr<R>::mac_from(Wy[(q * T + k) * LDW + row]));
     }
 #pragma unroll
     for (int k = 0; k < T; ++k) {
-        w[k] = s_tau[k] * w[k];
+        const R y = s_tau[k] * MacAr<R>::fin(w[k]);
 #pragma unroll
-        for (int m = k + 1; m < T; ++m) w[m] = fma(-gram[k * (T + 1) + m], w[k], w[m]);
+        for (int m = k + 1; m < T; ++m) MacAr<R>::mac(w[m], -gram[k * (T + 1) + m], y);
+        Wy[k * LDW + row] = y;
     }
-#pragma unroll
-    for (int k = 0; k < T; ++k) Wy[k * LDW + row] = w[k];
 }
 
 template <int B, int T, typename R, int C>
@@ -428,11 +491,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                 // W = A V: thread = 4 rows x 4 reflectors, BK columns of the sum
                 {
                     const int g = tid % Cfg::NG4, k0 = (tid / Cfg::NG4) % (T / 4) * 4, ks = tid / (Cfg::NG4 * (T / 4));
-                    R acc[4][4];
+                    typename MacAr<R>::Mac acc[4][4];
 #pragma unroll
                     for (int a = 0; a < 4; ++a)
 #pragma unroll
-                        for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = R(0);
+                        for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = MacAr<R>::mac0();
 #pragma unroll 2
                     for (int c = ks * Cfg::BK; c < (ks + 1) * Cfg::BK; c += 4) {
                         R a4[4][4], v4[4][4];
@@ -445,12 +508,12 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
 #pragma unroll
                             for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-                                for (int rr = 0; rr < 4; ++rr) acc[kk][rr] = fma(a4[cc][rr], v4[kk][cc], acc[kk][rr]);
+                                for (int rr = 0; rr < 4; ++rr) MacAr<R>::mac(acc[kk][rr], a4[cc][rr], v4[kk][cc]);
                     }
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                        for (int rr = 0; rr < 4; ++rr) Wy[(ks * T + k0 + kk) * LDW + 4 * g + rr] = acc[kk][rr];
+                        for (int rr = 0; rr < 4; ++rr) Wy[(ks * T + k0 + kk) * LDW + 4 * g + rr] = MacAr<R>::fin(acc[kk][rr]);
                 }
                 __syncthreads();
                 if (tid < RPC) substitute<R, T, Cfg::KS, LDW>(s_tau, gram, Wy, tid);
@@ -460,11 +523,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                     constexpr int CPT = Cfg::CPT2R;
                     const int g = tid % Cfg::NG4, cgp = tid / Cfg::NG4;
                     const int cb = cgp * CPT;
-                    R acc[4][CPT];
+                    typename MacAr<R>::Mac acc[4][CPT];
 #pragma unroll
                     for (int cc = 0; cc < CPT; ++cc)
 #pragma unroll
-                        for (int rr = 0; rr < 4; ++rr) acc[rr][cc] = As[(cb + cc) * Cfg::LDA_R + 4 * g + rr];
+                        for (int rr = 0; rr < 4; ++rr) acc[rr][cc] = MacAr<R>::mac_from(As[(cb + cc) * Cfg::LDA_R + 4 * g + rr]);
                     for (int k = 0; k < T; ++k) {
                         R y4[4];
                         Vec4<R>::ld(Wy + k * LDW + 4 * g, y4);
@@ -476,7 +539,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                             for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
                                 for (int rr = 0; rr < 4; ++rr)
-                                    acc[rr][c4 + cc] = fma(-y4[rr], v4[cc], acc[rr][c4 + cc]);
+                                    MacAr<R>::mac(acc[rr][c4 + cc], -y4[rr], v4[cc]);
                         }
                     }
                     constexpr int VN = Vec16<R>::N;
@@ -490,12 +553,12 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                                 if (r + VN <= r_hi) {
                                     R v[VN];
 #pragma unroll
-                                    for (int e = 0; e < VN; ++e) v[e] = acc[r0 + e][cc];
+                                    for (int e = 0; e < VN; ++e) v[e] = MacAr<R>::fin(acc[r0 + e][cc]);
                                     Vec16<R>::st(at(r, c0 + c), v);
                                 } else {
 #pragma unroll
                                     for (int e = 0; e < VN; ++e)
-                                        if (r + e < r_hi) *at(r + e, c0 + c) = acc[r0 + e][cc];
+                                        if (r + e < r_hi) *at(r + e, c0 + c) = MacAr<R>::fin(acc[r0 + e][cc]);
                                 }
                             }
                         }
@@ -554,11 +617,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                 // their column reads spread over the banks) x 4 reflectors, BK rows of the sum
                 {
                     const int g = tid % Cfg::NG4, k0 = (tid / Cfg::NG4) % (T / 4) * 4, ks = tid / (Cfg::NG4 * (T / 4));
-                    R acc[4][4];
+                    typename MacAr<R>::Mac acc[4][4];
 #pragma unroll
                     for (int a = 0; a < 4; ++a)
 #pragma unroll
-                        for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = R(0);
+                        for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = MacAr<R>::mac0();
 #pragma unroll 2
                     for (int i = ks * Cfg::BK; i < (ks + 1) * Cfg::BK; i += 4) {
                         R a4[4][4], v4[4][4];
@@ -572,12 +635,12 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
 #pragma unroll
                             for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
-                                for (int ii = 0; ii < 4; ++ii) acc[kk][cc] = fma(v4[kk][ii], a4[cc][ii], acc[kk][cc]);
+                                for (int ii = 0; ii < 4; ++ii) MacAr<R>::mac(acc[kk][cc], v4[kk][ii], a4[cc][ii]);
                     }
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) Wy[(ks * T + k0 + kk) * LDW + g + cc * Cfg::NG4] = acc[kk][cc];
+                        for (int cc = 0; cc < 4; ++cc) Wy[(ks * T + k0 + kk) * LDW + g + cc * Cfg::NG4] = MacAr<R>::fin(acc[kk][cc]);
                 }
                 __syncthreads();
                 if (tid < RPC) substitute<R, T, Cfg::KS, LDW>(s_tau, gram, Wy, tid);
@@ -587,11 +650,11 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                     constexpr int CPT = Cfg::CPT2L;
                     const int ig = tid % Cfg::NIG, cgp = tid / Cfg::NIG;
                     const int cb = cgp * CPT;
-                    R acc[4][CPT];
+                    typename MacAr<R>::Mac acc[4][CPT];
 #pragma unroll
                     for (int cc = 0; cc < CPT; ++cc)
 #pragma unroll
-                        for (int ii = 0; ii < 4; ++ii) acc[ii][cc] = As[(cb + cc) * Cfg::LDA_L + 4 * ig + ii];
+                        for (int ii = 0; ii < 4; ++ii) acc[ii][cc] = MacAr<R>::mac_from(As[(cb + cc) * Cfg::LDA_L + 4 * ig + ii]);
                     for (int k = 0; k < T; ++k) {
                         R v4[4];
                         Vec4<R>::ld(P + k * LDP + 4 * ig, v4);
@@ -603,7 +666,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                             for (int cc = 0; cc < 4; ++cc)
 #pragma unroll
                                 for (int ii = 0; ii < 4; ++ii)
-                                    acc[ii][c4 + cc] = fma(-v4[ii], y4[cc], acc[ii][c4 + cc]);
+                                    MacAr<R>::mac(acc[ii][c4 + cc], -v4[ii], y4[cc]);
                         }
                     }
                     constexpr int VN = Vec16<R>::N;
@@ -617,12 +680,12 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                                 if (i + VN <= L) {
                                     R v[VN];
 #pragma unroll
-                                    for (int e = 0; e < VN; ++e) v[e] = acc[i0 + e][cc];
+                                    for (int e = 0; e < VN; ++e) v[e] = MacAr<R>::fin(acc[i0 + e][cc]);
                                     Vec16<R>::st(at(c0 + i, c), v);
                                 } else {
 #pragma unroll
                                     for (int e = 0; e < VN; ++e)
-                                        if (i + e < L) *at(c0 + i + e, c) = acc[i0 + e][cc];
+                                        if (i + e < L) *at(c0 + i + e, c) = MacAr<R>::fin(acc[i0 + e][cc]);
                                 }
                             }
                         }
@@ -705,7 +768,9 @@ __global__ void band_to_band_kernel(const R *ab1, int64_t n, int bw1, int64_t ld
         const int64_t r = c - ku2 + i;
         const bool in = (r >= 0 && r <= c && c - r <= bw2);
         const R v = in ? src[(ku1 + r - c) + c * ldab1] : R(0);
-        if constexpr (std::is_same<St, float2>::value) {
+        if constexpr (std::is_same<R, dfx>::value) {
+            dst[i] = make_float2(v.v.hi, v.v.lo);
+        } else if constexpr (std::is_same<St, float2>::value) {
             const float h = (float)v;
             dst[i] = make_float2(h, (float)((double)v - (double)h));
         } else {
@@ -757,6 +822,8 @@ template int band_stage<float>(float *, int64_t, int, int, int64_t, const Stage2
                                int64_t, int64_t);
 template int band_stage<double>(double *, int64_t, int, int, int64_t, const Stage2Work &, cudaStream_t, int, int,
                                 int64_t, int64_t);
+template int band_stage<dfx>(dfx *, int64_t, int, int, int64_t, const Stage2Work &, cudaStream_t, int, int, int64_t,
+                             int64_t);
 
 bool band_stage_supported(int bw, int tbw) {
     return ((bw == 256 || bw == 128) && (tbw == 32 || tbw == 16)) || (bw == 64 && tbw == 16);
@@ -774,6 +841,8 @@ template int dense_to_band<float, float>(const float *, int64_t, int64_t, int64_
                                          int, cudaStream_t);
 template int dense_to_band<double, double>(const double *, int64_t, int64_t, int64_t, int, double *, int64_t,
                                            int64_t, int, cudaStream_t);
+template int dense_to_band<double, dfx>(const double *, int64_t, int64_t, int64_t, int, dfx *, int64_t, int64_t, int,
+                                        cudaStream_t);
 
 template <typename R, typename St>
 int band_to_band(const R *dAB1, int64_t n, int bw1, int64_t ldab1, int64_t sAB1, int bw2, St *dAB2, int64_t ldab2,
@@ -788,6 +857,8 @@ template int band_to_band<float, float2>(const float *, int64_t, int, int64_t, i
                                          int64_t, int, cudaStream_t);
 template int band_to_band<double, double>(const double *, int64_t, int, int64_t, int64_t, int, double *, int64_t,
                                           int64_t, int, cudaStream_t);
+template int band_to_band<dfx, float2>(const dfx *, int64_t, int, int64_t, int64_t, int, float2 *, int64_t, int64_t,
+                                       int, cudaStream_t);
 
 template <typename R>
 int band_to_dense(const R *dAB, int64_t n, int bw, int64_t ldab, R *dA, int64_t lda, cudaStream_t s) {

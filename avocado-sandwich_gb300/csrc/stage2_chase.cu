@@ -725,15 +725,16 @@ template int stage2_chase_df<double>(const double *, int64_t, int64_t, int, floa
 // Hierarchical stage 2: the blocked band reduction bw -> tbw (stage2_band.cu;
 // the reference's bidiag! stage, BRD/src/bulgechasing2.jl:22-45), then the
 // element chase tbw -> 1 above.
-int stage2_chase_hier_df(const float *dW, int64_t n, int64_t ldw, int bw, int tbw, float *dAB1, float2 *dAB2,
+template <typename T, typename R>
+int stage2_chase_hier_df(const T *dW, int64_t n, int64_t ldw, int bw, int tbw, R *dAB1, float2 *dAB2,
                          double *dd, double *de, const Stage2Work &w, cudaStream_t s, int num_sms, int64_t *launches,
                          bool window, cudaEvent_t after_band) {
     const int64_t ldab1 = band_ldab(bw), ldab2 = 3 * (int64_t)tbw;
     int rc;
-    if ((rc = dense_to_band<float, float>(dW, n, ldw, 0, bw, dAB1, ldab1, 0, 1, s)) != AVS_SUCCESS) return rc;
-    if ((rc = band_stage<float>(dAB1, n, bw, tbw, ldab1, w, s, num_sms, 1, 0, 0)) != AVS_SUCCESS) return rc;
+    if ((rc = dense_to_band<T, R>(dW, n, ldw, 0, bw, dAB1, ldab1, 0, 1, s)) != AVS_SUCCESS) return rc;
+    if ((rc = band_stage<R>(dAB1, n, bw, tbw, ldab1, w, s, num_sms, 1, 0, 0)) != AVS_SUCCESS) return rc;
     if (after_band) AVS_CUDA_TRY(cudaEventRecord(after_band, s));
-    if ((rc = band_to_band<float, float2>(dAB1, n, bw, ldab1, 0, tbw, dAB2, ldab2, 0, 1, s)) != AVS_SUCCESS)
+    if ((rc = band_to_band<R, float2>(dAB1, n, bw, ldab1, 0, tbw, dAB2, ldab2, 0, 1, s)) != AVS_SUCCESS)
         return rc;
     if (window && chase_window_supported(tbw)) {
         if ((rc = stage2_chase_window_df(dAB2, n, tbw, w, s, num_sms)) != AVS_SUCCESS) return rc;
@@ -747,6 +748,13 @@ int stage2_chase_hier_df(const float *dW, int64_t n, int64_t ldw, int bw, int tb
     if (launches) *launches += 5;
     return AVS_SUCCESS;
 }
+
+template int stage2_chase_hier_df<float, float>(const float *, int64_t, int64_t, int, int, float *, float2 *, double *,
+                                                double *, const Stage2Work &, cudaStream_t, int, int64_t *, bool,
+                                                cudaEvent_t);
+template int stage2_chase_hier_df<double, dfx>(const double *, int64_t, int64_t, int, int, dfx *, float2 *, double *,
+                                               double *, const Stage2Work &, cudaStream_t, int, int64_t *, bool,
+                                               cudaEvent_t);
 
 int stage2_chase_hier_fp64(const double *dW, int64_t n, int64_t ldw, int bw, int tbw, double *dAB1, double *dAB2,
                            double *dd, double *de, const Stage2Work &w, cudaStream_t s, int num_sms,
@@ -809,23 +817,23 @@ __global__ void bidiag_out_batched(const typename ChaseAr<S>::St *ab, int64_t n,
 
 // Batched stage 2, the same choices as a single call's run_stages23 (so a
 // matrix's values do not depend on its batch): tbw > 0: the blocked band
-// reduction bw -> tbw (arithmetic T, band dAB as T elements, band_stride(bw,
+// reduction bw -> tbw (arithmetic R, band dAB as R elements, band_stride(bw,
 // n) per matrix), then the element chase of the narrow band (dAB2, 3 tbw x n per
 // matrix); tbw == 0: the element chase from width bw.  window: the element
 // chase in the shared-memory window (bands 8/16/32) instead of clusters.
-template <typename T, typename S>
+template <typename T, typename S, typename R = T>
 int stage2_chase_batched(const T *dW, int64_t n, int bw, int batch, typename ChaseAr<S>::St *dAB, int64_t ldab,
                          double *dd, double *de, const Stage2Work &w, cudaStream_t s, int num_sms,
                          int64_t *launches, int tbw, bool window, typename ChaseAr<S>::St *dAB2) {
     using St = typename ChaseAr<S>::St;
     if (tbw > 0) {
-        T *ab1 = reinterpret_cast<T *>(dAB);
+        R *ab1 = reinterpret_cast<R *>(dAB);
         const int64_t ldab1 = band_ldab(bw), sAB1 = band_stride(bw, n), ldab2 = 3 * (int64_t)tbw, sAB2 = ldab2 * n;
         int rc;
-        if ((rc = dense_to_band<T, T>(dW, n, n, n * n, bw, ab1, ldab1, sAB1, batch, s)) != AVS_SUCCESS) return rc;
-        if ((rc = band_stage<T>(ab1, n, bw, tbw, ldab1, w, s, num_sms, batch, sAB1, n + 1)) != AVS_SUCCESS)
+        if ((rc = dense_to_band<T, R>(dW, n, n, n * n, bw, ab1, ldab1, sAB1, batch, s)) != AVS_SUCCESS) return rc;
+        if ((rc = band_stage<R>(ab1, n, bw, tbw, ldab1, w, s, num_sms, batch, sAB1, n + 1)) != AVS_SUCCESS)
             return rc;
-        if ((rc = band_to_band<T, St>(ab1, n, bw, ldab1, sAB1, tbw, dAB2, ldab2, sAB2, batch, s)) != AVS_SUCCESS)
+        if ((rc = band_to_band<R, St>(ab1, n, bw, ldab1, sAB1, tbw, dAB2, ldab2, sAB2, batch, s)) != AVS_SUCCESS)
             return rc;
         if (window && chase_window_supported(tbw)) {
             rc = std::is_same<S, df64>::value
@@ -912,10 +920,10 @@ int stage2_chase_df_batched(const float *dW, int64_t n, int bw, int batch, float
 }
 
 int stage2_chase_df_batched(const double *dW, int64_t n, int bw, int batch, float2 *dAB, int64_t ldab, double *dd,
-                            double *de, const Stage2Work &w, cudaStream_t s, int num_sms, int64_t *launches,
-                            bool window) {
-    return stage2_chase_batched<double, df64>(dW, n, bw, batch, dAB, ldab, dd, de, w, s, num_sms, launches, 0, window,
-                                              nullptr);
+                            double *de, const Stage2Work &w, cudaStream_t s, int num_sms, int64_t *launches, int tbw,
+                            bool window, float2 *dAB2) {
+    return stage2_chase_batched<double, df64, dfx>(dW, n, bw, batch, dAB, ldab, dd, de, w, s, num_sms, launches, tbw,
+                                                   window, dAB2);
 }
 
 int stage2_chase_fp64_batched(const double *dW, int64_t n, int bw, int batch, double *dAB, int64_t ldab, double *dd,

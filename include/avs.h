@@ -82,11 +82,12 @@ extern "C" {
  * override that choice. */
 #define AVS_FLAG_FP64_STAGES 1
 #define AVS_FLAG_DF64_STAGES 2
-/* Stage 2 is hierarchical by default in the FP32-class modes, as the
+/* Stage 2 is hierarchical by default with double-float stages, as the
  * reference's bidiag! (BRD/src/bulgechasing2.jl:22-45) and the halving of
  * bidiagonalize (KAbasedSVD/src/bulgechasing.jl:33-42): a blocked band
- * reduction (T rows per sweep, compact-WY applies, FP32 arithmetic) takes the
- * band of width tile (64, 128 or 256) to width 16, then the element chase
+ * reduction (T rows per sweep, compact-WY applies; FP32 arithmetic on FP32
+ * tiles, double-float on the FP64 tiles of AVS_PREC_FP64X2) takes the band of
+ * width tile (64, 128 or 256) to width 16, then the element chase
  * (double-float) takes it to the bidiagonal.  With FP64 stages the element
  * chase runs from the band of width tile (the FP64 block stage is slower on
  * GB300's FP64 pipe) unless AVS_FLAG_HIER_CHASE asks for the hierarchy (FP64
