@@ -365,6 +365,7 @@ int run_pipeline(avs_handle *h, const Layout &L, int64_t n, int b, const TI *src
     w1.tblk = ws_at(h, L.off_tblk);
     w1.flags = reinterpret_cast<int *>(ws_at(h, L.off_flags1));
     w1.uflags = reinterpret_cast<int *>(ws_at(h, L.off_flags2));  // stage 2's, idle in stage 1
+    w1.mail = ws_at(h, L.off_ab2);                                // the same
     w1.err = err;
     w1.tfull = ws_at(h, L.off_tfull);
     w1.tc_split = tc_split;
@@ -662,6 +663,7 @@ int blockbidiag_dev(avs_handle *h, int64_t n, int64_t lda, int32_t tile, T *dA, 
     w1.tblk = ws_at(h, L.off_tblk);
     w1.flags = reinterpret_cast<int *>(ws_at(h, L.off_flags1));
     w1.uflags = reinterpret_cast<int *>(ws_at(h, L.off_flags2));  // stage 2's, idle in stage 1
+    w1.mail = ws_at(h, L.off_ab2);                                // the same
     w1.err = err;
     w1.tfull = ws_at(h, L.off_tfull);
     w1.tc_split = split;
@@ -720,6 +722,7 @@ int geqrf_dev(avs_handle *h, int64_t n, int64_t lda, int32_t tile, T *dA, T *dta
     w1.tblk = ws_at(h, L.off_tblk);
     w1.flags = reinterpret_cast<int *>(ws_at(h, L.off_flags1));
     w1.uflags = reinterpret_cast<int *>(ws_at(h, L.off_flags2));  // stage 2's, idle in stage 1
+    w1.mail = ws_at(h, L.off_ab2);                                // the same
     w1.err = err;
     w1.tfull = ws_at(h, L.off_tfull);
     w1.tc_split = split;
@@ -786,6 +789,7 @@ int tile_kernel(avs_handle *h, int32_t b, T *dA, T *dB, T *dtau, bool ts) {
     w1.tblk = ws_at(h, L.off_tblk);
     w1.flags = reinterpret_cast<int *>(ws_at(h, L.off_flags1));
     w1.uflags = reinterpret_cast<int *>(ws_at(h, L.off_flags2));  // stage 2's, idle in stage 1
+    w1.mail = ws_at(h, L.off_ab2);                                // the same
     w1.err = err;
     w1.tfull = ws_at(h, L.off_tfull);
     if (!ts) {
@@ -1270,6 +1274,8 @@ int group_launches(avs_handle *h, const BatchLayout &L, int64_t n, int b, int cn
     w1.flags = reinterpret_cast<int *>(base + L.f1);
     w1.uflags = reinterpret_cast<int *>(base + L.f2);  // stage 2's, idle in stage 1
     w1.sUflags = n + 1;
+    w1.mail = base + L.ab2;
+    w1.sMail = 3 * kMaxNarrowBand * n;
     w1.err = err;
     w1.batch = cnt;
     w1.sA = n * n;

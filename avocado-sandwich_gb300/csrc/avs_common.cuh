@@ -108,6 +108,10 @@ struct Stage1Work {
     int *flags;       // ticket (1) + two progress counters per tile (2 nt), reset per launch
     int *uflags = nullptr;  // optional: counters of the update of tiles 16-64 (n / 8 + 1 ints, stage 2's flags)
     int64_t sUflags = 0;    // ints between matrices (batched)
+    // optional: the panel's mailbox, 32 n elements of T (the narrow band's buffer,
+    // idle in stage 1); without it (out of core) the diagonal blocks go through the matrix
+    void *mail = nullptr;
+    int64_t sMail = 0;      // doubles between matrices (batched)
     int *err;         // device status word (shared with other stages)
     void *tfull;      // [nt][b*b] of T: full compact-WY factors (tiles 128, 256)
     void *tc_ws = nullptr;  // tensor-core update buffers (stage1_tc_bytes), FP32 tiles

@@ -14,16 +14,17 @@
 //
 // Panel kernel.  Role 0 runs GEQRT on the top tile; role p >= 1 runs TSQRT on
 // [R; tile p], exactly the flat tree of the reference.  Reflectors of
-// different roles that touch different rows commute, so role p may process
-// its column block cb as soon as role p-1 has finished block cb: the roles form
-// a systolic pipeline over the row tiles whose critical path is
-// (#tiles + b/16) block steps instead of #tiles * b reflector steps.  Within a
-// block the 16 reflectors are generated one column at a time, and the block is
-// applied to the rest of the tile in compact-WY form (16 reflectors).  A role hands block cb on in two parts: the 16 x 16
-// diagonal block of the top rows right after its reflectors (all the next
-// role's reflectors read), and the trailing top rows after its apply (which the
-// next role reads only in its own apply), so the step between roles is one
-// reflector loop.  Roles are handed out by an atomic ticket in launch order,
+// different roles that touch different rows commute, and step i of a TSQRT block
+// reads row i of the block's diagonal block only, so role p runs its step i as soon
+// as role p-1 has finished step i: the roles form a systolic pipeline over the row
+// tiles whose critical path is one hand-off per tile plus the reflector steps of one
+// tile, instead of #tiles * b reflector steps.  Within a block the 16 reflectors are
+// generated one column at a time, and the block is applied to the rest of the tile
+// in compact-WY form (16 reflectors).  A role hands block cb on in two parts: the
+// rows of the 16 x 16 diagonal block one by one as its reflectors make them (all the
+// next role's reflectors read), and the trailing top rows after its apply (which the
+// next role reads only in its own apply).  Roles are handed out by an atomic ticket in
+// launch order,
 // so a role only ever waits on a role already running: no co-residency
 // assumption, and every wait is bounded.  The panel computes in its tile type,
 // except with the double-float trailing updates of FP64 tiles (AVS_PREC_FP64X2),
@@ -70,7 +71,9 @@ struct PanelArgs {
     int *err;
     const int *ready;  // optional: role p's tile is final once ready[p] >= ready_need
     int ready_need;
-    int64_t sA, sTau, sTblk, sFlags;  // per-matrix strides (blockIdx.y = matrix)
+    unsigned long long *mail;  // optional: rows of the diagonal blocks, role to role (tagged words)
+    unsigned tag;              // this launch's tag, never 0
+    int64_t sA, sTau, sTblk, sFlags, sMail;  // per-matrix strides (blockIdx.y = matrix)
 };
 
 struct UpdateArgs {
@@ -300,6 +303,50 @@ __device__ __forceinline__ void bar_named(int id, int cnt) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(cnt) : "memory");
 }
 
+// One value with its tag, role to role through L2: a 64-bit word {32 bits, tag},
+// two of them for an 8-byte type.  A word is written and read whole, so a value
+// whose tags are this launch's is complete, with no flag and no fence beside it.
+__device__ __forceinline__ void mail_put(unsigned long long *at, float v, unsigned tag) {
+    const unsigned long long w = ((unsigned long long)tag << 32) | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(at), "l"(w) : "memory");
+}
+__device__ __forceinline__ void mail_put2(unsigned long long *at, unsigned a, unsigned b, unsigned tag) {
+    const unsigned long long t = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(at), "l"(t | a), "l"(t | b) : "memory");
+}
+__device__ __forceinline__ void mail_put(unsigned long long *at, double v, unsigned tag) {
+    mail_put2(at, (unsigned)__double2loint(v), (unsigned)__double2hiint(v), tag);
+}
+__device__ __forceinline__ void mail_put(unsigned long long *at, dfx v, unsigned tag) {
+    mail_put2(at, __float_as_uint(v.v.hi), __float_as_uint(v.v.lo), tag);
+}
+__device__ __forceinline__ bool mail_get(const unsigned long long *at, float &v, unsigned tag) {
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(at) : "memory");
+    v = __uint_as_float((unsigned)w);
+    return (unsigned)(w >> 32) == tag;
+}
+__device__ __forceinline__ bool mail_get2(const unsigned long long *at, unsigned &a, unsigned &b, unsigned tag) {
+    unsigned long long x, y;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(at) : "memory");
+    a = (unsigned)x;
+    b = (unsigned)y;
+    return (unsigned)(x >> 32) == tag && (unsigned)(y >> 32) == tag;
+}
+__device__ __forceinline__ bool mail_get(const unsigned long long *at, double &v, unsigned tag) {
+    unsigned a, b;
+    const bool ok = mail_get2(at, a, b, tag);
+    v = __hiloint2double((int)b, (int)a);
+    return ok;
+}
+__device__ __forceinline__ bool mail_get(const unsigned long long *at, dfx &v, unsigned tag) {
+    unsigned a, b;
+    const bool ok = mail_get2(at, a, b, tag);
+    v = dfx(df64{__uint_as_float(a), __uint_as_float(b)});
+    return ok;
+}
+__device__ __forceinline__ int ld_shared_volatile(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
+
 // ---------------------------------------------------------------------------
 // Panel kernel (roles, schedule and outputs as described at the top).
 //
@@ -313,8 +360,14 @@ __device__ __forceinline__ void bar_named(int id, int cnt) {
 //     pairs beside them.  (With a row per lane the 16 dot products took a warp
 //     reduce-scatter of 423 cycles a step.)  Across warps one shared-memory pass
 //     and one barrier of the b / 32 reflector warps, none for tiles 16 and 32;
-//   * a TSQRT step changes one row of the diagonal block only, so that block is
-//     read once per block and each new row goes straight to global memory;
+//   * a TSQRT step changes one row of the diagonal block only: each new row goes to
+//     the next role at once, as tagged words through L2 that the next role's fetch warp
+//     polls and lays in shared memory ahead of its reflectors (about 1.5 k cycles from
+//     role to role; with whole blocks behind a counter the hand-off cost the 16 steps
+//     too, 9.5 k: stage 1 of FP32 n = 1296 tile 16 49.3 -> 17.7 ms, n = 2048 tile 64 17.2
+//     -> 11.3, n = 4096 tile 128 39.1 -> 32.5, split BF16 n = 5760 tile 128 49.2 -> 36.1,
+//     FP64 n = 1024 tile 64 28.2 -> 20.6).  Only the last role writes the rows to the
+//     matrix;
 //   * the block reflector is applied from the Gram matrix, not from T: with
 //     G = Y^T Y and T^-1 = diag(1/tau) + striu(G), W = T^T Z is the forward
 //     substitution w_l = tau_l (z_l - sum_{m<l} G_ml w_m), one thread per
@@ -331,15 +384,23 @@ __device__ __forceinline__ void bar_named(int id, int cnt) {
 // shared memory, a row per lane, explicit T): FP32 n = 1296 tile 16 195 -> 75 ms,
 // n = 1024 tile 64 20.4 -> 14.1, n = 4096 tile 128 91.8 -> 63.8, split BF16 n =
 // 5760 tile 128 96.8 -> 49.8, n = 16384 tile 256 344 -> 276; FP64 n = 1024 tile 64
-// 78.0 -> 43.0, double-float n = 2048 tile 128 103 -> 66.  A block of 16
+// 78.0 -> 43.0, double-float n = 2048 tile 128 103 -> 66; then the row hand-off above.
+// A block of 16
 // reflectors: 9.5 k cycles (tile 16), 14.5 k (64), 17 k (128), 21 k (256), before
 // about 48 k.
+// Who fetches a block's top rows: a warp of its own, a warp that the reflectors leave
+// idle, or the first reflector warp (whole blocks, no mailbox).
+enum : int { kFetchNone, kFetchIdle, kFetchOwn };
 template <typename CT, int B>
 struct PanelCfg {
     static constexpr int NB = B / kIB;
     static constexpr int NWR = B >= 32 ? B / 32 : 1;  // reflector warps
     static constexpr int RPL = (B >= 32 ? 32 : B) / 2;  // rows per lane
     static constexpr int NT = B >= 128 ? 256 : (B == 64 ? 128 : (B == 32 ? 64 : 32));
+    // tiles up to 64 have the registers for one more warp (a ninth one would leave the
+    // others 168), 128 has idle ones; at 256 every warp has reflector rows
+    static constexpr int FETCH = B <= 64 ? kFetchOwn : (B == 128 ? kFetchIdle : (sizeof(CT) == 4 ? kFetchOwn : kFetchNone));
+    static constexpr int NTL = NT + (FETCH == kFetchOwn ? 32 : 0);  // threads launched
     static constexpr int NW = NT / 32;
     static constexpr bool F4 = sizeof(CT) == 4;
     static constexpr int YLD = F4 ? 20 : 18;      // row stride of Y and W (16-byte rows, conflict-free vectors)
@@ -371,14 +432,118 @@ struct PanelCfg {
         return m;
     }
     static constexpr size_t smem_bytes() {  // in the order of the kernel's carving
-        return 16 * NWR + sizeof(CT) * (2 * NWR * kIB + 2 * NWR * 32 + 2 * kIB + kIB + kIB * (kIB + 4) + kIB * kIB +
+        return 16 * NWR + sizeof(CT) * (2 * NWR * kIB + 2 * NWR * 32 + 2 * kIB + kIB + 2 * kIB * (kIB + 4) + kIB * kIB +
                                        (F4 ? NW * kIB * kIB : 0) + (size_t)B * YLD +
                                        (NB > 1 ? (size_t)NR * YLD + (size_t)kIB * zcols() + (size_t)RESC * CLD : 0));
     }
 };
 
+// The fetch warp of a TSQRT role, block cb: top row i from the role ahead, as soon as
+// that role has made it, into dst; `rows` counts the rows in place.  Four rows are
+// polled at a time, so that the poll's round trip is paid once for them.  Without a
+// mailbox the whole block comes from the matrix, once the role ahead (if one runs)
+// counts it done.  False: gave up (the reflector warps stop waiting and the role ends
+// at their barrier).
+template <typename T, int LAYOUT, typename CT, int NB>
+__device__ __forceinline__ bool fetch_top(const View<T, LAYOUT> &V, int64_t top0, int64_t col0, int cb, bool follow,
+                                          const unsigned long long *box, unsigned tag, const int *progress, CT *dst,
+                                          int *rows, int *fail, int *err) {
+    constexpr int MW = sizeof(CT) / 4;
+    const int lane = threadIdx.x & 31, jc = lane & (kIB - 1), rr = lane >> 4;
+    const int c0 = cb * kIB;
+    auto give_up = [&]() {
+        if (lane == 0) {
+            *reinterpret_cast<volatile int *>(fail) = 1;
+            __threadfence_block();
+            *reinterpret_cast<volatile int *>(rows) = kIB * NB;
+        }
+        return false;
+    };
+    if (follow && box) {
+        const unsigned long long *src = box + (size_t)cb * kIB * kIB * MW;
+        const long long t0 = clock64();
+        int done = 0;
+#pragma unroll 1
+        for (long long it = 0; done < kIB; ++it) {
+            const int r0 = done + rr, r1 = done + 2 + rr;
+            CT v0 = CT(0), v1 = CT(0);
+            bool ok0 = r0 < kIB, ok1 = r1 < kIB;
+            if (ok0 && jc >= r0) ok0 = mail_get(src + (r0 * kIB + jc) * MW, v0, tag);
+            if (ok1 && jc >= r1) ok1 = mail_get(src + (r1 * kIB + jc) * MW, v1, tag);
+            const unsigned b0 = __ballot_sync(0xffffffffu, ok0), b1 = __ballot_sync(0xffffffffu, ok1);
+            int got = 0;  // rows done, done + 1, ... that are all here
+            if ((b0 & 0xffffu) == 0xffffu) {
+                got = 1;
+                if ((b0 >> 16) == 0xffffu) {
+                    got = 2;
+                    if ((b1 & 0xffffu) == 0xffffu) got = (b1 >> 16) == 0xffffu ? 4 : 3;
+                }
+            }
+            if (rr < got) dst[r0 * (kIB + 4) + jc] = v0;
+            if (2 + rr < got) dst[r1 * (kIB + 4) + jc] = v1;
+            if (got > 0) {
+                __threadfence_block();
+                __syncwarp();
+                done += got;
+                if (lane == 0) *reinterpret_cast<volatile int *>(rows) = c0 + done;
+            } else if ((it & 15) == 15) {  // another role's failure, the bounds: every 16 polls
+                int stop = 0;
+                if (lane == 0) {
+                    stop = ld_acquire(err) != kDevOk;
+                    if (!stop && (it > kSpinLimit || clock64() - t0 > 2 * kWaitNs)) {
+                        atomicCAS(err, kDevOk, kDevTimeout);
+                        stop = 1;
+                    }
+                }
+                if (__shfl_sync(0xffffffffu, stop, 0)) return give_up();
+                if (it > 64) __nanosleep(20);
+            }
+        }
+    } else {
+        int ok = 1;
+        if (follow && lane == 0) ok = wait_geq(progress, cb + 1, err) ? 1 : 0;
+        if (!__shfl_sync(0xffffffffu, ok, 0)) return give_up();
+        constexpr int RU = kIB * kIB / 32;  // all loads in flight
+        T v[RU];
+#pragma unroll
+        for (int u = 0; u < RU; ++u) {
+            const int idx = lane + u * 32;
+            const int l = LAYOUT == 0 ? idx % kIB : idx / kIB;
+            const int j = LAYOUT == 0 ? idx / kIB : idx % kIB;
+            v[u] = __ldcg(&V(top0 + c0 + l, col0 + c0 + j));
+        }
+#pragma unroll
+        for (int u = 0; u < RU; ++u) {
+            const int idx = lane + u * 32;
+            const int l = LAYOUT == 0 ? idx % kIB : idx / kIB;
+            const int j = LAYOUT == 0 ? idx / kIB : idx % kIB;
+            dst[l * (kIB + 4) + j] = CT(v[u]);
+        }
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) *reinterpret_cast<volatile int *>(rows) = c0 + kIB;
+    }
+    return true;
+}
+// The reflector warps' wait for `need` top rows; returns the rows in place.
+__device__ __forceinline__ int wait_rows(const int *rows, int need, int *fail, int *err) {
+    int have = ld_shared_volatile(rows);
+    if (have < need) {
+        const long long t0 = clock64();
+        for (long long it = 0; (have = ld_shared_volatile(rows)) < need; ++it) {
+            if ((it & 1023) == 1023 && clock64() - t0 > 4 * kWaitNs) {  // the fetch warp gives up before this
+                *reinterpret_cast<volatile int *>(fail) = 1;
+                atomicCAS(err, kDevOk, kDevTimeout);
+                break;
+            }
+        }
+    }
+    __syncwarp();
+    return have;
+}
+
 template <typename T, int LAYOUT, typename CT, int B>
-__global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs args) {
+__global__ void __launch_bounds__(PanelCfg<CT, B>::NTL) panel_kernel(PanelArgs args) {
     using Cfg = PanelCfg<CT, B>;
     using Ar = PAr<CT>;
     using Sq = typename Ar::Sq;
@@ -386,6 +551,7 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
     constexpr int NB = Cfg::NB, NWR = Cfg::NWR, NT = Cfg::NT, NW = Cfg::NW, YLD = Cfg::YLD, CLD = Cfg::CLD;
     constexpr int RPL = Cfg::RPL, RESC = Cfg::RESC, S0 = Cfg::S0;
     constexpr int TV = PVec<T>::VN, CV = PVec<CT>::VN;
+    constexpr int MW = sizeof(CT) / 4;  // mailbox words per value
     static_assert(sizeof(Sq) == 8 && sizeof(CT) == sizeof(T), "panel types");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Sq *spart = reinterpret_cast<Sq *>(smem_raw);                 // [2][NWR]
@@ -393,8 +559,8 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
     CT *xs = part + 2 * NWR * kIB;                                // [2][NWR][32] the step's column
     CT *rowb = xs + 2 * NWR * 32;                                 // [2][16]
     CT *stau = rowb + 2 * kIB;                                    // [16]
-    CT *Rts = stau + kIB;                                         // [16][20], Rts[l * 20 + j]
-    CT *G = Rts + kIB * (kIB + 4);                                // [16][16], G[l * 16 + m] = y_l^T y_m
+    CT *Rbuf = stau + kIB;                                        // [2][16][20], block cb's top rows [l * 20 + j]
+    CT *G = Rbuf + 2 * kIB * (kIB + 4);                              // [16][16], G[l * 16 + m] = y_l^T y_m
     CT *Gp = G + kIB * kIB;                                       // FP32: [NW][16][16]
     CT *Yr = Gp + (Cfg::F4 ? NW * kIB * kIB : 0);                 // [B][YLD]
     CT *Ws = Yr + (size_t)B * YLD;                                // [columns][YLD]
@@ -402,12 +568,14 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
     CT *Cs = Zp + (NB > 1 ? (size_t)kIB * Cfg::zcols() : 0);      // [column - S0][CLD]
 
     __shared__ int s_role, s_ok, s_fail;
+    __shared__ int s_rows, s_used;  // top rows fetched, blocks whose reflectors are done
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int64_t zb = blockIdx.y;
     int *progress = args.progress + zb * args.sFlags;
     if (tid == 0) {
         s_role = atomicAdd(args.ticket + zb * args.sFlags, 1) + args.first_role;
         s_fail = 0;
+        s_rows = s_used = 0;
     }
     __syncthreads();
     const int p = s_role;
@@ -428,6 +596,32 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
         if (!s_ok) return;
     }
     int *full = progress + args.P;  // per role: block cb's trailing top rows are final
+
+    const bool mail = Cfg::FETCH != kFetchNone && args.mail != nullptr;
+    const bool last = p == args.P - 1;
+    unsigned long long *box = mail ? args.mail + zb * args.sMail + (size_t)p * NB * kIB * kIB * MW : nullptr;
+    const unsigned long long *from = mail && !geqrt ? box - (size_t)NB * kIB * kIB * MW : nullptr;
+    if constexpr (Cfg::FETCH == kFetchOwn) {  // a warp of its own: a block ahead of the reflectors
+        if (wid == NW) {
+            if (geqrt) return;
+            const long long t0 = clock64();
+            for (int cb = 0; cb < NB; ++cb) {
+                for (long long it = 0; ld_shared_volatile(&s_used) < cb - 1; ++it) {  // block cb - 2 still in use
+                    if (ld_shared_volatile(&s_fail)) return;
+                    if (it > kSpinLimit || clock64() - t0 > 8 * kWaitNs) {
+                        if (lane == 0) *reinterpret_cast<volatile int *>(&s_fail) = 1;
+                        return;
+                    }
+                    __nanosleep(64);
+                }
+                __syncwarp();
+                if (!fetch_top<T, LAYOUT, CT, NB>(V, top0, col0, cb, follow, from, args.tag, progress + p - 1,
+                                                  Rbuf + (cb & 1) * kIB * (kIB + 4), &s_rows, &s_fail, args.err))
+                    return;
+            }
+            return;
+        }
+    }
 
     // my column of the block and my rows of it (reflector warps)
     const bool refl = wid < NWR;
@@ -467,35 +661,13 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
         CT *ZpS = Zp + (size_t)kIB * KR * nr;  // the streamed part's partial Z
 
         if (refl) {
-            // ---- the diagonal 16 x 16 block of the top rows, once the previous
-            // role's reflectors of this block are in it (TSQRT)
-            if (!geqrt) {
-                if (follow) {
-                    if (lane == 0 && !wait_geq(progress + p - 1, cb + 1, args.err)) s_fail = 1;
-                    __syncwarp();
+            const CT *Rts = Rbuf + (cb & 1) * kIB * (kIB + 4);  // this block's top rows (TSQRT)
+            if constexpr (Cfg::FETCH == kFetchNone) {  // read by the reflector warps themselves
+                if (!geqrt) {
+                    if (wid == 0) fetch_top<T, LAYOUT, CT, NB>(V, top0, col0, cb, follow, nullptr, args.tag, progress + p - 1,
+                                                     Rbuf + (cb & 1) * kIB * (kIB + 4), &s_rows, &s_fail, args.err);
+                    bar_named(1, NWR * 32);
                 }
-                {
-                    constexpr int RU = kIB * kIB / (NWR * 32);  // all loads in flight
-                    T v[RU];
-#pragma unroll
-                    for (int u = 0; u < RU; ++u) {
-                        const int idx = tid + u * NWR * 32;
-                        const int l = LAYOUT == 0 ? idx % kIB : idx / kIB;
-                        const int j = LAYOUT == 0 ? idx / kIB : idx % kIB;
-                        v[u] = __ldcg(&V(top0 + c0 + l, col0 + c0 + j));
-                    }
-#pragma unroll
-                    for (int u = 0; u < RU; ++u) {
-                        const int idx = tid + u * NWR * 32;
-                        const int l = LAYOUT == 0 ? idx % kIB : idx / kIB;
-                        const int j = LAYOUT == 0 ? idx / kIB : idx % kIB;
-                        Rts[l * (kIB + 4) + j] = CT(v[u]);
-                    }
-                }
-                // a hardware barrier for one warp too: after the divergent wait it puts the
-                // warp back in step (with __syncwarp alone a block of a 16-wide tile took
-                // 65 us instead of 7)
-                bar_named(1, NWR * 32);
             }
             // ---- the 16 reflectors of the block, one per step: a loop, not unrolled
             // (a step is some 200 instructions, and straight-line code that a single
@@ -521,7 +693,10 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
             const int nstep = (geqrt && cb == NB - 1) ? kIB - 1 : kIB;  // the last column has no reflector
             T *ptop = &V(top0 + c0, col0 + c0 + jc);
             const int64_t dtop = LAYOUT == 0 ? 1 : args.lda;
-            const bool out_top = !geqrt && tid < kIB;
+            const bool out_top = tid < kIB && (!geqrt || (mail && !last));
+            const bool post = mail && !last;  // the new top row: to the next role, from the last one to the matrix
+            unsigned long long *pbox = box + ((size_t)cb * kIB * kIB + jc) * MW;
+            int avail = geqrt ? kIB * NB : 0;
 #pragma unroll 1
             for (int i = 0; i < nstep; ++i) {
                 const int pb = i & 1;
@@ -581,6 +756,7 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
                 } else {
                     __syncwarp();
                 }
+                if (avail <= cb * kIB + i) avail = wait_rows(&s_rows, cb * kIB + i + 1, &s_fail, args.err);
                 const CT *prow = geqrt ? rowb + pb * kIB : Rts + i * (kIB + 4);
                 const CT rj = prow[jc];
                 const PRefl<CT> r = Ar::scalars(sq, prow[i]);
@@ -595,7 +771,10 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
                     for (int q = 0; q < RPL; ++q) col[q] = (own && jc >= i && i % RPL == q) ? top : col[q];
                 }
                 if (i < kIB - 1) put_x(i + 1);
-                if (out_top && jc >= i) ptop[i * dtop] = (T)top;
+                if (out_top && jc >= i) {
+                    if (post) mail_put(pbox + i * kIB * MW, top, args.tag);
+                    else ptop[i * dtop] = (T)top;
+                }
                 mytau = jc == i ? r.tau : mytau;
                 myinv = jc == i ? r.inv : myinv;
                 __syncwarp();
@@ -603,15 +782,23 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
             if (bad && lane == 0) atomicCAS(args.err, kDevOk, kDevNonfinite);
             if (tid < kIB) stau[tid] = mytau;
             __syncwarp();
-            // the diagonal block of the top rows is final for this role: handed on -- a
-            // TSQRT role's successor needs only this block for its own reflectors
-            if (!geqrt && tid == 0) st_release(progress + p, cb + 1);
+            // without the mailbox the diagonal block is handed on whole, here; the last
+            // row of the last block has no reflector
+            if (!geqrt && !mail && tid == 0) st_release(progress + p, cb + 1);
+            if (geqrt && post && cb == NB - 1 && jc == kIB - 1 && rb + RPL == B)
+                mail_put(pbox + (kIB - 1) * kIB * MW, col[RPL - 1], args.tag);
             // ---- V (each column scaled by its 1 / nu) back to the tile, and the
             // masked Y (unit lower for GEQRT)
 #pragma unroll
             for (int r = 0; r < RPL; ++r)
                 if (!geqrt || rb + r > c0 + jc) col[r] = col[r] * myinv;
-            if (!geqrt || rb >= c0) store_col<T, LAYOUT, CT, RPL>(V, row0 + rb, col0 + c0 + jc, col);
+            if (geqrt && post && rb >= c0 && rb < c0 + kIB) {  // the rows above the diagonal are the last role's to write
+#pragma unroll
+                for (int r = 0; r < RPL; ++r)
+                    if (rb + r > c0 + jc) V(row0 + rb + r, col0 + c0 + jc) = (T)col[r];
+            } else if (!geqrt || rb >= c0) {
+                store_col<T, LAYOUT, CT, RPL>(V, row0 + rb, col0 + c0 + jc, col);
+            }
 #pragma unroll
             for (int r = 0; r < RPL; ++r) {
                 CT y = col[r];
@@ -619,11 +806,18 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
                 Yr[(size_t)(rb + r) * YLD + jc] = y;
             }
         }
-        __syncthreads();
-        if (s_fail) return;
-        // the block's rows of the top tile are written back above (the release
-        // covers what the barrier ordered before it)
-        if (geqrt && tid == 0) st_release(progress, cb + 1);
+        if constexpr (Cfg::FETCH == kFetchIdle) {
+            if (wid == NWR && !geqrt)
+                fetch_top<T, LAYOUT, CT, NB>(V, top0, col0, cb, follow, from, args.tag, progress + p - 1,
+                                             Rbuf + (cb & 1) * kIB * (kIB + 4), &s_rows, &s_fail, args.err);
+        }
+        if (tid == 0) s_ok = !ld_shared_volatile(&s_fail);
+        bar_named(2, NT);
+        if (!s_ok) return;
+        if (tid == 0) *reinterpret_cast<volatile int *>(&s_used) = cb + 1;
+        // without the mailbox: the block's rows of the top tile are written back above
+        // (the release covers what the barrier ordered before it)
+        if (geqrt && !mail && tid == 0) st_release(progress, cb + 1);
         if (tid < kIB) tau_out[c0 + tid] = (T)stau[tid];
 
         // ---- Gram matrix of the block's reflectors
@@ -768,7 +962,7 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
                 }
             }
         }
-        __syncthreads();
+        bar_named(2, NT);
         if constexpr (Cfg::F4) {
             for (int idx = tid; idx < kIB * kIB; idx += NT) {
                 CT v = Gp[idx];
@@ -778,8 +972,11 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
             }
         }
         // the trailing top rows, once the previous role's are in them
-        if (tid == 0) s_ok = (follow && nrest > 0) ? wait_geq(full + p - 1, cb + 1, args.err) : true;
-        __syncthreads();
+        if (tid == 0) {
+            s_ok = (follow && nrest > 0) ? wait_geq(full + p - 1, cb + 1, args.err) : true;
+            if (!s_ok) *reinterpret_cast<volatile int *>(&s_fail) = 1;  // for the fetch warp
+        }
+        bar_named(2, NT);
         if (!s_ok) return;
 
         // ---- W = T^T (Z + top rows) by forward substitution; top rows -= W.  The 16
@@ -828,7 +1025,7 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
                 }
             }
         }
-        __syncthreads();
+        bar_named(2, NT);
         if constexpr (NB > 1) {
             // a TSQRT role hands the trailing top rows on before updating its own tile
             if (!geqrt && tid == 0) st_release(full + p, cb + 1);
@@ -954,7 +1151,7 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NT) panel_kernel(PanelArgs ar
                     }
                 }
             }
-            __syncthreads();
+            bar_named(2, NT);
         }
         if (geqrt && tid == 0) st_release(full, cb + 1);
     }
@@ -1231,7 +1428,7 @@ int launch_panel_b(const PanelArgs &a, dim3 grid, cudaStream_t s) {
                                           (int)smem));
         attr_set = true;
     }
-    panel_kernel<T, LAYOUT, CT, B><<<grid, Cfg::NT, smem, s>>>(a);
+    panel_kernel<T, LAYOUT, CT, B><<<grid, Cfg::NTL, smem, s>>>(a);
     AVS_CUDA_TRY(cudaGetLastError());
     return AVS_SUCCESS;
 }
@@ -1245,6 +1442,18 @@ int launch_panel_ct(const PanelArgs &a, dim3 grid, cudaStream_t s) {
         case 256: return launch_panel_b<T, LAYOUT, CT, 256>(a, grid, s);
         default: return AVS_ERR_UNSUPPORTED;
     }
+}
+
+// The panels' mailbox, cleared of any word that could pass for one of this call's
+// (tags 1, 2, ...): b rows of 16 values for each of nt tiles.
+template <typename T>
+int panel_mail_reset(const Stage1Work &w, int64_t n, cudaStream_t s) {
+    if (!w.mail) return AVS_SUCCESS;
+    const size_t bytes = 2 * sizeof(T) * (size_t)n * kIB;
+    const int batch = w.batch > 0 ? w.batch : 1;
+    if (batch == 1) AVS_CUDA_TRY(cudaMemsetAsync(w.mail, 0, bytes, s));
+    else AVS_CUDA_TRY(cudaMemset2DAsync(w.mail, sizeof(double) * (size_t)w.sMail, 0, bytes, batch, s));
+    return AVS_SUCCESS;
 }
 
 // FP64 tiles with the double-float trailing updates (AVS_PREC_FP64X2) run
@@ -1274,6 +1483,9 @@ int launch_panel(T *dA, int64_t lda, int b, int pr, int pc, int P, int first_rol
     a.sTau = w.sTau;
     a.sTblk = w.sTblk;
     a.sFlags = w.sFlags;
+    a.mail = P - first_role > 1 && first_role == 0 ? static_cast<unsigned long long *>(w.mail) : nullptr;
+    a.tag = (unsigned)(pr + pc + 1);  // half-step k of a call: 2 k + 1 (QR) or 2 k + 2 (LQ)
+    a.sMail = w.sMail;
     a.ready = ready;
     a.ready_need = b / kChainStrip;
     const dim3 grid(P - first_role, batch);
@@ -1406,6 +1618,7 @@ int stage1_ge2bnd_tc(float *X, int64_t n, int b, const Stage1Work &w, cudaStream
     int rc, dev = 0, sms = 0;
     AVS_CUDA_TRY(cudaGetDevice(&dev));
     AVS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if ((rc = panel_mail_reset<float>(w, n, s)) != AVS_SUCCESS) return rc;
     if ((rc = stage1_tc_planes(X, n, fmt, tb, s)) != AVS_SUCCESS) return rc;
     // panel + tau copy + T build of one half-step on the aux stream, after the
     // caller's stream has reached this point (or the point where it recorded
@@ -1489,6 +1702,7 @@ int stage1_ge2bnd(T *dA, int64_t n, int64_t lda, int b, const Stage1Work &w, cud
         if (w.tc_split && w.tc_ws && b >= 128 && lda == n && (w.batch <= 1))
             return stage1_ge2bnd_tc(reinterpret_cast<float *>(dA), n, b, w, s, launches);
     }
+    if ((rc = panel_mail_reset<T>(w, n, s)) != AVS_SUCCESS) return rc;
     for (int k = 0; k < nt; ++k) {
         // QR half-step: GEQRT(k,k) + TSQRT(row,k), Q^T applied to the row panels.
         const int P = nt - k;
@@ -1528,6 +1742,7 @@ int stage1_geqrf(T *dA, int64_t n, int64_t lda, int b, const Stage1Work &w, T *d
     const bool tc = sizeof(T) == 4 && w.tc_split && w.tc_ws && b >= 128 && lda == n && w.batch <= 1;
     TcBufs tb{};
     if (tc) tb = stage1_tc_carve(w.tc_ws, n, b, w.tc_split);
+    if ((rc = panel_mail_reset<T>(w, n, s)) != AVS_SUCCESS) return rc;
     for (int k = 0; k < nt; ++k) {
         const int P = nt - k;
         if ((rc = launch_panel<T, 0>(dA, lda, b, k, k, P, 0, w, s)) != AVS_SUCCESS) return rc;
