@@ -25,6 +25,44 @@ __device__ __forceinline__ df64 df_from_double(double x) {
     return df64{h, (float)(x - (double)h)};
 }
 __device__ __forceinline__ double df_to_double(df64 a) { return (double)a.hi + (double)a.lo; }
+// FP64 <-> double-float on the integer pipe: hi + lo rounded as (float)x and
+// (float)(x - hi), and (double)hi + (double)lo, exactly (an exact tie of hi goes up
+// instead of to even; hi + lo is the same).  The FP64 instructions for them, three
+// either way, issue at 64 cycles per warp on GB300: with all warps converting they took
+// as long as the products of a double-float trailing update.  Some 15 instructions,
+// so a loss where few warps convert (the panels: FP64 tiles of 64 n = 1024 stage 1 14.9
+// -> 15.8 ms).  Exponents within [-74, 126] and zeros; anything else takes the FP64
+// instructions.
+__device__ __forceinline__ df64 df_from_double_int(double x) {
+    const unsigned lo32 = (unsigned)__double2loint(x), hi32 = (unsigned)__double2hiint(x);
+    const unsigned ahi = hi32 & 0x7fffffffu, sgn = hi32 & 0x80000000u;
+    const unsigned ex = ahi >> 20;
+    if (ex - (1023u - 74u) <= 200u) {
+        const unsigned rl = lo32 + 0x10000000u, rh = ahi + (rl < lo32 ? 1u : 0u);  // + half a unit of hi
+        const unsigned h = __funnelshift_r(rl, rh, 29) - ((1023u - 127u) << 23);
+        const int rem = (int)(lo32 - (rl & 0xe0000000u));  // in units of 2^(ex - 1023 - 52)
+        const float sc = __uint_as_float((ex - (1023u - 127u) - 52u) << 23);
+        return df64{__uint_as_float(h | sgn), __uint_as_float(__float_as_uint(__fmul_rn((float)rem, sc)) ^ sgn)};
+    }
+    if ((ahi | lo32) == 0u) return df64{0.0f, 0.0f};
+    return df_from_double(x);
+}
+__device__ __forceinline__ double df_to_double_int(df64 a) {
+    const unsigned hb = __float_as_uint(a.hi), ah = hb & 0x7fffffffu, sgn = hb & 0x80000000u;
+    const unsigned ex = ah >> 23;
+    if (ex - (127u - 74u) <= 200u && fabsf(a.lo) <= __fmul_rn(fabsf(a.hi), 0x1p-22f)) {
+        // hi + lo in units of 2^(ex - 127 - 52), half of that just below a power of two
+        const float sl = __uint_as_float(__float_as_uint(a.lo) ^ sgn);  // lo relative to |hi|
+        const unsigned half = ((ah & 0x7fffffu) == 0u && sl < 0.0f) ? 1u : 0u;
+        const float sc = __uint_as_float((52u + 127u - (ex - 127u) + half) << 23);
+        const int k = __float2int_rn(__fmul_rn(sl, sc));
+        const unsigned l0 = ah << 29, h0 = (ah >> 3) + ((1023u - 127u) << 20);
+        const unsigned l1 = l0 + (unsigned)k;
+        const unsigned h1 = h0 + (unsigned)(k >> 31) + (l1 < l0 ? 1u : 0u);
+        return __hiloint2double((int)(h1 | sgn), (int)l1);
+    }
+    return df_to_double(a);
+}
 
 // |a| >= |b| (or a == 0): s + e == a + b exactly
 __device__ __forceinline__ df64 fast_two_sum(float a, float b) {

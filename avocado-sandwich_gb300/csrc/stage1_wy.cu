@@ -50,6 +50,18 @@ struct WCfg {
     static constexpr int KC = sizeof(T) == 8 ? 8 : 16;   // K chunk
 };
 
+// Memory type <-> compute type (all warps convert here: double-float on the integer pipe).
+template <typename CT, typename T>
+__device__ __forceinline__ CT to_ct(T v) {
+    if constexpr (std::is_same<CT, dfx>::value) return dfx(df_from_double_int(v));
+    else return CT(v);
+}
+template <typename T, typename CT>
+__device__ __forceinline__ T from_ct(CT v) {
+    if constexpr (std::is_same<CT, dfx>::value) return df_to_double_int(v.v);
+    else return (T)v;
+}
+
 struct TBuildArgs {
     const void *a;
     int64_t lda;
@@ -233,7 +245,7 @@ __global__ void __launch_bounds__(kWNT) gram_kernel(TBuildArgs args) {
         for (int e = 0; e < PER; ++e) {
             const int idx = tid + e * kWNT;
             const int k = LAYOUT == 0 ? idx % kGK : idx / kGT, m = LAYOUT == 0 ? idx / kGK : idx % kGT;
-            s[k * LD + m] = CT(v[e]);
+            s[k * LD + m] = to_ct<CT>(v[e]);
         }
     };
     const int l0 = 4 * (tid % 16), i0 = 4 * (tid / 16);
@@ -298,11 +310,11 @@ __global__ void __launch_bounds__(kWNT) tdouble_kernel(TBuildArgs args) {
     // the Gram blocks above the diagonal blocks, and the diagonal blocks of T
     for (int idx = tid; idx < B * B; idx += kWNT) {
         const int r = idx % B, i = idx / B;
-        if (r / kWIB < i / kWIB) col(i)[r] = CT(__ldcg(Tf + r + (size_t)i * B));
+        if (r / kWIB < i / kWIB) col(i)[r] = to_ct<CT>(__ldcg(Tf + r + (size_t)i * B));
     }
     for (int idx = tid; idx < NB * kWIB * kWIB; idx += kWNT) {
         const int J = idx / (kWIB * kWIB), e = idx % (kWIB * kWIB);
-        col(J * kWIB + e / kWIB)[J * kWIB + e % kWIB] = CT(tb[idx]);
+        col(J * kWIB + e / kWIB)[J * kWIB + e % kWIB] = to_ct<CT>(tb[idx]);
     }
     __syncthreads();
 #pragma unroll 1
@@ -383,7 +395,7 @@ __global__ void __launch_bounds__(kWNT) tdouble_kernel(TBuildArgs args) {
     // out, zeros below the diagonal blocks
     for (int idx = tid; idx < B * B; idx += kWNT) {
         const int r = idx % B, i = idx / B;
-        Tf[idx] = (r < kWIB * (i / kWIB + 1)) ? (T)col(i)[r] : T(0);
+        Tf[idx] = (r < kWIB * (i / kWIB + 1)) ? from_ct<T>(col(i)[r]) : T(0);
     }
 }
 
@@ -440,12 +452,12 @@ struct UpdCtx {
     __device__ __forceinline__ CT a_elem(int s, int k, int m) const {
         if (s == kVrows) {  // V(k, m): Z = V^T ...
             if (geqrt && k <= m) return (k == m) ? CT(1) : CT(0);
-            return CT(V(row0 + k, col0 + m));
+            return to_ct<CT>(V(row0 + k, col0 + m));
         } else if (s == kTrows) {  // T(k, m)
-            return CT(Tf[k + (size_t)m * B]);
+            return to_ct<CT>(Tf[k + (size_t)m * B]);
         } else {  // V(m, k): ... -= V W
             if (geqrt && m <= k) return (m == k) ? CT(1) : CT(0);
-            return CT(V(row0 + m, col0 + k));
+            return to_ct<CT>(V(row0 + m, col0 + k));
         }
     }
     // chunk element index -> (k, m), coalesced for the source
@@ -599,14 +611,14 @@ __global__ void __launch_bounds__(kWNT) update_full_kernel(UpdFullArgs args) {
         for (int idx = tid; idx < B * C::W; idx += kWNT) {
             int t, c;
             if (LAYOUT == 0) { t = idx % B; c = idx / B; } else { c = idx % C::W; t = idx / C::W; }
-            S[t * C::LDW + c] = (c < wc) ? CT(__ldcg(&V(r0 + t, j0 + c))) : CT(0);
+            S[t * C::LDW + c] = (c < wc) ? to_ct<CT>(__ldcg(&V(r0 + t, j0 + c))) : CT(0);
         }
     };
     auto store_strip = [&](const CT *S, int64_t r0) {
         for (int idx = tid; idx < B * C::W; idx += kWNT) {
             int t, c;
             if (LAYOUT == 0) { t = idx % B; c = idx / B; } else { c = idx % C::W; t = idx / C::W; }
-            if (c < wc) V(r0 + t, j0 + c) = (T)S[t * C::LDW + c];
+            if (c < wc) V(r0 + t, j0 + c) = from_ct<T>(S[t * C::LDW + c]);
         }
     };
     auto get_blk = [&](const CT *S, CT (&r)[8][C::CB]) {
