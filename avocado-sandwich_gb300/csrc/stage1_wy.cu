@@ -22,15 +22,20 @@
 // CTA only waits on one that already runs.  What bounded it with one CTA per strip
 // looping over the tiles: the strips were the launch's only parallelism (64
 // columns each, 2 to 62 CTAs on 152 SMs at n = 4096) and every tile's three
-// products ran in sequence.  Now the FP32 pipe while there are many tiles (n = 4096:
-// about 19 TFLOP/s in the first half-steps), the chain of W (about 6 us a tile)
-// towards the end.  Measured (GB300, all updates of a call, before -> after): FP32 n
-// = 4096 tile 128 45.8 -> 20.2 ms, double-float n = 2048 tile 128 34.5 -> 24.0 ms.
-// Each of the three products is a register-blocked GEMM (8 rows x CB columns per
+// products ran in sequence; then the chain of W through the tiles (two CTAs on an SM
+// instead of one gained nothing, warps stood at the barrier behind the wait).  So W
+// runs by row blocks of 32: T is upper triangular, a block of W needs the top strip's
+// rows up to that block only, and each block has its own counter and is handed on as
+// soon as it is made, so the blocks of a strip pipeline through the tiles; T's block is
+// loaded before the wait.  Two CTAs (16-column FP64 strips: three) share an SM.
+// Measured (GB300, all updates of a call: one CTA per strip -> CTA per tile and strip
+// -> row blocks): FP32 n = 4096 tile 128 45.8 -> 20.2 -> 12 ms, double-float n = 2048
+// tile 128 34.5 -> 18.6 -> 11 ms (24.0 before the integer conversions).
+// The two products with V are register-blocked GEMMs (8 rows x CB columns per
 // thread, K = b streamed through shared memory in chunks that the next chunk's
-// loads overlap); T's zeros are skipped by row groups.  FP64 tiles use 16-column
-// strips when 32-column strips would leave SMs idle; in double-float the products
-// accumulate with the compensated dot product.
+// loads overlap).  FP64 tiles use 16-column strips when 32-column strips would leave
+// SMs idle; in double-float the products accumulate with the compensated dot
+// product.
 #include <algorithm>
 #include <type_traits>
 
@@ -411,13 +416,14 @@ struct UpdFullArgs {
     int64_t sA, sTfull;  // per-matrix strides (blockIdx.y = matrix)
     int first_role;      // 1: the top tile's own reflectors were applied earlier
     int nstrip;
-    int *flags;          // [0] ticket, [1 + strip] tiles finished with the top strip; zeroed
+    int fine;            // 1: a counter per row block of a strip, 0: one per strip
+    int *flags;          // [0] ticket, then the counters: tiles finished with the row block (strip); zeroed
     int64_t sFlags;      // ints between matrices
     int *err;
 };
 
-// A-operand sources for the three products.
-enum ASrc { kVrows = 0, kTrows = 1, kVcols = 2 };
+// A-operand sources of the products with V.
+enum ASrc { kVrows = 0, kVcols = 1 };
 
 template <typename T, int B, int WW = WCfg<T>::W>
 struct UCfg {
@@ -436,6 +442,14 @@ struct UCfg {
     static constexpr int LDW = W + VN;            // row stride of the strip buffers
     static constexpr int LDC = B + 4;             // leading dimension of A chunks (m)
     static constexpr int PER = KC * B / kWNT;     // chunk elements per thread
+    // W = T^T Z: row blocks of KB; a thread's 8 rows are pairs, one per quarter of the tile
+    static constexpr int KB = sizeof(T) == 8 && B == 256 ? 16 : 32;
+    static constexpr int NBK = B / KB;
+    static constexpr int GSC = B / 4;
+    static __device__ __forceinline__ int crow(int m0, int i) { return (i / 2) * GSC + m0 * 2 + i % 2; }
+    static constexpr int CHUNK = (2 * KC > KB ? 2 * KC : KB) * LDC;  // A operands staged
+    // CTAs per SM (shared memory allows them; the registers are held to it)
+    static constexpr int MINB = B == 128 ? (sizeof(T) == 8 && W == 16 ? 3 : 2) : (sizeof(T) == 8 && W == 16 ? 2 : 1);
     static_assert(CB >= 1 && PER >= 1, "update configuration");
 };
 
@@ -453,8 +467,6 @@ struct UpdCtx {
         if (s == kVrows) {  // V(k, m): Z = V^T ...
             if (geqrt && k <= m) return (k == m) ? CT(1) : CT(0);
             return to_ct<CT>(V(row0 + k, col0 + m));
-        } else if (s == kTrows) {  // T(k, m)
-            return to_ct<CT>(Tf[k + (size_t)m * B]);
         } else {  // V(m, k): ... -= V W
             if (geqrt && m <= k) return (m == k) ? CT(1) : CT(0);
             return to_ct<CT>(V(row0 + m, col0 + k));
@@ -462,10 +474,25 @@ struct UpdCtx {
     }
     // chunk element index -> (k, m), coalesced for the source
     __device__ __forceinline__ void map(int s, int idx, int &k, int &m) const {
-        const bool kfast = (s == kTrows) || (s == kVrows && LAYOUT == 0) || (s == kVcols && LAYOUT == 1);
+        const bool kfast = (s == kVrows) == (LAYOUT == 0);
         if (kfast) { k = idx % C::KC; m = idx / C::KC; } else { m = idx % B; k = idx / B; }
     }
 };
+
+// Double-float: compensated accumulation (Dot2, Ogita-Rump-Oishi) on the pair
+// (s, c) = (a.hi, a.lo): the product's error terms and the sum's rounding error go
+// to c, renormalised once per product.
+__device__ __forceinline__ void dot2(df64 &a, df64 x, df64 y) {
+    const float pr = __fmul_rn(x.hi, y.hi);
+    float ep = __fmaf_rn(x.hi, y.hi, -pr);
+    ep = __fmaf_rn(x.hi, y.lo, ep);
+    ep = __fmaf_rn(x.lo, y.hi, ep);
+    const float t = __fadd_rn(a.hi, pr);
+    const float z = __fsub_rn(t, a.hi);
+    const float es = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(t, z)), __fsub_rn(pr, z));
+    a.hi = t;
+    a.lo = __fadd_rn(a.lo, __fadd_rn(es, ep));
+}
 
 // acc (+|-)= A(k, m)^T-view ... : acc[i][j] += sign * sum_k A(k, m0+i) * Bop(k, c0+j)
 template <typename T, int LAYOUT, int B, int WW = WCfg<T>::W, typename CT = T>
@@ -521,9 +548,7 @@ __device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, co
         }
         const int k0 = ch * C::KC;
         if constexpr (std::is_same<CT, dfx>::value) {
-            // double-float: compensated accumulation (Dot2, Ogita-Rump-Oishi) on
-            // the pairs (s, c) = (acc.hi, acc.lo): the product's error terms and
-            // the sum's rounding error go to c, renormalised once per call below
+            // renormalised once per call below
 #pragma unroll 4
             for (int k = 0; k < C::KC; ++k) {
                 CT av[8], bv[C::CB];
@@ -534,20 +559,9 @@ __device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, co
                     if (neg) bv[j] = -bv[j];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    if (src == kTrows && (i / C::VN + 1) * C::GS <= k0) continue;  // T(k, m) = 0 below the diagonal
 #pragma unroll
                     for (int j = 0; j < C::CB; ++j) {
-                        const df64 x = av[i].v, y = bv[j].v;
-                        const float pr = __fmul_rn(x.hi, y.hi);
-                        float ep = __fmaf_rn(x.hi, y.hi, -pr);
-                        ep = __fmaf_rn(x.hi, y.lo, ep);
-                        ep = __fmaf_rn(x.lo, y.hi, ep);
-                        df64 &a = acc[i][j].v;
-                        const float t = __fadd_rn(a.hi, pr);
-                        const float z = __fsub_rn(t, a.hi);
-                        const float es = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(t, z)), __fsub_rn(pr, z));
-                        a.hi = t;
-                        a.lo = __fadd_rn(a.lo, __fadd_rn(es, ep));
+                        dot2(acc[i][j].v, av[i].v, bv[j].v);
                     }
                 }
             }
@@ -566,7 +580,6 @@ __device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, co
             } else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    if (src == kTrows && (i / C::VN + 1) * C::GS <= k0) continue;  // T(k, m) = 0 below the diagonal
 #pragma unroll
                     for (int j = 0; j < C::CB; ++j) acc[i][j] += av[i] * bv[j];
                 }
@@ -583,13 +596,14 @@ __device__ __forceinline__ void gemm(const UpdCtx<T, LAYOUT, B, WW, CT> &ctx, co
 }
 
 template <typename T, int LAYOUT, int B, typename CT = T, int WW = WCfg<T>::W>
-__global__ void __launch_bounds__(kWNT) update_full_kernel(UpdFullArgs args) {
+__global__ void __launch_bounds__(kWNT, UCfg<T, B, WW>::MINB) update_full_kernel(UpdFullArgs args) {
     using C = UCfg<T, B, WW>;
     static_assert(sizeof(CT) == sizeof(T), "compute type of the element's size");
+    constexpr int KB = C::KB, NBK = C::NBK, W = C::W;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CT *Buf = reinterpret_cast<CT *>(smem_raw);    // B x LDW, row-major: the tile's strip
-    CT *Zb = Buf + (size_t)B * C::LDW;             // B x LDW: top strip, Z, W
-    CT *ch0 = Zb + (size_t)B * C::LDW;             // KC x LDC
+    CT *Zb = Buf + (size_t)B * C::LDW;             // B x LDW: Z, then W
+    CT *ch0 = Zb + (size_t)B * C::LDW;             // KC x LDC, twice; KB x LDC for T
     CT *ch1 = ch0 + (size_t)C::KC * C::LDC;
     __shared__ int s_t, s_ok;
     const int tid = threadIdx.x;
@@ -599,112 +613,191 @@ __global__ void __launch_bounds__(kWNT) update_full_kernel(UpdFullArgs args) {
     __syncthreads();
     const int p = args.first_role + s_t / args.nstrip, strip = s_t % args.nstrip;
     if (p >= args.P) return;
-    int *done = flags + 1 + strip;
-    const int64_t j0 = (int64_t)(args.pc + 1) * B + (int64_t)strip * C::W;
-    const int wc = (int)min((int64_t)C::W, args.n - j0);
+    int *done = flags + 1 + strip * (args.fine ? NBK : 1);
+    const int64_t j0 = (int64_t)(args.pc + 1) * B + (int64_t)strip * W;  // whole tiles of columns: strips are full
     View<T, LAYOUT> V{reinterpret_cast<T *>(args.a) + zb * args.sA, args.lda};
     const int64_t top0 = (int64_t)args.pr * B;
     const int m0 = tid % C::TM;
     const int c0 = (tid / C::TM) * C::CB;
-
-    auto load_strip = [&](CT *S, int64_t r0) {
-        for (int idx = tid; idx < B * C::W; idx += kWNT) {
-            int t, c;
-            if (LAYOUT == 0) { t = idx % B; c = idx / B; } else { c = idx % C::W; t = idx / C::W; }
-            S[t * C::LDW + c] = (c < wc) ? to_ct<CT>(__ldcg(&V(r0 + t, j0 + c))) : CT(0);
-        }
-    };
-    auto store_strip = [&](const CT *S, int64_t r0) {
-        for (int idx = tid; idx < B * C::W; idx += kWNT) {
-            int t, c;
-            if (LAYOUT == 0) { t = idx % B; c = idx / B; } else { c = idx % C::W; t = idx / C::W; }
-            if (c < wc) V(r0 + t, j0 + c) = from_ct<T>(S[t * C::LDW + c]);
-        }
-    };
-    auto get_blk = [&](const CT *S, CT (&r)[8][C::CB]) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < C::CB; ++j) r[i][j] = S[C::row(m0, i) * C::LDW + c0 + j];
-    };
-    auto put_blk = [&](CT *S, const CT (&r)[8][C::CB]) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < C::CB; ++j) S[C::row(m0, i) * C::LDW + c0 + j] = r[i][j];
-    };
-    auto zero = [&](CT (&r)[8][C::CB]) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < C::CB; ++j) r[i][j] = CT(0);
+    // rows [0, R) of a strip: element u of the thread (tid + u kWNT) in memory order
+    auto elem = [&](int R, int idx, int &t, int &c) {
+        t = LAYOUT == 0 ? idx % R : idx / W;
+        c = LAYOUT == 0 ? idx / R : idx % W;
     };
 
     CT acc[8][C::CB];
-    CT blk[8][C::CB];
     UpdCtx<T, LAYOUT, B, WW, CT> ctx;
     ctx.V = V;
-    ctx.Tf = reinterpret_cast<const T *>(args.tfull) + zb * args.sTfull + (size_t)p * B * B;
     ctx.row0 = (int64_t)(args.pr + p) * B;
     ctx.col0 = (int64_t)args.pc * B;
     ctx.geqrt = (p == 0);
-    load_strip(Buf, ctx.row0);
-    __syncthreads();
-    zero(acc);
-    gemm(ctx, kVrows, acc, Buf, ch0, ch1, false);   // V_p^T A_p (the top tile: Y0^T Top)
-    if (p == 0) {
-        put_blk(Zb, acc);
-        __syncthreads();
-        zero(acc);
-        gemm(ctx, kTrows, acc, Zb, ch0, ch1, false);   // W = T0^T Z
-        put_blk(Zb, acc);
-        __syncthreads();
-        get_blk(Buf, acc);
-        gemm(ctx, kVcols, acc, Zb, ch0, ch1, true);    // Top -= Y0 W
-        put_blk(Buf, acc);
-        __syncthreads();
-        store_strip(Buf, top0);
-        __syncthreads();
-        if (tid == 0) st_release(done, 1);
-        return;
+    const T *Tf = reinterpret_cast<const T *>(args.tfull) + zb * args.sTfull + (size_t)p * B * B;
+    {  // the tile's strip, NL loads in flight
+        constexpr int NL = 8;
+        static_assert(B * W % (kWNT * NL) == 0, "strip loads");
+#pragma unroll 1
+        for (int base = tid; base < B * W; base += kWNT * NL) {
+            T v[NL];
+            int t, c;
+#pragma unroll
+            for (int u = 0; u < NL; ++u) {
+                elem(B, base + u * kWNT, t, c);
+                v[u] = __ldcg(&V(ctx.row0 + t, j0 + c));
+            }
+#pragma unroll
+            for (int u = 0; u < NL; ++u) {
+                elem(B, base + u * kWNT, t, c);
+                Buf[t * C::LDW + c] = to_ct<CT>(v[u]);
+            }
+        }
     }
-    // the top strip, once the previous tile is done with it
-    if (tid == 0) s_ok = p > args.first_role ? wait_geq(done, p - args.first_role, args.err) : true;
     __syncthreads();
-    if (!s_ok) return;
-    load_strip(Zb, top0);
-    __syncthreads();
-    get_blk(Zb, blk);
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < C::CB; ++j) acc[i][j] += blk[i][j];
-    put_blk(Zb, acc);                                // Z = Top + V^T A_p (each thread its own entries)
-    __syncthreads();
-    zero(acc);
-    gemm(ctx, kTrows, acc, Zb, ch0, ch1, false);    // W = T^T Z
+        for (int j = 0; j < C::CB; ++j) acc[i][j] = CT(0);
+    gemm(ctx, kVrows, acc, Buf, ch0, ch1, false);   // V_p^T A_p (the top tile: Y0^T Top)
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < C::CB; ++j) blk[i][j] -= acc[i][j];
-    put_blk(Zb, blk);                                // Top -= W, handed on
+        for (int j = 0; j < C::CB; ++j) {
+            Zb[C::row(m0, i) * C::LDW + c0 + j] = acc[i][j];
+            acc[i][j] = CT(0);
+        }
+
+    // ---- W = T^T (Z + Top), Top -= W, row block by row block: T is upper triangular,
+    // so a block of W needs the top strip's rows up to that block only, and each block
+    // is handed on at once
+    constexpr int PT = KB * W / kWNT;   // top elements per thread and block
+    constexpr int PF = KB * B / kWNT;   // T elements per thread and block
+    static_assert(PT >= 1 && PF >= 1, "chain split");
+#pragma unroll 1
+    for (int m = 0; m < NBK; ++m) {
+        T tv[PF], top[PT];
+#pragma unroll
+        for (int e = 0; e < PF; ++e) {  // T(k, i), k in the block, i >= m KB
+            const int idx = tid + e * kWNT, k = idx % KB, i = idx / KB;
+            tv[e] = i >= m * KB ? Tf[m * KB + k + (size_t)i * B] : T(0);
+        }
+        if (p > args.first_role && (args.fine || m == 0)) {
+            if (tid == 0) s_ok = wait_geq(done + (args.fine ? m : 0), p - args.first_role, args.err);
+            __syncthreads();
+            if (!s_ok) return;
+        }
+        if (p > 0) {
+            int t, c;
+#pragma unroll
+            for (int u = 0; u < PT; ++u) {
+                elem(KB, tid + u * kWNT, t, c);
+                top[u] = __ldcg(&V(top0 + m * KB + t, j0 + c));
+            }
+        }
+        __syncthreads();  // Zb complete (m = 0), the previous block's T no longer read
+#pragma unroll
+        for (int e = 0; e < PF; ++e) {
+            const int idx = tid + e * kWNT, k = idx % KB, i = idx / KB;
+            ch0[k * C::LDC + i] = to_ct<CT>(tv[e]);
+        }
+        if (p > 0) {
+            int t, c;
+#pragma unroll
+            for (int u = 0; u < PT; ++u) {
+                elem(KB, tid + u * kWNT, t, c);
+                CT &z = Zb[(m * KB + t) * C::LDW + c];
+                z = z + to_ct<CT>(top[u]);
+            }
+        }
+        __syncthreads();
+        auto product = [&](auto first_c) {  // the thread's pairs from `first` on reach past the block
+            constexpr int G0 = decltype(first_c)::value;
+#pragma unroll 4
+            for (int k = 0; k < KB; ++k) {
+                CT av[8], bv[C::CB];
+#pragma unroll
+                for (int g = G0; g < 4; ++g) {
+                    if constexpr (sizeof(CT) == 8) {
+                        PVec<CT>::ld(ch0 + k * C::LDC + C::crow(m0, 2 * g), av + 2 * g);
+                    } else {
+                        const float2 v = *reinterpret_cast<const float2 *>(ch0 + k * C::LDC + C::crow(m0, 2 * g));
+                        av[2 * g] = v.x;
+                        av[2 * g + 1] = v.y;
+                    }
+                }
+                const CT *bp = Zb + (m * KB + k) * C::LDW + c0;
+                if constexpr (C::CB % C::VN == 0) {
+#pragma unroll
+                    for (int j = 0; j < C::CB; j += C::VN) PVec<CT>::ld(bp + j, bv + j);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < C::CB; ++j) bv[j] = bp[j];
+                }
+#pragma unroll
+                for (int i = 2 * G0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < C::CB; ++j) {
+                        if constexpr (std::is_same<CT, dfx>::value) dot2(acc[i][j].v, av[i].v, bv[j].v);
+                        else acc[i][j] += av[i] * bv[j];
+                    }
+            }
+        };
+        switch (m * KB / C::GSC) {
+            case 0: product(std::integral_constant<int, 0>{}); break;
+            case 1: product(std::integral_constant<int, 1>{}); break;
+            case 2: product(std::integral_constant<int, 2>{}); break;
+            default: product(std::integral_constant<int, 3>{}); break;
+        }
+        __syncthreads();  // the block's Z no longer read: W in its place
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = C::crow(m0, i);
+            if (r >= m * KB && r < (m + 1) * KB) {
+#pragma unroll
+                for (int j = 0; j < C::CB; ++j) {
+                    if constexpr (std::is_same<CT, dfx>::value) acc[i][j].v = two_sum(acc[i][j].v.hi, acc[i][j].v.lo);
+                    Zb[r * C::LDW + c0 + j] = acc[i][j];
+                }
+            }
+        }
+        __syncthreads();
+        if (p > 0) {
+            int t, c;
+#pragma unroll
+            for (int u = 0; u < PT; ++u) {
+                elem(KB, tid + u * kWNT, t, c);
+                V(top0 + m * KB + t, j0 + c) = from_ct<T>(to_ct<CT>(top[u]) - Zb[(m * KB + t) * C::LDW + c]);
+            }
+            __syncthreads();
+            if (tid == 0 && (args.fine || m == NBK - 1))
+                st_release(done + (args.fine ? m : 0), p - args.first_role + 1);
+        }
+    }
+
+    // ---- A_p -= V W (the top tile: Top -= Y0 W)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < C::CB; ++j) acc[i][j] = Buf[C::row(m0, i) * C::LDW + c0 + j];
+    gemm(ctx, kVcols, acc, Zb, ch0, ch1, true);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < C::CB; ++j) Buf[C::row(m0, i) * C::LDW + c0 + j] = acc[i][j];
     __syncthreads();
-    store_strip(Zb, top0);
-    __syncthreads();
-    if (tid == 0) st_release(done, p - args.first_role + 1);
-    put_blk(Zb, acc);
-    __syncthreads();
-    get_blk(Buf, blk);
-    gemm(ctx, kVcols, blk, Zb, ch0, ch1, true);     // A_p -= V W
-    put_blk(Buf, blk);
-    __syncthreads();
-    store_strip(Buf, ctx.row0);
+    for (int idx = tid; idx < B * W; idx += kWNT) {
+        int t, c;
+        elem(B, idx, t, c);
+        V(ctx.row0 + t, j0 + c) = from_ct<T>(Buf[t * C::LDW + c]);
+    }
+    if (p == 0) {
+        __syncthreads();
+        if (tid < (args.fine ? NBK : 1)) st_release(done + tid, 1);
+    }
 }
 
 template <typename T, int B, int WW = WCfg<T>::W>
 size_t upd_full_smem() {
     using C = UCfg<T, B, WW>;
-    return sizeof(T) * (2 * (size_t)B * C::LDW + 2 * (size_t)C::KC * C::LDC);
+    return sizeof(T) * (2 * (size_t)B * C::LDW + (size_t)C::CHUNK);
 }
 
 template <typename T, int LAYOUT, int B, typename CT = T, int WW = WCfg<T>::W>
@@ -725,14 +818,15 @@ int launch_upd_full(T *dA, int64_t lda, int64_t n, int pr, int pc, int P, const 
     // ticket and strip counters take the place of the panel's 16 x 16 T blocks,
     // which the T build has read
     const int64_t sFl = w.sTblk * (int64_t)(sizeof(T) / sizeof(int));
-    if (sizeof(int) * (size_t)(1 + nstrip) > sizeof(T) * (size_t)(P - first_role) * (B / kWIB) * kWIB * kWIB)
-        return AVS_ERR_INTERNAL;
+    const size_t room = sizeof(T) * (size_t)(P - first_role) * (B / kWIB) * kWIB * kWIB;
+    // (out of core, one tile at a time, they may hold one counter per strip only)
+    const int fine = sizeof(int) * (size_t)(1 + nstrip * C::NBK) <= room ? 1 : 0;
+    const size_t used = sizeof(int) * (size_t)(1 + nstrip * (fine ? C::NBK : 1));
+    if (used > room) return AVS_ERR_INTERNAL;
     int *flags = reinterpret_cast<int *>(w.tblk);
-    if (batch > 1)
-        AVS_CUDA_TRY(cudaMemset2DAsync(flags, sizeof(int) * (size_t)sFl, 0, sizeof(int) * (size_t)(1 + nstrip), batch, s));
-    else
-        AVS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)(1 + nstrip), s));
-    UpdFullArgs a{dA, lda, n, B, pr, pc, P, w.tfull, w.sA, w.sTfull, first_role, nstrip, flags, sFl, w.err};
+    if (batch > 1) AVS_CUDA_TRY(cudaMemset2DAsync(flags, sizeof(int) * (size_t)sFl, 0, used, batch, s));
+    else AVS_CUDA_TRY(cudaMemsetAsync(flags, 0, used, s));
+    UpdFullArgs a{dA, lda, n, B, pr, pc, P, w.tfull, w.sA, w.sTfull, first_role, nstrip, fine, flags, sFl, w.err};
     update_full_kernel<T, LAYOUT, B, CT, WW><<<dim3((unsigned)nstrip * (P - first_role), batch), kWNT, smem, s>>>(a);
     AVS_CUDA_TRY(cudaGetLastError());
     return AVS_SUCCESS;
