@@ -17,11 +17,13 @@
 //     are factored QR (T reflectors from the left); the columns to their
 //     right, [c0+T, c0+2B), are multiplied by Q^T = I - V T^T V^T.
 // Every index range is clipped to n.  With T = 1 this is the element chase
-// of stage2_chase.cu.  Op k of sweep s touches nothing that ops >= k+4 of
-// sweep s-1 touch (the same lag as the element chase: R op m of sweep s
-// overlaps sweep s-1's ops up to L op m+1 in a T x T corner, L op m up to R
-// op m+2), so sweep s runs op k once sweep s-1 has finished k+4 ops, and the
-// result is bit-identical to running the sweeps one after another.
+// of stage2_chase.cu.  Op k of sweep s touches nothing that ops >= k+4 of sweep s-1
+// touch, and of op k+3 one T x T corner only: the triangle its factorisation leaves in
+// its pivot rows (columns), at the far end of op k's rows (columns), final before op
+// k+3's apply.  So op k starts once sweep s-1 has finished op k+2, and reads the corner
+// between its own factorisation and its apply, when sweep s-1 has announced it (done
+// counts 2 per op and 1 for the corner); the result is bit-identical to running the
+// sweeps one after another.
 //
 // One thread-block cluster of C CTAs owns a sweep.  Every CTA loads the
 // panel and factors it itself (same data, same code: the same bits) and applies
@@ -35,7 +37,8 @@
 // reflectors are half of it: 12 to 15 k of about 20 to 37 k cycles).  Measured (GB300,
 // the whole stage, before: every column's work inside the panel's chain, T formed
 // by one warp, one reflector per thread in the first product): band 64 n = 1024 3.3
-// -> 2.4 ms, 128 n = 4096 15.4 -> 11.6 ms, 256 n = 16384 115 -> 84 ms.
+// -> 2.4 ms, 128 n = 4096 15.4 -> 11.6 ms, 256 n = 16384 115 -> 84 ms; then, with a lag
+// of three ops instead of four, 2.4 -> 2.0, 11.6 -> 9.6, 84 -> 67 ms.
 // The band is in compact storage A(r, c) at AB[(r - c + 2B) + c * ldab],
 // ldab = 3B + 1 (band_ku / band_ldab): rows c-2B .. c+B of column c (band,
 // upper bulge up to 2B-1, lower bulge up to B-1), laid out so that every
@@ -107,6 +110,12 @@ __device__ __forceinline__ dfx wsum(df64 s) {
     for (int o = 16; o > 0; o >>= 1)
         s = MacAr<dfx>::mac_merge(s, df64{__shfl_xor_sync(0xffffffffu, s.hi, o), __shfl_xor_sync(0xffffffffu, s.lo, o)});
     return MacAr<dfx>::fin(s);
+}
+__device__ __forceinline__ float ldcg_elem(const float *p) { return __ldcg(p); }
+__device__ __forceinline__ double ldcg_elem(const double *p) { return __ldcg(p); }
+__device__ __forceinline__ dfx ldcg_elem(const dfx *p) {
+    const float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
+    return dfx(df64{v.x, v.y});
 }
 __device__ __forceinline__ float wshfl(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 __device__ __forceinline__ double wshfl(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
@@ -436,7 +445,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
             // A wait that runs out records kDevTimeout; the cluster still runs its
             // barriers to the end (later waits return at once), so no CTA is left
             // at a cluster barrier.
-            if (tid == 0 && sw > 0) wait_geq(done + sw - 1, min(op + 4, ops_prev), err);
+            if (tid == 0 && sw > 0) wait_geq(done + sw - 1, 2 * min(op + 3, ops_prev), err);
+            const bool corner = sw > 0 && op + 3 < ops_prev;  // op + 3's pivot corner is still to come
             __syncthreads();
             const int L = (int)(n - c0 < B ? n - c0 : (int64_t)B);  // R op: columns; L op: rows
             if (rop) {
@@ -480,14 +490,33 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                 cl_wait();  // every CTA has read the pivot rows: L and zeros, a share per CTA
                 for (int idx = q * (T * B / C) + tid; idx < (q + 1) * (T * B / C); idx += NT) {
                     const int k = idx % T, j = idx / T;
-                    if (j < L) *at(rho + k, c0 + j) = (j <= k) ? P[k * LDP + j] : R(0);
+                    if (j >= T && j < L) *at(rho + k, c0 + j) = R(0);
+                }
+                if (q == 0) {  // the T x T corner, the next sweep's
+                    for (int idx = tid; idx < T * T; idx += NT) {
+                        const int k = idx % T, j = idx / T;
+                        if (j < L) *at(rho + k, c0 + j) = (j <= k) ? P[k * LDP + j] : R(0);
+                    }
                 }
                 __syncthreads();
+                if (q == 0 && tid == 0) st_release(done + sw, 2 * op + 1);
+                const int64_t rc = c0 + B - T - r_lo;  // the corner's first row in this CTA's rows
+                const bool mine = corner && rc > -T && rc < RPC;
+                if (mine && tid == 0) wait_geq(done + sw - 1, 2 * (op + 3) + 1, err);
                 for (int idx = tid; idx < T * T; idx += NT) {  // explicit V: unit diagonal, zeros above
                     const int k = idx / T, i = idx % T;
                     if (i <= k) P[k * LDP + i] = (i == k) ? R(1) : R(0);
                 }
                 __syncthreads();
+                if (mine) {
+                    for (int idx = tid; idx < T * T; idx += NT) {
+                        const int64_t r = rc + idx % T;
+                        const int c = B - T + idx / T;
+                        if (r >= 0 && r < RPC && r_lo + r < r_hi && c < L)
+                            As[c * Cfg::LDA_R + r] = ldcg_elem(at(r_lo + r, c0 + c));
+                    }
+                    __syncthreads();
+                }
                 // W = A V: thread = 4 rows x 4 reflectors, BK columns of the sum
                 {
                     const int g = tid % Cfg::NG4, k0 = (tid / Cfg::NG4) % (T / 4) * 4, ks = tid / (Cfg::NG4 * (T / 4));
@@ -605,14 +634,33 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                 cl_wait();  // R and zeros, a share per CTA
                 for (int idx = q * (T * B / C) + tid; idx < (q + 1) * (T * B / C); idx += NT) {
                     const int i = idx % B, k = idx / B;
-                    if (i < L && k < Tc) *at(c0 + i, c0 + k) = (i <= k) ? P[k * LDP + i] : R(0);
+                    if (i >= T && i < L && k < Tc) *at(c0 + i, c0 + k) = R(0);
+                }
+                if (q == 0) {  // the T x T corner, the next sweep's
+                    for (int idx = tid; idx < T * T; idx += NT) {
+                        const int i = idx % T, k = idx / T;
+                        if (i < L && k < Tc) *at(c0 + i, c0 + k) = (i <= k) ? P[k * LDP + i] : R(0);
+                    }
                 }
                 __syncthreads();
+                if (q == 0 && tid == 0) st_release(done + sw, 2 * op + 1);
+                const int64_t rc = c0 + 2 * B - T - cc_lo;  // the corner's first column in this CTA's columns
+                const bool mine = corner && rc > -T && rc < RPC;
+                if (mine && tid == 0) wait_geq(done + sw - 1, 2 * (op + 3) + 1, err);
                 for (int idx = tid; idx < T * T; idx += NT) {
                     const int k = idx / T, i = idx % T;
                     if (i <= k) P[k * LDP + i] = (i == k) ? R(1) : R(0);
                 }
                 __syncthreads();
+                if (mine) {
+                    for (int idx = tid; idx < T * T; idx += NT) {
+                        const int i = B - T + idx % T;
+                        const int64_t c = rc + idx / T;
+                        if (c >= 0 && c < RPC && cc_lo + c < c_hi && i < L)
+                            As[c * Cfg::LDA_L + i] = ldcg_elem(at(c0 + i, cc_lo + c));
+                    }
+                    __syncthreads();
+                }
                 // Z = V^T A: thread = 4 columns (g + cc NG4: lanes one column apart, so
                 // their column reads spread over the banks) x 4 reflectors, BK rows of the sum
                 {
@@ -697,7 +745,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
             __syncthreads();
             if (tid == 0) __threadfence();
             cluster.sync();
-            if (q == 0 && tid == 0) st_release(done + sw, op + 1);
+            if (q == 0 && tid == 0) st_release(done + sw, 2 * (op + 1));
         }
     }
 }
@@ -729,8 +777,8 @@ int launch_band_stage(R *dAB, int64_t n, int64_t ldab, const Stage2Work &w, cuda
     }
     const int64_t nsw = (n - 2 - T >= 0) ? (n - 2 - T) / T + 1 : 0;
     if (nsw == 0) return AVS_SUCCESS;
-    // sweeps in flight: a sweep's 2 n / B ops over a lag of 4 ops
-    const int64_t want = std::max<int64_t>(1, ((n / B) / 2 + 2) * (int64_t)batch);
+    // sweeps in flight: a sweep's 2 n / B ops over a lag of 3 ops
+    const int64_t want = std::max<int64_t>(1, (2 * (n / B) / 3 + 2) * (int64_t)batch);
     const int64_t clusters = std::min<int64_t>(std::min<int64_t>(want, max_clusters), nsw * (int64_t)batch);
     cfg.gridDim = dim3((unsigned)(clusters * C));
     AVS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, dAB, n, ldab, w.flags, w.flags + 1, w.err, batch, sAB, sDone));
