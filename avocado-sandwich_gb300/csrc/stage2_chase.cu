@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(ChaseCfg<BW, CC, NTT>::NT, ChaseCfg<BW, CC, NT
 #pragma unroll
                         for (int k = 0; k < Cfg::CPG; ++k) {
                             const int ci = g * Cfg::CPG + k;
-                            if (ci < L) Ar::st(A.at(r, c0 + ci), Ar::sub(vals[k], Ar::mul(w, sv[ci])));
+                            if (ci < L) Ar::st(A.at(r, c0 + ci), ChaseRefl<S>::sub_mul(vals[k], w, sv[ci]));
                         }
                     }
                 }
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(ChaseCfg<BW, CC, NTT>::NT, ChaseCfg<BW, CC, NT
 #pragma unroll
                             for (int t = 0; t < Cfg::RPL; ++t) {
                                 const int ri = lane + 32 * t;
-                                if (ri < L) Ar::st(A.at(c0 + ri, c), Ar::sub(vals[k][t], Ar::mul(w, sv[ri])));
+                                if (ri < L) Ar::st(A.at(c0 + ri, c), ChaseRefl<S>::sub_mul(vals[k][t], w, sv[ri]));
                             }
                         }
                     }
@@ -444,6 +444,9 @@ int launch_chase_cluster(typename ChaseAr<S>::St *dAB, int64_t n, int64_t ldab, 
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (Cfg::C > 8)
+        AVS_CUDA_TRY(cudaFuncSetAttribute(chase_cluster_kernel<BW, S, CC, NTT>,
+                                          cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     int max_clusters = 0;
     cfg.gridDim = dim3(Cfg::C * 64);
     if (cudaOccupancyMaxActiveClusters(&max_clusters, chase_cluster_kernel<BW, S, CC, NTT>, &cfg) != cudaSuccess ||
@@ -460,14 +463,28 @@ int launch_chase_cluster(typename ChaseAr<S>::St *dAB, int64_t n, int64_t ldab, 
     return AVS_SUCCESS;
 }
 
+// Twice the CTAs per cluster while the sweeps in flight then still have an SM per CTA:
+// an op's latency falls with the SMs that share its rows and columns, FP64 instructions
+// above all (FP64, the stage, before -> after: band 64 n = 256 5.3 -> 4.4 ms, n = 1024 24.0
+// -> 19.9, n = 2048 48.9 -> 43.4; band 128 n = 512 12.9 -> 10.4, n = 1024 28.2 -> 22.4, n =
+// 1536 43.3 -> 36.2; with more sweeps than that they would wait for SMs).
+inline bool chase_room(int64_t n, int bw, int cc, int num_sms) {
+    return ((n / bw) / 2 + 2) * cc <= (int64_t)num_sms;
+}
+
 template <typename S>
 int launch_chase_any(typename ChaseAr<S>::St *dAB, int64_t n, int bw, int64_t ldab, const Stage2Work &w,
                      cudaStream_t s, int num_sms) {
     switch (bw) {
         case 16: return launch_chase_cluster<16, S>(dAB, n, ldab, w, s, num_sms);
         case 32: return launch_chase_cluster<32, S>(dAB, n, ldab, w, s, num_sms);
-        case 64: return launch_chase_cluster<64, S>(dAB, n, ldab, w, s, num_sms);
-        case 128: return launch_chase_cluster<128, S>(dAB, n, ldab, w, s, num_sms);
+        case 64:
+            if (chase_room(n, 64, 8, num_sms)) return launch_chase_cluster<64, S, 8, 256>(dAB, n, ldab, w, s, num_sms);
+            return launch_chase_cluster<64, S>(dAB, n, ldab, w, s, num_sms);
+        case 128:
+            if (chase_room(n, 128, 16, num_sms))
+                return launch_chase_cluster<128, S, 16, 256>(dAB, n, ldab, w, s, num_sms);
+            return launch_chase_cluster<128, S>(dAB, n, ldab, w, s, num_sms);
         case 256: return launch_chase_cluster<256, S>(dAB, n, ldab, w, s, num_sms);
         default: return AVS_ERR_UNSUPPORTED;
     }
