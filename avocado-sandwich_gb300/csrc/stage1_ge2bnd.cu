@@ -1158,8 +1158,8 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NTL) panel_kernel(PanelArgs a
 }
 
 // ---------------------------------------------------------------------------
-// Trailing update of tiles 16, 32 and 64, 16 reflectors at a time (tiles 128 and
-// 256: the full-T update).
+// Trailing update of tiles 32 and 64 and of FP64 tiles of 16, 16 reflectors at a time
+// (FP32 tiles of 16: update16_kernel; tiles 128 and 256: the full-T update).
 //
 // A CTA takes a column strip and `group` consecutive tiles; a thread owns 16 rows
 // of one column of the current tile, in registers from its load to its store.
@@ -1190,7 +1190,7 @@ struct UpdCfg {
     static constexpr int LDV = F4 ? 20 : 18;       // row stride of V (16-byte rows)
     static constexpr int VSZ = B * LDV + kIB * kIB;  // one staged block: V, then T (row l: T(0..15, l))
     static constexpr int PER = (B * kIB + NT - 1) / NT;
-    static constexpr int MINB = F4 ? (B == 64 ? 2 : (B == 32 ? 3 : 6)) : 1;  // CTAs per SM the registers allow
+    static constexpr int MINB = F4 ? (B == 64 ? 2 : 3) : 1;  // CTAs per SM the registers allow
     static constexpr size_t smem_bytes() {
         return sizeof(T) * (3 * (size_t)VSZ + (size_t)B * W + (NB > 1 ? 2 * (size_t)NB * kIB * W + kIB * W : 0));
     }
@@ -1416,6 +1416,162 @@ __global__ void __launch_bounds__(UpdCfg<T, B>::NT, UpdCfg<T, B>::MINB) update_k
     }
 }
 
+// ---------------------------------------------------------------------------
+// Trailing update of FP32 tiles of 16: a CTA takes a strip of 16 columns through all
+// tiles, four threads per column, four rows (and four reflectors) each.
+//
+// What bounds it: the latency of a tile, times the tiles; a 16 x 16 product is too
+// little work to pass the strip on for.  With one thread per column a tile was 650
+// dependent-ish instructions of one warp (3.1 k cycles); four threads share them (Z by
+// a reduce-scatter over the quad, W and Z gathered through shared memory), V, T and the
+// strip's tile arrive by asynchronous copies five tiles ahead, and 16 columns a CTA
+// give each warp a scheduler to itself.  Measured (GB300, n = 1296, all updates of the
+// call): 11.2 -> 5.0 ms.
+constexpr int kU16W = 16, kU16T = 4 * kU16W, kU16S = 6;  // columns, threads, stages
+__device__ __forceinline__ void copy16_async(float *dst, const float *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+template <int LAYOUT>
+__global__ void __launch_bounds__(kU16T) update16_kernel(UpdateArgs args) {
+    constexpr int VS = 272, TS = 272, AS = 288, ST = VS + TS + AS;
+    __shared__ __align__(16) float sm[kU16S * ST];
+    __shared__ __align__(16) float ex[kU16T / 32][8 * 20];  // a quad's 16 values
+    const int tid = threadIdx.x, qd = tid & 3, col = tid >> 2;
+    const int64_t zb = blockIdx.y;
+    View<float, LAYOUT> V{reinterpret_cast<float *>(args.a) + zb * args.sA, args.lda};
+    const float *tblk = reinterpret_cast<const float *>(args.tblk) + zb * args.sTblk;
+    const int64_t col0 = (int64_t)args.pc * 16, j0 = col0 + 16 + (int64_t)blockIdx.x * kU16W;
+    const int64_t top0 = (int64_t)args.pr * 16;
+    const int p0 = args.first_role, P = args.P;
+    // 16-word rows, every four of them 4 (8) words further: the quad's 16-byte (4-byte) reads spread over the banks
+    auto pad4 = [](int r) { return r * 16 + (r / 4) * 4; };
+    auto pad8 = [](int r) { return r * 16 + (r / 4) * 8; };
+    auto fetch = [&](int p) {
+        if (p < P) {
+            float *st = sm + (p % kU16S) * ST;
+            const int64_t row0 = (int64_t)(args.pr + p) * 16;
+            const int i = tid >> 2, q4 = 4 * (tid & 3);
+            if (LAYOUT == 0) {  // [reflector][row], [column][row]
+                copy16_async(st + i * 16 + q4, &V(row0 + q4, col0 + i));
+                copy16_async(st + VS + TS + i * 16 + q4, &V(row0 + q4, j0 + i));
+            } else {  // [row][reflector], [row][column]
+                copy16_async(st + pad4(i) + q4, &V(row0 + i, col0 + q4));
+                copy16_async(st + VS + TS + pad8(i) + q4, &V(row0 + i, j0 + q4));
+            }
+            copy16_async(st + VS + pad4(i) + q4, tblk + (size_t)p * kIB * kIB + i * 16 + q4);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float *exq = ex[tid >> 5] + ((tid & 31) >> 2) * 20;
+    auto gather = [&](const float (&own)[4], float (&all)[16]) {  // the quad's 4 x 4 values
+        __syncwarp();
+        *reinterpret_cast<float4 *>(exq + 4 * qd) = make_float4(own[0], own[1], own[2], own[3]);
+        __syncwarp();
+        ld16<float>(exq, all);
+    };
+    auto load4 = [&](int64_t r0, float (&v)[4]) {
+        load_col<float, LAYOUT, float, 4>(V, r0 + 4 * qd, j0 + col, v);
+    };
+    auto store4 = [&](int64_t r0, const float (&v)[4]) {
+        store_col<float, LAYOUT, float, 4>(V, r0 + 4 * qd, j0 + col, v);
+    };
+
+    float top[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (p0 > 0) load4(top0, top);
+    for (int i = 0; i < kU16S - 1; ++i) fetch(p0 + i);
+#pragma unroll 1
+    for (int p = p0; p < P; ++p) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kU16S - 2) : "memory");
+        __syncthreads();  // tile p is here; the slot of tile p - 1 is free
+        fetch(p + kU16S - 1);
+        const float *st = sm + (p % kU16S) * ST;
+        const bool head = p == 0;  // the top tile itself (GEQRT): unit lower V, W = T^T Z
+        float v[4][16], a[4];
+        if (LAYOUT == 0) {
+#pragma unroll
+            for (int l = 0; l < 16; ++l) {
+                const float4 x = *reinterpret_cast<const float4 *>(st + l * 16 + 4 * qd);
+                v[0][l] = x.x;
+                v[1][l] = x.y;
+                v[2][l] = x.z;
+                v[3][l] = x.w;
+            }
+            const float4 x = *reinterpret_cast<const float4 *>(st + VS + TS + col * 16 + 4 * qd);
+            a[0] = x.x;
+            a[1] = x.y;
+            a[2] = x.z;
+            a[3] = x.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                ld16<float>(st + pad4(4 * qd + e), v[e]);
+                a[e] = st[VS + TS + pad8(4 * qd + e) + col];
+            }
+        }
+        if (head) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int l = 0; l < 16; ++l)
+                    v[e][l] = 4 * qd + e > l ? v[e][l] : (4 * qd + e == l ? 1.0f : 0.0f);
+        }
+        // Z = V^T A: the quad's partial sums, reflectors 4 qd .. 4 qd + 3 to this thread
+        float z[16], k8[8], zo[4];
+#pragma unroll
+        for (int l = 0; l < 16; ++l) {
+            z[l] = v[0][l] * a[0];
+#pragma unroll
+            for (int e = 1; e < 4; ++e) z[l] = fmaf(v[e][l], a[e], z[l]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float keep = (qd & 2) ? z[8 + i] : z[i], send = (qd & 2) ? z[i] : z[8 + i];
+            k8[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float keep = (qd & 1) ? k8[4 + i] : k8[i], send = (qd & 1) ? k8[i] : k8[4 + i];
+            zo[i] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+            if (!head) zo[i] += top[i];
+        }
+        // W = T^T Z, top rows -= W
+        float wo[4], w[16];
+        gather(zo, z);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float t[16], s0 = 0.0f, s1 = 0.0f;
+            ld16<float>(st + VS + pad4(4 * qd + e), t);
+#pragma unroll
+            for (int m = 0; m < 16; m += 2) {
+                s0 = fmaf(t[m], z[m], s0);
+                s1 = fmaf(t[m + 1], z[m + 1], s1);
+            }
+            wo[e] = s0 + s1;
+            if (!head) top[e] -= wo[e];
+        }
+        gather(wo, w);
+        // A -= V W
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+            for (int l = 0; l < 16; l += 2) {
+                s0 = fmaf(v[e][l], w[l], s0);
+                s1 = fmaf(v[e][l + 1], w[l + 1], s1);
+            }
+            a[e] -= s0 + s1;
+        }
+        if (head) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) top[e] = a[e];
+        } else {
+            store4((int64_t)(args.pr + p) * 16, a);
+        }
+    }
+    store4(top0, top);
+}
+
 // One panel kernel per tile size.
 template <typename T, int LAYOUT, typename CT, int B>
 int launch_panel_b(const PanelArgs &a, dim3 grid, cudaStream_t s) {
@@ -1508,14 +1664,12 @@ int launch_update_b(UpdateArgs a, int64_t ncols, const Stage1Work &w, cudaStream
     }
     const int batch = w.batch > 0 ? w.batch : 1;
     a.nstrip = (int)((ncols + C::W - 1) / C::W);
-    // Tiles per CTA.  Passing the strip on costs about what a 16-wide FP32 tile costs,
-    // so those go to one CTA per strip (n = 1296: stage 1 49 ms, one tile per CTA
-    // 54).  Otherwise one tile per CTA where latency counts (FP32 n = 1024 tile 64
+    // Tiles per CTA.  One tile per CTA where latency counts (FP32 n = 1024 tile 64
     // 5.0 ms, all tiles in one CTA 6.5; FP64 n = 512 tile 32 18.0 against 27.7, and
     // FP64 always: its tiles take long), and all of them once the strips fill the GPU
     // twice over by themselves (32 matrices of order 1024 tile 64 10.5 ms against
     // 15.0, 256 of order 256 tile 32 2.2 against 3.0).  The values do not depend on it.
-    const bool whole = C::F4 && (B == 16 || (int64_t)a.nstrip * batch >= 304);
+    const bool whole = C::F4 && (int64_t)a.nstrip * batch >= 304;
     a.group = whole ? a.P : 1;
     // ticket and counters: one per block and strip in the work's own array, else (out
     // of core) one per strip in the panel's flags, which are free again
@@ -1529,6 +1683,12 @@ int launch_update_b(UpdateArgs a, int64_t ncols, const Stage1Work &w, cudaStream
         AVS_CUDA_TRY(cudaMemsetAsync(a.flags, 0, fb, s));
     const int ngrp = (a.P - a.first_role + a.group - 1) / a.group;
     update_kernel<T, LAYOUT, B><<<dim3((unsigned)a.nstrip * ngrp, batch), C::NT, smem, s>>>(a);
+    AVS_CUDA_TRY(cudaGetLastError());
+    return AVS_SUCCESS;
+}
+template <int LAYOUT>
+int launch_update16(const UpdateArgs &a, int64_t ncols, const Stage1Work &w, cudaStream_t s) {
+    update16_kernel<LAYOUT><<<dim3((unsigned)(ncols / kU16W), w.batch > 0 ? w.batch : 1), kU16T, 0, s>>>(a);
     AVS_CUDA_TRY(cudaGetLastError());
     return AVS_SUCCESS;
 }
@@ -1551,7 +1711,9 @@ int launch_update(T *dA, int64_t lda, int64_t n, int b, int pr, int pc, int P, c
     a.sA = w.sA;
     a.sTblk = w.sTblk;
     switch (b) {
-        case 16: return launch_update_b<T, LAYOUT, 16>(a, ncols, w, s);
+        case 16:
+            if constexpr (sizeof(T) == 4) return launch_update16<LAYOUT>(a, ncols, w, s);
+            else return launch_update_b<T, LAYOUT, 16>(a, ncols, w, s);
         case 32: return launch_update_b<T, LAYOUT, 32>(a, ncols, w, s);
         case 64: return launch_update_b<T, LAYOUT, 64>(a, ncols, w, s);
         default: return AVS_ERR_UNSUPPORTED;  // the full-T update
