@@ -10,7 +10,9 @@
 // where S_p = Y_p^T A_p came from the batched tensor-core GEMM.  Each product
 // is one tcgen05 MMA sequence: the b x b factor (T_p^T, or Y0) is the A
 // operand, loaded by TMA from its K-major operand planes through a two-stage
-// ring; the strip operand (Top + S_p, or W0) is the B operand, written into
+// ring (192 KB a tile at b = 256 in split BF16, which is most of a tile's time; two
+// K blocks of the next tile load under this tile's epilogue: n = 16384 stage 1 262 ->
+// 250 ms); the strip operand (Top + S_p, or W0) is the B operand, written into
 // shared memory by the CTA's threads in the canonical 128-byte-swizzled
 // K-major layout; the accumulator (b rows x 32 columns, two 128-lane halves
 // for b = 256) lives in tensor memory.  Both factors are triangular (T_p^T
@@ -50,6 +52,7 @@ struct CCfg {
     static constexpr int EB = BF16 ? 2 : 4;
     static constexpr int BK = 128 / EB;           // K elements per 128-byte block
     static constexpr int NKB = B / BK;            // K blocks
+    static_assert(NKB >= 2, "two K blocks of the next product in the ring");
     static constexpr int HALVES = B / 128;        // 128-row halves of the factor
     static constexpr int PL = SPLIT ? 2 : 1;      // operand planes
     static constexpr int ZT = NS * 128;           // bytes of one B tile (32 rows x 128 B)
@@ -131,23 +134,30 @@ __global__ void __launch_bounds__(CCfg<B, SPLIT, BF16>::CNT, 1)
     // halves of the factor that are nonzero in K block kb (lower triangular)
     auto halves_in = [&](int kb) { return (kb * C::BK < 128) ? 0 : 1; };  // first half used
 
+    // K block kb of a factor into ring slot g & 1, once the products have read it
+    auto load_a = [&](int g, const CUtensorMap *ah, const CUtensorMap *al, int a_row0, int kb) -> bool {
+        const int s = g & 1;
+        if (g >= 2 && !mbar_wait(smem_u32(&empty[s]), (uint32_t)(((g >> 1) - 1) & 1), args.err)) return false;
+        const int h0 = halves_in(kb);
+        const uint32_t fb = smem_u32(&full[s]);
+        mbar_expect_tx(fb, (uint32_t)((C::HALVES - h0) * C::PL * C::AT));
+        for (int h = h0; h < C::HALVES; ++h) {
+            tma_load_2d(a_tile(s, h, 0), ah, kb * C::BK, a_row0 + h * 128, fb);
+            if (SPLIT) tma_load_2d(a_tile(s, h, 1), al, kb * C::BK, a_row0 + h * 128, fb);
+        }
+        return true;
+    };
     // One product: accumulator = factor rows [a_row0, a_row0 + B) (A) x strip operand (B).
-    auto product = [&](const CUtensorMap *ah, const CUtensorMap *al, int a_row0) {
+    // Its first two K blocks are in the ring already (but for the first product); the
+    // next product's (rows n_row0 of nh, nl; nh null: none) follow its own, so that they
+    // cross from L2 under this product's epilogue and the next operand's preparation.
+    auto product = [&](const CUtensorMap *ah, const CUtensorMap *al, int a_row0, const CUtensorMap *nh,
+                       const CUtensorMap *nl, int n_row0) {
         if (tid == 0) {
-            for (int kb = 0; kb < C::NKB; ++kb) {
-                const int g = gblk + kb, s = g & 1;
-                if (g >= 2 && !mbar_wait(smem_u32(&empty[s]), (uint32_t)(((g >> 1) - 1) & 1), args.err)) {
-                    s_fail = 1;
-                    break;
-                }
-                const int h0 = halves_in(kb);
-                const uint32_t fb = smem_u32(&full[s]);
-                mbar_expect_tx(fb, (uint32_t)((C::HALVES - h0) * C::PL * C::AT));
-                for (int h = h0; h < C::HALVES; ++h) {
-                    tma_load_2d(a_tile(s, h, 0), ah, kb * C::BK, a_row0 + h * 128, fb);
-                    if (SPLIT) tma_load_2d(a_tile(s, h, 1), al, kb * C::BK, a_row0 + h * 128, fb);
-                }
-            }
+            bool go = true;
+            for (int kb = gblk > 0 ? 2 : 0; go && kb < C::NKB; ++kb) go = load_a(gblk + kb, ah, al, a_row0, kb);
+            for (int kb = 0; go && nh && kb < 2; ++kb) go = load_a(gblk + C::NKB + kb, nh, nl, n_row0, kb);
+            if (!go) s_fail = 1;
         } else if (tid == 32) {
             for (int kb = 0; kb < C::NKB; ++kb) {
                 const int g = gblk + kb, s = g & 1;
@@ -240,7 +250,9 @@ __global__ void __launch_bounds__(CCfg<B, SPLIT, BF16>::CNT, 1)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (p + 1 < args.P) load_s(p + 1);
-        product(&tT_hi, &tT_lo, p * B);  // W = T_p^T Z
+        // W = T_p^T Z
+        if (p == 0) product(&tT_hi, &tT_lo, 0, &tY_hi, &tY_lo, 0);
+        else product(&tT_hi, &tT_lo, p * B, p + 1 < args.P ? &tT_hi : nullptr, &tT_lo, (p + 1) * B);
         if (p == 0) {
             // W0 becomes the strip operand of Top -= Y0 W0
             {
@@ -253,7 +265,7 @@ __global__ void __launch_bounds__(CCfg<B, SPLIT, BF16>::CNT, 1)
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            product(&tY_hi, &tY_lo, 0);  // Y0 W0
+            product(&tY_hi, &tY_lo, 0, args.P > 1 ? &tT_hi : nullptr, &tT_lo, B);  // Y0 W0
             {
                 float v[EC];
                 read_acc(v);
