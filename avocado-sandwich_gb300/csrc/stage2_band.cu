@@ -106,7 +106,7 @@ __device__ __forceinline__ bool positive(dfx a) { return a.v.hi > 0.0f; }
 __device__ __forceinline__ float wsum(float v) { return warp_sum(v); }
 __device__ __forceinline__ double wsum(double v) { return warp_sum(v); }
 __device__ __forceinline__ dfx wsum(df64 s) {
-#pragma unroll
+#pragma unroll 1
     for (int o = 16; o > 0; o >>= 1)
         s = MacAr<dfx>::mac_merge(s, df64{__shfl_xor_sync(0xffffffffu, s.hi, o), __shfl_xor_sync(0xffffffffu, s.lo, o)});
     return MacAr<dfx>::fin(s);
@@ -405,12 +405,38 @@ __device__ __forceinline__ void substitute(const R *s_tau, const R *gram, R *Wy,
         Wy[k * LDW + row] = y;
     }
 }
+// The same with a lane per reflector: lane l of a group of T holds w_l of one row, y_k
+// passes by shuffle.  A loop of T short steps instead of T^2 / 2 multiply-adds in a row.
+template <typename R, int T, int KS, int LDW, int RPC, int NT>
+__device__ __forceinline__ void substitute_lanes(const R *s_tau, const R *gram, R *Wy) {
+    constexpr int GRP = NT / T;
+    static_assert(RPC % GRP == 0, "rows per group");
+    const int l = threadIdx.x % T, grp = threadIdx.x / T;
+#pragma unroll 1
+    for (int row = grp; row < RPC; row += GRP) {
+        auto w = MacAr<R>::mac_from(Wy[l * LDW + row]);
+#pragma unroll 1
+        for (int q = 1; q < KS; ++q) w = MacAr<R>::mac_merge(w, MacAr<R>::mac_from(Wy[(q * T + l) * LDW + row]));
+        R y = R(0);
+#pragma unroll 1
+        for (int k = 0; k < T; ++k) {
+            const R yk = wshfl(s_tau[k] * MacAr<R>::fin(w), (threadIdx.x & 31 & ~(T - 1)) + k);
+            if (l == k) y = yk;
+            if (l > k) MacAr<R>::mac(w, -gram[k * (T + 1) + l], yk);
+        }
+        Wy[l * LDW + row] = y;
+    }
+}
 
 template <int B, int T, typename R, int C>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel(R *ab_base, int64_t n, int64_t ldab, int *ticket,
                                                           int *done_base, int *err, int batch, int64_t sAB,
                                                           int64_t sDone) {
     using Cfg = BandCfg<B, T, C>;
+    // double-float: short loops (one row or column of the products at a time, the
+    // substitution a lane per reflector), since unrolled as FP32 is the op's code does not
+    // fit the instruction caches (band 64 n = 1024 7.0 -> 6.5 ms, 128 n = 2048 14.5 -> 12.6)
+    constexpr bool kSmall = std::is_same<R, dfx>::value;
     constexpr int NT = Cfg::NT, NW = Cfg::NW, LDP = Cfg::LDP, RPC = Cfg::RPC, LDW = Cfg::LDW;
     constexpr int ku = band_ku(B);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -525,6 +551,19 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                     for (int a = 0; a < 4; ++a)
 #pragma unroll
                         for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = MacAr<R>::mac0();
+                    if constexpr (kSmall) {
+#pragma unroll 1
+                        for (int c = ks * Cfg::BK; c < (ks + 1) * Cfg::BK; ++c) {
+                            R a4[4];
+                            Vec4<R>::ld(As + c * Cfg::LDA_R + 4 * g, a4);
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk) {
+                                const R vk = P[(k0 + kk) * LDP + c];
+#pragma unroll
+                                for (int rr = 0; rr < 4; ++rr) MacAr<R>::mac(acc[kk][rr], a4[rr], vk);
+                            }
+                        }
+                    } else {
 #pragma unroll 2
                     for (int c = ks * Cfg::BK; c < (ks + 1) * Cfg::BK; c += 4) {
                         R a4[4][4], v4[4][4];
@@ -539,13 +578,15 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
 #pragma unroll
                                 for (int rr = 0; rr < 4; ++rr) MacAr<R>::mac(acc[kk][rr], a4[cc][rr], v4[kk][cc]);
                     }
+                    }
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
                         for (int rr = 0; rr < 4; ++rr) Wy[(ks * T + k0 + kk) * LDW + 4 * g + rr] = MacAr<R>::fin(acc[kk][rr]);
                 }
                 __syncthreads();
-                if (tid < RPC) substitute<R, T, Cfg::KS, LDW>(s_tau, gram, Wy, tid);
+                if constexpr (kSmall) substitute_lanes<R, T, Cfg::KS, LDW, RPC, NT>(s_tau, gram, Wy);
+                else if (tid < RPC) substitute<R, T, Cfg::KS, LDW>(s_tau, gram, Wy, tid);
                 __syncthreads();
                 // A -= Y V^T: thread = 4 rows x CPT2R columns; straight to global
                 {
@@ -557,6 +598,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                     for (int cc = 0; cc < CPT; ++cc)
 #pragma unroll
                         for (int rr = 0; rr < 4; ++rr) acc[rr][cc] = MacAr<R>::mac_from(As[(cb + cc) * Cfg::LDA_R + 4 * g + rr]);
+#pragma unroll(kSmall ? 1 : 16)
                     for (int k = 0; k < T; ++k) {
                         R y4[4];
                         Vec4<R>::ld(Wy + k * LDW + 4 * g, y4);
@@ -670,6 +712,20 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                     for (int a = 0; a < 4; ++a)
 #pragma unroll
                         for (int b2 = 0; b2 < 4; ++b2) acc[a][b2] = MacAr<R>::mac0();
+                    if constexpr (kSmall) {
+#pragma unroll 1
+                        for (int i = ks * Cfg::BK; i < (ks + 1) * Cfg::BK; ++i) {
+                            R a4[4];
+#pragma unroll
+                            for (int cc = 0; cc < 4; ++cc) a4[cc] = As[(g + cc * Cfg::NG4) * Cfg::LDA_L + i];
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk) {
+                                const R vk = P[(k0 + kk) * LDP + i];
+#pragma unroll
+                                for (int cc = 0; cc < 4; ++cc) MacAr<R>::mac(acc[kk][cc], vk, a4[cc]);
+                            }
+                        }
+                    } else {
 #pragma unroll 2
                     for (int i = ks * Cfg::BK; i < (ks + 1) * Cfg::BK; i += 4) {
                         R a4[4][4], v4[4][4];
@@ -685,13 +741,15 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
 #pragma unroll
                                 for (int ii = 0; ii < 4; ++ii) MacAr<R>::mac(acc[kk][cc], v4[kk][ii], a4[cc][ii]);
                     }
+                    }
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
                         for (int cc = 0; cc < 4; ++cc) Wy[(ks * T + k0 + kk) * LDW + g + cc * Cfg::NG4] = MacAr<R>::fin(acc[kk][cc]);
                 }
                 __syncthreads();
-                if (tid < RPC) substitute<R, T, Cfg::KS, LDW>(s_tau, gram, Wy, tid);
+                if constexpr (kSmall) substitute_lanes<R, T, Cfg::KS, LDW, RPC, NT>(s_tau, gram, Wy);
+                else if (tid < RPC) substitute<R, T, Cfg::KS, LDW>(s_tau, gram, Wy, tid);
                 __syncthreads();
                 // A -= V Y: thread = 4 rows x CPT2L columns; straight to global
                 {
@@ -703,6 +761,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) band_stage_kernel
                     for (int cc = 0; cc < CPT; ++cc)
 #pragma unroll
                         for (int ii = 0; ii < 4; ++ii) acc[ii][cc] = MacAr<R>::mac_from(As[(cb + cc) * Cfg::LDA_L + 4 * ig + ii]);
+#pragma unroll(kSmall ? 1 : 16)
                     for (int k = 0; k < T; ++k) {
                         R v4[4];
                         Vec4<R>::ld(P + k * LDP + 4 * ig, v4);
