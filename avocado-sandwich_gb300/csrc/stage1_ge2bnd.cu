@@ -1799,7 +1799,7 @@ int stage1_ge2bnd_tc(float *X, int64_t n, int b, const Stage1Work &w, cudaStream
         if ((int64_t)(pc + 1) * b < n && (r = stage1_tbuild<float>(M, n, b, 0, pr, pc, P, w, a)) != AVS_SUCCESS)
             return r;
         if (la) AVS_CUDA_TRY(cudaEventRecord(w.la_tb, a));
-        if (launches) *launches += 2;
+        if (launches) *launches += (int64_t)(pc + 1) * b < n ? 3 : 1;
         return AVS_SUCCESS;
     };
     // one half-step's update on the caller's stream, with the next panel
@@ -1875,7 +1875,7 @@ int stage1_ge2bnd(T *dA, int64_t n, int64_t lda, int b, const Stage1Work &w, cud
         else
             rc = launch_update<T, 0>(dA, lda, n, b, k, k, P, w, s);
         if (rc != AVS_SUCCESS) return rc;
-        if (launches) *launches += (k + 1 < nt) ? ((b >= 128 && w.tfull) ? 3 : 2) : 1;
+        if (launches) *launches += (k + 1 < nt) ? ((b >= 128 && w.tfull) ? 4 : 2) : 1;
         if (k == nt - 1) break;
         // LQ half-step: the same on the transposed view, top tile (k, k+1).
         const int PL = nt - k - 1;
@@ -1886,7 +1886,7 @@ int stage1_ge2bnd(T *dA, int64_t n, int64_t lda, int b, const Stage1Work &w, cud
         else
             rc = launch_update<T, 1>(dA, lda, n, b, k + 1, k, PL, w, s);
         if (rc != AVS_SUCCESS) return rc;
-        if (launches) *launches += (b >= 128 && w.tfull) ? 3 : 2;
+        if (launches) *launches += (b >= 128 && w.tfull) ? 4 : 2;
     }
     return AVS_SUCCESS;
 }
@@ -1925,7 +1925,7 @@ int stage1_geqrf(T *dA, int64_t n, int64_t lda, int b, const Stage1Work &w, T *d
                 if ((rc = timed_update(reinterpret_cast<float *>(dA), n, b, k, k, P, w, tb, s, launches)) !=
                     AVS_SUCCESS)
                     return rc;
-                if (launches) *launches += 2;
+                if (launches) *launches += 3;
                 continue;
             }
         }
@@ -1934,7 +1934,7 @@ int stage1_geqrf(T *dA, int64_t n, int64_t lda, int b, const Stage1Work &w, T *d
         else
             rc = launch_update<T, 0>(dA, lda, n, b, k, k, P, w, s);
         if (rc != AVS_SUCCESS) return rc;
-        if (launches) *launches += (b >= 128 && w.tfull) ? 2 : 1;
+        if (launches) *launches += (b >= 128 && w.tfull) ? 3 : 1;
     }
     return AVS_SUCCESS;
 }
