@@ -189,7 +189,7 @@ inline int flags_of(const avs_opts *opts) { return opts ? opts->flags : 0; }
 // bidiagonal by the element chase (0: the element chase from width b).  FP64
 // stages keep the one-stage chase unless asked (the FP64 block stage runs on
 // the FP64 pipe, 1/64 of the FP32 rate: slower than the one-stage FP64 chase,
-// measured 537 vs 315 ms at n = 8192, tile 128).
+// measured 32 vs 20 ms at n = 1024, tile 64).
 int narrow_band_of(int b, int flags, bool fp64) {
     if (flags & AVS_FLAG_ONE_STAGE_CHASE) return 0;
     if (fp64 && !(flags & AVS_FLAG_HIER_CHASE)) return 0;
@@ -283,9 +283,9 @@ int run_stages23(avs_handle *h, const Layout &L, int64_t n, int b, const S *W, i
         if (band_ran) *band_ran = true;
     } else if (tbw > 0 && sizeof(S) == 8 && !fp64_stages) {
         // FP64 tiles, double-float stages: the block stage in double-float too.  One
-        // stage against two (GB300, stage 2): tile 64 n = 256 3.3 / 2.9 ms, n = 1024 15.1
-        // / 13.2; tile 128 n = 512 8.1 / 6.6, n = 2048 36.6 / 29.0; tile 256 n = 2048 72.5
-        // / 37.0.
+        // stage against two (GB300, stage 2): tile 64 n = 256 3.3 / 2.6 ms, n = 1024 15.1
+        // / 11.5; tile 128 n = 512 8.1 / 5.4, n = 2048 36.6 / 22.8; tile 256 n = 2048 72.5
+        // / 29.4.
         if ((rc = stage2_chase_hier_df<double, dfx>(
                  reinterpret_cast<const double *>(W), n, ldw, b, tbw, reinterpret_cast<dfx *>(AB),
                  reinterpret_cast<float2 *>(ws_at(h, L.off_ab2)), dd, de, w2, s, h->num_sms, launches,
