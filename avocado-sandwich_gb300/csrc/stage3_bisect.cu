@@ -25,37 +25,50 @@
 namespace avs {
 namespace {
 
-// scratch[0] = Gershgorin bound of TGK, scratch[1] = pivmin, scratch[2] = exponent k
-// of the scaling by 2^-k (one block).
+// scratch[0] = Gershgorin bound of TGK (Inf when it overflows, or an entry is Inf),
+// scratch[1] = pivmin, scratch[2] = exponent k of the scaling by 2^-k, scratch[3] =
+// the bound of the scaled matrix: below 1 for finite entries (taken from quarters of
+// the entries, whose sums don't overflow), else Inf (one block).
 __device__ void tgk_bound_body(const double *d, const double *e, int64_t n, double *scratch) {
-    __shared__ double sb[32], sm[32];
-    double bound = 0.0, maxsq = 0.0;
+    __shared__ double sb[32], sq[32], sm[32];
+    double bound = 0.0, quarter = 0.0, maxsq = 0.0;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
         const double di = fabs(d[i]);
         const double el = i > 0 ? fabs(e[i - 1]) : 0.0;
         const double er = i + 1 < n ? fabs(e[i]) : 0.0;
         bound = fmax(bound, di + el + er);
+        quarter = fmax(quarter, 0.25 * di + 0.25 * el + 0.25 * er);
         maxsq = fmax(maxsq, fmax(di * di, er * er));
     }
     for (int o = 16; o > 0; o >>= 1) {
         bound = fmax(bound, __shfl_xor_sync(0xffffffffu, bound, o));
+        quarter = fmax(quarter, __shfl_xor_sync(0xffffffffu, quarter, o));
         maxsq = fmax(maxsq, __shfl_xor_sync(0xffffffffu, maxsq, o));
     }
     if ((threadIdx.x & 31) == 0) {
         sb[threadIdx.x >> 5] = bound;
+        sq[threadIdx.x >> 5] = quarter;
         sm[threadIdx.x >> 5] = maxsq;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double b2 = 0.0, m2 = 0.0;
+        double b2 = 0.0, b4 = 0.0, m2 = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
             b2 = fmax(b2, sb[w]);
+            b4 = fmax(b4, sq[w]);
             m2 = fmax(m2, sm[w]);
         }
         scratch[0] = b2;
         scratch[1] = DBL_MIN * fmax(m2, 1.0);
         // exponent of the scale: b2 2^-k < 1, with room for the bound's rounding
-        scratch[2] = (b2 > 0.0 && b2 <= DBL_MAX) ? (double)(ilogb(b2 * (1.0 + 1e-6)) + 1) : 0.0;
+        int k = 0;
+        double scaled = b4;
+        if (b4 <= DBL_MAX && b2 > 0.0) {
+            k = b4 >= 1.0 ? ilogb(b4 * (1.0 + 1e-6)) + 3 : ilogb(b2 * (1.0 + 1e-6)) + 1;
+            scaled = b4 >= 1.0 ? scalbn(b4, 2 - k) : scalbn(b2, -k);
+        }
+        scratch[2] = (double)k;
+        scratch[3] = scaled;
     }
 }
 
@@ -281,7 +294,7 @@ __device__ __forceinline__ int tgk_count_d(const double *__restrict__ sq, int m,
         q = tgk_step_d(__ldg(sq + i), q, x);
         // |q| < DBL_MIN (no exponent): the pivot guard
         if ((__double2hiint(q) & 0x7ff00000) == 0) q = -DBL_MIN;
-        cnt += (unsigned)__double2hiint(q) >> 31;
+        cnt += (unsigned)__double2hiint(q) - 0x80000000u <= 0x7ff00000u;  // q < 0, no NaN
     }
     return cnt;
 }
@@ -336,13 +349,13 @@ __device__ __forceinline__ Bracket widen(const Bracket &b) {
 template <int G, bool F64>
 __device__ double bisect_grp(const float2 *a, const double *sq, int64_t n, int64_t k, double rel_tol,
                              const double *scratch, int gl, unsigned gmask) {
-    const double bound = scratch[0];
-    if (!(bound > 0.0)) return bound;  // 0, or NaN
+    const double bound = scratch[0], scaled = scratch[3];
+    if (!(bound > 0.0 && scaled <= 1.0)) return bound;  // 0, or an entry is Inf
     const int ke = (int)scratch[2];
     const int m = (int)(2 * n - 1);
     const int target = (int)(2 * n - 1 - k);  // TGK index (ascending) of the k-th largest sigma
     // depth whose cells are at most rel_tol * bound wide
-    const double tol = fmin(fmax(rel_tol * scalbn(bound, -ke), 1e-17), 0.5);
+    const double tol = fmin(fmax(rel_tol * scaled, 1e-17), 0.5);
     int want = -ilogb(tol);
     if (pow2d(-want) > tol) ++want;
     want = max(want, kDepthF + 2);
@@ -387,6 +400,9 @@ __device__ double bisect_grp(const float2 *a, const double *sq, int64_t n, int64
             multisect<G, 1>(b, wd, gl, gmask, ex_d);
         }
     }
+    // no count reached the target below the bound (a NaN entry, which no comparison
+    // counts): the bound
+    if ((double)b.lo * pow2d(-b.depth) > scaled) return bound;
     return scalbn(((double)b.lo + 0.5) * pow2d(-b.depth), ke);
 }
 
