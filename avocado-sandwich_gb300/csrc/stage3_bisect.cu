@@ -400,10 +400,25 @@ __device__ double bisect_grp(const float2 *a, const double *sq, int64_t n, int64
             multisect<G, 1>(b, wd, gl, gmask, ex_d);
         }
     }
+    double lo = (double)b.lo * pow2d(-b.depth), hi = ((double)b.lo + 1.0) * pow2d(-b.depth);
     // no count reached the target below the bound (a NaN entry, which no comparison
     // counts): the bound
-    if ((double)b.lo * pow2d(-b.depth) > scaled) return bound;
-    return scalbn(((double)b.lo + 0.5) * pow2d(-b.depth), ke);
+    if (lo > scaled) return bound;
+    if constexpr (F64) {
+        // a width below the grid's cells (2^-52 of the scale): halving, as far down as
+        // FP64 numbers and the requested width go.  Every lane of the group runs the
+        // same counts; the default width ends on the grid (one halving more for a bound
+        // within 1e-6 below a power of two).
+        for (int it = 0; it < 128 && hi - lo > rel_tol * scaled; ++it) {
+            const double mid = 0.5 * (lo + hi);
+            if (mid <= lo || mid >= hi) break;
+            if (tgk_count_d(sq, m, mid) > target)
+                hi = mid;
+            else
+                lo = mid;
+        }
+    }
+    return scalbn(0.5 * (lo + hi), ke);
 }
 
 // Lanes per value.  A pass costs one count's latency while every scheduler has
