@@ -307,7 +307,8 @@ struct Bracket {
 };
 
 constexpr int kDepthF = 18;      // cells of the FP32 phase: its counts err by up to a few 1e-7
-constexpr int kDepthDfMax = 47;  // the double-float grid: shifts are exact pairs
+constexpr int kDepthDfMax = 51;  // the double-float grid: exact pairs to depth 48, below it shifts near 1
+                                 // round at 2^-50 (a width of 1e-15 of the bound, the least in double-float)
 constexpr int kDepthDfD = 40;    // double-float cells before the FP64 phase
 
 // One group (G consecutive lanes) splits the bracket at G K points per pass until
@@ -355,7 +356,7 @@ __device__ double bisect_grp(const float2 *a, const double *sq, int64_t n, int64
     const int m = (int)(2 * n - 1);
     const int target = (int)(2 * n - 1 - k);  // TGK index (ascending) of the k-th largest sigma
     // depth whose cells are at most rel_tol * bound wide
-    const double tol = fmin(fmax(rel_tol * scaled, 1e-17), 0.5);
+    const double tol = fmin(F64 ? fmax(rel_tol * scaled, 1e-17) : fmax(rel_tol, 1e-15) * scaled, 0.5);
     int want = -ilogb(tol);
     if (pow2d(-want) > tol) ++want;
     want = max(want, kDepthF + 2);
@@ -375,9 +376,11 @@ __device__ double bisect_grp(const float2 *a, const double *sq, int64_t n, int64
         df64 x[K];
         int c[K];
 #pragma unroll
-        for (int j = 0; j < K; ++j) {  // 24 + 23 bits, both exact
+        for (int j = 0; j < K; ++j) {  // the upper bits rounded to 24, the rest
             const long long v = v0 + j;
-            x[j] = fast_two_sum((float)(int)(v >> 24) * pow2f(24 - depth), (float)(int)(v & 0xffffff) * pow2f(-depth));
+            const float h = (float)(unsigned)(v >> 20);
+            const int r = (int)(v - ((long long)(unsigned)h << 20));
+            x[j] = fast_two_sum(h * pow2f(20 - depth), (float)r * pow2f(-depth));
         }
         tgk_count_df<K>(a, m, x, c);
 #pragma unroll

@@ -98,3 +98,15 @@ def test_width_below_the_grid_whole_call(avs_mod, batch):
     else:
         got = avs_mod.my_CU_svdval(a, 16, rel_tol=1e-26)
     assert np.all(np.abs(got.cpu().numpy() - d) <= 1e-26 + 2 * d.size * 2.0 ** -46 * d)
+
+
+def test_narrowest_width_in_double_float(avs_mod):
+    """A width of 1e-15 of the bound (here 0.9): the values, midpoints of brackets no wider
+    than that, cannot all be midpoints of cells of 2^-47."""
+    torch = cuda()
+    d = np.random.default_rng(5).uniform(0.0, 0.9, 64)
+    d[0] = 0.9
+    a = torch.diag(torch.from_numpy(d)).cuda()
+    got = avs_mod.my_CU_svdval(a, 16, precision="fp64x2", rel_tol=1e-15).cpu().numpy()
+    assert np.any((got * 2.0 ** 48) % 1.0 != 0.0)
+    assert np.max(np.abs(got - np.sort(d)[::-1])) <= 2e-14
