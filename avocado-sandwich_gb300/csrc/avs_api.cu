@@ -46,7 +46,8 @@ struct avs_handle {
         int64_t kernels = 0;
         cudaEvent_t ev[4] = {};  // recorded inside the graph: start, after stage 1, 2, 3
     };
-    std::map<std::tuple<int64_t, int, int, int>, Graph> graphs;  // (n, tile, count, output form)
+    // (n, tile, count, output form and flags, bisection width)
+    std::map<std::tuple<int64_t, int, int, int, double>, Graph> graphs;
     void drop_graphs() {
         for (auto &kv : graphs) {
             cudaGraphExecDestroy(kv.second.exec);
@@ -1444,7 +1445,8 @@ static int batched_call(avs_handle *h, int32_t count, const int64_t *n, const in
                                              AVS_FLAG_HIER_CHASE);
         const auto key = std::make_tuple(gn, gb, cnt,
                                          (bidiag ? 1 : 0) + (sizeof(T) == 8 ? 2 : 0) + (dfu ? 4 : 0) + (f64s ? 8 : 0) +
-                                             (cflags << 4));
+                                             (cflags << 4),
+                                         bidiag ? 0.0 : tol);
         auto it = h->graphs.find(key);
         if (it == h->graphs.end()) {
             avs_handle::Graph gr;

@@ -294,7 +294,7 @@ int avs_bidiag_svals_noalloc(int64_t n, const double *dd, const double *de, doub
  * group: stage-1 launches cover the whole group, one cluster chase kernel runs
  * all the group's sweeps, one bisection kernel all its values.  Each group's
  * launch sequence is captured once in a CUDA graph (kept per (n, tile, group
- * size) on the handle) and replayed.  Results of a matrix do not depend on the
+ * size, bisection width) on the handle) and replayed.  Results of a matrix do not depend on the
  * other matrices of the call.  Precision: FP32 tiles with double-float stages
  * 2 and 3 (the `precision` field of opts is ignored; bisect_rel_tol is used;
  * the Float64 form below takes AVS_PREC_FP64X2).
