@@ -207,8 +207,11 @@ struct PAr<double> : MacAr<double> {
     static __device__ __forceinline__ PRefl<double> scalars(Sq s, double alpha) {
         PRefl<double> r;
         const double x = fma(alpha, alpha, s);
-        if (x == 0.0) {
-            r.nu = r.tau = r.tc = r.f = r.inv = 0.0;
+        if (x == 0.0) {  // zero column: identity reflector
+            r.nu = r.tc = r.f = r.inv = 0.0;
+            // but not when alpha's square underflowed: the factorisation is refused
+            // (non-finite tau), as every column is whose norm FP64 cannot square
+            r.tau = alpha == 0.0 ? 0.0 : __longlong_as_double(0x7ff0000000000000ll);
             r.beta = alpha;
             return r;
         }
