@@ -112,6 +112,9 @@ struct Stage1Work {
     // idle in stage 1); without it (out of core) the diagonal blocks go through the matrix
     void *mail = nullptr;
     int64_t sMail = 0;      // doubles between matrices (batched)
+    // optional (one matrix; out of core): the b diagonal values of the call's first
+    // panel, contiguous (in core they are read from the matrix)
+    const void *ref = nullptr;
     int *err;         // device status word (shared with other stages)
     void *tfull;      // [nt][b*b] of T: full compact-WY factors (tiles 128, 256)
     void *tc_ws = nullptr;  // tensor-core update buffers (stage1_tc_bytes), FP32 tiles

@@ -76,10 +76,12 @@ int copy2d(T *dst, int64_t dld, const T *src, int64_t sld, int64_t width, int64_
 // One half-step through slab buffers.  layout 0 (QR, tile rows of the block
 // rows r0.., columns c0..n-1) or 1 (LQ, tile columns of the block columns c0..,
 // rows r0..n-1).  `tiles` tiles in the panel; the top tile is tile 0.  tau of
-// role p goes to tau_host + p*b (QR only).
+// role p goes to tau_host + p*b (QR only); first_diag (optional) receives the b
+// diagonal values of the finished top tile (device).
 template <typename T>
 int half_step(T *A, int64_t n, int64_t lda, int b, int layout, int64_t r0, int64_t c0, int tiles, int slab,
-              const OocBufs &ob, const Stage1Work &w, T *tau_host, cudaStream_t s, OocStats *st) {
+              const OocBufs &ob, const Stage1Work &w, T *tau_host, cudaStream_t s, OocStats *st,
+              T *first_diag = nullptr) {
     // the block: QR: rows r0 + [0, tiles*b), columns c0..n-1 (m columns);
     //            LQ: columns c0 + [0, tiles*b), rows r0..n-1 (m rows)
     const int64_t m = layout == 0 ? n - c0 : n - r0;
@@ -129,6 +131,9 @@ int half_step(T *A, int64_t n, int64_t lda, int b, int layout, int64_t r0, int64
         if ((rc = move(X[nx], 1, 1 + done, std::min(slab, tiles - 1 - done), true)) != AVS_SUCCESS) return rc;
         cur = nx;
     }
+    if (first_diag)  // for the later panels
+        AVS_CUDA_TRY(cudaMemcpy2DAsync(first_diag, sizeof(T), X[cur], sizeof(T) * (size_t)(ld + 1), sizeof(T), (size_t)b,
+                                       cudaMemcpyDeviceToDevice, s));
     return move(X[cur], 0, 0, 1, false);
 }
 
@@ -160,6 +165,7 @@ int ooc_ge2bnd(T *A, int64_t n, int64_t lda, int b, bool qr_only, T *tau_host, c
     w.flags = ob.flags;
     w.err = err;
     w.tfull = ob.tfull;  // full-T updates for tiles >= 128, as in core
+    T *diag = static_cast<T *>(ob.tau) + (size_t)nt * b;  // tau's last slot: no panel has nt + 1 tiles
     int rc;
     for (int k = 0; k < nt; ++k) {
         const int64_t kb = (int64_t)k * b, m = n - kb;
@@ -193,8 +199,10 @@ int ooc_ge2bnd(T *A, int64_t n, int64_t lda, int b, bool qr_only, T *tau_host, c
         }
         // QR half-step k: tile rows k..nt-1 of tile column k
         if ((rc = half_step<T>(A, n, lda, b, 0, kb, kb, ntt, plan.slab, ob, w,
-                               tau_host ? tau_host + ((size_t)k * nt + k) * b : nullptr, s, st)) != AVS_SUCCESS)
+                               tau_host ? tau_host + ((size_t)k * nt + k) * b : nullptr, s, st,
+                               k == 0 ? diag : nullptr)) != AVS_SUCCESS)
             return rc;
+        w.ref = diag;
         if (qr_only || k == nt - 1) continue;
         // LQ half-step k: tile columns k+1..nt-1 of tile row k
         if ((rc = half_step<T>(A, n, lda, b, 1, kb, kb + b, ntt - 1, plan.slab, ob, w, nullptr, s, st)) !=

@@ -73,6 +73,8 @@ struct PanelArgs {
     int ready_need;
     unsigned long long *mail;  // optional: rows of the diagonal blocks, role to role (tagged words)
     unsigned tag;              // this launch's tag, never 0
+    const void *ref;  // optional: the b diagonal values of the call's first panel, at ref_ld, sRef per matrix
+    int64_t ref_ld, sRef;
     int64_t sA, sTau, sTblk, sFlags, sMail;  // per-matrix strides (blockIdx.y = matrix)
 };
 
@@ -100,7 +102,10 @@ struct UpdateArgs {
 // tau = 2 nu^2 / (s + nu^2) = |nu| / n1, tc = tau / nu = sign(nu) / n1,
 // f = tau / nu^2 = 1 / (n1 |nu|), inv = 1 / nu, beta = -sign(alpha) n1 (the new
 // diagonal); evaluated in double-float for FP32 tiles and rounded once, in FP64
-// for FP64 tiles (reflect.cuh: hardware estimates and one residual each).
+// for FP64 tiles (reflect.cuh: hardware estimates and one residual each).  They are
+// meaningless for a zero column; small: the squared norm is 0, or so small that f may
+// overflow (or NaN); vanished: it is 0.  kRefuse: alpha != 0 whose square vanishes is
+// an error (FP32 and double-float take the column for zero).
 template <typename CT>
 struct PRefl {
     CT nu, tc, f, inv, beta, tau;
@@ -108,6 +113,7 @@ struct PRefl {
 
 template <typename CT>
 struct PAr;
+constexpr float kSmallF = 0x1.02p-128f;  // n1 |nu| >= n1^2 above it: f below 2^128
 
 struct PSqPair {
     using Sq = float2;
@@ -129,14 +135,12 @@ struct PAr<float> : PSqPair, MacAr<float> {
     // FP32 and everything else is a residual of them: with r ~ 1/n1 and z ~ 1/|nu|,
     // n1 = x r (1 + g), 1/n1 = r (1 + g), 1/|nu| = z (1 + k); relative errors
     // below 2^-44 before the one rounding of each result.
+    static constexpr bool kRefuse = false;
+    static __device__ __forceinline__ bool small(Sq s, float alpha) { return !(fmaf(alpha, alpha, s.x) > kSmallF); }
+    static __device__ __forceinline__ bool vanished(Sq s, float alpha) { return fmaf(alpha, alpha, s.x) <= 0.0f; }
     static __device__ __forceinline__ PRefl<float> scalars(Sq s, float alpha) {
         PRefl<float> o;
         const float xa = fmaf(alpha, alpha, s.x);  // n1^2 to FP32
-        if (xa <= 0.0f) {  // zero column: identity reflector
-            o.nu = o.tau = o.tc = o.f = o.inv = 0.0f;
-            o.beta = alpha;
-            return o;
-        }
         const float r = rsqrt_hw(xa);
         const df64 a2 = two_prod(alpha, alpha);
         const df64 x = two_sum(a2.hi, s.x);
@@ -174,16 +178,20 @@ struct PAr<dfx> : PSqPair, MacAr<dfx> {
         const float p = __fmul_rn(x.hi, x.hi);
         return make_float2(p, __fmaf_rn(2.0f * x.hi, x.lo, __fmaf_rn(x.hi, x.hi, -p)));
     }
+    static constexpr bool kRefuse = false;
+    static __device__ __forceinline__ bool small(Sq s, dfx al) {
+        const Sq m = merge(s, sq(al));
+        return !(__fadd_rn(m.x, m.y) > kSmallF);
+    }
+    static __device__ __forceinline__ bool vanished(Sq s, dfx al) {
+        const Sq m = merge(s, sq(al));
+        return __fadd_rn(m.x, m.y) <= 0.0f;
+    }
     static __device__ __forceinline__ PRefl<dfx> scalars(Sq s, dfx al) {
         PRefl<dfx> r;
         const df64 alpha = al.v;
         const Sq m = merge(s, sq(al));
         const df64 x = fast_two_sum(m.x, m.y);
-        if (x.hi <= 0.0f) {
-            r.nu = r.tau = r.tc = r.f = r.inv = dfx(0);
-            r.beta = al;
-            return r;
-        }
         df64 rn, n1;
         rsqrt_sqrt(x, rn, n1);
         const bool neg = df_lt0(alpha);
@@ -204,17 +212,14 @@ struct PAr<double> : MacAr<double> {
     static __device__ __forceinline__ Sq sq(double x) { return x * x; }
     static __device__ __forceinline__ Sq merge(Sq a, Sq b) { return a + b; }
     static __device__ __forceinline__ Sq merge_xor(Sq a, int o) { return a + __shfl_xor_sync(0xffffffffu, a, o); }
+    static constexpr bool kRefuse = true;
+    static __device__ __forceinline__ bool small(Sq s, double alpha) {
+        return (__double2hiint(fma(alpha, alpha, s)) & 0x7ff00000) == 0;  // below 2^-1022
+    }
+    static __device__ __forceinline__ bool vanished(Sq s, double alpha) { return fma(alpha, alpha, s) == 0.0; }
     static __device__ __forceinline__ PRefl<double> scalars(Sq s, double alpha) {
         PRefl<double> r;
         const double x = fma(alpha, alpha, s);
-        if (x == 0.0) {  // zero column: identity reflector
-            r.nu = r.tc = r.f = r.inv = 0.0;
-            // but not when alpha's square underflowed: the factorisation is refused
-            // (non-finite tau), as every column is whose norm FP64 cannot square
-            r.tau = alpha == 0.0 ? 0.0 : __longlong_as_double(0x7ff0000000000000ll);
-            r.beta = alpha;
-            return r;
-        }
         double rn, n1;
         rsqrt_sqrt(x, rn, n1);
         const bool neg = alpha < 0.0;
@@ -237,8 +242,26 @@ __device__ __forceinline__ dfx vshfl_xor(dfx v, int o) {
     return dfx(df64{__shfl_xor_sync(0xffffffffu, v.v.hi, o), __shfl_xor_sync(0xffffffffu, v.v.lo, o)});
 }
 __device__ __forceinline__ bool vfinite(float v) { return isfinite(v); }
-__device__ __forceinline__ bool vfinite(double v) { return isfinite(v); }
+__device__ __forceinline__ bool vfinite(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 __device__ __forceinline__ bool vfinite(dfx v) { return isfinite(v.v.hi) && isfinite(v.v.lo); }
+
+// Magnitudes in order, as integers: the bits of |v| (FP64: of its upper word), -1 for
+// Inf and NaN; and whether a magnitude is nothing against another (below the unit
+// roundoff of the type, and less).
+__device__ __forceinline__ int mag_bits(float v) {
+    const int m = __float_as_int(v) & 0x7fffffff;
+    return m < 0x7f800000 ? m : -1;
+}
+__device__ __forceinline__ int mag_bits(double v) {
+    const int m = __double2hiint(v) & 0x7fffffff;
+    return m < 0x7ff00000 ? m : -1;
+}
+__device__ __forceinline__ int mag_bits(dfx v) { return mag_bits(v.v.hi); }
+template <typename CT>
+__device__ __forceinline__ bool negligible(int m, int big) {
+    constexpr int k = std::is_same<CT, float>::value ? (30 << 23) : (std::is_same<CT, dfx>::value ? (56 << 23) : (60 << 20));
+    return m >= 0 && m < big - k;
+}
 
 // two sums of squares at a 16-byte aligned address
 template <typename Sq>
@@ -631,6 +654,7 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NTL) panel_kernel(PanelArgs a
     const int jc = lane & (kIB - 1), half = lane >> 4;
     const int rb = wid * 32 + half * RPL;
     CT col[RPL];
+    int big = 0;  // the largest column so far
     if (refl) load_col<T, LAYOUT, CT, RPL>(V, row0 + rb, col0 + jc, col);
     if constexpr (RESC > 0 && NB > 1) {  // the trailing columns, kept until the role is done
         constexpr int U = 16;
@@ -678,7 +702,13 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NTL) panel_kernel(PanelArgs a
             // or above the pivot row do not take part (zeros in the broadcast column);
             // the pivot row is row i % RPL of the lanes of its segment.
             CT myinv = CT(0), mytau = CT(0);
-            bool bad = false;
+            bool bad = false;  // a reflector that its type cannot hold
+            // the largest column of this block up to the i-th (within a factor of two) and of
+            // the blocks before it
+            auto largest = [&](int i) {
+                const int m = mag_bits(myinv);
+                return max(big, __reduce_max_sync(0xffffffffu, jc < i && m > 0 ? 2 * mag_bits(CT(1)) - m : 0));
+            };
             auto put_x = [&](int i) {  // column i's live rows for every lane of the warp
                 if (jc == i) {
                     CT *dst = xs + ((i & 1) * NWR + wid) * 32 + half * RPL;
@@ -762,7 +792,29 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NTL) panel_kernel(PanelArgs a
                 if (avail <= cb * kIB + i) avail = wait_rows(&s_rows, cb * kIB + i + 1, &s_fail, args.err);
                 const CT *prow = geqrt ? rowb + pb * kIB : Rts + i * (kIB + 4);
                 const CT rj = prow[jc];
-                const PRefl<CT> r = Ar::scalars(sq, prow[i]);
+                PRefl<CT> r = Ar::scalars(sq, prow[i]);
+                if (Ar::small(sq, prow[i])) {  // known well before the scalars
+                    bool zero = Ar::vanished(sq, prow[i]);
+                    if (zero ? Ar::kRefuse && prow[i] != CT(0) : !vfinite(r.f)) {
+                        // A column too small for its type (its squares vanish, or tau / nu^2
+                        // overflows), or NaN.  One that is nothing against the columns before
+                        // it counts as zero: what cancellation leaves of dependent columns,
+                        // each some 1e-8 (1e-16) of the one before
+                        int m = largest(i);
+                        if (args.ref) {
+                            const T *ref = reinterpret_cast<const T *>(args.ref) + zb * args.sRef;
+                            for (int q = lane; q < B; q += 32) m = max(m, mag_bits(__ldcg(ref + q * args.ref_ld)));
+                            m = __reduce_max_sync(0xffffffffu, m);
+                        }
+                        const bool drop = negligible<CT>(mag_bits(zero ? prow[i] : r.nu), m);
+                        bad = bad || (!drop && (zero || i < kIB - 1));  // the last column needs no tau / nu^2
+                        zero = zero || drop;
+                    }
+                    if (zero) {  // identity reflector
+                        r.nu = r.tau = r.tc = r.f = r.inv = CT(0);
+                        r.beta = prow[i];
+                    }
+                }
                 bad = bad || !vfinite(r.tau) || !vfinite(r.nu);
                 const CT h = r.nu * rj + d;
                 const CT w = jc > i ? r.f * h : CT(0);  // columns up to i are finished
@@ -782,6 +834,7 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NTL) panel_kernel(PanelArgs a
                 myinv = jc == i ? r.inv : myinv;
                 __syncwarp();
             }
+            big = largest(kIB);
             if (bad && lane == 0) atomicCAS(args.err, kDevOk, kDevNonfinite);
             if (tid < kIB) stau[tid] = mytau;
             __syncwarp();
@@ -1621,7 +1674,7 @@ int panel_mail_reset(const Stage1Work &w, int64_t n, cudaStream_t s) {
 // the FP32 rate and the panel's reflectors and applies are FP64-issue-bound.
 template <typename T, int LAYOUT>
 int launch_panel(T *dA, int64_t lda, int b, int pr, int pc, int P, int first_role, const Stage1Work &w,
-                 cudaStream_t s, const int *ready = nullptr) {
+                 cudaStream_t s, const int *ready = nullptr, const T *ref = nullptr) {
     const bool dfp = sizeof(T) == 8 && w.df_update;
     const int batch = w.batch > 0 ? w.batch : 1;
     AVS_CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(int) * (size_t)(batch > 1 ? w.sFlags * batch : 2 * P + 1), s));
@@ -1644,6 +1697,10 @@ int launch_panel(T *dA, int64_t lda, int b, int pr, int pc, int P, int first_rol
     a.sFlags = w.sFlags;
     a.mail = P - first_role > 1 && first_role == 0 ? static_cast<unsigned long long *>(w.mail) : nullptr;
     a.tag = (unsigned)(pr + pc + 1);  // half-step k of a call: 2 k + 1 (QR) or 2 k + 2 (LQ)
+    // the diagonal of the call's first panel: given (out of core), or in the matrix once that panel is through
+    a.ref = w.ref ? w.ref : (pr + pc > 0 ? (ref ? ref : dA) : nullptr);
+    a.ref_ld = w.ref ? 1 : lda + 1;
+    a.sRef = w.sA;
     a.sMail = w.sMail;
     a.ready = ready;
     a.ready_need = b / kChainStrip;
@@ -1796,7 +1853,7 @@ int stage1_ge2bnd_tc(float *X, int64_t n, int b, const Stage1Work &w, cudaStream
             if (!forked) AVS_CUDA_TRY(cudaEventRecord(w.la_fork, s));
             AVS_CUDA_TRY(cudaStreamWaitEvent(a, w.la_fork, 0));
         }
-        if ((r = launch_panel<float, 0>(M, n, b, pr, pc, P, 0, w, a, ready)) != AVS_SUCCESS) return r;
+        if ((r = launch_panel<float, 0>(M, n, b, pr, pc, P, 0, w, a, ready, X)) != AVS_SUCCESS) return r;
         if ((r = copy_tau_out<float>(tau_out, w, nt, k, first, P, b, a)) != AVS_SUCCESS) return r;
         if (la) AVS_CUDA_TRY(cudaEventRecord(w.la_panel, a));
         if ((int64_t)(pc + 1) * b < n && (r = stage1_tbuild<float>(M, n, b, 0, pr, pc, P, w, a)) != AVS_SUCCESS)
