@@ -104,8 +104,8 @@ struct UpdateArgs {
 // diagonal); evaluated in double-float for FP32 tiles and rounded once, in FP64
 // for FP64 tiles (reflect.cuh: hardware estimates and one residual each).  They are
 // meaningless for a zero column; small: the squared norm is 0, or so small that f may
-// overflow (or NaN); vanished: it is 0.  kRefuse: alpha != 0 whose square vanishes is
-// an error (FP32 and double-float take the column for zero).
+// overflow (or NaN); vanished: it is 0, a zero column for FP32 and double-float, an
+// error for FP64 if alpha != 0.
 template <typename CT>
 struct PRefl {
     CT nu, tc, f, inv, beta, tau;
@@ -135,7 +135,7 @@ struct PAr<float> : PSqPair, MacAr<float> {
     // FP32 and everything else is a residual of them: with r ~ 1/n1 and z ~ 1/|nu|,
     // n1 = x r (1 + g), 1/n1 = r (1 + g), 1/|nu| = z (1 + k); relative errors
     // below 2^-44 before the one rounding of each result.
-    static constexpr bool kRefuse = false;
+    static constexpr bool kFp64 = false;
     static __device__ __forceinline__ bool small(Sq s, float alpha) { return !(fmaf(alpha, alpha, s.x) > kSmallF); }
     static __device__ __forceinline__ bool vanished(Sq s, float alpha) { return fmaf(alpha, alpha, s.x) <= 0.0f; }
     static __device__ __forceinline__ PRefl<float> scalars(Sq s, float alpha) {
@@ -178,7 +178,7 @@ struct PAr<dfx> : PSqPair, MacAr<dfx> {
         const float p = __fmul_rn(x.hi, x.hi);
         return make_float2(p, __fmaf_rn(2.0f * x.hi, x.lo, __fmaf_rn(x.hi, x.hi, -p)));
     }
-    static constexpr bool kRefuse = false;
+    static constexpr bool kFp64 = false;
     static __device__ __forceinline__ bool small(Sq s, dfx al) {
         const Sq m = merge(s, sq(al));
         return !(__fadd_rn(m.x, m.y) > kSmallF);
@@ -212,7 +212,7 @@ struct PAr<double> : MacAr<double> {
     static __device__ __forceinline__ Sq sq(double x) { return x * x; }
     static __device__ __forceinline__ Sq merge(Sq a, Sq b) { return a + b; }
     static __device__ __forceinline__ Sq merge_xor(Sq a, int o) { return a + __shfl_xor_sync(0xffffffffu, a, o); }
-    static constexpr bool kRefuse = true;
+    static constexpr bool kFp64 = true;
     static __device__ __forceinline__ bool small(Sq s, double alpha) {
         return (__double2hiint(fma(alpha, alpha, s)) & 0x7ff00000) == 0;  // below 2^-1022
     }
@@ -795,19 +795,19 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NTL) panel_kernel(PanelArgs a
                 PRefl<CT> r = Ar::scalars(sq, prow[i]);
                 if (Ar::small(sq, prow[i])) {  // known well before the scalars
                     bool zero = Ar::vanished(sq, prow[i]);
-                    if (zero ? Ar::kRefuse && prow[i] != CT(0) : !vfinite(r.f)) {
-                        // A column too small for its type (its squares vanish, or tau / nu^2
-                        // overflows), or NaN.  One that is nothing against the columns before
+                    if (Ar::kFp64 ? (zero ? prow[i] != CT(0) : !vfinite(r.f)) : !zero) {
+                        // A column too small for its type (FP64: its squares vanish, or tau /
+                        // nu^2 overflows), or NaN.  One that is nothing against the columns before
                         // it counts as zero: what cancellation leaves of dependent columns,
                         // each some 1e-8 (1e-16) of the one before
                         int m = largest(i);
                         if (args.ref) {
                             const T *ref = reinterpret_cast<const T *>(args.ref) + zb * args.sRef;
-                            for (int q = lane; q < B; q += 32) m = max(m, mag_bits(__ldcg(ref + q * args.ref_ld)));
+                            for (int q = lane; q < B; q += 32) m = max(m, mag_bits(CT(__ldcg(ref + q * args.ref_ld))));
                             m = __reduce_max_sync(0xffffffffu, m);
                         }
                         const bool drop = negligible<CT>(mag_bits(zero ? prow[i] : r.nu), m);
-                        bad = bad || (!drop && (zero || i < kIB - 1));  // the last column needs no tau / nu^2
+                        bad = bad || (!drop && (zero || i < kIB - 1 || !Ar::kFp64));  // (FP64's last column needs no f)
                         zero = zero || drop;
                     }
                     if (zero) {  // identity reflector

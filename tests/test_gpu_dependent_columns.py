@@ -95,3 +95,14 @@ def test_end_of_the_fp32_range(avs_mod, tile, tiles, scale):
     a = a.astype(np.float64) / scale
     assert np.all(np.isfinite(band))
     assert np.max(np.abs(sl.svdvals(band) - sl.svdvals(a))) <= 1e-5 * sl.svdvals(a)[0]
+
+
+@pytest.mark.parametrize("tile,tiles", [(16, 3), (16, 8), (32, 3), (64, 3), (128, 3)])
+def test_end_of_the_fp32_range_in_double_float(avs_mod, tile, tiles):
+    """Where FP32's range ends, double-float loses its second word: refused, not answered to
+    a few digits (these Gaussian matrices have a column below 5e-20 in one of their panels)."""
+    cuda()
+    a = np.random.default_rng(7).standard_normal((tile * tiles, tile * tiles)) * 1e-19
+    with pytest.raises(avs_mod.AvsError) as e:
+        avs_mod.my_CU_svdval(avs_mod.to_device(a), tile, precision="fp64x2")
+    assert e.value.status == 4  # AVS_ERR_NONFINITE
