@@ -630,12 +630,15 @@ __global__ void __launch_bounds__(PanelCfg<CT, B>::NTL) panel_kernel(PanelArgs a
     if constexpr (Cfg::FETCH == kFetchOwn) {  // a warp of its own: a block ahead of the reflectors
         if (wid == NW) {
             if (geqrt) return;
-            const long long t0 = clock64();
             for (int cb = 0; cb < NB; ++cb) {
+                const long long t0 = clock64();
                 for (long long it = 0; ld_shared_volatile(&s_used) < cb - 1; ++it) {  // block cb - 2 still in use
                     if (ld_shared_volatile(&s_fail)) return;
                     if (it > kSpinLimit || clock64() - t0 > 8 * kWaitNs) {
-                        if (lane == 0) *reinterpret_cast<volatile int *>(&s_fail) = 1;
+                        if (lane == 0) {
+                            atomicCAS(args.err, kDevOk, kDevTimeout);
+                            *reinterpret_cast<volatile int *>(&s_fail) = 1;
+                        }
                         return;
                     }
                     __nanosleep(64);
