@@ -15,6 +15,7 @@
 
 #include "avs_common.cuh"
 #include "df64.cuh"
+#include "tblk.cuh"
 #include "tc_gemm.cuh"
 
 namespace avs {
@@ -88,7 +89,7 @@ Layout make_layout(int64_t n, int b, size_t elem, size_t stage_elem, int tc_fmt 
     L.off_tau = o;
     o = align_up(o + elem * (size_t)(nt + 1) * (size_t)b);
     L.off_tblk = o;
-    o = align_up(o + elem * (size_t)(nt + 1) * (size_t)(b / 16) * 256);
+    o = align_up(o + elem * tblk_elems(n, b));
     L.off_tfull = o;
     o = align_up(o + (b >= 128 ? elem * (size_t)(nt + 1) * (size_t)b * (size_t)b : 0));
     L.off_flags1 = o;
@@ -1179,7 +1180,7 @@ BatchLayout batch_layout(int64_t n, int b, int cnt, size_t elem = 4) {
     L.err = take(64);
     L.W = take(elem * (size_t)cnt * n * n);
     L.tau = take(elem * (size_t)cnt * (nt + 1) * b);
-    L.tblk = take(elem * (size_t)cnt * (nt + 1) * (b / 16) * 256);
+    L.tblk = take(elem * (size_t)cnt * tblk_elems(n, b));
     L.tfull = take(b >= 128 ? elem * (size_t)cnt * (nt + 1) * b * b : 0);
     L.f1 = take(sizeof(int) * (size_t)cnt * (2 * nt + 4));
     L.ab = take(sizeof(double) * (size_t)cnt * (size_t)band_stride(b, n));
@@ -1281,7 +1282,7 @@ int group_launches(avs_handle *h, const BatchLayout &L, int64_t n, int b, int cn
     w1.batch = cnt;
     w1.sA = n * n;
     w1.sTau = (nt + 1) * b;
-    w1.sTblk = (nt + 1) * (b / 16) * 256;
+    w1.sTblk = (int64_t)tblk_elems(n, b);
     w1.sTfull = (nt + 1) * (int64_t)b * b;
     w1.sFlags = 2 * nt + 4;
     w1.df_update = (sizeof(T) == 8 && df_update) ? 1 : 0;

@@ -21,6 +21,7 @@
 #include <utility>
 
 #include "avs_common.cuh"
+#include "tblk.cuh"
 
 namespace avs {
 namespace {
@@ -43,7 +44,7 @@ OocBufs carve(void *ws, int64_t n, int b, size_t elem, int slab) {
     o.tau = p + off;
     off = al256(off + elem * (size_t)(nt + 1) * b);
     o.tblk = p + off;
-    off = al256(off + elem * (size_t)(nt + 1) * (b / 16) * 256);
+    off = al256(off + elem * tblk_elems(n, b));
     o.tfull = b >= 128 ? p + off : nullptr;
     off = al256(off + (b >= 128 ? elem * (size_t)(nt + 1) * b * b : 0));
     o.flags = reinterpret_cast<int *>(p + off);
@@ -58,7 +59,7 @@ OocBufs carve(void *ws, int64_t n, int b, size_t elem, int slab) {
 
 size_t fixed_bytes(int64_t n, int b, size_t elem) {
     const int64_t nt = n / b;
-    return al256(elem * (size_t)(nt + 1) * b) + al256(elem * (size_t)(nt + 1) * (b / 16) * 256) +
+    return al256(elem * (size_t)(nt + 1) * b) + al256(elem * tblk_elems(n, b)) +
            al256(b >= 128 ? elem * (size_t)(nt + 1) * b * b : 0) + al256(sizeof(int) * (size_t)(2 * nt + 4)) + 256;
 }
 

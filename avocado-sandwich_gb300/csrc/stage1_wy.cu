@@ -41,6 +41,7 @@
 
 #include "avs_common.cuh"
 #include "df64.cuh"
+#include "tblk.cuh"
 #include "vec16.cuh"
 
 namespace avs {
@@ -51,7 +52,7 @@ constexpr int kWNT = 256;    // threads per CTA
 
 template <typename T>
 struct WCfg {
-    static constexpr int W = sizeof(T) == 8 ? 32 : 64;   // strip width
+    static constexpr int W = upd_strip(sizeof(T), false);  // strip width
     static constexpr int KC = sizeof(T) == 8 ? 8 : 16;   // K chunk
 };
 
@@ -357,8 +358,7 @@ struct UpdFullArgs {
     int64_t sA, sTfull;  // per-matrix strides (blockIdx.y = matrix)
     int first_role;      // 1: the top tile's own reflectors were applied earlier
     int nstrip;
-    int fine;            // 1: a counter per row block of a strip, 0: one per strip
-    int *flags;          // [0] ticket, then the counters: tiles finished with the row block (strip); zeroed
+    int *flags;          // [0] ticket, then a counter per row block of each strip: tiles finished with it; zeroed
     int64_t sFlags;      // ints between matrices
     int *err;
 };
@@ -384,7 +384,7 @@ struct UCfg {
     static constexpr int LDC = B + 4;             // leading dimension of A chunks (m)
     static constexpr int PER = KC * B / kWNT;     // chunk elements per thread
     // W = T^T Z: row blocks of KB; a thread's 8 rows are pairs, one per quarter of the tile
-    static constexpr int KB = sizeof(T) == 8 && B == 256 ? 16 : 32;
+    static constexpr int KB = upd_row_block(sizeof(T), B);
     static constexpr int NBK = B / KB;
     static constexpr int GSC = B / 4;
     static __device__ __forceinline__ int crow(int m0, int i) { return (i / 2) * GSC + m0 * 2 + i % 2; }
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(kWNT, UCfg<T, B, WW>::MINB) update_full_kernel
     __syncthreads();
     const int p = args.first_role + s_t / args.nstrip, strip = s_t % args.nstrip;
     if (p >= args.P) return;
-    int *done = flags + 1 + strip * (args.fine ? NBK : 1);
+    int *done = flags + 1 + strip * NBK;
     const int64_t j0 = (int64_t)(args.pc + 1) * B + (int64_t)strip * W;  // whole tiles of columns: strips are full
     View<T, LAYOUT> V{reinterpret_cast<T *>(args.a) + zb * args.sA, args.lda};
     const int64_t top0 = (int64_t)args.pr * B;
@@ -620,8 +620,8 @@ __global__ void __launch_bounds__(kWNT, UCfg<T, B, WW>::MINB) update_full_kernel
             const int idx = tid + e * kWNT, k = idx % KB, i = idx / KB;
             tv[e] = i >= m * KB ? Tf[m * KB + k + (size_t)i * B] : T(0);
         }
-        if (p > args.first_role && (args.fine || m == 0)) {
-            if (tid == 0) s_ok = wait_geq(done + (args.fine ? m : 0), p - args.first_role, args.err);
+        if (p > args.first_role) {
+            if (tid == 0) s_ok = wait_geq(done + m, p - args.first_role, args.err);
             __syncthreads();
             if (!s_ok) return;
         }
@@ -708,8 +708,7 @@ __global__ void __launch_bounds__(kWNT, UCfg<T, B, WW>::MINB) update_full_kernel
                 V(top0 + m * KB + t, j0 + c) = from_ct<T>(to_ct<CT>(top[u]) - Zb[(m * KB + t) * C::LDW + c]);
             }
             __syncthreads();
-            if (tid == 0 && (args.fine || m == NBK - 1))
-                st_release(done + (args.fine ? m : 0), p - args.first_role + 1);
+            if (tid == 0) st_release(done + m, p - args.first_role + 1);
         }
     }
 
@@ -731,7 +730,7 @@ __global__ void __launch_bounds__(kWNT, UCfg<T, B, WW>::MINB) update_full_kernel
     }
     if (p == 0) {
         __syncthreads();
-        if (tid < (args.fine ? NBK : 1)) st_release(done + tid, 1);
+        if (tid < NBK) st_release(done + tid, 1);
     }
 }
 
@@ -754,20 +753,17 @@ int launch_upd_full(T *dA, int64_t lda, int64_t n, int pr, int pc, int P, const 
     }
     const int64_t ncols = n - (int64_t)(pc + 1) * B;
     if (ncols <= 0) return AVS_SUCCESS;
-    const int nstrip = (int)((ncols + C::W - 1) / C::W);
+    const int nstrip = (int)upd_strips(ncols, C::W);
     const int batch = w.batch > 0 ? w.batch : 1;
-    // ticket and strip counters take the place of the panel's 16 x 16 T blocks,
-    // which the T build has read
+    // ticket and counters take the place of the panel's 16 x 16 T blocks, which the T
+    // build has read; the buffer's size goes with the order (tblk_elems), not with the
+    // tiles of this launch, and holds them for every order
     const int64_t sFl = w.sTblk * (int64_t)(sizeof(T) / sizeof(int));
-    const size_t room = sizeof(T) * (size_t)(P - first_role) * (B / kWIB) * kWIB * kWIB;
-    // (out of core, one tile at a time, they may hold one counter per strip only)
-    const int fine = sizeof(int) * (size_t)(1 + nstrip * C::NBK) <= room ? 1 : 0;
-    const size_t used = sizeof(int) * (size_t)(1 + nstrip * (fine ? C::NBK : 1));
-    if (used > room) return AVS_ERR_INTERNAL;
+    const size_t used = sizeof(int) * (size_t)upd_counters(ncols, B, sizeof(T), C::W);
     int *flags = reinterpret_cast<int *>(w.tblk);
     if (batch > 1) AVS_CUDA_TRY(cudaMemset2DAsync(flags, sizeof(int) * (size_t)sFl, 0, used, batch, s));
     else AVS_CUDA_TRY(cudaMemsetAsync(flags, 0, used, s));
-    UpdFullArgs a{dA, lda, n, B, pr, pc, P, w.tfull, w.sA, w.sTfull, first_role, nstrip, fine, flags, sFl, w.err};
+    UpdFullArgs a{dA, lda, n, B, pr, pc, P, w.tfull, w.sA, w.sTfull, first_role, nstrip, flags, sFl, w.err};
     update_full_kernel<T, LAYOUT, B, CT, WW><<<dim3((unsigned)nstrip * (P - first_role), batch), kWNT, smem, s>>>(a);
     AVS_CUDA_TRY(cudaGetLastError());
     return AVS_SUCCESS;
@@ -792,9 +788,9 @@ int launch_upd_full_any(T *dA, int64_t lda, int64_t n, int pr, int pc, int P, co
         const int64_t ncols = n - (int64_t)(pc + 1) * B;
         const bool narrow = ((ncols + 31) / 32) * (int64_t)(w.batch > 0 ? w.batch : 1) < 2 * (int64_t)sms;
         if (w.df_update)
-            return narrow ? launch_upd_full<T, LAYOUT, B, dfx, 16>(dA, lda, n, pr, pc, P, w, s, first_role)
+            return narrow ? launch_upd_full<T, LAYOUT, B, dfx, upd_strip(8, true)>(dA, lda, n, pr, pc, P, w, s, first_role)
                           : launch_upd_full<T, LAYOUT, B, dfx>(dA, lda, n, pr, pc, P, w, s, first_role);
-        return narrow ? launch_upd_full<T, LAYOUT, B, T, 16>(dA, lda, n, pr, pc, P, w, s, first_role)
+        return narrow ? launch_upd_full<T, LAYOUT, B, T, upd_strip(8, true)>(dA, lda, n, pr, pc, P, w, s, first_role)
                       : launch_upd_full<T, LAYOUT, B>(dA, lda, n, pr, pc, P, w, s, first_role);
     }
     return launch_upd_full<T, LAYOUT, B>(dA, lda, n, pr, pc, P, w, s, first_role);
