@@ -31,8 +31,8 @@ __device__ __forceinline__ double df_to_double(df64 a) { return (double)a.hi + (
 // either way, issue at 64 cycles per warp on GB300: with all warps converting they took
 // as long as the products of a double-float trailing update.  Some 15 instructions,
 // so a loss where few warps convert (the panels: FP64 tiles of 64 n = 1024 stage 1 14.9
-// -> 15.8 ms).  Exponents within [-74, 126] and zeros; anything else takes the FP64
-// instructions.
+// -> 15.8 ms).  Exponents within [-74, 126] and zeros, and normalised pairs; anything
+// else takes the FP64 instructions.
 __device__ __forceinline__ df64 df_from_double_int(double x) {
     const unsigned lo32 = (unsigned)__double2loint(x), hi32 = (unsigned)__double2hiint(x);
     const unsigned ahi = hi32 & 0x7fffffffu, sgn = hi32 & 0x80000000u;
@@ -50,8 +50,9 @@ __device__ __forceinline__ df64 df_from_double_int(double x) {
 __device__ __forceinline__ double df_to_double_int(df64 a) {
     const unsigned hb = __float_as_uint(a.hi), ah = hb & 0x7fffffffu, sgn = hb & 0x80000000u;
     const unsigned ex = ah >> 23;
-    if (ex - (127u - 74u) <= 200u && fabsf(a.lo) <= __fmul_rn(fabsf(a.hi), 0x1p-22f)) {
-        // hi + lo in units of 2^(ex - 127 - 52), half of that just below a power of two
+    if (ex - (127u - 74u) <= 200u && fabsf(a.lo) <= __fmul_rn(fabsf(a.hi), 0x1p-24f)) {
+        // hi + lo in units of 2^(ex - 127 - 52), half of that just below a power of two: a
+        // normalised pair (|lo| <= 2^-24 |hi|) leaves hi's binade only there
         const float sl = __uint_as_float(__float_as_uint(a.lo) ^ sgn);  // lo relative to |hi|
         const unsigned half = ((ah & 0x7fffffu) == 0u && sl < 0.0f) ? 1u : 0u;
         const float sc = __uint_as_float((52u + 127u - (ex - 127u) + half) << 23);
