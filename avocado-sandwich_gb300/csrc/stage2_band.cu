@@ -237,44 +237,6 @@ __device__ __forceinline__ void stage_in_vec(int tid, Src src, Dst dst) {
 __device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 
-// Scalars of the LAPACK-convention reflector of x = (alpha, x2) with s =
-// ||x2||^2 > 0: beta = -sign(alpha) ||x||, tau = (beta - alpha) / beta =
-// 1 + |alpha| / ||x||, scal = 1 / (alpha - beta): the hardware estimates with one
-// Newton step each in FP32 (within an ulp), reflect.cuh's in FP64 -- a short
-// dependent chain on the panel's critical path.
-__device__ __forceinline__ void reflector_scalars(float alpha, float s, float &tau, float &beta, float &scal) {
-    const float a2s = fmaf(alpha, alpha, s);
-    const float r = rsqrt_hw(a2s);
-    const float t = a2s * r;
-    const float h = 0.5f * fmaf(-t, r, 1.0f);
-    const float nrm = fmaf(t, h, t), rn = fmaf(r, h, r);
-    const float u = fabsf(alpha) + nrm;
-    float z = rcp_hw(u);
-    z = fmaf(z, fmaf(-u, z, 1.0f), z);
-    beta = alpha >= 0.0f ? -nrm : nrm;
-    scal = alpha >= 0.0f ? z : -z;
-    tau = fmaf(fabsf(alpha), rn, 1.0f);
-}
-__device__ __forceinline__ void reflector_scalars(double alpha, double s, double &tau, double &beta, double &scal) {
-    double rn, nrm;
-    rsqrt_sqrt(fma(alpha, alpha, s), rn, nrm);
-    beta = alpha >= 0.0 ? -nrm : nrm;
-    tau = fma(fabs(alpha), rn, 1.0);
-    const double z = rcp_est(fabs(alpha) + nrm);
-    scal = alpha >= 0.0 ? z : -z;
-}
-
-__device__ __forceinline__ void reflector_scalars(dfx al, dfx s, dfx &tau, dfx &beta, dfx &scal) {
-    df64 rn, nrm;
-    rsqrt_sqrt((al * al + s).v, rn, nrm);
-    const bool neg = df_lt0(al.v);
-    const df64 aa = neg ? df_neg(al.v) : al.v;
-    beta = dfx(neg ? nrm : df_neg(nrm));
-    tau = dfx(aa) * dfx(rn) + dfx(1);
-    const df64 z = rcp_est(df_add(aa, nrm));
-    scal = dfx(neg ? df_neg(z) : z);
-}
-
 // Householder QR of the panel P (B rows x T columns, column k at P + k*LDP,
 // zero rows below the valid part), LAPACK convention per column: beta =
 // -sign(alpha) ||x||, v = x / (alpha - beta) below the diagonal, v_k = 1,
