@@ -49,12 +49,6 @@ __device__ __forceinline__ void st_release(int *p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // Bounded wait until *flag >= target.  Called by one thread; returns false on
 // timeout (after recording kDevTimeout in *err) or when another CTA already
 // failed.  Never spins forever: at most kSpinLimit polls and limit_ns, measured

@@ -27,15 +27,9 @@ struct ChaseAr<double> {
     static __device__ __forceinline__ V mul(V a, V b) { return a * b; }
     static __device__ __forceinline__ V fma(V a, V b, V c) { return ::fma(a, b, c); }
     static __device__ __forceinline__ V neg(V a) { return -a; }
-    static __device__ __forceinline__ V div(V a, V b) { return a / b; }
-    static __device__ __forceinline__ V sqrt(V a) { return ::sqrt(a); }
     static __device__ __forceinline__ bool ge0(V a) { return a >= 0.0; }
-    static __device__ __forceinline__ bool gt0(V a) { return a > 0.0; }
     static __device__ __forceinline__ bool iszero(V a) { return a == 0.0; }
-    static __device__ __forceinline__ V shfl_xor(V a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
     static __device__ __forceinline__ V shfl(V a, int src) { return __shfl_sync(0xffffffffu, a, src); }
-    static __device__ __forceinline__ V rcp(V a) { return 1.0 / a; }
-    static __device__ __forceinline__ double to_double(V a) { return a; }
     static __device__ __forceinline__ St from_double(double a) { return a; }
     static __device__ __forceinline__ V v_from_double(double a) { return a; }
     // dot-product accumulator: plain FMA chain
@@ -65,19 +59,11 @@ struct ChaseAr<df64> {
     static __device__ __forceinline__ V mul(V a, V b) { return df_mul(a, b); }
     static __device__ __forceinline__ V fma(V a, V b, V c) { return df_add(df_mul(a, b), c); }
     static __device__ __forceinline__ V neg(V a) { return df_neg(a); }
-    static __device__ __forceinline__ V div(V a, V b) { return df_div(a, b); }
-    static __device__ __forceinline__ V sqrt(V a) { return df_sqrt(a); }
     static __device__ __forceinline__ bool ge0(V a) { return !df_lt0(a); }
-    static __device__ __forceinline__ bool gt0(V a) { return a.hi > 0.0f || (a.hi == 0.0f && a.lo > 0.0f); }
     static __device__ __forceinline__ bool iszero(V a) { return a.hi == 0.0f && a.lo == 0.0f; }
-    static __device__ __forceinline__ V shfl_xor(V a, int o) {
-        return df64{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
-    }
     static __device__ __forceinline__ V shfl(V a, int src) {
         return df64{__shfl_sync(0xffffffffu, a.hi, src), __shfl_sync(0xffffffffu, a.lo, src)};
     }
-    static __device__ __forceinline__ V rcp(V a) { return df_rcp(a); }
-    static __device__ __forceinline__ double to_double(V a) { return df_to_double(a); }
     // Dot-product accumulator in compensated FP32 (Ogita, Rump & Oishi,
     // "Accurate sum and dot product", SIAM J. Sci. Comput. 26 (2005), Dot2):
     // s carries the running FP32 sum, c the exact rounding errors of the sums

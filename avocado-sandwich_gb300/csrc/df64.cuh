@@ -18,8 +18,6 @@ struct df64 {
     float hi, lo;
 };
 
-__device__ __forceinline__ df64 df_make(float h, float l) { return df64{h, l}; }
-
 __device__ __forceinline__ df64 df_from_double(double x) {
     const float h = (float)x;
     return df64{h, (float)(x - (double)h)};
@@ -96,36 +94,8 @@ __device__ __forceinline__ df64 df_mul(df64 a, df64 b) {
     p.lo = __fmaf_rn(a.lo, b.hi, p.lo);
     return fast_two_sum(p.hi, p.lo);
 }
-__device__ __forceinline__ df64 df_mul_f(df64 a, float b) {
-    df64 p = two_prod(a.hi, b);
-    p.lo = __fmaf_rn(a.lo, b, p.lo);
-    return fast_two_sum(p.hi, p.lo);
-}
-// a * b + c
-__device__ __forceinline__ df64 df_fma(df64 a, df64 b, df64 c) { return df_add(df_mul(a, b), c); }
-
-// 1 / a: FP32 reciprocal estimate refined by one Newton-Raphson step in df64,
-// r' = r + r (1 - a r).
-__device__ __forceinline__ df64 df_rcp(df64 a) {
-    const float r = __frcp_rn(a.hi);
-    // e = 1 - a * r, computed in df64
-    df64 ar = df_mul_f(a, r);
-    df64 e = df_sub(df64{1.0f, 0.0f}, ar);
-    return df_add(df64{r, 0.0f}, df_mul_f(e, r));
-}
-__device__ __forceinline__ df64 df_div(df64 a, df64 b) { return df_mul(a, df_rcp(b)); }
-
-// sqrt(a), a >= 0: FP32 estimate s, one Newton step s' = s + (a - s^2) / (2 s).
-__device__ __forceinline__ df64 df_sqrt(df64 a) {
-    if (a.hi <= 0.0f) return df64{0.0f, 0.0f};
-    const float s = __fsqrt_rn(a.hi);
-    const df64 s2 = two_prod(s, s);
-    const df64 r = df_sub(a, s2);
-    return fast_two_sum(s, __fdiv_rn(r.hi, 2.0f * s));
-}
 
 __device__ __forceinline__ bool df_lt0(df64 a) { return a.hi < 0.0f || (a.hi == 0.0f && a.lo < 0.0f); }
-__device__ __forceinline__ float df_abs_hi(df64 a) { return fabsf(a.hi); }
 
 // A double-float value with arithmetic operators: the compute type of kernels
 // templated on their element type when the data is stored in FP64 (converted
