@@ -268,6 +268,7 @@ int run_stages23(avs_handle *h, const Layout &L, int64_t n, int b, const S *W, i
     Stage2Work w2;
     w2.flags = reinterpret_cast<int *>(ws_at(h, L.off_flags2));
     w2.err = err;
+    w2.scale = reinterpret_cast<int *>(ws_at(h, L.off_scr));  // stage 3's, idle in stage 2
     const int tbw = narrow_band_of(b, flags, fp64_stages);
     if (tbw > 0 && sizeof(S) == 8 && fp64_stages) {
         if ((rc = stage2_chase_hier_fp64(reinterpret_cast<const double *>(W), n, ldw, b, tbw, AB,
@@ -295,7 +296,8 @@ int run_stages23(avs_handle *h, const Layout &L, int64_t n, int b, const S *W, i
             return rc;
         if (band_ran) *band_ran = true;
     } else if (fp64_stages) {
-        if ((rc = extract_band_compact<S>(W, n, ldw, b, AB, L.ldab, s)) != AVS_SUCCESS) return rc;
+        if ((rc = band_scale<S>(W, n, ldw, 0, b, 1, w2, s, launches)) != AVS_SUCCESS) return rc;
+        if ((rc = extract_band_compact<S>(W, n, ldw, b, AB, L.ldab, w2.scale, s)) != AVS_SUCCESS) return rc;
         ++*launches;
         if ((rc = stage2_chase(AB, n, b, L.ldab, dd, de, w2, s, h->num_sms, launches,
                                !(flags & AVS_FLAG_CLUSTER_CHASE))) != AVS_SUCCESS)
@@ -945,18 +947,20 @@ int band_reduce_dev(avs_handle *h, int64_t n, int32_t bw, int32_t tbw, R *dB, in
     AVS_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), s));
     R *AB = reinterpret_cast<R *>(ws_at(h, ab_off));
     AVS_CUDA_TRY(cudaEventRecord(h->ev[0], s));
-    if ((rc = dense_to_band<R, R>(dB, n, ldb, 0, bw, AB, ldab, 0, 1, s)) != AVS_SUCCESS) return rc;
     Stage2Work w2;
     w2.flags = reinterpret_cast<int *>(ws_at(h, fl_off));
     w2.err = err;
+    w2.scale = reinterpret_cast<int *>(ws_at(h, L.off_scr));
+    if ((rc = band_scale<R>(dB, n, ldb, 0, bw, 1, w2, s, nullptr)) != AVS_SUCCESS) return rc;
+    if ((rc = dense_to_band<R, R>(dB, n, ldb, 0, bw, AB, ldab, 0, 1, w2.scale, s)) != AVS_SUCCESS) return rc;
     if ((rc = band_stage<R>(AB, n, bw, tbw, ldab, w2, s, h->num_sms, 1, 0, 0)) != AVS_SUCCESS) return rc;
     AVS_CUDA_TRY(cudaEventRecord(h->ev[1], s));
-    if ((rc = band_to_dense<R>(AB, n, bw, ldab, dB, ldb, s)) != AVS_SUCCESS) return rc;
+    if ((rc = band_to_dense<R>(AB, n, bw, ldab, dB, ldb, w2.scale, s)) != AVS_SUCCESS) return rc;
     AVS_CUDA_TRY(cudaMemcpyAsync(h->h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
     rc = finish_status(h, s);
     if (rep) {
         rep->t_stage2_ms = rep->t_total_ms = ev_ms(h->ev[0], h->ev[1]);
-        rep->kernel_launches = 3;
+        rep->kernel_launches = 4;
         rep->status = rc;
     }
     return rc;
@@ -1075,11 +1079,13 @@ int avs_band_to_bidiag_dev(avs_handle *h, int64_t n, int32_t bw, const double *d
     double *td = reinterpret_cast<double *>(ws_at(h, d_off));
     double *te = reinterpret_cast<double *>(ws_at(h, e_off));
     AVS_CUDA_TRY(cudaEventRecord(h->ev[0], s));
-    if ((rc = dense_band_to_compact(dB, n, ldb, bw, AB, ldab, s)) != AVS_SUCCESS) return rc;
     Stage2Work w2;
     w2.flags = reinterpret_cast<int *>(ws_at(h, fl_off));
     w2.err = err;
+    w2.scale = reinterpret_cast<int *>(ws_at(h, L.off_scr));
     int64_t launches = 1;
+    if ((rc = band_scale<double>(dB, n, ldb, 0, bw, 1, w2, s, &launches)) != AVS_SUCCESS) return rc;
+    if ((rc = extract_band_compact<double>(dB, n, ldb, bw, AB, ldab, w2.scale, s)) != AVS_SUCCESS) return rc;
     if ((rc = stage2_chase(AB, n, bw, ldab, td, te, w2, s, h->num_sms, &launches)) != AVS_SUCCESS) return rc;
     AVS_CUDA_TRY(cudaEventRecord(h->ev[1], s));
     AVS_CUDA_TRY(cudaMemcpyAsync(dd, td, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, s));
@@ -1292,6 +1298,7 @@ int group_launches(avs_handle *h, const BatchLayout &L, int64_t n, int b, int cn
     Stage2Work w2;
     w2.flags = reinterpret_cast<int *>(base + L.f2);
     w2.err = err;
+    w2.scale = reinterpret_cast<int *>(base + L.scr);  // stage 3's, idle in stage 2
     double *dd = reinterpret_cast<double *>(base + L.d);
     double *de = reinterpret_cast<double *>(base + L.e);
     // stage 2 as a single call of the same mode runs it (run_stages23)

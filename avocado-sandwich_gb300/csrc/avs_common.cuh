@@ -217,16 +217,21 @@ template <typename T>
 int stage1_tsqrt_pair(T *dRB, int b, T *dtau, const Stage1Work &w, cudaStream_t s);
 
 template <typename T>
-int extract_band_compact(const T *dA, int64_t n, int64_t lda, int bw, double *dAB, int64_t ldab, cudaStream_t s);
+int extract_band_compact(const T *dA, int64_t n, int64_t lda, int bw, double *dAB, int64_t ldab, const int *scale,
+                         cudaStream_t s);
 template <typename T>
 int extract_band_dense(const T *dA, int64_t n, int64_t lda, int bw, double *dB, int64_t ldb, cudaStream_t s);
-int dense_band_to_compact(const double *dB, int64_t n, int64_t ldb, int bw, double *dAB, int64_t ldab,
-                          cudaStream_t s);
 
 struct Stage2Work {
     int *flags;  // ticket (1) + done (n) ; reset per launch
     int *err;
+    int *scale = nullptr;  // one word per matrix: the band's largest exponent (band_scale.cuh)
 };
+// The band's largest exponent into w.scale (W[r + c*ldw], 0 <= c - r <= bw; matrices at
+// stride sW): what the copies in and out of stage 2 scale by.
+template <typename T>
+int band_scale(const T *dW, int64_t n, int64_t ldw, int64_t sW, int bw, int batch, const Stage2Work &w, cudaStream_t s,
+               int64_t *launches);
 // window: bands 8/16/32 by the shared-memory window kernel (ldab == 3 bw)
 int stage2_chase(double *dAB, int64_t n, int bw, int64_t ldab, double *dd, double *de, const Stage2Work &w,
                  cudaStream_t s, int num_sms, int64_t *launches, bool window = false);
@@ -261,12 +266,13 @@ int band_stage(R *dAB, int64_t n, int bw, int tbw, int64_t ldab, const Stage2Wor
 bool band_stage_supported(int bw, int tbw);
 template <typename TI, typename R>
 int dense_to_band(const TI *dA, int64_t n, int64_t lda, int64_t sA, int bw, R *dAB, int64_t ldab, int64_t sAB,
-                  int batch, cudaStream_t s);
+                  int batch, const int *scale, cudaStream_t s);
 template <typename R, typename St>
 int band_to_band(const R *dAB1, int64_t n, int bw1, int64_t ldab1, int64_t sAB1, int bw2, St *dAB2, int64_t ldab2,
                  int64_t sAB2, int batch, cudaStream_t s);
 template <typename R>
-int band_to_dense(const R *dAB, int64_t n, int bw, int64_t ldab, R *dA, int64_t lda, cudaStream_t s);
+int band_to_dense(const R *dAB, int64_t n, int bw, int64_t ldab, R *dA, int64_t lda, const int *scale,
+                  cudaStream_t s);
 // Hierarchical stage 2 (stage2_chase.cu): the band of width bw of dW
 // (W[r + c*ldw]) -> width tbw by the blocked band reduction, then the element
 // chase tbw -> 1; d and e out.  _df: band reduction in FP32 (R = float, FP32 tiles)

@@ -54,6 +54,7 @@
 #include <type_traits>
 
 #include "avs_common.cuh"
+#include "band_scale.cuh"
 #include "df64.cuh"
 #include "reflect.cuh"
 #include "vec16.cuh"
@@ -807,18 +808,19 @@ int launch_band_stage(R *dAB, int64_t n, int64_t ldab, const Stage2Work &w, cuda
 }
 
 // dense (leading dimension lda, matrix stride sA) -> compact band of width
-// bw (ku = band_ku(bw)), zeros outside 0 <= c - r <= bw
+// bw (ku = band_ku(bw)), scaled (band_scale.cuh), zeros outside 0 <= c - r <= bw
 template <typename TI, typename R>
 __global__ void dense_to_band_kernel(const TI *a, int64_t n, int64_t lda, int64_t sA, int bw, R *ab, int64_t ldab,
-                                     int64_t sAB) {
+                                     int64_t sAB, const int *scale) {
     const int64_t c = blockIdx.x;
     const int64_t zb = blockIdx.y;
     const int ku = band_ku(bw);
+    const TI f = pow2<TI>(-band_exponent(scale, zb));
     const TI *az = a + zb * sA;
     R *abz = ab + zb * sAB + c * ldab;
     for (int i = threadIdx.x; i < ldab; i += blockDim.x) {
         const int64_t r = c - ku + i;
-        abz[i] = (r >= 0 && r <= c && c - r <= bw) ? (R)az[r + c * lda] : R(0);
+        abz[i] = (r >= 0 && r <= c && c - r <= bw) ? (R)(az[r + c * lda] * f) : R(0);
     }
 }
 
@@ -849,14 +851,16 @@ __global__ void band_to_band_kernel(const R *ab1, int64_t n, int bw1, int64_t ld
 }
 
 // compact band (width bw storage) -> dense column-major n x n: every entry the
-// compact storage holds (rows c-2bw .. c+bw of column c), zeros elsewhere
+// compact storage holds (rows c-2bw .. c+bw of column c), scaled back, zeros elsewhere
 template <typename R>
-__global__ void band_to_dense_kernel(const R *ab, int64_t n, int bw, int64_t ldab, R *a, int64_t lda) {
+__global__ void band_to_dense_kernel(const R *ab, int64_t n, int bw, int64_t ldab, R *a, int64_t lda,
+                                     const int *scale) {
     const int64_t c = blockIdx.x;
     const int ku = band_ku(bw);
+    const R f = pow2<R>(band_exponent(scale, 0));
     for (int64_t r = threadIdx.x; r < n; r += blockDim.x) {
         const int64_t i = ku + r - c;
-        a[r + c * lda] = (i >= 0 && i < ldab) ? ab[i + c * ldab] : R(0);
+        a[r + c * lda] = (i >= 0 && i < ldab) ? ab[i + c * ldab] * f : R(0);
     }
 }
 
@@ -900,18 +904,19 @@ bool band_stage_supported(int bw, int tbw) {
 
 template <typename TI, typename R>
 int dense_to_band(const TI *dA, int64_t n, int64_t lda, int64_t sA, int bw, R *dAB, int64_t ldab, int64_t sAB,
-                  int batch, cudaStream_t s) {
+                  int batch, const int *scale, cudaStream_t s) {
     if (n <= 0) return AVS_SUCCESS;
-    dense_to_band_kernel<TI, R><<<dim3((unsigned)n, (unsigned)batch), 128, 0, s>>>(dA, n, lda, sA, bw, dAB, ldab, sAB);
+    dense_to_band_kernel<TI, R><<<dim3((unsigned)n, (unsigned)batch), 128, 0, s>>>(dA, n, lda, sA, bw, dAB, ldab, sAB,
+                                                                                  scale);
     AVS_CUDA_TRY(cudaGetLastError());
     return AVS_SUCCESS;
 }
 template int dense_to_band<float, float>(const float *, int64_t, int64_t, int64_t, int, float *, int64_t, int64_t,
-                                         int, cudaStream_t);
+                                         int, const int *, cudaStream_t);
 template int dense_to_band<double, double>(const double *, int64_t, int64_t, int64_t, int, double *, int64_t,
-                                           int64_t, int, cudaStream_t);
+                                           int64_t, int, const int *, cudaStream_t);
 template int dense_to_band<double, dfx>(const double *, int64_t, int64_t, int64_t, int, dfx *, int64_t, int64_t, int,
-                                        cudaStream_t);
+                                        const int *, cudaStream_t);
 
 template <typename R, typename St>
 int band_to_band(const R *dAB1, int64_t n, int bw1, int64_t ldab1, int64_t sAB1, int bw2, St *dAB2, int64_t ldab2,
@@ -930,13 +935,16 @@ template int band_to_band<dfx, float2>(const dfx *, int64_t, int, int64_t, int64
                                        int, cudaStream_t);
 
 template <typename R>
-int band_to_dense(const R *dAB, int64_t n, int bw, int64_t ldab, R *dA, int64_t lda, cudaStream_t s) {
+int band_to_dense(const R *dAB, int64_t n, int bw, int64_t ldab, R *dA, int64_t lda, const int *scale,
+                  cudaStream_t s) {
     if (n <= 0) return AVS_SUCCESS;
-    band_to_dense_kernel<R><<<(unsigned)n, 256, 0, s>>>(dAB, n, bw, ldab, dA, lda);
+    band_to_dense_kernel<R><<<(unsigned)n, 256, 0, s>>>(dAB, n, bw, ldab, dA, lda, scale);
     AVS_CUDA_TRY(cudaGetLastError());
     return AVS_SUCCESS;
 }
-template int band_to_dense<float>(const float *, int64_t, int, int64_t, float *, int64_t, cudaStream_t);
-template int band_to_dense<double>(const double *, int64_t, int, int64_t, double *, int64_t, cudaStream_t);
+template int band_to_dense<float>(const float *, int64_t, int, int64_t, float *, int64_t, const int *,
+                                  cudaStream_t);
+template int band_to_dense<double>(const double *, int64_t, int, int64_t, double *, int64_t, const int *,
+                                   cudaStream_t);
 
 }  // namespace avs

@@ -40,6 +40,7 @@
 #include <cmath>
 
 #include "avs_common.cuh"
+#include "band_scale.cuh"
 #include "chase_ar.cuh"
 #include "df64.cuh"
 
@@ -490,18 +491,20 @@ int launch_chase_any(typename ChaseAr<S>::St *dAB, int64_t n, int bw, int64_t ld
     }
 }
 
-// float2 band (double-float) <-> extraction
+// float2 band (double-float) <-> extraction; scaled (band_scale.cuh)
 template <typename T>
-__global__ void extract_band_df_kernel(const T *a, int64_t n, int64_t lda, int bw, float2 *ab, int64_t ldab) {
+__global__ void extract_band_df_kernel(const T *a, int64_t n, int64_t lda, int bw, float2 *ab, int64_t ldab,
+                                       const int *scale) {
     const int64_t c = blockIdx.x;
     const int ku = 2 * bw - 1;
+    const T f = pow2<T>(-band_exponent(scale, 0));
     for (int i = threadIdx.x; i <= bw; i += blockDim.x) {
         const int64_t r = c - bw + i;
         if (r >= 0) {
             if (sizeof(T) == 4) {
-                ab[(ku + r - c) + c * ldab] = make_float2((float)a[r + c * lda], 0.0f);  // exact
+                ab[(ku + r - c) + c * ldab] = make_float2((float)(a[r + c * lda] * f), 0.0f);  // exact
             } else {
-                const double v = (double)a[r + c * lda];
+                const double v = (double)(a[r + c * lda] * f);
                 const float h = (float)v;
                 ab[(ku + r - c) + c * ldab] = make_float2(h, (float)(v - (double)h));
             }
@@ -509,25 +512,29 @@ __global__ void extract_band_df_kernel(const T *a, int64_t n, int64_t lda, int b
     }
 }
 
-__global__ void bidiag_out_df_kernel(const float2 *ab, int64_t n, int bw, int64_t ldab, double *d, double *e) {
+__global__ void bidiag_out_df_kernel(const float2 *ab, int64_t n, int bw, int64_t ldab, double *d, double *e,
+                                     const int *scale) {
     const int ku = 2 * bw - 1;
+    const double f = pow2<double>(band_exponent(scale, 0));
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float2 x = ab[ku + i * ldab];
-        d[i] = (double)x.x + (double)x.y;
+        d[i] = ((double)x.x + (double)x.y) * f;
         if (i + 1 < n) {
             const float2 y = ab[(ku - 1) + (i + 1) * ldab];
-            e[i] = (double)y.x + (double)y.y;
+            e[i] = ((double)y.x + (double)y.y) * f;
         }
     }
 }
 
 template <typename T>
-__global__ void extract_band_compact_kernel(const T *a, int64_t n, int64_t lda, int bw, double *ab, int64_t ldab) {
+__global__ void extract_band_compact_kernel(const T *a, int64_t n, int64_t lda, int bw, double *ab, int64_t ldab,
+                                            const int *scale) {
     const int64_t c = blockIdx.x;
     const int ku = 2 * bw - 1;
+    const double f = pow2<double>(-band_exponent(scale, 0));
     for (int i = threadIdx.x; i <= bw; i += blockDim.x) {
         const int64_t r = c - bw + i;
-        if (r >= 0) ab[(ku + r - c) + c * ldab] = (double)a[r + c * lda];
+        if (r >= 0) ab[(ku + r - c) + c * ldab] = (double)a[r + c * lda] * f;
     }
 }
 
@@ -540,20 +547,13 @@ __global__ void extract_band_dense_kernel(const T *a, int64_t n, int64_t lda, in
     }
 }
 
-__global__ void dense_to_compact_kernel(const double *bm, int64_t n, int64_t ldb, int bw, double *ab, int64_t ldab) {
-    const int64_t c = blockIdx.x;
+__global__ void bidiag_out_kernel(const double *ab, int64_t n, int bw, int64_t ldab, double *d, double *e,
+                                  const int *scale) {
     const int ku = 2 * bw - 1;
-    for (int i = threadIdx.x; i <= bw; i += blockDim.x) {
-        const int64_t r = c - bw + i;
-        if (r >= 0) ab[(ku + r - c) + c * ldab] = bm[r + c * ldb];
-    }
-}
-
-__global__ void bidiag_out_kernel(const double *ab, int64_t n, int bw, int64_t ldab, double *d, double *e) {
-    const int ku = 2 * bw - 1;
+    const double f = pow2<double>(band_exponent(scale, 0));
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        d[i] = ab[ku + i * ldab];
-        if (i + 1 < n) e[i] = ab[(ku - 1) + (i + 1) * ldab];
+        d[i] = ab[ku + i * ldab] * f;
+        if (i + 1 < n) e[i] = ab[(ku - 1) + (i + 1) * ldab] * f;
     }
 }
 
@@ -658,14 +658,37 @@ int stage2_rate(int fp64, int num_sms, double *flops_per_s) {
 }
 
 template <typename T>
-int extract_band_compact(const T *dA, int64_t n, int64_t lda, int bw, double *dAB, int64_t ldab, cudaStream_t s) {
+int band_scale(const T *dW, int64_t n, int64_t ldw, int64_t sW, int bw, int batch, const Stage2Work &w, cudaStream_t s,
+               int64_t *launches) {
+    // one block while it reads the band in a few rounds (no word to zero first)
+    const int64_t total = n * (bw + 1);
+    const bool one = total <= 16384;
+    const dim3 grid(one ? 1u : (unsigned)std::min<int64_t>((total + 4095) / 4096, 608), (unsigned)batch);
+    if (!one) AVS_CUDA_TRY(cudaMemsetAsync(w.scale, 0, sizeof(int) * (size_t)batch, s));
+    // (a 32-bit index with room for a stride)
+    if (total < ((int64_t)1 << 31)) band_scale_kernel<T, unsigned><<<grid, 1024, 0, s>>>(dW, n, ldw, sW, bw, w.scale);
+    else band_scale_kernel<T, uint64_t><<<grid, 1024, 0, s>>>(dW, n, ldw, sW, bw, w.scale);
+    AVS_CUDA_TRY(cudaGetLastError());
+    if (launches) *launches += 1;
+    return AVS_SUCCESS;
+}
+template int band_scale<float>(const float *, int64_t, int64_t, int64_t, int, int, const Stage2Work &, cudaStream_t,
+                               int64_t *);
+template int band_scale<double>(const double *, int64_t, int64_t, int64_t, int, int, const Stage2Work &, cudaStream_t,
+                                int64_t *);
+
+template <typename T>
+int extract_band_compact(const T *dA, int64_t n, int64_t lda, int bw, double *dAB, int64_t ldab, const int *scale,
+                         cudaStream_t s) {
     AVS_CUDA_TRY(cudaMemsetAsync(dAB, 0, sizeof(double) * (size_t)ldab * (size_t)n, s));
-    extract_band_compact_kernel<T><<<(unsigned)n, 128, 0, s>>>(dA, n, lda, bw, dAB, ldab);
+    extract_band_compact_kernel<T><<<(unsigned)n, 128, 0, s>>>(dA, n, lda, bw, dAB, ldab, scale);
     AVS_CUDA_TRY(cudaGetLastError());
     return AVS_SUCCESS;
 }
-template int extract_band_compact<float>(const float *, int64_t, int64_t, int, double *, int64_t, cudaStream_t);
-template int extract_band_compact<double>(const double *, int64_t, int64_t, int, double *, int64_t, cudaStream_t);
+template int extract_band_compact<float>(const float *, int64_t, int64_t, int, double *, int64_t, const int *,
+                                         cudaStream_t);
+template int extract_band_compact<double>(const double *, int64_t, int64_t, int, double *, int64_t, const int *,
+                                          cudaStream_t);
 
 template <typename T>
 int extract_band_dense(const T *dA, int64_t n, int64_t lda, int bw, double *dB, int64_t ldb, cudaStream_t s) {
@@ -675,14 +698,6 @@ int extract_band_dense(const T *dA, int64_t n, int64_t lda, int bw, double *dB, 
 }
 template int extract_band_dense<float>(const float *, int64_t, int64_t, int, double *, int64_t, cudaStream_t);
 template int extract_band_dense<double>(const double *, int64_t, int64_t, int, double *, int64_t, cudaStream_t);
-
-int dense_band_to_compact(const double *dB, int64_t n, int64_t ldb, int bw, double *dAB, int64_t ldab,
-                          cudaStream_t s) {
-    AVS_CUDA_TRY(cudaMemsetAsync(dAB, 0, sizeof(double) * (size_t)ldab * (size_t)n, s));
-    dense_to_compact_kernel<<<(unsigned)n, 128, 0, s>>>(dB, n, ldb, bw, dAB, ldab);
-    AVS_CUDA_TRY(cudaGetLastError());
-    return AVS_SUCCESS;
-}
 
 int stage2_chase(double *dAB, int64_t n, int bw, int64_t ldab, double *dd, double *de, const Stage2Work &w,
                  cudaStream_t s, int num_sms, int64_t *launches, bool window) {
@@ -707,7 +722,7 @@ int stage2_chase(double *dAB, int64_t n, int bw, int64_t ldab, double *dd, doubl
         if (launches) *launches += 1;
     }
     const int nb = (int)std::min<int64_t>((n + 255) / 256, 4096);
-    bidiag_out_kernel<<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB, n, bw, ldab, dd, de);
+    bidiag_out_kernel<<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB, n, bw, ldab, dd, de, w.scale);
     AVS_CUDA_TRY(cudaGetLastError());
     if (launches) *launches += 1;
     return AVS_SUCCESS;
@@ -717,19 +732,19 @@ int stage2_chase(double *dAB, int64_t n, int bw, int64_t ldab, double *dd, doubl
 template <typename T>
 int stage2_chase_df(const T *dW, int64_t n, int64_t ldw, int bw, float2 *dAB, int64_t ldab, double *dd, double *de,
                     const Stage2Work &w, cudaStream_t s, int num_sms, int64_t *launches, bool window) {
+    int rc;
+    if ((rc = band_scale<T>(dW, n, ldw, 0, bw, 1, w, s, launches)) != AVS_SUCCESS) return rc;
     AVS_CUDA_TRY(cudaMemsetAsync(dAB, 0, sizeof(float2) * (size_t)ldab * (size_t)n, s));
-    extract_band_df_kernel<T><<<(unsigned)n, 128, 0, s>>>(dW, n, ldw, bw, dAB, ldab);
+    extract_band_df_kernel<T><<<(unsigned)n, 128, 0, s>>>(dW, n, ldw, bw, dAB, ldab, w.scale);
     AVS_CUDA_TRY(cudaGetLastError());
     if (window && chase_window_supported(bw) && ldab == 3 * (int64_t)bw) {
-        const int rc = stage2_chase_window_df(dAB, n, bw, w, s, num_sms);
-        if (rc != AVS_SUCCESS) return rc;
+        if ((rc = stage2_chase_window_df(dAB, n, bw, w, s, num_sms)) != AVS_SUCCESS) return rc;
     } else if (n >= 2) {
         AVS_CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(int) * (size_t)(n + 1), s));
-        const int rc = launch_chase_any<df64>(dAB, n, bw, ldab, w, s, num_sms);
-        if (rc != AVS_SUCCESS) return rc;
+        if ((rc = launch_chase_any<df64>(dAB, n, bw, ldab, w, s, num_sms)) != AVS_SUCCESS) return rc;
     }
     const int nb = (int)std::min<int64_t>((n + 255) / 256, 4096);
-    bidiag_out_df_kernel<<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB, n, bw, ldab, dd, de);
+    bidiag_out_df_kernel<<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB, n, bw, ldab, dd, de, w.scale);
     AVS_CUDA_TRY(cudaGetLastError());
     if (launches) *launches += 3;
     return AVS_SUCCESS;
@@ -748,7 +763,8 @@ int stage2_chase_hier_df(const T *dW, int64_t n, int64_t ldw, int bw, int tbw, R
                          bool window, cudaEvent_t after_band) {
     const int64_t ldab1 = band_ldab(bw), ldab2 = 3 * (int64_t)tbw;
     int rc;
-    if ((rc = dense_to_band<T, R>(dW, n, ldw, 0, bw, dAB1, ldab1, 0, 1, s)) != AVS_SUCCESS) return rc;
+    if ((rc = band_scale<T>(dW, n, ldw, 0, bw, 1, w, s, launches)) != AVS_SUCCESS) return rc;
+    if ((rc = dense_to_band<T, R>(dW, n, ldw, 0, bw, dAB1, ldab1, 0, 1, w.scale, s)) != AVS_SUCCESS) return rc;
     if ((rc = band_stage<R>(dAB1, n, bw, tbw, ldab1, w, s, num_sms, 1, 0, 0)) != AVS_SUCCESS) return rc;
     if (after_band) AVS_CUDA_TRY(cudaEventRecord(after_band, s));
     if ((rc = band_to_band<R, float2>(dAB1, n, bw, ldab1, 0, tbw, dAB2, ldab2, 0, 1, s)) != AVS_SUCCESS)
@@ -760,7 +776,7 @@ int stage2_chase_hier_df(const T *dW, int64_t n, int64_t ldw, int bw, int tbw, R
         if ((rc = launch_chase_any<df64>(dAB2, n, tbw, ldab2, w, s, num_sms)) != AVS_SUCCESS) return rc;
     }
     const int nb = (int)std::min<int64_t>((n + 255) / 256, 4096);
-    bidiag_out_df_kernel<<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB2, n, tbw, ldab2, dd, de);
+    bidiag_out_df_kernel<<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB2, n, tbw, ldab2, dd, de, w.scale);
     AVS_CUDA_TRY(cudaGetLastError());
     if (launches) *launches += 5;
     return AVS_SUCCESS;
@@ -778,7 +794,9 @@ int stage2_chase_hier_fp64(const double *dW, int64_t n, int64_t ldw, int bw, int
                            int64_t *launches, bool window, cudaEvent_t after_band) {
     const int64_t ldab1 = band_ldab(bw), ldab2 = 3 * (int64_t)tbw;
     int rc;
-    if ((rc = dense_to_band<double, double>(dW, n, ldw, 0, bw, dAB1, ldab1, 0, 1, s)) != AVS_SUCCESS) return rc;
+    if ((rc = band_scale<double>(dW, n, ldw, 0, bw, 1, w, s, launches)) != AVS_SUCCESS) return rc;
+    if ((rc = dense_to_band<double, double>(dW, n, ldw, 0, bw, dAB1, ldab1, 0, 1, w.scale, s)) != AVS_SUCCESS)
+        return rc;
     if ((rc = band_stage<double>(dAB1, n, bw, tbw, ldab1, w, s, num_sms, 1, 0, 0)) != AVS_SUCCESS) return rc;
     if (after_band) AVS_CUDA_TRY(cudaEventRecord(after_band, s));
     if ((rc = band_to_band<double, double>(dAB1, n, bw, ldab1, 0, tbw, dAB2, ldab2, 0, 1, s)) != AVS_SUCCESS)
@@ -790,7 +808,7 @@ int stage2_chase_hier_fp64(const double *dW, int64_t n, int64_t ldw, int bw, int
         if ((rc = launch_chase_any<double>(dAB2, n, tbw, ldab2, w, s, num_sms)) != AVS_SUCCESS) return rc;
     }
     const int nb = (int)std::min<int64_t>((n + 255) / 256, 4096);
-    bidiag_out_kernel<<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB2, n, tbw, ldab2, dd, de);
+    bidiag_out_kernel<<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB2, n, tbw, ldab2, dd, de, w.scale);
     AVS_CUDA_TRY(cudaGetLastError());
     if (launches) *launches += 5;
     return AVS_SUCCESS;
@@ -802,9 +820,11 @@ int stage2_chase_hier_fp64(const double *dW, int64_t n, int64_t ldw, int bw, int
 // S = df64 (FP32 tiles, the FP32-class modes) or double (FP64 tiles).
 namespace {
 template <typename T, typename S>
-__global__ void extract_band_batched(const T *a, int64_t n, int bw, typename ChaseAr<S>::St *ab, int64_t ldab) {
+__global__ void extract_band_batched(const T *a, int64_t n, int bw, typename ChaseAr<S>::St *ab, int64_t ldab,
+                                     const int *scale) {
     const int64_t c = blockIdx.x, zb = blockIdx.y;
     const int ku = 2 * bw - 1;
+    const T f = pow2<T>(-band_exponent(scale, zb));
     const T *az = a + zb * n * n;
     typename ChaseAr<S>::St *abz = ab + zb * ldab * n;
     for (int i = threadIdx.x; i <= bw; i += blockDim.x) {
@@ -812,22 +832,23 @@ __global__ void extract_band_batched(const T *a, int64_t n, int bw, typename Cha
         if (r >= 0) {
             if constexpr (sizeof(typename ChaseAr<S>::St) == sizeof(float2) && sizeof(T) == 4 &&
                           !std::is_same<S, double>::value)
-                abz[(ku + r - c) + c * ldab] = make_float2((float)az[r + c * n], 0.0f);  // exact
+                abz[(ku + r - c) + c * ldab] = make_float2((float)(az[r + c * n] * f), 0.0f);  // exact
             else
-                abz[(ku + r - c) + c * ldab] = ChaseAr<S>::from_double((double)az[r + c * n]);
+                abz[(ku + r - c) + c * ldab] = ChaseAr<S>::from_double((double)(az[r + c * n] * f));
         }
     }
 }
 template <typename S>
 __global__ void bidiag_out_batched(const typename ChaseAr<S>::St *ab, int64_t n, int bw, int64_t ldab, double *d,
-                                   double *e, int batch, int64_t sAB) {
+                                   double *e, int batch, int64_t sAB, const int *scale) {
     const int ku = 2 * bw - 1;
     const int64_t total = n * (int64_t)batch;
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
         const int64_t zb = g / n, i = g % n;
         const typename ChaseAr<S>::St *abz = ab + zb * sAB;
-        d[zb * n + i] = st_to_double(abz[ku + i * ldab]);
-        e[zb * n + i] = (i + 1 < n) ? st_to_double(abz[(ku - 1) + (i + 1) * ldab]) : 0.0;
+        const double f = pow2<double>(band_exponent(scale, zb));
+        d[zb * n + i] = st_to_double(abz[ku + i * ldab]) * f;
+        e[zb * n + i] = (i + 1 < n) ? st_to_double(abz[(ku - 1) + (i + 1) * ldab]) * f : 0.0;
     }
 }
 }  // namespace
@@ -843,11 +864,13 @@ int stage2_chase_batched(const T *dW, int64_t n, int bw, int batch, typename Cha
                          double *dd, double *de, const Stage2Work &w, cudaStream_t s, int num_sms,
                          int64_t *launches, int tbw, bool window, typename ChaseAr<S>::St *dAB2) {
     using St = typename ChaseAr<S>::St;
+    int rc;
+    if ((rc = band_scale<T>(dW, n, n, n * n, bw, batch, w, s, launches)) != AVS_SUCCESS) return rc;
     if (tbw > 0) {
         R *ab1 = reinterpret_cast<R *>(dAB);
         const int64_t ldab1 = band_ldab(bw), sAB1 = band_stride(bw, n), ldab2 = 3 * (int64_t)tbw, sAB2 = ldab2 * n;
-        int rc;
-        if ((rc = dense_to_band<T, R>(dW, n, n, n * n, bw, ab1, ldab1, sAB1, batch, s)) != AVS_SUCCESS) return rc;
+        if ((rc = dense_to_band<T, R>(dW, n, n, n * n, bw, ab1, ldab1, sAB1, batch, w.scale, s)) != AVS_SUCCESS)
+            return rc;
         if ((rc = band_stage<R>(ab1, n, bw, tbw, ldab1, w, s, num_sms, batch, sAB1, n + 1)) != AVS_SUCCESS)
             return rc;
         if ((rc = band_to_band<R, St>(ab1, n, bw, ldab1, sAB1, tbw, dAB2, ldab2, sAB2, batch, s)) != AVS_SUCCESS)
@@ -864,24 +887,21 @@ int stage2_chase_batched(const T *dW, int64_t n, int bw, int batch, typename Cha
         }
         if (rc != AVS_SUCCESS) return rc;
         const int nb = (int)std::min<int64_t>((n * batch + 255) / 256, 8192);
-        bidiag_out_batched<S><<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB2, n, tbw, ldab2, dd, de, batch, sAB2);
+        bidiag_out_batched<S><<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB2, n, tbw, ldab2, dd, de, batch, sAB2, w.scale);
         AVS_CUDA_TRY(cudaGetLastError());
         if (launches) *launches += 5;
         return AVS_SUCCESS;
     }
     AVS_CUDA_TRY(cudaMemsetAsync(dAB, 0, sizeof(St) * (size_t)ldab * (size_t)n * batch, s));
-    extract_band_batched<T, S><<<dim3((unsigned)n, (unsigned)batch), 128, 0, s>>>(dW, n, bw, dAB, ldab);
+    extract_band_batched<T, S><<<dim3((unsigned)n, (unsigned)batch), 128, 0, s>>>(dW, n, bw, dAB, ldab, w.scale);
     AVS_CUDA_TRY(cudaGetLastError());
     if (window && chase_window_supported(bw) && ldab == 3 * (int64_t)bw) {
-        const int rc = std::is_same<S, df64>::value
-                           ? stage2_chase_window_df(reinterpret_cast<float2 *>(dAB), n, bw, w, s, num_sms, batch,
-                                                    ldab * n)
-                           : stage2_chase_window_fp64(reinterpret_cast<double *>(dAB), n, bw, w, s, num_sms, batch,
-                                                      ldab * n);
+        rc = std::is_same<S, df64>::value
+                 ? stage2_chase_window_df(reinterpret_cast<float2 *>(dAB), n, bw, w, s, num_sms, batch, ldab * n)
+                 : stage2_chase_window_fp64(reinterpret_cast<double *>(dAB), n, bw, w, s, num_sms, batch, ldab * n);
         if (rc != AVS_SUCCESS) return rc;
     } else if (n >= 2) {
         AVS_CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(int) * (size_t)((n + 1) * (int64_t)batch + 1), s));
-        int rc;
         // small bands: few, small CTAs per sweep (the batch supplies the
         // parallelism).  Measured on the 4096-matrix workload (orders 64..1024;
         // the matrices each band divides), stage 2, CTAs per cluster x threads:
@@ -923,7 +943,7 @@ int stage2_chase_batched(const T *dW, int64_t n, int bw, int batch, typename Cha
         if (rc != AVS_SUCCESS) return rc;
     }
     const int nb = (int)std::min<int64_t>((n * batch + 255) / 256, 8192);
-    bidiag_out_batched<S><<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB, n, bw, ldab, dd, de, batch, ldab * n);
+    bidiag_out_batched<S><<<nb > 0 ? nb : 1, 256, 0, s>>>(dAB, n, bw, ldab, dd, de, batch, ldab * n, w.scale);
     AVS_CUDA_TRY(cudaGetLastError());
     if (launches) *launches += 3;
     return AVS_SUCCESS;
