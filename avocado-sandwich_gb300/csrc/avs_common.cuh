@@ -17,10 +17,13 @@ enum DeviceError : int {
     kDevInternal = 3,  // a kernel found its own bookkeeping inconsistent
 };
 
-// Bounds of any dependency wait: at most kSpinLimit polls (an acquire load and
-// a short sleep each, about 1 us with the load's latency) and at most kWaitNs,
-// whichever comes first -- far beyond any legitimate wait, short enough that a
-// lost dependency returns AVS_ERR_TIMEOUT instead of hanging the GPU.
+// Bounds of a dependency wait: at most kSpinLimit polls (an acquire load and
+// a short sleep each, about 1 us with the load's latency) and at most 2 kWaitNs cycles
+// of the SM clock, whichever comes first: 4 s at 2 GHz, more at a lower clock (7 s at
+// 1.1 GHz) -- far beyond any legitimate wait, short enough that a lost dependency
+// returns AVS_ERR_TIMEOUT instead of hanging the GPU.  (The panel's waits between its
+// own warps have two and four times as many cycles, so that the wait on the other CTA
+// gives up first.)
 constexpr long long kSpinLimit = 1ll << 27;
 constexpr long long kWaitNs = 4000000000ll;  // 4 s
 
@@ -51,9 +54,9 @@ __device__ __forceinline__ void st_release(int *p, int v) {
 
 // Bounded wait until *flag >= target.  Called by one thread; returns false on
 // timeout (after recording kDevTimeout in *err) or when another CTA already
-// failed.  Never spins forever: at most kSpinLimit polls and limit_ns, measured
-// on the SM's clock at 2 cycles per ns (its maximum is 2.07 GHz; reading it takes
-// a few cycles, %globaltimer hundreds).  The first polls follow one another at
+// failed.  Never spins forever: at most kSpinLimit polls and 2 limit_ns cycles of the
+// SM's clock (limit_ns at 2 GHz, its maximum is 2.07; reading it takes a few cycles,
+// %globaltimer hundreds).  The first polls follow one another at
 // the load's latency: most waits are shorter than a sleep.
 __device__ __forceinline__ bool wait_geq_n(const int *flag, int target, int *err, long long limit_ns) {
     if (ld_acquire(flag) >= target) return true;

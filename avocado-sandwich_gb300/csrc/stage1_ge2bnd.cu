@@ -32,11 +32,14 @@
 // tensor-core path (stage1_ge2bnd_tc) a role may also wait for its own tile,
 // which the previous update's chain finishes on the other stream.
 //
-// Trailing update kernel.  One CTA owns a column strip of the trailing matrix,
-// keeps the strip of the top tile row in shared memory, and applies the GEQRT
-// blocks and then, row tile by row tile, the TSQRT blocks (compact WY per 16
-// reflectors) -- the serial order of the reference's Qtapply1_par! /
-// Qtapply2_par! (TiledMatrix.jl:107-113) per column, all columns in parallel.
+// Trailing update kernels: per column the serial order of the reference's
+// Qtapply1_par! / Qtapply2_par! (TiledMatrix.jl:107-113) -- the GEQRT blocks, then row
+// tile by row tile the TSQRT blocks, compact WY per 16 reflectors -- all columns in
+// parallel.  update_kernel (tiles of 32 and 64, and FP64 tiles of 16): a CTA takes a
+// ticket for a (tile group, column strip) and receives the strip of the top tile row
+// from the CTA of the group before through global memory, block of 16 rows by block,
+// behind counters.  update16_kernel (FP32 tiles of 16): a CTA per 16-column strip
+// walks all tiles.  Tiles of 128 and 256: update_full_kernel (stage1_wy.cu).
 //
 // Householder vectors stay where the reference leaves them before it zeroes
 // them (tiledalgos.jl:40,46,52,58); later stages read only the band, so the
@@ -1730,7 +1733,7 @@ int launch_update_b(UpdateArgs a, int64_t ncols, const Stage1Work &w, cudaStream
     // Tiles per CTA.  One tile per CTA where latency counts (FP32 n = 1024 tile 64
     // 5.0 ms, all tiles in one CTA 6.5; FP64 n = 512 tile 32 18.0 against 27.7, and
     // FP64 always: its tiles take long), and all of them once the strips fill the GPU
-    // twice over by themselves (32 matrices of order 1024 tile 64 10.5 ms against
+    // twice over by themselves (2 x 152 SMs; 32 matrices of order 1024 tile 64 10.5 ms against
     // 15.0, 256 of order 256 tile 32 2.2 against 3.0).  The values do not depend on it.
     const bool whole = C::F4 && (int64_t)a.nstrip * batch >= 304;
     a.group = whole ? a.P : 1;

@@ -27,7 +27,8 @@
 // cluster barrier separates the ops.  Dependencies are tracked per op: the
 // counter of sweep j counts finished ops (R, L, R, L, ...), and op k of sweep
 // j waits until sweep j-1 has finished op k+3 -- the tightest lag for which
-// the wavefront stays bit-identical to the sequential order.  Along the
+// whole ops stay in the sequential order (the other two chases read the one element,
+// or corner, that ops three apart share inside the op, and lag by three).  Along the
 // critical path a sweep therefore costs 4 ops instead of 6.
 //
 // Band storage: A(r, c) at AB[(r - c + 2bw - 1) + c * ldab], ldab >= 3bw - 1,
@@ -914,9 +915,10 @@ int stage2_chase_batched(const T *dW, int64_t n, int bw, int batch, typename Cha
         // a short batch is latency-bound and keeps 512-thread CTAs.  Every
         // configuration of a band width computes the same bits (fixed
         // reduction order), so a matrix's values do not depend on its batch.
-        // A batch whose sweeps in flight fit twice in the GPU with the single
-        // call's clusters (C = 8 at bands >= 128, 4 at 64, 2 at 32) is
-        // latency-bound and takes them: e.g. one n = 8192 matrix at band 128.
+        // A batch whose sweeps in flight fit twice in the GPU with clusters of
+        // C = 8 at bands >= 128, 4 at 64 and 2 at 32 is latency-bound and takes
+        // them: e.g. one n = 8192 matrix at band 128.  (A single call takes twice
+        // that where chase_room allows; measured for single calls only.)
         const int64_t inflight = (int64_t)batch * std::max<int64_t>(1, (n / bw) / 2);
         const bool wide = inflight >= 4 * (int64_t)num_sms;
         const int cdef = bw >= 128 ? 8 : (bw == 64 ? 4 : (bw == 32 ? 2 : 1));

@@ -37,7 +37,8 @@
 // What bounds it: the latency of one op times the ops on the critical path (3
 // per sweep, plus 5 to 6 and the hand-off per group); the band stays in L2 and
 // shared memory.  The op's chain is kept short: the reflector is used unscaled
-// (u = x with u_0 = alpha - beta), so the dot products do not wait for the norm;
+// (u = x with u_0 = alpha - beta; the band comes scaled, band_scale.cuh), so the dot
+// products do not wait for the norm;
 // the norm's butterfly merges compensated pairs without renormalising; the
 // scalars come from the hardware estimates with one residual each
 // (reflect.cuh); full ops that do not wrap in the window have immediate
@@ -124,7 +125,7 @@ __device__ __forceinline__ int ld_relaxed(const int *p) {
 }
 
 // Bounded waits of the CTA's warps on one another: kWaitCycles of the SM clock
-// (about 4 s; reading it costs a few cycles, %globaltimer hundreds) and
+// (4 s at 2 GHz; reading it costs a few cycles, %globaltimer hundreds) and
 // kSpinLimit polls.  A wait that runs out records kDevTimeout and raises *fail,
 // on which every later wait of the CTA returns at once: the group runs to its
 // end on whatever data it has.

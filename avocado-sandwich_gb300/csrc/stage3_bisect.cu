@@ -14,7 +14,8 @@
 // FP64 counts on that cell and its neighbours, each on a group of G lanes that
 // splits the bracket at G K points a pass.  A bracket whose edges a finer
 // arithmetic does not confirm is dropped and that arithmetic starts again from
-// [0, 1).
+// [0, 1).  Widths below the grid's cells (2^-52 of the scale): halving in FP64 from
+// there.  An infinite entry gives the infinite bound for every value.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
